@@ -66,11 +66,22 @@ struct tmx_ctx {
   // observables (get_table): cached Clebsch-Gordan table and work buffers
   DevBuf cg, cg_off;
   int cg_nmax = 0;
-  DevBuf Ta, o_angles, o_phis, o_wts, o_coef, o_shw, o_og, o_work, o_sj, o_qj,
-      o_S, o_gq, o_gz, o_cq, o_cz, o_pairs, o_grp, o_x;
-  // plan of the observable kernels (first pair of each grain, job groups)
-  int64_t o_ngrains = 0, o_npairs = 0;
-  int o_nbmax = 1, o_ngrp = 0;
+  DevBuf Ta, o_angles, o_phis, o_wts, o_coef, o_shw, o_og, o_work, o_qj,
+      o_S, o_gq, o_gz, o_cq, o_cz, o_pairs, o_grp, o_ins, o_prs, o_rng, o_x;
+  // plan of the observable kernels: the amplitude groups in chunks that share
+  // the buffer of m sums (o_xcap complex per matrix set), one launch per block
+  // size (ranges [rng0, rng0 + nrng) of o_rng)
+  int64_t o_npairs = 0, o_xcap = 1;
+  int o_nbmax = 1;
+  struct AmpLaunch {
+    int rng0 = 0, nrng = 0, lcap = 1;
+    int64_t nitems = 0;
+  };
+  struct AmpChunk {
+    int g0 = 0, g1 = 0, nin = 1, nitem_max = 1;
+    std::vector<AmpLaunch> launches;
+  };
+  std::vector<AmpChunk> o_chunks;
   // orientation-average work order: pair-major item starts (o_pairs, pmax^2
   // + 1) and the grains by descending order (o_ord)
   DevBuf o_ord;
@@ -210,7 +221,7 @@ struct tmx_ctx {
   std::vector<ItemTemplate> item_tpl; // indexed by N
   int64_t p2_scr_total = 0, p2_t_total = 0;
   DevBuf lu, dT, tscr, dTa, dS; // tangent buffers
-  int o_nsj = 0, o_nqj = 0;     // per-grain observable job counts
+  int o_nqj = 0;                // per-grain observable job count
   // events that order a free on `stream` after the work queued so far on the
   // round streams, their bucket streams (stream2, stream3, aux[0..5]) and
   // the copy stream

@@ -239,21 +239,32 @@ struct TmxAngle {
   double c, s, si;
 };
 
-// forward-amplitude job: S(theta_in -> theta_out) for nphi azimuths
-struct TmxSJob {
-  int32_t grain;
-  int32_t angle_in;
-  int32_t angle_out;
+// Amplitude plan. A group is a set of up to TMX_AMP_NIN incoming angles of one
+// grain with the (incoming, outgoing) pairs that use them; groups of grains
+// with the same angles share one list of angles and pairs.
+#define TMX_AMP_NIN 16
+// S(theta_in -> theta_out) for nphi azimuths
+struct TmxAmpPair {
+  int32_t in;        // position of the incoming angle in the group's list
+  int32_t angle_out; // outgoing angle
   int32_t nphi;
-  int64_t phi0; // first e^{i phi} of the job in the azimuth table
-  int64_t out;  // first S (4 complex each) of the job
+  int32_t pref;      // azimuths of the group's pairs before this one
+  int64_t phi0;      // first e^{i phi} of the pair in the azimuth table
+  int64_t out;       // first S (4 complex each), after the group's out0
 };
-
-// consecutive amplitude jobs of one grain handled by one CTA (at most 32)
 struct TmxAmpGroup {
   int32_t grain;
-  int32_t njobs;
-  int64_t job0;
+  int32_t nin, in0;     // incoming angles: list entries [in0, in0 + nin)
+  int32_t npair, pair0; // pairs [pair0, pair0 + npair)
+  int32_t nitem;        // azimuths of all pairs
+  int64_t out0;         // first S of the group's grain
+  int64_t x0;           // m sums of the group: X[x0 + (pair (N + 1) + m) 4 + q]
+};
+// work items of one amplitude launch: items [base, next entry's base) are
+// block m of groups first, first + 1, ...
+struct TmxAmpRange {
+  int64_t base;
+  int32_t m, first;
 };
 
 // Q job for one (grain, theta): main amplitude and, with the scattering
@@ -288,17 +299,23 @@ void tmx_launch_orient_pairs(const TmxObsGrain *og, const int64_t *pstart,
                              const int64_t *cg_off, const double *cg,
                              int cg_nmax, int mmax, int fold,
                              cudaStream_t stream);
-// CTAs of the amplitude kernel at full occupancy for nbmax and nmat (its
-// work slots: grid x nmat x 32 x (nbmax + 1) x 4 complex)
-int tmx_amp_grid(int nbmax, int nmat);
-// amplitudes of nmat (1 or 4) averaged sets: src[k] -> S at dst[k]
-// wpi / wtau (may be NULL: the kernel runs the recurrences itself): the
-// plan's pi and tau columns from tmx_launch_wigner_cols for nmax wnmax
-void tmx_launch_amp(const TmxAmpGroup *groups, int ngroups, const TmxSJob *jobs,
-                    const TmxObsGrain *og, const TmxMatSet &mats, int nmat,
-                    const TmxAngle *angles, const double2 *phis, double2 *xslot,
-                    int nbmax, int grid, const double *wpi, const double *wtau,
-                    int wnmax, cudaStream_t stream);
+// m sums X of nmat (1 .. 4) averaged sets (compact class layout, src[k]) into
+// x + k xstride: nitems items in the nrng ranges, blocks of at most lcap
+// orders, groups of at most nin incoming angles; wpi / wtau: the plan's pi and
+// tau columns (tmx_launch_wigner_cols for nmax wnmax)
+void tmx_launch_amp(const TmxAmpGroup *groups, const int32_t *ins,
+                    const TmxAmpPair *pairs, const TmxAmpRange *rng, int nrng,
+                    int64_t nitems, const TmxObsGrain *og, const TmxMatSet &mats,
+                    int nmat, const double *wpi, const double *wtau, int wnmax,
+                    double2 *x, int64_t xstride, int lcap, int nin,
+                    cudaStream_t stream);
+// S of every pair and azimuth of ngroups groups from their m sums, to
+// mats.dst[k]; nitem_max: the largest group's azimuths
+void tmx_launch_azimuth(const TmxAmpGroup *groups, int ngroups,
+                        const TmxAmpPair *pairs, const TmxObsGrain *og,
+                        const TmxMatSet &mats, int nmat, const double2 *phis,
+                        const double2 *x, int64_t xstride, int nitem_max,
+                        cudaStream_t stream);
 // pi and tau columns of every (angle, m <= nmax): column (a, m) holds orders
 // max(m, 1) .. nmax at ((a (nmax + 1) + m) nmax)
 void tmx_launch_wigner_cols(const TmxAngle *angles, int nangles, int nmax,

@@ -7,13 +7,13 @@
 //                   115-215), restructured: the m1 sum does not depend on m,
 //                   so it is formed once per (n1, n2, N) and reused for every
 //                   m (O(N^4) instead of O(N^5))
-//   k_forward_s     the forward-scattering amplitude S of
+//   k_amp           the per-m sums of the forward-scattering amplitude S of
 //                   ExtinctionCoefficientTask.hpp:517-619 (and its copies in
 //                   AbsorptionCoefficientTask.hpp:612-715 and
-//                   ScatteringMatrixTask.hpp:588-691) for one (theta_in,
-//                   theta_out) pair and a list of azimuths: the per-m sums
-//                   over (n, n') are formed once, each azimuth then costs
-//                   O(nmax)
+//                   ScatteringMatrixTask.hpp:588-691): T times the vectors of
+//                   a set of incoming angles on the FP64 tensor pipe, then
+//                   the product with each pair's outgoing vector
+//   k_azimuth       S of every pair and azimuth from those sums, O(nmax) each
 //   k_q_epilogue    Q_ext/Q_extpol/Q_extcpol and Q_abs/Q_abspol (with the
 //                   optional scattering subtraction of
 //                   AbsorptionCoefficientTask.hpp:742-773)
@@ -126,6 +126,14 @@ __device__ __forceinline__ int64_t telem(int N, int m, int i1, int n1, int i2,
          n2 - nmin;
 }
 
+// matrix k of a set (selects, so that the pointers stay in constant memory)
+__device__ __forceinline__ const cplx *mat_src(const TmxMatSet &s, int k) {
+  return k == 0 ? s.src[0] : k == 1 ? s.src[1] : k == 2 ? s.src[2] : s.src[3];
+}
+__device__ __forceinline__ cplx *mat_dst(const TmxMatSet &s, int k) {
+  return k == 0 ? s.dst[0] : k == 1 ? s.dst[1] : k == 2 ? s.dst[2] : s.dst[3];
+}
+
 // acc += t * a (complex times real), fused; this file is compiled without
 // automatic contraction, so the contractions are spelled out
 __device__ __forceinline__ void cfma(cplx &acc, cplx t, double a) {
@@ -136,6 +144,32 @@ __device__ __forceinline__ void cfma(cplx &acc, cplx t, double a) {
 // sqrt((2n + 1) / ((n + 1) n)), the factor of a_{n n'} for one order
 __device__ __forceinline__ double a_fac(int n) {
   return sqrt((2. * n + 1.) / ((n + 1.) * n));
+}
+
+// element (i1, n1; i2, n2) of block m of an averaged T-matrix of order N in
+// the compact class layout the amplitude kernel reads: the entries of the
+// parity classes (i + n) % 2 of block m (m = 0: of each (i, n % 2)) one after
+// the other as dense row-major matrices, members by i, then n. Half the size
+// of the block; -1 for the entries between classes, which are zero.
+__device__ __forceinline__ int64_t celem(int N, int m, int i1, int n1, int i2,
+                                         int n2) {
+  if (((i1 + n1 + i2 + n2) & 1) || (m == 0 && i1 != i2)) {
+    return -1;
+  }
+  if (m == 0) {
+    const int no = (N + 1) >> 1, ne = N >> 1;
+    const int ld = (n1 & 1) ? no : ne;
+    const int64_t off = (int64_t)i1 * (no * no + ne * ne) + ((n1 & 1) ? 0 : no * no);
+    return off + (int64_t)((n1 - 1) >> 1) * ld + ((n2 - 1) >> 1);
+  }
+  const int cls = (i1 + n1) & 1;
+  const int L = N + 1 - m;
+  // first order of the members with i = 0 and i = 1, and their number
+  const int f0 = m + ((m & 1) != cls), f1 = m + ((m & 1) == cls);
+  const int r0 = (N >= f0) ? (N - f0) / 2 + 1 : 0;
+  const int a = i1 ? r0 + ((n1 - f1) >> 1) : (n1 - f0) >> 1;
+  const int b = i2 ? r0 + ((n2 - f1) >> 1) : (n2 - f0) >> 1;
+  return tblock(N, m) / 2 + ((int64_t)cls * L + a) * L + b;
 }
 
 // c_{n' n} z for c_{n' n} = i^{n' - n - 1} a_{n' n} (NBasedResources::get_cnn,
@@ -212,9 +246,14 @@ k_orient_pairs(const TmxObsGrain *__restrict__ og,
         for (int q = 0; q < 4; ++q) {
           const int i1 = q >> 1, i2 = q & 1;
           const int64_t e = telem(N, m, i1, n1, i2, n2);
+          const int64_t ed = fold ? celem(N, m, i1, n1, i2, n2) : e;
+          if (ed < 0) {
+            continue;
+          }
 #pragma unroll
           for (int k = 0; k < NMAT; ++k) {
-            mats.dst[k][G.t_off + e] = c_fold(n2, nfold, afold, mats.src[k][G.t_off + e]);
+            mats.dst[k][(fold ? G.t_off / 2 : G.t_off) + ed] =
+                c_fold(n2, nfold, afold, mats.src[k][G.t_off + e]);
           }
         }
       }
@@ -291,6 +330,19 @@ k_orient_pairs(const TmxObsGrain *__restrict__ og,
       }
 #pragma unroll
       for (int k = 0; k < NMAT; ++k) {
+        if (fold) {
+          cplx *Tag = mats.dst[k] + G.t_off / 2;
+          const bool same = ((n1 + n2) & 1) == 0;
+          const int64_t ea = celem(N, m, 0, n1, same ? 0 : 1, n2);
+          const int64_t eb = celem(N, m, 1, n1, same ? 1 : 0, n2);
+          if (ea >= 0) {
+            Tag[ea] = c_fold(n2, nfold, afold, same ? e00[k] : e01[k]);
+          }
+          if (eb >= 0) {
+            Tag[eb] = c_fold(n2, nfold, afold, same ? e11[k] : e10[k]);
+          }
+          continue;
+        }
         cplx *Tag = mats.dst[k] + G.t_off;
         Tag[telem(N, m, 0, n1, 0, n2)] = c_fold(n2, nfold, afold, e00[k]);
         Tag[telem(N, m, 1, n1, 1, n2)] = c_fold(n2, nfold, afold, e11[k]);
@@ -337,12 +389,14 @@ __device__ static void wigner_col(double cosx, double sinx, double sinx_inv,
   if (m == 0) {
     double d1 = 1.;
     double d2 = cosx;
+#pragma unroll 4
     for (int n = 0; n < nmax; ++n) {
       const double np1 = n + 1.;
       const double np2 = n + 2.;
       const double np12p1 = 2. * np1 + 1.;
-      const double dnp1 = (np12p1 * cosx * d2 - np1 * d1) / np2;
-      const double ddn = sinx_inv * np1 * np2 * (dnp1 - d1) / np12p1;
+      const double r2 = 1. / np2;
+      const double dnp1 = __fma_rn(np12p1 * cosx * r2, d2, -(np1 * r2 * d1));
+      const double ddn = (sinx_inv * np1 * np2 / np12p1) * (dnp1 - d1);
       pi[n * stride] = 0.;
       tau[n * stride] = ddn;
       d1 = d2;
@@ -350,31 +404,37 @@ __device__ static void wigner_col(double cosx, double sinx, double sinx_inv,
     }
     return;
   }
+  // the square roots and quotients of a step do not depend on the step before
+  // it: only one fused multiply-add per order is serial
   const double m2 = (double)(m * m);
   double d1 = 0.;
   double d2 = 1.;
+#pragma unroll 4
   for (int i = 0; i < m; ++i) {
     const double i2 = 2. * (i + 1.);
     d2 *= sqrt((i2 - 1.) / i2) * sinx;
   }
+  double s12 = 0.; // sqrt(n^2 - m^2) at n = m
+#pragma unroll 4
   for (int n = m - 1; n < nmax; ++n) {
     const double np1 = n + 1.;
     const double np2 = n + 2.;
     const double np12p1 = 2. * np1 + 1.;
-    const double s12 = sqrt(np1 * np1 - m2);
     const double s22 = sqrt(np2 * np2 - m2);
-    const double dnp1 = (np12p1 * cosx * d2 - s12 * d1) / s22;
-    const double ddn = sinx_inv * (np1 * s22 * dnp1 - np2 * s12 * d1) / np12p1;
+    const double r22 = 1. / s22;
+    const double dnp1 = __fma_rn(np12p1 * cosx * r22, d2, -(s12 * r22 * d1));
+    const double ddn =
+        (sinx_inv / np12p1) * (np1 * s22 * dnp1 - np2 * s12 * d1);
     pi[(n + 1 - nmin) * stride] = m * (d2 * sinx_inv);
     tau[(n + 1 - nmin) * stride] = ddn;
     d1 = d2;
     d2 = dnp1;
+    s12 = s22;
   }
 }
 
-// pi and tau columns of every (angle, m <= nmax) of an amplitude plan, the
-// recurrence of k_amp done once for all grains and jobs that share an angle:
-// column (a, m) holds orders n = max(m, 1) .. nmax at ((a (nmax + 1) + m)
+// pi and tau columns of every (angle, m <= nmax) of an amplitude plan, once
+// for all grains and jobs that share an angle: column (a, m) holds orders n = max(m, 1) .. nmax at ((a (nmax + 1) + m)
 // nmax). (The values of orders <= N do not depend on how far the
 // recurrence runs, so a grain of order N reads the first entries.)
 __global__ void k_wigner_cols(const TmxAngle *__restrict__ angles, int nangles,
@@ -389,185 +449,258 @@ __global__ void k_wigner_cols(const TmxAngle *__restrict__ angles, int nangles,
   wigner_col(A.c, A.s, A.si, nmax, m, pi + u * nmax, tau + u * nmax, 1);
 }
 
-// One CTA per group of up to 32 amplitude jobs of one grain (lane = job).
-// For every m, with u = (pi_n, tau_n) at the outgoing angle and v at the
-// incoming one (n the row order, n' the column order of block m),
+// D += A B for one m8n8k4 FP64 tensor-core tile: lane l holds A[l / 4][l % 4],
+// B[l % 4][l / 4] and D[l / 4][2 (l % 4) + {0, 1}]
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, "
+      "{%0, %1};\n"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
+// parity class c of block m of order N: members (i = 0, n = f0 + 2 j), j <
+// r0, then (i = 1, n = f1 + 2 j), nb in all (celem's order), and its offset
+struct AmpClass {
+  int nb, r0, f0, f1;
+  int64_t off;
+};
+__device__ __forceinline__ AmpClass amp_class(int N, int m, int c) {
+  AmpClass A;
+  if (m == 0) {
+    const int no = (N + 1) >> 1, ne = N >> 1;
+    A.f0 = A.f1 = 1 + (c & 1);
+    A.nb = (c & 1) ? ne : no;
+    A.r0 = (c >> 1) ? 0 : A.nb;
+    A.off = (int64_t)(c >> 1) * (no * no + ne * ne) + ((c & 1) ? no * no : 0);
+    return A;
+  }
+  A.nb = N + 1 - m;
+  A.f0 = m + ((m & 1) != c);
+  A.f1 = m + ((m & 1) == c);
+  A.r0 = (N >= A.f0) ? (N - A.f0) / 2 + 1 : 0;
+  A.off = tblock(N, m) / 2 + (int64_t)c * A.nb * A.nb;
+  return A;
+}
+
+// One CTA per (group, block m): with u = (pi_n, tau_n) at the outgoing angle
+// and v at the incoming one (n the row order, n' the column order of block m),
 //   X0 = u^T Tc v,  X1 = u^T Tc v',  X2 = u'^T Tc v,  X3 = u'^T Tc v'
 // where Tc is block m with the c_{n' n} factors folded in and u', v' swap
 // the pi and tau halves: the four (n, n') sums of
-// ExtinctionCoefficientTask.hpp:517-619 as one (2nb x 2nb) x (2nb x 64)
-// product per m. Warps own rows; lanes own jobs; the T row is read once per
-// warp (a broadcast) and the angle vectors come from shared memory. X is
-// kept in this CTA's global slot; the azimuth pass then forms
-//   S = (1/k) sum_m (2 cos m phi, 2 sin m phi) X_m
-// with e^{i m phi} built by repeated multiplication as in the reference.
-template <int NMAT>
-__global__ void __launch_bounds__(256, (NMAT > 1) ? 2 : 3)
-k_amp(const TmxAmpGroup *__restrict__ groups, int ngroups,
-      const TmxSJob *__restrict__ jobs, const TmxObsGrain *__restrict__ og,
-      TmxMatSet mats, const TmxAngle *__restrict__ angles,
-      const cplx *__restrict__ phis, cplx *__restrict__ xslot, int nbmax,
-      const double *__restrict__ wpi, const double *__restrict__ wtau,
-      int wnmax) {
-  extern __shared__ double ash[];
-  double *po = ash;
-  double *to = po + nbmax * 32;
-  double *pi = to + nbmax * 32;
-  double *ti = pi + nbmax * 32;
-  cplx *red = (cplx *)(ti + nbmax * 32); // [NMAT][8 warps][4][32 lanes]
-  __shared__ TmxSJob sj[32];
-  __shared__ int pref[33];
+// ExtinctionCoefficientTask.hpp:517-619.
+// Phase 1 forms y = Tc v, y' = Tc v' of every incoming angle: per parity class
+// an (nb x nb) complex by (nb x 2 nin) real product, 8-row tiles over the
+// warps, columns (angle, v or v') on the FP64 tensor pipe, T entries straight
+// from memory (each is used once per CTA), eight K steps in flight. Phase 2
+// multiplies with the outgoing vectors pair by pair, 2^k lanes per pair.
+// Splitting over m (rather than one CTA looping over a grain's blocks) fills
+// the chip from a few grains on, and an incoming angle's product is formed
+// once however many outgoing angles it goes with. Only the entries of the
+// parity classes are read (half of a block, the rest is zero).
+// Measured (B200): 96 grains of orders 16..50, 16 angles: 2.11 ms with one CTA
+// of FMA dot products per grain -> 0.093 ms; a 1920-grain table, orders 10..99,
+// 32 angles: 29.0 -> 0.84 ms; the three tangents of 1024 grains, 32 angles:
+// 1.92 -> 0.72 ms. Bound by the latency of the T reads and of phase 2's
+// shared-memory reads at small L, well below the FP64 and HBM rates.
+template <int NT, int NTH>
+__global__ void __launch_bounds__(NTH, (NTH == 128) ? 4 : 2)
+k_amp(const TmxAmpGroup *__restrict__ groups, const int32_t *__restrict__ ins,
+      const TmxAmpPair *__restrict__ pairs, const TmxAmpRange *__restrict__ rng,
+      int nrng, const TmxObsGrain *__restrict__ og, TmxMatSet mats,
+      const double *__restrict__ wpi, const double *__restrict__ wtau, int wnmax,
+      cplx *__restrict__ X, int64_t xstride, int lcap) {
+  constexpr int NA = 4 * NT;              // angle slots
+  constexpr int VS = (NA > 8) ? 18 : 10;  // row stride: k steps of 2 orders hit
+                                          // distinct bank groups
+  extern __shared__ cplx ash[];
+  cplx *Y = ash;                          // [2 L][NA][2]: row (i, n), (y, y')
+  double *V = reinterpret_cast<double *>(Y + (int64_t)2 * lcap * NA * 2); // [2][L][VS]
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  cplx *X = xslot + (int64_t)blockIdx.x * 32 * (nbmax + 1) * 4 * NMAT;
-  for (int gi = blockIdx.x; gi < ngroups; gi += gridDim.x) {
-    const TmxAmpGroup grp = groups[gi];
-    const TmxObsGrain G = og[grp.grain];
-    const int N = G.nmax;
-    const int nj = grp.njobs;
-    if (tid < nj) {
-      sj[tid] = jobs[grp.job0 + tid];
+  int lo = 0, hi = nrng - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (rng[mid].base <= (int64_t)blockIdx.x) {
+      lo = mid;
+    } else {
+      hi = mid - 1;
     }
-    __syncthreads();
-    if (tid == 0) {
-      pref[0] = 0;
-      for (int p = 0; p < nj; ++p) {
-        pref[p + 1] = pref[p] + sj[p].nphi;
+  }
+  const TmxAmpRange R = rng[lo];
+  const int m = R.m;
+  const TmxAmpGroup grp = groups[R.first + (int)(blockIdx.x - R.base)];
+  const TmxObsGrain G = og[grp.grain];
+  const int N = G.nmax;
+  const int nmin = (m > 1) ? m : 1;
+  const int L = N + 1 - nmin;
+  const cplx *T = mat_src(mats, blockIdx.y) + G.t_off / 2;
+  // incoming vectors: V[0] = pi, V[1] = tau
+  for (int u = tid; u < NA * L; u += NTH) {
+    const int a = u / L;
+    const int k = u - a * L;
+    double p = 0., t = 0.;
+    if (a < grp.nin) {
+      const int64_t off = ((int64_t)ins[grp.in0 + a] * (wnmax + 1) + m) * wnmax + k;
+      p = wpi[off];
+      t = wtau[off];
+    }
+    V[k * VS + a] = p;
+    V[(L + k) * VS + a] = t;
+  }
+  __syncthreads();
+  {
+    const int rr = lane >> 2;
+    const int kq = lane & 3;
+    const int ncls = (m == 0) ? 4 : 2;
+    int tile0 = 0; // tiles of the classes before this one
+    for (int c = 0; c < ncls; ++c) {
+      const AmpClass C = amp_class(N, m, c);
+      const int nrt = (C.nb + 7) >> 3;
+      const cplx *Tc = T + C.off;
+      // this warp's row tiles of the class
+      for (int rt = (warp - tile0 % (NTH / 32) + NTH / 32) % (NTH / 32); rt < nrt;
+           rt += NTH / 32) {
+        double acc[NT][4];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.;
+        }
+        const int row = rt * 8 + rr;
+        const cplx *Tr = Tc + (int64_t)row * C.nb;
+        for (int k0 = 0; k0 < C.nb; k0 += 32) {
+          cplx t[8];
+#pragma unroll
+          for (int s = 0; s < 8; ++s) {
+            const int col = k0 + 4 * s + kq;
+            t[s] = (row < C.nb && col < C.nb) ? Tr[col] : mkc(0., 0.);
+          }
+#pragma unroll
+          for (int s = 0; s < 8; ++s) {
+            if (k0 + 4 * s < C.nb) {
+              const int col = min(k0 + 4 * s + kq, C.nb - 1);
+              const int i = (col < C.r0) ? 0 : 1;
+              const int n = i ? C.f1 + 2 * (col - C.r0) : C.f0 + 2 * col;
+              // column rr of the tile: angle rr / 2, v (0) or v' (1)
+              const double *v = V + (((rr & 1) ^ i) * L + n - nmin) * VS + (rr >> 1);
+#pragma unroll
+              for (int j = 0; j < NT; ++j) {
+                const double b = v[4 * j];
+                dmma(acc[j][0], acc[j][1], t[s].x, b);
+                dmma(acc[j][2], acc[j][3], t[s].y, b);
+              }
+            }
+          }
+        }
+        if (row < C.nb) {
+          const int i = (row < C.r0) ? 0 : 1;
+          const int n = i ? C.f1 + 2 * (row - C.r0) : C.f0 + 2 * row;
+          cplx *y = Y + ((int64_t)(i * L + n - nmin) * NA + kq) * 2;
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            y[8 * j] = mkc(acc[j][0], acc[j][2]);
+            y[8 * j + 1] = mkc(acc[j][1], acc[j][3]);
+          }
+        }
+      }
+      tile0 += nrt;
+    }
+  }
+  __syncthreads();
+  // lanes per pair: as many as keep every thread busy
+  int ns = 1;
+  while (ns < 32 && grp.npair * ns * 2 <= NTH) {
+    ns *= 2;
+  }
+  const int sl = tid & (ns - 1);
+  for (int p0 = 0; p0 < grp.npair; p0 += NTH / ns) {
+    const int p = p0 + tid / ns;
+    const bool act = p < grp.npair;
+    const TmxAmpPair P = pairs[grp.pair0 + (act ? p : 0)];
+    cplx x0 = mkc(0., 0.), x1 = x0, x2 = x0, x3 = x0;
+    if (act) {
+      const int64_t off = ((int64_t)P.angle_out * (wnmax + 1) + m) * wnmax;
+      for (int k = sl; k < L; k += ns) {
+        const double a = wpi[off + k], b = wtau[off + k];
+        const cplx *y = Y + ((int64_t)k * NA + P.in) * 2;
+        const cplx *z = y + (int64_t)L * NA * 2;
+        const cplx y0 = y[0], y1 = y[1], z0 = z[0], z1 = z[1];
+        cfma(x0, y0, a);
+        cfma(x0, z0, b);
+        cfma(x1, y1, a);
+        cfma(x1, z1, b);
+        cfma(x2, y0, b);
+        cfma(x2, z0, a);
+        cfma(x3, y1, b);
+        cfma(x3, z1, a);
       }
     }
-    for (int m = 0; m <= N; ++m) {
-      const int nmin = (m > 1) ? m : 1;
-      const int nb = N + 1 - nmin;
-      if (wpi) {
-        // the columns of this m from the plan's table (k_wigner_cols)
-        for (int u = tid; u < 64 * nb; u += blockDim.x) {
-          const int side = u / (32 * nb); // 0: outgoing angle, 1: incoming
-          const int k = (u - side * 32 * nb) >> 5;
-          const int p = u & 31;
-          double pv = 0., tv = 0.;
-          if (p < nj) {
-            const int a = side ? sj[p].angle_in : sj[p].angle_out;
-            const int64_t off = ((int64_t)a * (wnmax + 1) + m) * wnmax + k;
-            pv = wpi[off];
-            tv = wtau[off];
-          }
-          (side ? pi : po)[k * 32 + p] = pv;
-          (side ? ti : to)[k * 32 + p] = tv;
-        }
-      } else if (tid < 64) {
-        const int p = tid & 31;
-        const int side = tid >> 5; // 0: outgoing angle, 1: incoming angle
-        double *P = side ? pi : po;
-        double *Tt = side ? ti : to;
-        if (p < nj) {
-          const TmxAngle a = angles[side ? sj[p].angle_in : sj[p].angle_out];
-          wigner_col(a.c, a.s, a.si, N, m, P + p, Tt + p, 32);
-        } else {
-          for (int k = 0; k < nb; ++k) {
-            P[k * 32 + p] = 0.;
-            Tt[k * 32 + p] = 0.;
-          }
-        }
+    for (int o = ns >> 1; o > 0; o >>= 1) {
+      x0.x += __shfl_xor_sync(0xffffffffu, x0.x, o);
+      x0.y += __shfl_xor_sync(0xffffffffu, x0.y, o);
+      x1.x += __shfl_xor_sync(0xffffffffu, x1.x, o);
+      x1.y += __shfl_xor_sync(0xffffffffu, x1.y, o);
+      x2.x += __shfl_xor_sync(0xffffffffu, x2.x, o);
+      x2.y += __shfl_xor_sync(0xffffffffu, x2.y, o);
+      x3.x += __shfl_xor_sync(0xffffffffu, x3.x, o);
+      x3.y += __shfl_xor_sync(0xffffffffu, x3.y, o);
+    }
+    if (act && sl == 0) {
+      cplx *o = X + blockIdx.y * xstride + grp.x0 + ((int64_t)p * (N + 1) + m) * 4;
+      o[0] = x0;
+      o[1] = x1;
+      o[2] = x2;
+      o[3] = x3;
+    }
+  }
+}
+
+// S of every pair and azimuth of a group (blockIdx.x; blockIdx.y shares the
+// azimuths of a group, blockIdx.z the matrices):
+//   S = (1/k) sum_m (2 cos m phi, 2 sin m phi) X_m
+// with e^{i m phi} built by repeated multiplication as in the reference.
+__global__ void __launch_bounds__(128)
+k_azimuth(const TmxAmpGroup *__restrict__ groups, const TmxAmpPair *__restrict__ pairs,
+          const TmxObsGrain *__restrict__ og, TmxMatSet mats,
+          const cplx *__restrict__ phis, const cplx *__restrict__ X, int64_t xstride) {
+  const TmxAmpGroup grp = groups[blockIdx.x];
+  const TmxObsGrain G = og[grp.grain];
+  const int N = G.nmax;
+  const double kinv = 1. / G.k;
+  const TmxAmpPair *pr = pairs + grp.pair0;
+  for (int item = blockIdx.y * blockDim.x + threadIdx.x; item < grp.nitem;
+       item += gridDim.y * blockDim.x) {
+    int lo = 0, hi = grp.npair - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (pr[mid].pref <= item) {
+        lo = mid;
+      } else {
+        hi = mid - 1;
       }
-      __syncthreads();
-      cplx x0[NMAT], x1[NMAT], x2[NMAT], x3[NMAT];
-#pragma unroll
-      for (int q = 0; q < NMAT; ++q) {
-        x0[q] = x1[q] = x2[q] = x3[q] = mkc(0., 0.);
-      }
-      const int64_t tb = G.t_off + tblock(N, m);
-      for (int r = warp; r < 2 * nb; r += 8) {
-        cplx y0[NMAT], y1[NMAT];
-#pragma unroll
-        for (int q = 0; q < NMAT; ++q) {
-          y0[q] = y1[q] = mkc(0., 0.);
-        }
+    }
+    const TmxAmpPair P = pr[lo];
+    const int f = item - P.pref;
+    const cplx e1 = phis[P.phi0 + f];
+    const cplx *Xp = X + blockIdx.z * xstride + grp.x0 + (int64_t)lo * (N + 1) * 4;
+    cplx s0 = Xp[0], s1 = mkc(0., 0.), s2 = s1, s3 = Xp[3];
+    cplx e = cmul(mkc(1., 0.), e1);
 #pragma unroll 4
-        for (int k = 0; k < nb; ++k) {
-          const double a = pi[k * 32 + lane];
-          const double b = ti[k * 32 + lane];
-#pragma unroll
-          for (int q = 0; q < NMAT; ++q) {
-            const cplx *Tr = mats.src[q] + tb + (int64_t)r * 2 * nb;
-            const cplx t0 = Tr[k];
-            const cplx t1 = Tr[nb + k];
-            cfma(y0[q], t0, a);
-            cfma(y0[q], t1, b);
-            cfma(y1[q], t0, b);
-            cfma(y1[q], t1, a);
-          }
-        }
-        const int kr = (r < nb) ? r : r - nb;
-        const double u = (r < nb) ? po[kr * 32 + lane] : to[kr * 32 + lane];
-        const double up = (r < nb) ? to[kr * 32 + lane] : po[kr * 32 + lane];
-#pragma unroll
-        for (int q = 0; q < NMAT; ++q) {
-          cfma(x0[q], y0[q], u);
-          cfma(x1[q], y1[q], u);
-          cfma(x2[q], y0[q], up);
-          cfma(x3[q], y1[q], up);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < NMAT; ++q) {
-        cplx *rq = red + q * 8 * 4 * 32;
-        rq[(warp * 4 + 0) * 32 + lane] = x0[q];
-        rq[(warp * 4 + 1) * 32 + lane] = x1[q];
-        rq[(warp * 4 + 2) * 32 + lane] = x2[q];
-        rq[(warp * 4 + 3) * 32 + lane] = x3[q];
-      }
-      __syncthreads();
-      for (int v = tid; v < 128 * NMAT; v += blockDim.x) {
-        const int q = v >> 7;
-        const int k = (v >> 5) & 3;
-        const cplx *rq = red + q * 8 * 4 * 32;
-        cplx s = rq[k * 32 + lane];
-        for (int w = 1; w < 8; ++w) {
-          s = cadd(s, rq[(w * 4 + k) * 32 + lane]);
-        }
-        if (lane < nj) {
-          X[(((int64_t)q * 32 + lane) * (N + 1) + m) * 4 + k] = s;
-        }
-      }
+    for (int m = 1; m <= N; ++m) {
+      const double fcos = 2. * e.x;
+      const double fsin = 2. * e.y;
+      e = cmul(e, e1);
+      const cplx *x = Xp + m * 4;
+      s0 = cadd(s0, cscale(x[0], fcos));
+      s1 = cadd(s1, cscale(x[1], fsin));
+      s2 = csub(s2, cscale(x[2], fsin));
+      s3 = cadd(s3, cscale(x[3], fcos));
     }
-    __syncthreads();
-    const double kinv = 1. / G.k;
-    for (int item = tid; item < pref[nj]; item += blockDim.x) {
-      int p = 0;
-      while (pref[p + 1] <= item) {
-        ++p;
-      }
-      const TmxSJob J = sj[p];
-      const int f = item - pref[p];
-      const cplx e1 = phis[J.phi0 + f];
-#pragma unroll
-      for (int q = 0; q < NMAT; ++q) {
-        const cplx *Xp = X + ((int64_t)q * 32 + p) * (N + 1) * 4;
-        cplx e = mkc(1., 0.);
-        cplx s0 = mkc(0., 0.), s1 = s0, s2 = s0, s3 = s0;
-        for (int m = 0; m <= N; ++m) {
-          const double fcos = 2. * e.x;
-          const double fsin = 2. * e.y;
-          e = cmul(e, e1);
-          if (m == 0) {
-            s0 = cadd(s0, Xp[0]);
-            s3 = cadd(s3, Xp[3]);
-          } else {
-            s0 = cadd(s0, cscale(Xp[m * 4 + 0], fcos));
-            s1 = cadd(s1, cscale(Xp[m * 4 + 1], fsin));
-            s2 = csub(s2, cscale(Xp[m * 4 + 2], fsin));
-            s3 = cadd(s3, cscale(Xp[m * 4 + 3], fcos));
-          }
-        }
-        cplx *o = mats.dst[q] + (J.out + f) * 4;
-        o[0] = cscale(s0, kinv);
-        o[1] = cscale(s1, kinv);
-        o[2] = cscale(s2, kinv);
-        o[3] = cscale(s3, kinv);
-      }
-    }
-    __syncthreads();
+    cplx *o = mat_dst(mats, blockIdx.z) + (grp.out0 + P.out + f) * 4;
+    o[0] = cscale(s0, kinv);
+    o[1] = cscale(s1, kinv);
+    o[2] = cscale(s2, kinv);
+    o[3] = cscale(s3, kinv);
   }
 }
 
@@ -768,34 +901,6 @@ void tmx_launch_orient_pairs(const TmxObsGrain *og, const int64_t *pstart,
   }
 }
 
-static size_t amp_smem(int nbmax, int nmat) {
-  return (size_t)4 * nbmax * 32 * sizeof(double) +
-         (size_t)nmat * 8 * 4 * 32 * sizeof(double2);
-}
-
-int tmx_amp_grid(int nbmax, int nmat) {
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (nmat == 4) {
-    cudaFuncSetAttribute(k_amp<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)amp_smem(TMX_MAX_NB, 4));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_amp<4>, 256,
-                                                  amp_smem(nbmax, 4));
-  } else if (nmat == 3) {
-    cudaFuncSetAttribute(k_amp<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)amp_smem(TMX_MAX_NB, 3));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_amp<3>, 256,
-                                                  amp_smem(nbmax, 3));
-  } else {
-    cudaFuncSetAttribute(k_amp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)amp_smem(TMX_MAX_NB, 1));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_amp<1>, 256,
-                                                  amp_smem(nbmax, 1));
-  }
-  return std::max(1, sms * std::max(1, per_sm));
-}
-
 void tmx_launch_wigner_cols(const TmxAngle *angles, int nangles, int nmax,
                             double *pi, double *tau, cudaStream_t stream) {
   const int64_t n = (int64_t)nangles * (nmax + 1);
@@ -806,28 +911,53 @@ void tmx_launch_wigner_cols(const TmxAngle *angles, int nangles, int nmax,
                                                            pi, tau);
 }
 
-void tmx_launch_amp(const TmxAmpGroup *groups, int ngroups, const TmxSJob *jobs,
-                    const TmxObsGrain *og, const TmxMatSet &mats, int nmat,
-                    const TmxAngle *angles, const double2 *phis, double2 *xslot,
-                    int nbmax, int grid, const double *wpi, const double *wtau,
-                    int wnmax, cudaStream_t stream) {
+template <int NT, int NTH>
+static void launch_amp(const TmxAmpGroup *groups, const int32_t *ins,
+                       const TmxAmpPair *pairs, const TmxAmpRange *rng, int nrng,
+                       int64_t nitems, const TmxObsGrain *og, const TmxMatSet &mats,
+                       int nmat, const double *wpi, const double *wtau, int wnmax,
+                       double2 *x, int64_t xstride, int lcap, cudaStream_t stream) {
+  constexpr int NA = 4 * NT, VS = (NA > 8) ? 18 : 10;
+  const size_t smem = (size_t)lcap * (2 * NA * 2 * sizeof(double2) + 2 * VS * sizeof(double));
+  cudaFuncSetAttribute(k_amp<NT, NTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem);
+  k_amp<NT, NTH><<<dim3((unsigned)nitems, nmat), NTH, smem, stream>>>(
+      groups, ins, pairs, rng, nrng, og, mats, wpi, wtau, wnmax, x, xstride, lcap);
+}
+
+void tmx_launch_amp(const TmxAmpGroup *groups, const int32_t *ins,
+                    const TmxAmpPair *pairs, const TmxAmpRange *rng, int nrng,
+                    int64_t nitems, const TmxObsGrain *og, const TmxMatSet &mats,
+                    int nmat, const double *wpi, const double *wtau, int wnmax,
+                    double2 *x, int64_t xstride, int lcap, int nin,
+                    cudaStream_t stream) {
+  if (nitems <= 0) {
+    return;
+  }
+  // column tiles of four angles; blocks of more than 32 orders have enough
+  // row tiles for eight warps
+  const auto run = [&](auto f) {
+    f(groups, ins, pairs, rng, nrng, nitems, og, mats, nmat, wpi, wtau, wnmax, x,
+      xstride, lcap, stream);
+  };
+  if (lcap > 32) {
+    run(nin <= 4 ? launch_amp<1, 256> : nin <= 8 ? launch_amp<2, 256> : launch_amp<4, 256>);
+  } else {
+    run(nin <= 4 ? launch_amp<1, 128> : nin <= 8 ? launch_amp<2, 128> : launch_amp<4, 128>);
+  }
+}
+
+void tmx_launch_azimuth(const TmxAmpGroup *groups, int ngroups,
+                        const TmxAmpPair *pairs, const TmxObsGrain *og,
+                        const TmxMatSet &mats, int nmat, const double2 *phis,
+                        const double2 *x, int64_t xstride, int nitem_max,
+                        cudaStream_t stream) {
   if (ngroups <= 0) {
     return;
   }
-  const int blocks = std::min(grid, ngroups);
-  if (nmat == 4) {
-    k_amp<4><<<blocks, 256, amp_smem(nbmax, 4), stream>>>(groups, ngroups, jobs, og,
-                                                          mats, angles, phis, xslot,
-                                                          nbmax, wpi, wtau, wnmax);
-  } else if (nmat == 3) {
-    k_amp<3><<<blocks, 256, amp_smem(nbmax, 3), stream>>>(groups, ngroups, jobs, og,
-                                                          mats, angles, phis, xslot,
-                                                          nbmax, wpi, wtau, wnmax);
-  } else {
-    k_amp<1><<<blocks, 256, amp_smem(nbmax, 1), stream>>>(groups, ngroups, jobs, og,
-                                                          mats, angles, phis, xslot,
-                                                          nbmax, wpi, wtau, wnmax);
-  }
+  const int slices = std::max(1, std::min((nitem_max + 127) / 128, 1024));
+  k_azimuth<<<dim3(ngroups, slices, nmat), 128, 0, stream>>>(groups, pairs, og, mats,
+                                                             phis, x, xstride);
 }
 
 void tmx_launch_q_epilogue(const TmxQJob *jobs, int njobs, const TmxObsGrain *og,

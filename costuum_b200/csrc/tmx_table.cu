@@ -7,11 +7,14 @@
 // MishchenkoOrientationDistribution.hpp:107-118,
 // DavisGreensteinOrientationDistribution.hpp:81-102,
 // ShapeDistribution.hpp:95-106, DraineHensleyShapeDistribution.hpp.
+#include <algorithm>
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <map>
 #include <system_error>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "tmx_ctx.h"
@@ -367,13 +370,86 @@ int64_t est_nmax(double x, int min_order, int max_order) {
   return std::min<int64_t>((int64_t)e, max_order - 1);
 }
 
+// one amplitude job: an incoming and an outgoing angle, nphi azimuths from
+// phi0 on, the first S at out
+struct AmpJob {
+  int32_t ain, aout, nphi;
+  int64_t phi0, out;
+};
+
+// groups of a set of jobs (TmxAmpGroup without a grain): by distinct incoming
+// angle in order of first use, at most TMX_AMP_NIN of them and about
+// kGroupPairs pairs per group
+struct AmpPlan {
+  static constexpr int kGroupPairs = 512;
+  std::vector<int32_t> ins;
+  std::vector<TmxAmpPair> pairs;
+  std::vector<TmxAmpGroup> groups;
+
+  // returns the new groups [first, second)
+  std::pair<int, int> add(const std::vector<AmpJob> &jobs) {
+    const int g0 = (int)groups.size();
+    std::map<int32_t, int> seen;
+    std::vector<int32_t> angle;
+    std::vector<std::vector<const AmpJob *>> by;
+    for (const AmpJob &j : jobs) {
+      const auto it = seen.emplace(j.ain, (int)by.size());
+      if (it.second) {
+        angle.push_back(j.ain);
+        by.emplace_back();
+      }
+      by[it.first->second].push_back(&j);
+    }
+    TmxAmpGroup g = {};
+    const auto close = [&]() {
+      if (g.npair > 0) {
+        groups.push_back(g);
+      }
+      g = TmxAmpGroup{};
+    };
+    for (size_t a = 0; a < by.size(); ++a) {
+      for (size_t j = 0; j < by[a].size(); ++j) {
+        if (g.npair >= kGroupPairs || (j == 0 && g.nin == TMX_AMP_NIN)) {
+          close();
+        }
+        if (g.npair == 0) {
+          g.in0 = (int32_t)ins.size();
+          g.pair0 = (int32_t)pairs.size();
+        }
+        if (j == 0 || g.nin == 0) {
+          ins.push_back(angle[a]);
+          ++g.nin;
+        }
+        TmxAmpPair p;
+        p.in = g.nin - 1;
+        p.angle_out = by[a][j]->aout;
+        p.nphi = by[a][j]->nphi;
+        p.pref = g.nitem;
+        p.phi0 = by[a][j]->phi0;
+        p.out = by[a][j]->out;
+        pairs.push_back(p);
+        ++g.npair;
+        g.nitem += p.nphi;
+      }
+    }
+    close();
+    return {g0, (int)groups.size()};
+  }
+};
+
+// groups [g0, g1) of a plan for one grain, their S from out0 on
+struct AmpUse {
+  int32_t grain;
+  int g0, g1;
+  int64_t out0;
+};
+
 // Work plan of the observable kernels for the grains `og` (already on the
-// device in ctx->o_og) and the amplitude jobs `sj` (already in ctx->o_sj):
-// the first (n1, n2) pair of every grain for the orientation kernel and
-// groups of at most 32 consecutive jobs of one grain for the amplitude
-// kernel.
+// device in ctx->o_og): the orientation kernel's pair-major order and the
+// amplitude kernel's groups of every grain (`uses`, by descending order) in
+// launches of blocks of similar size.
 int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
-                    const std::vector<TmxSJob> &sj) {
+                    const AmpPlan &plan, std::vector<AmpUse> uses) {
   int rc0;
   ++ctx->plan_seq;
   cudaStream_t st = ctx->stream;
@@ -417,40 +493,104 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
     CK(cudaMemcpyAsync(ctx->o_ord.p, order.data(), order.size() * sizeof(int32_t),
                        cudaMemcpyHostToDevice, st));
   }
+  uses.erase(std::remove_if(uses.begin(), uses.end(),
+                            [&](const AmpUse &u) { return og[u.grain].nmax <= 0; }),
+             uses.end());
+  std::stable_sort(uses.begin(), uses.end(), [&](const AmpUse &a, const AmpUse &b) {
+    return og[a.grain].nmax > og[b.grain].nmax;
+  });
   std::vector<TmxAmpGroup> grp;
-  for (size_t j = 0; j < sj.size(); ++j) {
-    if (grp.empty() || grp.back().grain != sj[j].grain || grp.back().njobs == 32) {
-      TmxAmpGroup a;
-      a.grain = sj[j].grain;
-      a.njobs = 0;
-      a.job0 = (int64_t)j;
-      grp.push_back(a);
+  for (const AmpUse &u : uses) {
+    for (int k = u.g0; k < u.g1; ++k) {
+      TmxAmpGroup g = plan.groups[k];
+      g.grain = u.grain;
+      g.out0 = u.out0;
+      grp.push_back(g);
     }
-    grp.back().njobs += 1;
+  }
+  // chunks of groups whose m sums fit the X buffer, and per chunk one launch
+  // per block size: ranges of groups whose block m has lo < L <= hi orders
+  ctx->o_chunks.clear();
+  std::vector<TmxAmpRange> rng;
+  const int64_t x_cap = (int64_t)1 << 24; // complex elements per matrix
+  int64_t x_max = 1;
+  for (size_t g0 = 0; g0 < grp.size();) {
+    tmx_ctx::AmpChunk ch;
+    ch.g0 = (int)g0;
+    int64_t x = 0;
+    size_t g1 = g0;
+    for (; g1 < grp.size(); ++g1) {
+      const int64_t need = (int64_t)grp[g1].npair * (og[grp[g1].grain].nmax + 1) * 4;
+      if (g1 > g0 && x + need > x_cap) {
+        break;
+      }
+      grp[g1].x0 = x;
+      x += need;
+      ch.nitem_max = std::max(ch.nitem_max, grp[g1].nitem);
+      ch.nin = std::max(ch.nin, grp[g1].nin);
+    }
+    ch.g1 = (int)g1;
+    x_max = std::max(x_max, x);
+    const int top = og[grp[g0].grain].nmax;
+    // groups of the chunk of order >= k are its first at(k)
+    std::vector<int> at(top + 2, 0);
+    for (size_t g = g0; g < g1; ++g) {
+      at[og[grp[g].grain].nmax] += 1;
+    }
+    for (int k = top - 1; k >= 0; --k) {
+      at[k] += at[k + 1];
+    }
+    const int edges[] = {TMX_MAX_NB, 64, 32, 16, 0};
+    for (int b = 0; b < 4; ++b) {
+      const int hi = edges[b], lo = edges[b + 1];
+      tmx_ctx::AmpLaunch la;
+      la.rng0 = (int)rng.size();
+      for (int m = 0; m <= top; ++m) {
+        // L = N + 1 - max(m, 1): orders nlo .. nhi
+        const int nlo = std::max(m, 1) + lo, nhi = std::max(m, 1) - 1 + hi;
+        const int first = nhi + 1 <= top ? at[nhi + 1] : 0;
+        const int last = nlo <= top ? at[nlo] : 0;
+        if (last > first) {
+          rng.push_back({la.nitems, m, ch.g0 + first});
+          la.nitems += last - first;
+          la.lcap = std::max(la.lcap, std::min(hi, top + 1 - std::max(m, 1)));
+        }
+      }
+      la.nrng = (int)rng.size() - la.rng0;
+      if (la.nitems > 0) {
+        ch.launches.push_back(la);
+      }
+    }
+    ctx->o_chunks.push_back(ch);
+    g0 = g1;
   }
   int rc;
-  if ((rc = ensure(ctx, ctx->o_pairs, base.size() * sizeof(int64_t))) ||
-      (rc = ensure(ctx, ctx->o_grp, std::max<size_t>(1, grp.size()) * sizeof(TmxAmpGroup)))) {
+  const auto put = [&](DevBuf &buf, const void *src, size_t bytes) -> int {
+    const int r = ensure(ctx, buf, std::max<size_t>(16, bytes));
+    if (r || bytes == 0) {
+      return r;
+    }
+    CK(cudaMemcpyAsync(buf.p, src, bytes, cudaMemcpyHostToDevice, st));
+    return TMX_OK;
+  };
+  if ((rc = put(ctx->o_pairs, base.data(), base.size() * sizeof(int64_t))) ||
+      (rc = put(ctx->o_grp, grp.data(), grp.size() * sizeof(TmxAmpGroup))) ||
+      (rc = put(ctx->o_ins, plan.ins.data(), plan.ins.size() * sizeof(int32_t))) ||
+      (rc = put(ctx->o_prs, plan.pairs.data(), plan.pairs.size() * sizeof(TmxAmpPair))) ||
+      (rc = put(ctx->o_rng, rng.data(), rng.size() * sizeof(TmxAmpRange)))) {
     return rc;
   }
-  CK(cudaMemcpyAsync(ctx->o_pairs.p, base.data(), base.size() * sizeof(int64_t),
-                     cudaMemcpyHostToDevice, st));
-  if (!grp.empty()) {
-    CK(cudaMemcpyAsync(ctx->o_grp.p, grp.data(), grp.size() * sizeof(TmxAmpGroup),
-                       cudaMemcpyHostToDevice, st));
-  }
   CK(cudaStreamSynchronize(st));
-  ctx->o_ngrains = n;
   ctx->o_npairs = npairs;
   ctx->o_nbmax = nbmax;
   ctx->o_pmax = nbmax;
-  ctx->o_ngrp = (int)grp.size();
+  ctx->o_xcap = x_max;
   if (ctx->profiling) {
     // flops of one matrix set over the kernels' index spaces: the
     // orientation average 16 (2M + 1)(M + 1) per (n1, n2), M = min(n1, n2),
-    // of every averaged grain; the amplitudes 16 (2 nb)^2 per m block and job
+    // of every averaged grain; the amplitudes 16 L^2 per m block (L orders)
+    // and incoming angle and 32 L per pair
     double fo = 0., fa = 0.;
-    std::vector<double> per_job(nbmax + 1, -1.);
     for (int64_t g = 0; g < n; ++g) {
       const int N = og[g].nmax;
       if (N > 0 && og[g].coef_set >= 0) {
@@ -462,19 +602,12 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
         }
       }
     }
-    for (const TmxSJob &j : sj) {
-      const int N = og[j.grain].nmax;
-      if (N <= 0) {
-        continue;
+    for (const TmxAmpGroup &g : grp) {
+      const int N = og[g.grain].nmax;
+      for (int m = 0; m <= N; ++m) {
+        const double L = N + 1 - std::max(m, 1);
+        fa += 16. * L * L * g.nin + 32. * L * g.npair;
       }
-      if (per_job[N] < 0.) {
-        double s = 16. * 4. * N * N;
-        for (int k = 1; k <= N; ++k) {
-          s += 16. * 4. * k * k;
-        }
-        per_job[N] = s;
-      }
-      fa += per_job[N];
     }
     ctx->o_fl_orient = fo;
     ctx->o_fl_amp = fa;
@@ -483,15 +616,17 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
 }
 
 // Ta = orientation average (or copy) of Tsrc with the amplitude factors
-// folded in, then the amplitudes S of every job (zeroed first: grains with
+// folded in (compact class layout), then the amplitudes S of every job (zeroed first: grains with
 // nmax 0 have no jobs)
 int run_amplitudes(tmx_ctx *ctx, const cplx *const *Tsrc, int nmat,
                    int64_t t_total, int ncoef, cplx *const *S_out,
                    int64_t s_total) {
   cudaStream_t st = ctx->stream;
   int rc;
+  // (t_total is even: every T-matrix has a multiple of four elements)
+  const int64_t ta_total = (t_total + 1) / 2;
   if ((rc = ensure(ctx, ctx->Ta,
-                   std::max<int64_t>(1, nmat * t_total) * sizeof(cplx)))) {
+                   std::max<int64_t>(1, nmat * ta_total) * sizeof(cplx)))) {
     return rc;
   }
   for (int k = 0; k < nmat; ++k) {
@@ -504,13 +639,11 @@ int run_amplitudes(tmx_ctx *ctx, const cplx *const *Tsrc, int nmat,
   TmxMatSet avg = {}, amp = {};
   for (int k = 0; k < nmat; ++k) {
     avg.src[k] = Tsrc[k];
-    avg.dst[k] = (cplx *)ctx->Ta.p + k * t_total;
+    avg.dst[k] = (cplx *)ctx->Ta.p + k * ta_total;
     amp.src[k] = avg.dst[k];
     amp.dst[k] = S_out[k];
   }
-  const int grid = tmx_amp_grid(ctx->o_nbmax, nmat);
-  if ((rc = ensure(ctx, ctx->o_x,
-                   (size_t)grid * nmat * 32 * (ctx->o_nbmax + 1) * 4 * sizeof(cplx)))) {
+  if ((rc = ensure(ctx, ctx->o_x, (size_t)nmat * ctx->o_xcap * sizeof(cplx)))) {
     return rc;
   }
   cudaEvent_t pe = nullptr;
@@ -525,37 +658,43 @@ int run_amplitudes(tmx_ctx *ctx, const cplx *const *Tsrc, int nmat,
                           (const double *)ctx->cg.p, ctx->cg_nmax, ctx->o_nbmax, 1,
                           st);
   LAUNCHED();
-  // T-matrices in and averaged T-matrices out, once each
+  // T-matrices in and averaged T-matrices (compact, half the size) out
   if ((rc = prof_end(ctx, TMX_PROF_ORIENT, pe, nmat * ctx->o_fl_orient, st,
-                     2. * nmat * t_total * sizeof(cplx)))) {
+                     1.5 * nmat * t_total * sizeof(cplx)))) {
     return rc;
   }
   if ((rc = prof_begin(ctx, TMX_PROF_AMP, &pe))) {
     return rc;
   }
   // the pi / tau columns of every angle of the plan, once for all grains
-  // (unless the table would be large: then each CTA runs the recurrences)
-  const double *wpi = nullptr, *wtau = nullptr;
   const int wn = ctx->o_nbmax;
   const size_t wcol = (size_t)ctx->o_nangles * (wn + 1) * wn;
-  if (ctx->o_nangles > 0 && 2 * wcol * sizeof(double) <= ((size_t)512 << 20)) {
-    if ((rc = ensure(ctx, ctx->o_wcol, 2 * wcol * sizeof(double)))) {
-      return rc;
+  if ((rc = ensure(ctx, ctx->o_wcol, std::max<size_t>(1, 2 * wcol) * sizeof(double)))) {
+    return rc;
+  }
+  double *wpi = (double *)ctx->o_wcol.p, *wtau = wpi + wcol;
+  tmx_launch_wigner_cols((const TmxAngle *)ctx->o_angles.p, ctx->o_nangles, wn, wpi,
+                         wtau, st);
+  LAUNCHED();
+  const TmxAmpGroup *grp = (const TmxAmpGroup *)ctx->o_grp.p;
+  const TmxAmpPair *prs = (const TmxAmpPair *)ctx->o_prs.p;
+  const TmxObsGrain *og = (const TmxObsGrain *)ctx->o_og.p;
+  for (const tmx_ctx::AmpChunk &ch : ctx->o_chunks) {
+    for (const tmx_ctx::AmpLaunch &la : ch.launches) {
+      tmx_launch_amp(grp, (const int32_t *)ctx->o_ins.p, prs,
+                     (const TmxAmpRange *)ctx->o_rng.p + la.rng0, la.nrng, la.nitems,
+                     og, amp, nmat, wpi, wtau, wn, (cplx *)ctx->o_x.p, ctx->o_xcap,
+                     la.lcap, ch.nin, st);
+      LAUNCHED();
     }
-    wpi = (const double *)ctx->o_wcol.p;
-    wtau = wpi + wcol;
-    tmx_launch_wigner_cols((const TmxAngle *)ctx->o_angles.p, ctx->o_nangles, wn,
-                           (double *)ctx->o_wcol.p, (double *)ctx->o_wcol.p + wcol, st);
+    tmx_launch_azimuth(grp + ch.g0, ch.g1 - ch.g0, prs, og, amp, nmat,
+                       (const cplx *)ctx->o_phis.p, (const cplx *)ctx->o_x.p,
+                       ctx->o_xcap, ch.nitem_max, st);
     LAUNCHED();
   }
-  tmx_launch_amp((const TmxAmpGroup *)ctx->o_grp.p, ctx->o_ngrp,
-                 (const TmxSJob *)ctx->o_sj.p, (const TmxObsGrain *)ctx->o_og.p, amp,
-                 nmat, (const TmxAngle *)ctx->o_angles.p, (const cplx *)ctx->o_phis.p,
-                 (cplx *)ctx->o_x.p, ctx->o_nbmax, grid, wpi, wtau, wn, st);
-  LAUNCHED();
-  // averaged T-matrices in, four complex amplitudes per job and azimuth out
+  // averaged T-matrices in, four complex amplitudes per pair and azimuth out
   if ((rc = prof_end(ctx, TMX_PROF_AMP, pe, nmat * ctx->o_fl_amp, st,
-                     nmat * (t_total + 4. * s_total) * sizeof(cplx)))) {
+                     nmat * (t_total / 2. + 4. * s_total) * sizeof(cplx)))) {
     return rc;
   }
   return TMX_OK;
@@ -766,68 +905,47 @@ extern "C" int tmx_get_table(
     ++ctx->plan_seq; // the observable buffers change below
     CK(cudaMemcpyAsync(ctx->o_og.p, og.data(), ng * sizeof(TmxObsGrain),
                        cudaMemcpyHostToDevice, st));
-    // ---- amplitude jobs
-    std::vector<TmxSJob> sj;
+    // ---- amplitudes: the same angles for every grain
+    AmpPlan plan;
+    std::vector<AmpUse> uses;
     std::vector<TmxQJob> qj;
-    int64_t sidx = 0;
-    const int64_t sca_base = ng * ntheta * (1 + (account ? (int64_t)ngauss * ngauss : 0));
+    const int64_t per_theta = 1 + (account ? (int64_t)ngauss * ngauss : 0);
+    const int64_t sca_base = ng * ntheta * per_theta;
+    std::vector<AmpJob> jobs;
+    for (int t = 0; t < ntheta; ++t) {
+      jobs.push_back({t, t, 1, 0, t * per_theta});
+      for (int ti = 0; account && ti < ngauss; ++ti) {
+        jobs.push_back({acc_a0 + ti, t, ngauss, acc_p0,
+                        t * per_theta + 1 + (int64_t)ti * ngauss});
+      }
+    }
+    const auto main_groups = plan.add(jobs);
+    jobs.clear();
+    for (int t = 0; do_sca && t < ntheta; ++t) {
+      jobs.push_back({sca_ain, sca_a0 + t, nphi_sca, sca_p0, (int64_t)t * nphi_sca});
+    }
+    const auto sca_groups = plan.add(jobs);
     for (int64_t g = 0; g < ng; ++g) {
       if (og[g].nmax <= 0) {
         continue;
       }
+      const int64_t out0 = g * ntheta * per_theta;
+      uses.push_back({(int32_t)g, main_groups.first, main_groups.second, out0});
+      uses.push_back({(int32_t)g, sca_groups.first, sca_groups.second,
+                      sca_base + g * ntheta * nphi_sca});
       for (int t = 0; t < ntheta; ++t) {
         TmxQJob q;
         q.grain = (int32_t)g;
         q.pad = 0;
         q.out = g * ntheta + t;
-        TmxSJob j;
-        j.grain = (int32_t)g;
-        j.angle_in = t;
-        j.angle_out = t;
-        j.nphi = 1;
-        j.phi0 = 0;
-        j.out = sidx;
-        q.s_main = sidx;
-        sidx += 1;
-        sj.push_back(j);
-        q.s_acc = sidx;
-        if (account) {
-          for (int ti = 0; ti < ngauss; ++ti) {
-            TmxSJob a;
-            a.grain = (int32_t)g;
-            a.angle_in = acc_a0 + ti;
-            a.angle_out = t;
-            a.nphi = ngauss;
-            a.phi0 = acc_p0;
-            a.out = sidx;
-            sidx += ngauss;
-            sj.push_back(a);
-          }
-        }
+        q.s_main = out0 + t * per_theta;
+        q.s_acc = q.s_main + 1;
         qj.push_back(q);
       }
     }
-    int64_t nsca = 0;
-    if (do_sca) {
-      for (int64_t g = 0; g < ng; ++g) {
-        for (int t = 0; t < ntheta; ++t) {
-          if (og[g].nmax > 0) {
-            TmxSJob j;
-            j.grain = (int32_t)g;
-            j.angle_in = sca_ain;
-            j.angle_out = sca_a0 + t;
-            j.nphi = nphi_sca;
-            j.phi0 = sca_p0;
-            j.out = sca_base + (g * ntheta + t) * nphi_sca;
-            sj.push_back(j);
-          }
-        }
-      }
-      nsca = ng * ntheta * nphi_sca;
-    }
+    const int64_t nsca = do_sca ? ng * ntheta * nphi_sca : 0;
     const int64_t s_total = sca_base + nsca;
-    if ((rc = ensure(ctx, ctx->o_sj, std::max<size_t>(1, sj.size()) * sizeof(TmxSJob))) ||
-        (rc = ensure(ctx, ctx->o_qj, std::max<size_t>(1, qj.size()) * sizeof(TmxQJob))) ||
+    if ((rc = ensure(ctx, ctx->o_qj, std::max<size_t>(1, qj.size()) * sizeof(TmxQJob))) ||
         (rc = ensure(ctx, ctx->o_S, std::max<int64_t>(1, s_total) * 4 * sizeof(cplx))) ||
         (rc = ensure(ctx, ctx->o_gq, std::max<int64_t>(1, ng * ntheta * nq) * sizeof(double))) ||
         (rc = ensure(ctx, ctx->o_gz, std::max<int64_t>(1, do_sca ? nsca * 16 : 1) * sizeof(double))) ||
@@ -835,15 +953,11 @@ extern "C" int tmx_get_table(
         (rc = ensure(ctx, ctx->o_cz, std::max<int64_t>(1, do_sca ? nc * ntheta * nphi_sca * 16 : 1) * sizeof(double)))) {
       return rc;
     }
-    if (!sj.empty()) {
-      CK(cudaMemcpyAsync(ctx->o_sj.p, sj.data(), sj.size() * sizeof(TmxSJob),
-                         cudaMemcpyHostToDevice, st));
-    }
     if (!qj.empty()) {
       CK(cudaMemcpyAsync(ctx->o_qj.p, qj.data(), qj.size() * sizeof(TmxQJob),
                          cudaMemcpyHostToDevice, st));
     }
-    if ((rc = upload_obs_plan(ctx, og, sj)) ||
+    if ((rc = upload_obs_plan(ctx, og, plan, std::move(uses))) ||
         (ctx->obs_s_valid = false, false) ||
         (rc = run_amplitudes(ctx, (const cplx *)ctx->T.p, t_total, ncoef,
                              (cplx *)ctx->o_S.p, s_total))) {
@@ -968,9 +1082,14 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
   }
   std::vector<cplx> phis(1, mkc(1., 0.));
   std::vector<TmxObsGrain> og(n);
-  std::vector<TmxSJob> sj;
+  AmpPlan plan;
+  std::vector<AmpJob> jobs;
+  for (int t = 0; t < ntheta; ++t) {
+    jobs.push_back({t, t, 1, 0, t});
+  }
+  const auto groups = plan.add(jobs);
+  std::vector<AmpUse> uses;
   std::vector<TmxQJob> qj;
-  sj.reserve((size_t)n * ntheta);
   qj.reserve((size_t)n * ntheta);
   for (int64_t g = 0; g < n; ++g) {
     og[g].nmax = ctx->nmax_h[g];
@@ -985,15 +1104,8 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
     if (og[g].nmax <= 0) {
       continue;
     }
+    uses.push_back({(int32_t)g, groups.first, groups.second, g * ntheta});
     for (int t = 0; t < ntheta; ++t) {
-      TmxSJob j;
-      j.grain = (int32_t)g;
-      j.angle_in = t;
-      j.angle_out = t;
-      j.nphi = 1;
-      j.phi0 = 0;
-      j.out = g * ntheta + t;
-      sj.push_back(j);
       TmxQJob q;
       q.grain = (int32_t)g;
       q.pad = 0;
@@ -1006,7 +1118,6 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
   if ((rc = ensure(ctx, ctx->o_angles, std::max(1, ntheta) * sizeof(TmxAngle))) ||
       (rc = ensure(ctx, ctx->o_phis, sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->o_og, std::max<int64_t>(1, n) * sizeof(TmxObsGrain))) ||
-      (rc = ensure(ctx, ctx->o_sj, std::max<size_t>(1, sj.size()) * sizeof(TmxSJob))) ||
       (rc = ensure(ctx, ctx->o_qj, std::max<size_t>(1, qj.size()) * sizeof(TmxQJob))) ||
       (rc = ensure(ctx, ctx->o_coef, std::max(1, ncoef) * sizeof(double)))) {
     return rc;
@@ -1018,9 +1129,7 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
                      cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(ctx->o_og.p, og.data(), n * sizeof(TmxObsGrain),
                      cudaMemcpyHostToDevice, st));
-  if (!sj.empty()) {
-    CK(cudaMemcpyAsync(ctx->o_sj.p, sj.data(), sj.size() * sizeof(TmxSJob),
-                       cudaMemcpyHostToDevice, st));
+  if (!qj.empty()) {
     CK(cudaMemcpyAsync(ctx->o_qj.p, qj.data(), qj.size() * sizeof(TmxQJob),
                        cudaMemcpyHostToDevice, st));
   }
@@ -1028,7 +1137,6 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
     CK(cudaMemcpyAsync(ctx->o_coef.p, coeffs, ncoef * sizeof(double),
                        cudaMemcpyHostToDevice, st));
   }
-  ctx->o_nsj = (int)sj.size();
   ctx->o_nqj = (int)qj.size();
   if (coeffs) {
     int nmax_b = 1;
@@ -1039,7 +1147,7 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
       return rc;
     }
   }
-  if ((rc = upload_obs_plan(ctx, og, sj))) {
+  if ((rc = upload_obs_plan(ctx, og, plan, std::move(uses)))) {
     return rc;
   }
   key.valid = true;
@@ -1425,81 +1533,98 @@ void k_from_s(double k, const zc S[2][2], double *K) {
   K[14] = -K[11];
 }
 
-// Amplitude matrices S^P of jobs (grain, incoming angle index, outgoing
-// angle index, e^{i(phi_out - phi_in)}) for the T-matrices of the last batch
-// (plain or averaged): sorted by grain for the amplitude kernel's groups,
-// results in job order.
+// Amplitude matrices S^P of jobs (AmpJob with a grain each: incoming and
+// outgoing angle, azimuths e^{i(phi_out - phi_in)}) for the T-matrices of the
+// last batch (plain or averaged); ns amplitudes in all, at the jobs' places.
 int plain_amplitudes(tmx_ctx *ctx, const std::vector<int32_t> &grain,
-                     const std::vector<TmxAngle> &ang,
-                     const std::vector<int32_t> &ain,
-                     const std::vector<int32_t> &aout,
-                     const std::vector<cplx> &e1, std::vector<zc> &S) {
+                     const std::vector<TmxAngle> &ang, const std::vector<AmpJob> &jobs,
+                     const std::vector<cplx> &e1, int64_t ns, std::vector<zc> &S) {
   cudaStream_t st = ctx->stream;
   const int64_t n = ctx->n;
   const int64_t nj = (int64_t)grain.size();
   int rc;
   std::vector<TmxObsGrain> og(n);
+  int nbmax = 1;
   for (int64_t g = 0; g < n; ++g) {
     og[g].nmax = ctx->nmax_h[g];
     og[g].coef_set = -1;
     og[g].t_off = ctx->t_off_h[g];
     og[g].k = ctx->up_grains[g].k;
     og[g].r_ev = ctx->up_grains[g].r_ev;
-  }
-  std::vector<int64_t> order(nj);
-  for (int64_t j = 0; j < nj; ++j) {
-    order[j] = j;
-  }
-  std::stable_sort(order.begin(), order.end(),
-                   [&](int64_t a, int64_t b) { return grain[a] < grain[b]; });
-  std::vector<TmxSJob> sj;
-  sj.reserve(nj);
-  for (int64_t q = 0; q < nj; ++q) {
-    const int64_t j = order[q];
-    if (og[grain[j]].nmax <= 0) {
-      continue;
-    }
-    TmxSJob J;
-    J.grain = grain[j];
-    J.angle_in = ain[j];
-    J.angle_out = aout[j];
-    J.nphi = 1;
-    J.phi0 = j;
-    J.out = j;
-    sj.push_back(J);
+    nbmax = std::max(nbmax, og[g].nmax);
   }
   if ((rc = ensure(ctx, ctx->o_og, std::max<int64_t>(1, n) * sizeof(TmxObsGrain))) ||
-      (rc = ensure(ctx, ctx->o_angles, std::max<size_t>(1, ang.size()) * sizeof(TmxAngle))) ||
       (rc = ensure(ctx, ctx->o_phis, std::max<size_t>(1, e1.size()) * sizeof(cplx))) ||
-      (rc = ensure(ctx, ctx->o_sj, std::max<size_t>(1, sj.size()) * sizeof(TmxSJob))) ||
-      (rc = ensure(ctx, ctx->o_S, std::max<int64_t>(1, nj) * 4 * sizeof(cplx)))) {
+      (rc = ensure(ctx, ctx->o_S, std::max<int64_t>(1, ns) * 4 * sizeof(cplx)))) {
     return rc;
   }
+  std::vector<std::vector<AmpJob>> by(n);
+  // angles in use, renumbered per pass: a pass takes jobs until the table of
+  // its angles reaches 512 MB
+  const int64_t max_ang = std::max<int64_t>(
+      2, ((int64_t)512 << 20) / (16 * (int64_t)(nbmax + 1) * nbmax));
+  std::vector<int32_t> local(ang.size());
+  S.assign(4 * ns, zc(0., 0.));
+  std::vector<cplx> Sh(4 * ns);
   ++ctx->plan_seq; // the observable buffers change below
+  ctx->obs_s_valid = false;
   CK(cudaMemcpyAsync(ctx->o_og.p, og.data(), n * sizeof(TmxObsGrain),
                      cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(ctx->o_angles.p, ang.data(), ang.size() * sizeof(TmxAngle),
-                     cudaMemcpyHostToDevice, st));
-  ctx->o_nangles = (int)ang.size();
   CK(cudaMemcpyAsync(ctx->o_phis.p, e1.data(), e1.size() * sizeof(cplx),
                      cudaMemcpyHostToDevice, st));
-  if (!sj.empty()) {
-    CK(cudaMemcpyAsync(ctx->o_sj.p, sj.data(), sj.size() * sizeof(TmxSJob),
+  int64_t j0 = 0;
+  while (j0 < nj) {
+    std::fill(local.begin(), local.end(), -1);
+    std::vector<TmxAngle> used;
+    for (auto &v : by) {
+      v.clear();
+    }
+    const int64_t first = j0;
+    for (; j0 < nj; ++j0) {
+      if (og[grain[j0]].nmax <= 0) {
+        continue;
+      }
+      AmpJob J = jobs[j0];
+      const int fresh = (local[J.ain] < 0) + (local[J.aout] < 0 && J.aout != J.ain);
+      if (j0 > first && (int64_t)used.size() + fresh > max_ang) {
+        break;
+      }
+      for (int32_t *a : {&J.ain, &J.aout}) {
+        int32_t &l = local[*a];
+        if (l < 0) {
+          l = (int32_t)used.size();
+          used.push_back(ang[*a]);
+        }
+        *a = l;
+      }
+      by[grain[j0]].push_back(J);
+    }
+    AmpPlan plan;
+    std::vector<AmpUse> uses;
+    for (int64_t g = 0; g < n; ++g) {
+      if (!by[g].empty()) {
+        const auto gr = plan.add(by[g]);
+        uses.push_back({(int32_t)g, gr.first, gr.second, 0});
+      }
+    }
+    if ((rc = ensure(ctx, ctx->o_angles, std::max<size_t>(1, used.size()) * sizeof(TmxAngle)))) {
+      return rc;
+    }
+    CK(cudaMemcpyAsync(ctx->o_angles.p, used.data(), used.size() * sizeof(TmxAngle),
                        cudaMemcpyHostToDevice, st));
-  }
-  if ((rc = upload_obs_plan(ctx, og, sj)) ||
-      (ctx->obs_s_valid = false, false) ||
-      (rc = run_amplitudes(ctx, (const cplx *)ctx->T.p, ctx->p2_t_total, 1,
-                           (cplx *)ctx->o_S.p, nj))) {
-    return rc;
-  }
-  std::vector<cplx> Sh(4 * nj);
-  CK(cudaMemcpyAsync(Sh.data(), ctx->o_S.p, 4 * nj * sizeof(cplx),
-                     cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  S.resize(4 * nj);
-  for (int64_t i = 0; i < 4 * nj; ++i) {
-    S[i] = zc(Sh[i].x, Sh[i].y);
+    ctx->o_nangles = (int)used.size();
+    if ((rc = upload_obs_plan(ctx, og, plan, std::move(uses))) ||
+        (rc = run_amplitudes(ctx, (const cplx *)ctx->T.p, ctx->p2_t_total, 1,
+                             (cplx *)ctx->o_S.p, ns))) {
+      return rc;
+    }
+    CK(cudaMemcpyAsync(Sh.data(), ctx->o_S.p, 4 * ns * sizeof(cplx),
+                       cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    // each pass leaves zeros at the other passes' places
+    for (int64_t i = 0; i < 4 * ns; ++i) {
+      S[i] += zc(Sh[i].x, Sh[i].y);
+    }
   }
   return TMX_OK;
 }
@@ -1523,25 +1648,42 @@ int lab_amplitudes(tmx_ctx *ctx, int64_t njobs, const int64_t *grain,
                    const double *theta_in, const double *phi_in,
                    const double *theta_out, const double *phi_out,
                    std::vector<zc> &SL) {
-  std::vector<int32_t> g(njobs), ain(njobs), aout(njobs);
-  std::vector<TmxAngle> ang(2 * njobs);
+  std::vector<int32_t> g(njobs);
+  std::vector<AmpJob> jobs(njobs);
   std::vector<cplx> e1(njobs);
   std::vector<PDir> din(njobs), dout(njobs);
+  // one angle per distinct particle-frame zenith
+  std::vector<TmxAngle> ang;
+  std::unordered_map<uint64_t, int32_t> index;
+  const auto angle = [&](const TmxAngle &a) {
+    uint64_t h[3];
+    memcpy(h, &a, sizeof(h));
+    // (cos, sin) name the angle; 1 / sin follows from sin
+    uint64_t key = h[0] ^ (h[1] * 0x9E3779B97F4A7C15ull);
+    for (;;) {
+      const auto it = index.emplace(key, (int32_t)ang.size());
+      if (it.second) {
+        ang.push_back(a);
+      }
+      const int32_t i = it.first->second;
+      if (memcmp(&ang[i], &a, sizeof(a)) == 0) {
+        return i;
+      }
+      key = key * 6364136223846793005ull + 1442695040888963407ull;
+    }
+  };
   for (int64_t j = 0; j < njobs; ++j) {
     const double ca = cos(alpha[j]), sa = sin(alpha[j]);
     const double cb = cos(beta[j]), sb = sin(beta[j]);
     din[j] = particle_dir(ca, sa, cb, sb, theta_in[j], phi_in[j]);
     dout[j] = particle_dir(ca, sa, cb, sb, theta_out[j], phi_out[j]);
     g[j] = (int32_t)grain[j];
-    ang[2 * j] = din[j].a;
-    ang[2 * j + 1] = dout[j].a;
-    ain[j] = (int32_t)(2 * j);
-    aout[j] = (int32_t)(2 * j + 1);
+    jobs[j] = {angle(din[j].a), angle(dout[j].a), 1, j, j};
     e1[j] = mkc(dout[j].cphi * din[j].cphi + dout[j].sphi * din[j].sphi,
                 dout[j].sphi * din[j].cphi - dout[j].cphi * din[j].sphi);
   }
   std::vector<zc> SP;
-  int rc = plain_amplitudes(ctx, g, ang, ain, aout, e1, SP);
+  int rc = plain_amplitudes(ctx, g, ang, jobs, e1, njobs, SP);
   if (rc) {
     return rc;
   }
@@ -1587,26 +1729,25 @@ int absorption(tmx_ctx *ctx, int32_t grain, int32_t ntheta, const double *th,
   for (int t = 0; t < ntheta; ++t) {
     ang.push_back(plain_angle(th[t]));
   }
-  std::vector<int32_t> g, ain, aout;
-  std::vector<cplx> e1;
+  // per angle the forward amplitude, then every incoming zenith with its
+  // ngauss azimuths: e^{i(0 - phi_in)} as the reference forms it
+  std::vector<AmpJob> jobs;
+  std::vector<cplx> e1(1, mkc(1., 0.));
+  for (int ip = 0; ip < ngauss; ++ip) {
+    const double cp = cos(ph[ip]), sp = sin(ph[ip]);
+    e1.push_back(mkc(1. * cp + 0. * sp, 0. * cp - 1. * sp));
+  }
+  int64_t ns = 0;
   for (int t = 0; t < ntheta; ++t) {
-    g.push_back(grain);
-    ain.push_back(a0 + t);
-    aout.push_back(a0 + t);
-    e1.push_back(mkc(1., 0.));
+    jobs.push_back({a0 + t, a0 + t, 1, 0, ns++});
     for (int it = 0; it < ngauss; ++it) {
-      for (int ip = 0; ip < ngauss; ++ip) {
-        // e^{i(0 - phi_in)} as the reference forms it
-        const double cp = cos(ph[ip]), sp = sin(ph[ip]);
-        g.push_back(grain);
-        ain.push_back(it);
-        aout.push_back(a0 + t);
-        e1.push_back(mkc(1. * cp + 0. * sp, 0. * cp - 1. * sp));
-      }
+      jobs.push_back({it, a0 + t, ngauss, 1, ns});
+      ns += ngauss;
     }
   }
   std::vector<zc> S;
-  int rc = plain_amplitudes(ctx, g, ang, ain, aout, e1, S);
+  int rc = plain_amplitudes(ctx, std::vector<int32_t>(jobs.size(), grain), ang, jobs, e1,
+                            ns, S);
   if (rc) {
     return rc;
   }
@@ -1683,7 +1824,7 @@ extern "C" int tmx_batch_orientation_average(tmx_ctx *ctx, const double *coeffs,
     CK(cudaMemcpyAsync(ctx->o_coef.p, coeffs, (int64_t)nsets * ncoef * sizeof(double),
                        cudaMemcpyHostToDevice, st));
   }
-  if ((rc = upload_obs_plan(ctx, og, std::vector<TmxSJob>()))) {
+  if ((rc = upload_obs_plan(ctx, og, AmpPlan(), {}))) {
     return rc;
   }
   if (t_total > 0 && ctx->o_npairs > 0) {
