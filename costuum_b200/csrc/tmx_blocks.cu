@@ -1,4 +1,4 @@
-// Block kernel: for one (grain, m, parity class) work item, assemble the
+// Block kernels: for one (grain, m, parity class) work item, assemble the
 // class sub-matrices of Q and RgQ by quadrature, factor Q with partial
 // pivoting in shared memory and solve T_c Q_c = -RgQ_c.
 //
@@ -17,7 +17,7 @@
 //    the LUs of the independent classes. Each class is one work item here.
 //  * Assembly as a GEMM. Every entry is sum_g sum_{t<4} F_t(g, n1) W_t(g, n2)
 //    with A-side vectors built from h_n1 = j + i y (or j alone for RgQ) and
-//    B-side vectors built from j_n2(m k r); see build_chunk().
+//    B-side vectors built from j_n2(m k r); see below.
 //  * T = -RgQ Q^-1 by two triangular solves on the LU factors instead of the
 //    explicit inverse followed by a product.
 #include <algorithm>
@@ -40,11 +40,12 @@
 // A-side vectors (F^j, F^y) of row member a at node g, stored to f[t * ts].
 // LEAN: without the factor a_n (the caller scales the finished entries by
 // a_n1 a_n2) and, for m = 0, only the terms 1 and 3 that survive mu = 0.
+// (an: a_n of the row, not used by LEAN)
 template <bool LEAN = false>
 __device__ __forceinline__ void a_side_row(double j, double dj, double y,
                                            double dy, double d, double dd,
                                            const double *s, int n, cplx *f,
-                                           int ts, int m) {
+                                           int ts, int m, double an = 1.) {
   const double nn = n * (n + 1.);
   const double q = nn * s[TMX_NS_DRR] * s[TMX_NS_KRINV] * d;
   if (LEAN) {
@@ -56,7 +57,6 @@ __device__ __forceinline__ void a_side_row(double j, double dj, double y,
     f[3 * ts] = mkc(dd * dj + q * j, dd * dy + q * y);
     return;
   }
-  const double an = a_n(n);
   f[0] = mkc(an * d * j, an * d * y);
   f[ts] = mkc(an * dd * j, an * dd * y);
   f[2 * ts] = mkc(an * d * dj, an * d * dy);
@@ -77,50 +77,66 @@ __device__ __forceinline__ void a_side(const ClassDesc &D, int a, int N, int g,
                    S + (int64_t)g * TMX_NS, n, f, ts, m);
 }
 
-// B-side vectors of column member b at node g for each row group, stored to
+// B-side vectors of column member (ib, n) at one node for the rows of block
+// index ia, stored to wr[t * ts]. LEAN as for a_side.
+struct BSide {
+  cplx G1, G2, G3, G4;
+  double wr2, mu, beta;
+};
+template <bool LEAN>
+__device__ __forceinline__ BSide b_side_node(int n, int m, cplx jm, cplx djm, double d,
+                                             double dd, const double *s,
+                                             double an = 1.) {
+  BSide B;
+  const double nn = n * (n + 1.);
+  const cplx kmi = mkc(s[TMX_NS_KRMRINV_RE], s[TMX_NS_KRMRINV_IM]);
+  B.G1 = cscale(djm, an * d);
+  B.G2 = cscale(
+      cadd(cscale(djm, dd), cscale(cmul(kmi, jm), s[TMX_NS_DRR] * nn * d)), an);
+  B.G3 = cscale(jm, an * d);
+  B.G4 = cscale(jm, an * dd);
+  B.wr2 = s[TMX_NS_W] * s[TMX_NS_R2];
+  B.mu = (double)(m * m) * s[TMX_NS_SIN2INV];
+  B.beta = s[TMX_NS_SININV] * m * B.wr2;
+  return B;
+}
+template <bool LEAN>
+__device__ __forceinline__ void b_side_terms(const BSide &B, int ia, int ib, int m,
+                                             double k2, cplx k2mr, cplx *wr, int ts) {
+  if (ia == ib) {
+    // diagonal-type block: Q11 (i = 0) or Q22 (i = 1)
+    const cplx chi = (ia == 0) ? k2mr : mkc(k2, 0.);
+    const cplx clo = (ia == 0) ? mkc(-k2, 0.) : mkc(-k2mr.x, -k2mr.y);
+    if (!LEAN || m != 0) {
+      wr[0] = cmul(chi, cscale(B.G1, B.wr2 * B.mu));
+      wr[2 * ts] = cmul(clo, cscale(B.G3, B.wr2 * B.mu));
+    }
+    wr[ts] = cmul(chi, cscale(B.G2, B.wr2));
+    wr[3 * ts] = cmul(clo, cscale(B.G4, B.wr2));
+  } else {
+    // off-diagonal block: Q12 (ia = 0, ib = 1) or Q21 (ia = 1, ib = 0)
+    const cplx c1 = (ia == 0) ? k2mr : mkc(k2, 0.);
+    const cplx c2 = (ia == 0) ? mkc(k2, 0.) : k2mr;
+    const cplx ic1 = mkc(-c1.y * B.beta, c1.x * B.beta); // i c1 beta
+    const cplx ic2 = mkc(-c2.y * B.beta, c2.x * B.beta);
+    wr[0] = cmul(ic1, B.G4);
+    wr[ts] = cmul(ic1, B.G3);
+    wr[2 * ts] = cmul(ic2, B.G2);
+    wr[3 * ts] = cmul(ic2, B.G1);
+  }
+}
+
+// B-side vectors of a column member for each row group, stored to
 // w[rg * gs + t * ts] (rg = 0 rows of block index D.iA, rg = 1 rows of D.iB).
-// LEAN as for a_side.
 template <bool LEAN = false>
 __device__ __forceinline__ void b_side_row(const ClassDesc &D, int ib, int n,
                                            int m, cplx jm, cplx djm, double d,
                                            double dd, const double *s,
                                            int ngroups, double k2, cplx k2mr,
                                            cplx *w, int ts, int gs) {
-  const double an = LEAN ? 1. : a_n(n);
-  const double nn = n * (n + 1.);
-  const cplx kmi = mkc(s[TMX_NS_KRMRINV_RE], s[TMX_NS_KRMRINV_IM]);
-  const cplx G1 = cscale(djm, an * d);
-  const cplx G2 = cscale(
-      cadd(cscale(djm, dd), cscale(cmul(kmi, jm), s[TMX_NS_DRR] * nn * d)), an);
-  const cplx G3 = cscale(jm, an * d);
-  const cplx G4 = cscale(jm, an * dd);
-  const double wr2 = s[TMX_NS_W] * s[TMX_NS_R2];
-  const double mu = (double)(m * m) * s[TMX_NS_SIN2INV];
-  const double beta = s[TMX_NS_SININV] * m * wr2;
+  const BSide B = b_side_node<LEAN>(n, m, jm, djm, d, dd, s);
   for (int rg = 0; rg < ngroups; ++rg) {
-    const int ia = (rg == 0) ? D.iA : D.iB;
-    cplx *wr = w + rg * gs;
-    if (ia == ib) {
-      // diagonal-type block: Q11 (i = 0) or Q22 (i = 1)
-      const cplx chi = (ia == 0) ? k2mr : mkc(k2, 0.);
-      const cplx clo = (ia == 0) ? mkc(-k2, 0.) : mkc(-k2mr.x, -k2mr.y);
-      if (!LEAN || m != 0) {
-        wr[0] = cmul(chi, cscale(G1, wr2 * mu));
-        wr[2 * ts] = cmul(clo, cscale(G3, wr2 * mu));
-      }
-      wr[ts] = cmul(chi, cscale(G2, wr2));
-      wr[3 * ts] = cmul(clo, cscale(G4, wr2));
-    } else {
-      // off-diagonal block: Q12 (ia = 0, ib = 1) or Q21 (ia = 1, ib = 0)
-      const cplx c1 = (ia == 0) ? k2mr : mkc(k2, 0.);
-      const cplx c2 = (ia == 0) ? mkc(k2, 0.) : k2mr;
-      const cplx ic1 = mkc(-c1.y * beta, c1.x * beta); // i c1 beta
-      const cplx ic2 = mkc(-c2.y * beta, c2.x * beta);
-      wr[0] = cmul(ic1, G4);
-      wr[ts] = cmul(ic1, G3);
-      wr[2 * ts] = cmul(ic2, G2);
-      wr[3 * ts] = cmul(ic2, G1);
-    }
+    b_side_terms<LEAN>(B, (rg == 0) ? D.iA : D.iB, ib, m, k2, k2mr, w + rg * gs, ts);
   }
 }
 
@@ -144,345 +160,6 @@ __device__ __forceinline__ void b_side(const ClassDesc &D, int b, int N, int m,
 __device__ __forceinline__ void zero_side(cplx *f, int ts, int nt) {
   for (int t = 0; t < nt; ++t) {
     f[t * ts] = mkc(0., 0.);
-  }
-}
-
-template <int TC>
-__device__ void build_chunk(const ClassDesc &D, const AsmLayout &L, int N,
-                            int m, int ng, int g0, const double *__restrict__ T,
-                            const double *__restrict__ S,
-                            const double *__restrict__ Wg, double k2,
-                            cplx k2mr, cplx *Fs, cplx *Ws) {
-  const int G = L.G;
-  // A side
-  for (int u = threadIdx.x; u < G * L.NRp; u += blockDim.x) {
-    const int gl = u / L.NRp;
-    const int pr = u % L.NRp;
-    const int g = g0 + gl;
-    const int a = padded_member(D, pr);
-    cplx *fp = Fs + (int64_t)(4 * gl) * L.NRp + pr;
-    if (a >= 0 && g < ng) {
-      a_side(D, a, N, g, T, S, Wg, fp, L.NRp);
-    } else {
-      zero_side(fp, L.NRp, 4);
-    }
-  }
-  // B side
-  const int ncolp = L.CT * TC;
-  for (int u = threadIdx.x; u < G * ncolp; u += blockDim.x) {
-    const int gl = u / ncolp;
-    const int b = u % ncolp;
-    const int g = g0 + gl;
-    cplx *wp = Ws + (int64_t)(4 * gl) * ncolp + b;
-    const int gs = 4 * G * ncolp;
-    if (b < D.nb && g < ng) {
-      b_side(D, b, N, m, g, L.ngroups, T, S, Wg, k2, k2mr, wp, ncolp, gs);
-    } else {
-      for (int rg = 0; rg < L.ngroups; ++rg) {
-        zero_side(wp + rg * gs, ncolp, 4);
-      }
-    }
-  }
-}
-
-extern __shared__ __align__(16) unsigned char tmx_smem[];
-
-// one item `it` by the whole CTA (every thread calls it; the early returns
-// are uniform over the CTA)
-template <int TR, int TC, int NT>
-__device__ __forceinline__ void block_item(const TmxBlockArgs &A, int it,
-                                           size_t smem_bytes) {
-  const TmxItem item = A.items[it];
-  const TmxSlot sl = A.slots[item.slot];
-  const TmxGrain G = A.grains[sl.grain];
-  const int N = sl.nmax;
-  const int ng = sl.ngauss;
-  const int m = item.m;
-  const ClassDesc D = describe<TR>(N, m, item.cls);
-  const int nb = D.nb;
-  if (nb <= 0) {
-    return;
-  }
-  // (shared memory is sized for classes of at most max_nb members)
-  if (nb > TMX_MAX_NB || nb > A.max_nb) {
-    if (threadIdx.x == 0) {
-      atomicOr(&A.status[sl.grain], TMX_ST_TOO_LARGE);
-    }
-    return;
-  }
-  const double *T = A.tab + sl.tab;
-  const double *S = A.nsc + sl.nsc;
-  const double *Wg = A.wig + A.wig_off[sl.wig_n] + (int64_t)m * ng * N * 2;
-  const double k2 = G.k * G.k;
-  const cplx k2mr = mkc(G.mr * k2, G.mi * k2);
-  cplx *Qs = A.scratch + item.scratch;
-  cplx *Rs = Qs + (int64_t)nb * nb;
-
-  // ------------------------------------------------------------ assembly
-  AsmLayout L;
-  L.G = A.chunk_nodes;
-  L.NRp = D.NRp;
-  L.CT = (nb + TC - 1) / TC;
-  L.ncol = L.CT * TC;
-  L.ngroups = (D.R1 > 0 && m > 0) ? 2 : 1;
-  const int RT = D.NRp / TR;
-  cplx *Fs = reinterpret_cast<cplx *>(tmx_smem);
-  cplx *Ws = Fs + (int64_t)4 * L.G * L.NRp;
-  const int ntiles = RT * L.CT;
-  const int tstep = (m == 0) ? 2 : 1; // m = 0: mu = 0 kills t = 0, 2
-  const int t0 = (m == 0) ? 1 : 0;
-  for (int tile0 = 0; tile0 < ntiles; tile0 += NT) {
-    const int tile = tile0 + threadIdx.x;
-    const bool active = tile < ntiles;
-    const int ct = active ? tile % L.CT : 0;
-    const int rt = active ? tile / L.CT : 0;
-    const int rg = (rt * TR < D.R0p) ? 0 : 1;
-    double aj[TR][TC][2], ay[TR][TC][2];
-#pragma unroll
-    for (int r = 0; r < TR; ++r) {
-#pragma unroll
-      for (int c = 0; c < TC; ++c) {
-        aj[r][c][0] = aj[r][c][1] = ay[r][c][0] = ay[r][c][1] = 0.;
-      }
-    }
-    for (int g0 = 0; g0 < ng; g0 += L.G) {
-      __syncthreads();
-      build_chunk<TC>(D, L, N, m, ng, g0, T, S, Wg, k2, k2mr, Fs, Ws);
-      __syncthreads();
-      if (active) {
-        const int kmax = 4 * min(L.G, ng - g0);
-        for (int kk = t0; kk < kmax; kk += tstep) {
-          const cplx *fr = Fs + (int64_t)kk * L.NRp + rt * TR;
-          const cplx *wr = Ws + ((int64_t)rg * 4 * L.G + kk) * L.ncol + ct;
-          cplx f[TR], w[TC];
-#pragma unroll
-          for (int r = 0; r < TR; ++r) {
-            f[r] = fr[r];
-          }
-#pragma unroll
-          for (int c = 0; c < TC; ++c) {
-            w[c] = wr[c * L.CT];
-          }
-#pragma unroll
-          for (int r = 0; r < TR; ++r) {
-#pragma unroll
-            for (int c = 0; c < TC; ++c) {
-              aj[r][c][0] = fma(f[r].x, w[c].x, aj[r][c][0]);
-              aj[r][c][1] = fma(f[r].x, w[c].y, aj[r][c][1]);
-              ay[r][c][0] = fma(f[r].y, w[c].x, ay[r][c][0]);
-              ay[r][c][1] = fma(f[r].y, w[c].y, ay[r][c][1]);
-            }
-          }
-        }
-      }
-    }
-    if (active) {
-#pragma unroll
-      for (int r = 0; r < TR; ++r) {
-        const int a = padded_member(D, rt * TR + r);
-        if (a < 0) {
-          continue;
-        }
-#pragma unroll
-        for (int c = 0; c < TC; ++c) {
-          const int b = ct + c * L.CT;
-          if (b >= nb) {
-            continue;
-          }
-          // Q = G^j + i G^y, RgQ = G^j
-          Qs[(int64_t)a * nb + b] =
-              mkc(aj[r][c][0] - ay[r][c][1], aj[r][c][1] + ay[r][c][0]);
-          Rs[(int64_t)a * nb + b] = mkc(aj[r][c][0], aj[r][c][1]);
-        }
-      }
-    }
-  }
-  __syncthreads();
-
-  // ------------------------------------------------------------------ LU
-  // The factors live in shared memory (odd stride: conflict-free column
-  // access) when they fit beside a chunk of at least 8 right-hand-side rows;
-  // larger classes factor Q_c in place in its global scratch and solve on
-  // -RgQ_c in place (L2-resident), with only the pivots in shared memory.
-  const int lda_s = nb | 1;
-  size_t lu_need = ((size_t)nb * lda_s + nb) * sizeof(cplx) + (3 * nb + 1) * sizeof(int);
-  lu_need = (lu_need + 15) & ~(size_t)15;
-  const bool lu_global =
-      lu_need + (size_t)(nb < 8 ? nb : 8) * lda_s * sizeof(cplx) > smem_bytes;
-  const int lda = lu_global ? nb : lda_s;
-  cplx *Am = lu_global ? Qs : reinterpret_cast<cplx *>(tmx_smem);
-  cplx *uinv = lu_global ? reinterpret_cast<cplx *>(tmx_smem) : Am + (int64_t)nb * lda;
-  int *piv = reinterpret_cast<int *>(uinv + nb);
-  int *perm = piv + nb;
-  int *flag = perm + nb;
-  cplx *X = lu_global ? Rs : reinterpret_cast<cplx *>(tmx_smem + lu_need);
-  int Rchunk = lu_global ? nb : (int)((smem_bytes - lu_need) / (sizeof(cplx) * lda));
-  if (Rchunk > nb) {
-    Rchunk = nb;
-  }
-  if (!lu_global) {
-    for (int u = threadIdx.x; u < nb * nb; u += blockDim.x) {
-      Am[(u / nb) * lda + (u % nb)] = Qs[u];
-    }
-  }
-  if (threadIdx.x == 0) {
-    *flag = 0;
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  for (int i = 0; i < nb; ++i) {
-    if (warp == 0) {
-      double best = -1.;
-      int bi = i;
-      for (int j = i + lane; j < nb; j += 32) {
-        const double v = cabs_dev(Am[j * lda + i]);
-        if (v > best) {
-          best = v;
-          bi = j;
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_down_sync(0xffffffffu, best, o);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) {
-          best = ov;
-          bi = oi;
-        }
-      }
-      if (lane == 0) {
-        piv[i] = bi;
-        if (!(best > 0.)) {
-          *flag = 1;
-        }
-      }
-    }
-    __syncthreads();
-    const int ip = piv[i];
-    if (ip != i) {
-      for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-        const cplx t = Am[i * lda + j];
-        Am[i * lda + j] = Am[ip * lda + j];
-        Am[ip * lda + j] = t;
-      }
-      __syncthreads();
-    }
-    const cplx pinv = cinv_lu(Am[i * lda + i]);
-    for (int j = i + 1 + threadIdx.x; j < nb; j += blockDim.x) {
-      Am[j * lda + i] = cmul(Am[j * lda + i], pinv);
-    }
-    __syncthreads();
-    const int rem = nb - i - 1;
-    for (int u = threadIdx.x; u < rem * rem; u += blockDim.x) {
-      const int j = i + 1 + u / rem;
-      const int k = i + 1 + u % rem;
-      Am[j * lda + k] = csub(Am[j * lda + k], cmul(Am[j * lda + i], Am[i * lda + k]));
-    }
-    __syncthreads();
-  }
-  for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-    uinv[j] = cinv_lu(Am[j * lda + j]);
-  }
-  if (threadIdx.x == 0) {
-    // column exchanges of Matrix::plu_inverse step 4, as a gather index
-    for (int j = 0; j < nb; ++j) {
-      perm[j] = j;
-    }
-    for (int j = nb - 1; j >= 0; --j) {
-      const int p = piv[j];
-      const int t = perm[j];
-      perm[j] = perm[p];
-      perm[p] = t;
-    }
-    if (*flag) {
-      atomicOr(&A.status[sl.grain], TMX_ST_SINGULAR);
-    }
-  }
-  __syncthreads();
-  if (A.lu) {
-    // factors (unit-lower L below, U on and above the diagonal) and the
-    // column gather index, for the tangent solves
-    cplx *Ls = A.lu + item.scratch;
-    for (int u = threadIdx.x; u < nb * nb; u += blockDim.x) {
-      Ls[u] = Am[(u / nb) * lda + (u % nb)];
-    }
-    int *ps = reinterpret_cast<int *>(Ls + (int64_t)nb * nb);
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-      ps[j] = perm[j];
-    }
-  }
-
-  // --------------------------------------------- solve T_c Q_c = -RgQ_c
-  const bool chain = sl.tout < 0;
-  for (int r0 = 0; r0 < nb; r0 += Rchunk) {
-    const int R = min(Rchunk, nb - r0);
-    // (in place when X is Rs itself: each element is read and written by
-    // the same thread)
-    for (int u = threadIdx.x; u < R * nb; u += blockDim.x) {
-      const cplx v = Rs[(int64_t)(r0 + u / nb) * nb + (u % nb)];
-      X[(u / nb) * lda + (u % nb)] = mkc(-v.x, -v.y);
-    }
-    __syncthreads();
-    // Z U = X (forward over columns)
-    for (int j = 0; j < nb; ++j) {
-      for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        X[r * lda + j] = cmul(X[r * lda + j], uinv[j]);
-      }
-      __syncthreads();
-      const int rem = nb - j - 1;
-      for (int u = threadIdx.x; u < R * rem; u += blockDim.x) {
-        const int r = u / rem;
-        const int k = j + 1 + u % rem;
-        X[r * lda + k] = csub(X[r * lda + k], cmul(X[r * lda + j], Am[j * lda + k]));
-      }
-      __syncthreads();
-    }
-    // Y L = Z (backward over columns, L unit lower)
-    for (int j = nb - 1; j >= 1; --j) {
-      for (int u = threadIdx.x; u < R * j; u += blockDim.x) {
-        const int r = u / j;
-        const int k = u % j;
-        X[r * lda + k] = csub(X[r * lda + k], cmul(X[r * lda + j], Am[j * lda + k]));
-      }
-      __syncthreads();
-    }
-    // write out: T_c[a][b] = Y[a][perm[b]]
-    if (chain) {
-      for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        const int a = r0 + r;
-        int ia, na;
-        member(D, a, ia, na);
-        A.diag[sl.diag + ia * N + (na - 1)] = X[r * lda + perm[a]];
-      }
-    } else {
-      cplx *Tb = A.tout + sl.tout + block_offset(N, m);
-      const int w2 = 2 * D.nbb;
-      for (int u = threadIdx.x; u < R * nb; u += blockDim.x) {
-        const int r = u / nb;
-        const int b = u % nb;
-        const int a = r0 + r;
-        int ia, na, ib, nbn;
-        member(D, a, ia, na);
-        member(D, b, ib, nbn);
-        const int row = ia * D.nbb + (na - D.nmin);
-        const int col = ib * D.nbb + (nbn - D.nmin);
-        Tb[(int64_t)row * w2 + col] = X[r * lda + perm[b]];
-      }
-    }
-    __syncthreads();
-  }
-}
-
-template <int TR, int TC, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB)
-    k_blocks(TmxBlockArgs A, size_t smem_bytes) {
-  const int ilo = A.range ? A.range[0] : 0;
-  const int ihi = A.range ? min(A.range[1], A.nitems) : A.nitems;
-  for (int it = ilo + blockIdx.x; it < ihi; it += gridDim.x) {
-    block_item<TR, TC, NT>(A, it, smem_bytes);
-    // shared memory is reused by the next item
-    __syncthreads();
   }
 }
 
@@ -1343,280 +1020,6 @@ __global__ void __launch_bounds__(128, 4) k_blocks_cta32(TmxBlockArgs A) {
   }
 }
 
-// ------------------------------------------ eight warps per item (<= 64) --
-//
-// Classes of 33..64 members: one CTA of eight warps per item. As in
-// k_blocks_cta32 the warps build each chunk of TMX_WG32 nodes together and
-// warp w accumulates column tile w over all eight row tiles with DMMA, so
-// the node factors are built once per item; the LU pivots with warp 0 and
-// updates with all threads (four barriers per step), and the solves keep
-// each row in the registers of four lanes (row tid / 4).
-
-__host__ __device__ constexpr int cta64_elems() {
-  // F[WG][4][64] + W[2][WG][4][64], or Q, RgQ [64][65], 1/U_jj, pivot and
-  // gather indices and a flag
-  return (12 * TMX_WG32 * 64 > 2 * 64 * 65 + 64 + 66) ? 12 * TMX_WG32 * 64
-                                                        : 2 * 64 * 65 + 64 + 66;
-}
-
-__global__ void __launch_bounds__(256, 1) k_blocks_cta64(TmxBlockArgs A) {
-  constexpr int NBM = 64;
-  constexpr int LD = NBM + 1;
-  constexpr int NTH = 256;
-  extern __shared__ __align__(16) unsigned char tmx_c64smem[];
-  cplx *base = reinterpret_cast<cplx *>(tmx_c64smem);
-  cplx *Fs = base;                    // [WG][4][NBM]
-  cplx *Ws = Fs + TMX_WG32 * 4 * NBM; // [2][WG][4][NBM]
-  cplx *Qm = base;                    // [NBM][LD]  (after the assembly)
-  cplx *Rm = Qm + NBM * LD;           // [NBM][LD]
-  cplx *uinv = Rm + NBM * LD;         // [NBM]
-  int *perm = reinterpret_cast<int *>(uinv + NBM); // [NBM]
-  int *piv = perm + NBM;                           // [NBM]
-  int *flag = piv + NBM;
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int wib = tid >> 5;
-  const int q = lane & 3;
-  const int rr = lane >> 2;
-  const int ilo = A.range ? A.range[0] : 0;
-  const int ihi = A.range ? min(A.range[1], A.nitems) : A.nitems;
-  for (int it = ilo + blockIdx.x; it < ihi; it += gridDim.x) {
-    const TmxItem item = A.items[it];
-    const TmxSlot sl = A.slots[item.slot];
-    const TmxGrain Gr = A.grains[sl.grain];
-    const int N = sl.nmax;
-    const int ng = sl.ngauss;
-    const int m = item.m;
-    const ClassDesc D = describe<1>(N, m, item.cls);
-    const int nb = D.nb;
-    if (nb <= 0) {
-      continue;
-    }
-    if (nb > NBM) {
-      if (tid == 0) {
-        atomicOr(&A.status[sl.grain], TMX_ST_TOO_LARGE);
-      }
-      continue;
-    }
-    const double *T = A.tab + sl.tab;
-    const double *S = A.nsc + sl.nsc;
-    const double *Wg = A.wig + A.wig_off[sl.wig_n] + (int64_t)m * ng * N * 2;
-    const double k2 = Gr.k * Gr.k;
-    const cplx k2mr = mkc(Gr.mr * k2, Gr.mi * k2);
-    const int ngroups = (D.R1 > 0 && m > 0) ? 2 : 1;
-    const int nrt = (nb + 7) >> 3;
-    const int col = wib * 8 + rr; // B-fragment column of this lane
-    double acc[8][4][2];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        acc[r][p][0] = acc[r][p][1] = 0.;
-      }
-    }
-    for (int g0 = 0; g0 < ng; g0 += TMX_WG32) {
-      __syncthreads();
-      for (int u = tid; u < TMX_WG32 * nb; u += NTH) {
-        const int gl = u / nb;
-        const int a = u - gl * nb;
-        cplx *fp = Fs + gl * 4 * NBM + a;
-        cplx *wp = Ws + gl * 4 * NBM + a;
-        if (g0 + gl < ng) {
-          a_side<true>(D, a, N, g0 + gl, T, S, Wg, fp, NBM, m);
-          b_side<true>(D, a, N, m, g0 + gl, ngroups, T, S, Wg, k2, k2mr, wp, NBM,
-                       TMX_WG32 * 4 * NBM);
-        } else {
-          zero_side(fp, NBM, 4);
-          for (int g = 0; g < ngroups; ++g) {
-            zero_side(wp + g * TMX_WG32 * 4 * NBM, NBM, 4);
-          }
-        }
-      }
-      __syncthreads();
-      if (wib * 8 < nb) {
-        const int gmax = min(TMX_WG32, ng - g0);
-        const int nsl = (m == 0) ? (gmax + 1) >> 1 : gmax;
-        for (int sx = 0; sx < nsl; ++sx) {
-          const int gl = (m == 0) ? 2 * sx + (q >> 1) : sx;
-          const int t = (m == 0) ? 1 + 2 * (q & 1) : q;
-          cplx w[2];
-#pragma unroll
-          for (int g = 0; g < 2; ++g) {
-            w[g] = (col < nb && g < ngroups)
-                       ? Ws[((g * TMX_WG32 + gl) * 4 + t) * NBM + col]
-                       : mkc(0., 0.);
-          }
-#pragma unroll
-          for (int rti = 0; rti < 8; ++rti) {
-            if (rti < nrt) {
-              const int row = rti * 8 + rr;
-              const cplx f = (row < nb) ? Fs[(gl * 4 + t) * NBM + row] : mkc(0., 0.);
-              const int grp = (row < D.R0) ? 0 : 1;
-              const int lo = rti * 8, hi = min(rti * 8 + 8, nb);
-#pragma unroll
-              for (int g = 0; g < 2; ++g) {
-                const bool present = (g == 0) ? (lo < D.R0) : (ngroups == 2 && hi > D.R0);
-                if (present) {
-                  const double fj = (grp == g) ? f.x : 0.;
-                  const double fy = (grp == g) ? f.y : 0.;
-                  double *a4 = &acc[rti][0][0];
-                  dmma(a4[0], a4[1], fj, w[g].x);
-                  dmma(a4[2], a4[3], fj, w[g].y);
-                  dmma(a4[4], a4[5], fy, w[g].x);
-                  dmma(a4[6], a4[7], fy, w[g].y);
-                }
-              }
-            }
-          }
-        }
-      }
-    }
-    // a_n of each member once per item (in the 1/U_jj slots)
-    double *an_s = reinterpret_cast<double *>(uinv);
-    if (tid < nb) {
-      int ia, na;
-      member(D, tid, ia, na);
-      an_s[tid] = a_n(na);
-    }
-    if (tid == 0) {
-      *flag = 0;
-    }
-    __syncthreads();
-    // Q = G^j + i G^y, RgQ = G^j (times a_n1 a_n2), into the chunk buffers
-#pragma unroll
-    for (int rti = 0; rti < 8; ++rti) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int a = rti * 8 + rr;
-        const int b = wib * 8 + 2 * q + i;
-        if (a < nb && b < nb) {
-          const double sc = an_s[a] * an_s[b];
-          const double jr = acc[rti][0][i], ji = acc[rti][1][i];
-          const double yr = acc[rti][2][i], yi = acc[rti][3][i];
-          Qm[a * LD + b] = mkc((jr - yi) * sc, (ji + yr) * sc);
-          Rm[a * LD + b] = mkc(jr * sc, ji * sc);
-        }
-      }
-    }
-    __syncthreads();
-    // LU in place in Qm: pivot of column i by warp 0 (first row with the
-    // largest |Q_ri|), row exchange, column scaling, rank-1 update
-    for (int i = 0; i < nb; ++i) {
-      if (wib == 0) {
-        double best = -1.;
-        int bi = i;
-        for (int j = i + lane; j < nb; j += 32) {
-          const double v = cabs_dev(Qm[j * LD + i]);
-          if (v > best) {
-            best = v;
-            bi = j;
-          }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const double ov = __shfl_down_sync(0xffffffffu, best, o);
-          const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-          if (ov > best || (ov == best && oi < bi)) {
-            best = ov;
-            bi = oi;
-          }
-        }
-        if (lane == 0) {
-          piv[i] = bi;
-          if (!(best > 0.)) {
-            *flag = 1;
-          }
-        }
-      }
-      __syncthreads();
-      const int ip = piv[i];
-      if (ip != i) {
-        for (int j = tid; j < nb; j += NTH) {
-          const cplx t = Qm[i * LD + j];
-          Qm[i * LD + j] = Qm[ip * LD + j];
-          Qm[ip * LD + j] = t;
-        }
-        __syncthreads();
-      }
-      const cplx pinv = cinv_lu(Qm[i * LD + i]);
-      for (int j = i + 1 + tid; j < nb; j += NTH) {
-        Qm[j * LD + i] = cmul(Qm[j * LD + i], pinv);
-      }
-      __syncthreads();
-      const int rem = nb - i - 1;
-      for (int u = tid; u < rem * rem; u += NTH) {
-        const int j = i + 1 + u / rem;
-        const int k = i + 1 + u % rem;
-        Qm[j * LD + k] = csub(Qm[j * LD + k], cmul(Qm[j * LD + i], Qm[i * LD + k]));
-      }
-      __syncthreads();
-    }
-    for (int j = tid; j < nb; j += NTH) {
-      uinv[j] = cinv_lu(Qm[j * LD + j]);
-    }
-    if (tid == 0) {
-      // column exchanges of Matrix::plu_inverse step 4, as a gather index
-      for (int j = 0; j < nb; ++j) {
-        perm[j] = j;
-      }
-      for (int j = nb - 1; j >= 0; --j) {
-        const int p = piv[j];
-        const int t = perm[j];
-        perm[j] = perm[p];
-        perm[p] = t;
-      }
-      if (*flag) {
-        atomicOr(&A.status[sl.grain], TMX_ST_SINGULAR);
-      }
-    }
-    __syncthreads();
-    if (A.lu) {
-      cplx *Ls = A.lu + item.scratch;
-      for (int u = tid; u < nb * nb; u += NTH) {
-        Ls[u] = Qm[(u / nb) * LD + (u % nb)];
-      }
-      int *ps = reinterpret_cast<int *>(Ls + (int64_t)nb * nb);
-      for (int j = tid; j < nb; j += NTH) {
-        ps[j] = perm[j];
-      }
-    }
-    // solve T_c Q_c = -RgQ_c: four lanes per row
-    solve_rows<NBM, 4>(Rm, Qm, LD, uinv, nb, tid >> 2, tid & 3);
-    __syncthreads();
-    // write out: T_c[a][b] = Y[a][perm[b]]
-    if (sl.tout < 0) {
-      for (int a = tid; a < nb; a += NTH) {
-        int ia, na;
-        member(D, a, ia, na);
-        A.diag[sl.diag + ia * N + (na - 1)] = Rm[a * LD + perm[a]];
-      }
-    } else {
-      cplx *Tb = A.tout + sl.tout + block_offset(N, m);
-      const int w2 = 2 * D.nbb;
-      for (int u = tid; u < nb * nb; u += NTH) {
-        const int a = u / nb;
-        const int b = u - a * nb;
-        int ia, na, ib, nbn;
-        member(D, a, ia, na);
-        member(D, b, ib, nbn);
-        Tb[(int64_t)(ia * D.nbb + (na - D.nmin)) * w2 + ib * D.nbb + (nbn - D.nmin)] =
-            Rm[a * LD + perm[b]];
-      }
-    }
-    __syncthreads();
-  }
-}
-
-static void launch_cta64(const TmxBlockArgs &a, cudaStream_t stream) {
-  const size_t smem = (size_t)cta64_elems() * sizeof(cplx);
-  cudaFuncSetAttribute(k_blocks_cta64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
-  // one item per CTA (see launch_warp_variant)
-  const int blocks = (a.max_ctas > 0) ? std::min(std::max(1, a.nitems), a.max_ctas)
-                                       : std::max(1, a.nitems);
-  k_blocks_cta64<<<blocks, 256, smem, stream>>>(a);
-}
-
 static void launch_cta32(const TmxBlockArgs &a, cudaStream_t stream) {
   const size_t smem = (size_t)cta32_elems() * sizeof(cplx);
   cudaFuncSetAttribute(k_blocks_cta32, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1627,54 +1030,607 @@ static void launch_cta32(const TmxBlockArgs &a, cudaStream_t stream) {
   k_blocks_cta32<<<blocks, 128, smem, stream>>>(a);
 }
 
-// dynamic shared memory the CTA kernel may use (of the 227 KB per block)
-#define TMX_BLOCK_SMEM_MAX (227u * 1024u)
+// -------------------------------------- assembly, factors and solves apart --
+//
+// Classes of more than 32 members: one item is too much for a CTA's registers
+// and too little, in its factorisation, for a whole SM's FP64 pipe, and the
+// large orders come a few grains at a time. So the assembly of an item is
+// split over CTAs of 32 rows x 32 columns (k_assemble, Q and RgQ to the item's
+// scratch), one CTA per item factors Q (k_factor), and the solves are split by
+// rows again (k_solve).
+// Measured (B200), one CTA per item for everything -> the three kernels: 1154
+// items of 33..50 members, 66..100 nodes: 1.41 -> 0.50 + 0.23 + 0.16 ms; 1960
+// items of 65..99 members, 198 nodes: 15.4 -> 5.96 + 1.99 + 1.79 ms; the m = 0
+// classes of nine grains at orders 129..199: 1.42 -> 0.39 ms per order.
+// k_assemble is bound by the issue of its build phase (32 x 64 tiles with two
+// CTAs per SM took 0.53 and 6.9 ms; three chunks of table rows in flight
+// instead of one 0.56 and 7.1), k_factor by its shared-memory traffic, k_solve
+// by the FP64 pipe and the chain of its columns.
 
-// shared memory of one block: the larger of the assembly chunk buffers and
-// the LU phase (factors, pivots and a right-hand-side chunk, or the pivot
-// data alone for classes whose factors do not fit)
-size_t tmx_block_smem_bytes(int max_nb, int chunk_nodes) {
-  const int nrp = (max_nb + 3) / 4 * 4 + 4;
-  const int ncol = (max_nb + 3) / 4 * 4;
-  const size_t asm_bytes =
-      ((size_t)4 * chunk_nodes * nrp + (size_t)2 * 4 * chunk_nodes * ncol) *
-      sizeof(cplx);
-  const int lda = max_nb | 1;
-  size_t lu = ((size_t)max_nb * lda + max_nb) * sizeof(cplx) +
-              (3 * max_nb + 1) * sizeof(int);
-  lu = (lu + 15) & ~(size_t)15;
-  // at least 8 rows of the right-hand side per solve chunk
-  const int rows = max_nb < 8 ? max_nb : 8;
-  size_t lu_total = lu + (size_t)rows * lda * sizeof(cplx);
-  // prefer the whole right-hand side when it fits in 200 KB
-  const size_t full = lu + (size_t)max_nb * lda * sizeof(cplx);
-  if (full <= 200 * 1024) {
-    lu_total = full;
-  }
-  if (lu_total > TMX_BLOCK_SMEM_MAX) {
-    // the kernel factors such classes in global memory: shared memory holds
-    // the pivot data only
-    lu_total = ((size_t)max_nb * sizeof(cplx) + (3 * max_nb + 1) * sizeof(int) + 15) &
-               ~(size_t)15;
-  }
-  return asm_bytes > lu_total ? asm_bytes : lu_total;
+#define TMX_ASM_ROWS 32
+#define TMX_ASM_COLS 32
+#define TMX_ASM_WG 8 // quadrature nodes per chunk
+
+// row tiles of an item of at most max_nb members: each holds rows of one
+// group only (classes of m >= 1 have groups of at most (nb + 1) / 2 rows)
+__host__ __device__ constexpr int asm_row_tiles(int max_nb) {
+  return 2 * (((max_nb + 1) / 2 + TMX_ASM_ROWS - 1) / TMX_ASM_ROWS);
+}
+__host__ __device__ constexpr int asm_col_tiles(int max_nb) {
+  return (max_nb + TMX_ASM_COLS - 1) / TMX_ASM_COLS;
 }
 
-template <int TR, int TC, int NT, int MINB>
-static void launch_variant(const TmxBlockArgs &a, size_t smem,
-                           cudaStream_t stream) {
-  static int attr_dev = -1;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (attr_dev != dev) {
-    cudaFuncSetAttribute(k_blocks<TR, TC, NT, MINB>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         227 * 1024);
-    attr_dev = dev;
+// LEAN as for a_side_row: the factors a_n applied to the finished entries.
+//
+// Eight warps share the 8 x 8 tiles of the CTA's 32 x 32 entries (whatever is
+// left of them at the edges) evenly, each tile four DMMA accumulators: (j, y) x
+// (re, im). The K dimension is (node, term): four terms of a node for m >= 1,
+// two for m = 0 (mu = 0 removes terms 0 and 2), in ascending order; a DMMA
+// rounds as the four fused multiply-adds in that order. Thread t builds row
+// and column t % 32 of node t / 32 of a chunk;
+// the table rows of the next chunk are copied (cp.async) meanwhile. F and W
+// rows are padded by two entries, so that the four terms and two members that
+// eight lanes read fall into distinct banks.
+template <bool LEAN>
+__global__ void __launch_bounds__(256, 3) k_assemble(TmxBlockArgs A, int rtiles, int ctiles) {
+  constexpr int NR = TMX_ASM_ROWS, NC = TMX_ASM_COLS, WG = TMX_ASM_WG;
+  constexpr int LDF = NR + 2, LDW = NC + 2;
+  constexpr int NP = (NR + NC) * 3; // 16-byte pieces of a node: 3 per member
+  constexpr int NTILE = NR * NC / 64 / 8; // tiles per warp
+  static_assert(WG * NC == 256 && WG * NR <= 256 && NP <= 256, "thread layout");
+  extern __shared__ __align__(16) unsigned char asm_sm[];
+  cplx *Fs = reinterpret_cast<cplx *>(asm_sm);                 // [4 WG][LDF]
+  cplx *Ws = Fs + 4 * WG * LDF;                                // [4 WG][LDW]
+  double *stg = reinterpret_cast<double *>(Ws + 4 * WG * LDW); // [WG][NP] pieces
+  double *stgS = stg + WG * NP * 2;                            // [WG] node scalars
+  __shared__ double an_s[NR + NC]; // a_n of the row and column members
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const int q = lane & 3;
+  const int rr = lane >> 2;
+  const int tiles = rtiles * ctiles;
+  const int ilo = A.range ? A.range[0] : 0;
+  const int ihi = A.range ? min(A.range[1], A.nitems) : A.nitems;
+  for (int64_t u0 = (int64_t)ilo * tiles + blockIdx.x; u0 < (int64_t)ihi * tiles;
+       u0 += gridDim.x) {
+    const TmxItem item = A.items[u0 / tiles];
+    const int tile = (int)(u0 % tiles);
+    const TmxSlot sl = A.slots[item.slot];
+    const int N = sl.nmax;
+    const int ng = sl.ngauss;
+    const int m = item.m;
+    const ClassDesc D = describe<1>(N, m, item.cls);
+    const int nb = D.nb;
+    // rows [r0, r0 + nr) of group rg, columns [c0, c0 + nc)
+    const int n0 = (D.R0 + NR - 1) / NR;
+    const int rt = tile / ctiles;
+    const int rg = (rt < n0) ? 0 : 1;
+    const int r0 = (rg == 0) ? rt * NR : D.R0 + (rt - n0) * NR;
+    const int nr = min(NR, ((rg == 0) ? D.R0 : nb) - r0);
+    const int c0 = (tile % ctiles) * NC;
+    const int nc = min(NC, nb - c0);
+    if (nb > A.max_nb || nr <= 0 || nc <= 0) {
+      continue; // (k_factor flags classes above the launch's size)
+    }
+    const TmxGrain Gr = A.grains[sl.grain];
+    const double *T = A.tab + sl.tab;
+    const double *S = A.nsc + sl.nsc;
+    const double *Wg = A.wig + A.wig_off[sl.wig_n] + (int64_t)m * ng * N * 2;
+    const double k2 = Gr.k * Gr.k;
+    const cplx k2mr = mkc(Gr.mr * k2, Gr.mi * k2);
+    const int nt = (m == 0) ? 2 : 4; // terms per node
+    // this thread's piece: of row member r0 + tid / 3 (tid < 3 NR) or column
+    // member c0 + tid / 3 - NR, a half of its Bessel row or its Wigner pair
+    const int pm = tid / 3, piece = tid - 3 * pm;
+    const bool prow = pm < NR;
+    const bool have = tid < NP && (prow ? pm < nr : pm - NR < nc);
+    int pi, pn;
+    member(D, prow ? r0 + pm : c0 + pm - NR, pi, pn);
+    pn = have ? pn : 1;
+    const double *src = (piece < 2)
+                            ? T + (int64_t)(pn - 1) * TMX_NQ + (prow ? 0 : 4) + 2 * piece
+                            : Wg + (int64_t)(pn - 1) * 2;
+    const int stride = (piece < 2) ? N * TMX_NQ : 2 * N;
+    const auto issue = [&](int g0) {
+      if (have) {
+        const double *sp = src + (int64_t)g0 * stride;
+#pragma unroll
+        for (int gl = 0; gl < WG; ++gl) {
+          if (g0 + gl < ng) {
+            cp16(stg + (gl * NP + tid) * 2, sp);
+          }
+          sp += stride;
+        }
+      }
+      if (tid < WG * (TMX_NS / 2) && g0 + tid / (TMX_NS / 2) < ng) {
+        cp16(stgS + 2 * tid, S + (int64_t)g0 * TMX_NS + 2 * tid);
+      }
+      cp_commit();
+    };
+    issue(0);
+    // this thread's row and column of a chunk (padding up to whole 8 x 8 tiles
+    // is built as zeros; it is contracted but not written out)
+    const int fg = tid / NR, fm = tid % NR;
+    const int wg = tid / NC, wm = tid % NC;
+    const bool frow = tid < WG * NR && (fm & ~7) < nr;
+    const bool wcol = (wm & ~7) < nc;
+    int fi, fn, wi, wn;
+    member(D, r0 + fm, fi, fn);
+    member(D, c0 + wm, wi, wn);
+    if (tid < NR + NC && (tid < NR ? tid < nr : tid - NR < nc)) {
+      int ia, n;
+      member(D, tid < NR ? r0 + tid : c0 + tid - NR, ia, n);
+      an_s[tid] = a_n(n);
+    }
+    // this warp's tiles: fo, wo their first entries in F and W
+    const int nct = (nc + 7) >> 3;
+    const int ntl = ((nr + 7) >> 3) * nct;
+    int fo[NTILE], wo[NTILE];
+    double acc[NTILE][4][2];
+#pragma unroll
+    for (int i = 0; i < NTILE; ++i) {
+      const int t = warp + 8 * i;
+      fo[i] = q * LDF + (t / nct) * 8 + rr;
+      wo[i] = q * LDW + (t % nct) * 8 + rr;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        acc[i][p][0] = acc[i][p][1] = 0.;
+      }
+    }
+    for (int g0 = 0; g0 < ng; g0 += WG) {
+      cp_wait_all();
+      __syncthreads(); // the chunk's rows are there; F and W are free
+      if (frow) {
+        cplx v[4] = {mkc(0., 0.), mkc(0., 0.), mkc(0., 0.), mkc(0., 0.)};
+        if (fm < nr && g0 + fg < ng) {
+          const double *r = stg + (fg * NP + 3 * fm) * 2;
+          const double2 x = *reinterpret_cast<const double2 *>(r);
+          const double2 y = *reinterpret_cast<const double2 *>(r + 2);
+          const double2 w = *reinterpret_cast<const double2 *>(r + 4);
+          a_side_row<LEAN>(x.x, x.y, y.x, y.y, w.x, w.y, stgS + fg * TMX_NS, fn, v, 1, m,
+                           LEAN ? 1. : an_s[fm]);
+        }
+        cplx *o = Fs + fg * nt * LDF + fm;
+        if (m == 0) {
+          o[0] = v[1];
+          o[LDF] = v[3];
+        } else {
+          o[0] = v[0];
+          o[LDF] = v[1];
+          o[2 * LDF] = v[2];
+          o[3 * LDF] = v[3];
+        }
+      }
+      if (wcol) {
+        cplx v[4] = {mkc(0., 0.), mkc(0., 0.), mkc(0., 0.), mkc(0., 0.)};
+        if (wm < nc && g0 + wg < ng) {
+          const double *r = stg + (wg * NP + 3 * (NR + wm)) * 2;
+          const double2 x = *reinterpret_cast<const double2 *>(r);
+          const double2 y = *reinterpret_cast<const double2 *>(r + 2);
+          const double2 w = *reinterpret_cast<const double2 *>(r + 4);
+          const BSide B = b_side_node<LEAN>(wn, m, x, y, w.x, w.y, stgS + wg * TMX_NS,
+                                            LEAN ? 1. : an_s[NR + wm]);
+          b_side_terms<LEAN>(B, (rg == 0) ? D.iA : D.iB, wi, m, k2, k2mr, v, 1);
+        }
+        cplx *o = Ws + wg * nt * LDW + wm;
+        if (m == 0) {
+          o[0] = v[1];
+          o[LDW] = v[3];
+        } else {
+          o[0] = v[0];
+          o[LDW] = v[1];
+          o[2 * LDW] = v[2];
+          o[3 * LDW] = v[3];
+        }
+      }
+      __syncthreads();
+      if (g0 + WG < ng) {
+        issue(g0 + WG);
+      }
+      const int kmax = min(WG, ng - g0) * nt;
+      for (int k0 = 0; k0 < kmax; k0 += 4) {
+#pragma unroll
+        for (int i = 0; i < NTILE; ++i) {
+          if (warp + 8 * i < ntl) {
+            const cplx f = Fs[fo[i] + k0 * LDF];
+            const cplx w = Ws[wo[i] + k0 * LDW];
+            dmma(acc[i][0][0], acc[i][0][1], f.x, w.x); // jr
+            dmma(acc[i][1][0], acc[i][1][1], f.x, w.y); // ji
+            dmma(acc[i][2][0], acc[i][2][1], f.y, w.x); // yr
+            dmma(acc[i][3][0], acc[i][3][1], f.y, w.y); // yi
+          }
+        }
+      }
+    }
+    // Q = G^j + i G^y, RgQ = G^j
+    cplx *Qs = A.scratch + item.scratch;
+    cplx *Rs = Qs + (int64_t)nb * nb;
+#pragma unroll
+    for (int i = 0; i < NTILE; ++i) {
+      const int t = warp + 8 * i;
+      const int row = (t / nct) * 8 + rr;
+      if (t < ntl && row < nr) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int cl = (t % nct) * 8 + 2 * q + e;
+          if (cl < nc) {
+            const double jr = acc[i][0][e], ji = acc[i][1][e];
+            const double yr = acc[i][2][e], yi = acc[i][3][e];
+            const double sc = LEAN ? an_s[row] * an_s[NR + cl] : 1.;
+            const int64_t o = (int64_t)(r0 + row) * nb + c0 + cl;
+            Qs[o] = mkc((jr - yi) * sc, (ji + yr) * sc);
+            Rs[o] = mkc(jr * sc, ji * sc);
+          }
+        }
+      }
+    }
+    __syncthreads(); // stage and chunk buffers are reused by the next tile
   }
-  const int blocks = (a.max_ctas > 0) ? std::min(std::max(1, a.nitems), a.max_ctas)
-                                       : std::max(1, a.nitems);
-  k_blocks<TR, TC, NT, MINB><<<blocks, NT, smem, stream>>>(a, smem);
+}
+
+// Complex products with their roundings spelled out (the compiler may contract
+// either product of a sum, and large elongated grains amplify the last bit of
+// a factor by many orders of magnitude): mul_xy fuses the x x and y x products,
+// mul_xx the x x and x y ones, mul_yx the y y and x y ones. They are the forms
+// that keep T-matrices the same, bit for bit, as those of one-CTA-per-item
+// kernels with compiler-chosen contractions.
+__device__ __forceinline__ cplx mul_xy(cplx a, cplx b) {
+  return mkc(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
+             __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
+}
+__device__ __forceinline__ cplx mul_xx(cplx a, cplx b) {
+  return mkc(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
+             __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ cplx mul_yx(cplx a, cplx b) {
+  return mkc(__fma_rn(-a.y, b.y, __dmul_rn(a.x, b.x)),
+             __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
+
+// LU of Q_c, one item per CTA, in shared memory (in the scratch itself for
+// classes whose factors exceed it).
+//
+// Thread (tr, tc) of a (NTH / 16) x 16 grid owns rows tr, tr + NTH / 16, ..
+// and columns tc, tc + 16, ..; rows stay in place and carry a position (the
+// pivot of step i is the first position with the largest |Q_ri|, as in
+// Matrix::plu_inverse). A step has one barrier: the threads of column i + 1
+// post their largest candidate of the next step right after updating it,
+// behind the barrier every warp reduces the candidates itself, and the l of a
+// row are formed by the 16 threads that share it. The factors go back to the
+// scratch with their rows in place, and the row at each position beside them.
+template <int NBM, int NTH>
+__global__ void __launch_bounds__(NTH, (NBM > 64) ? 1 : 2)
+    k_factor(TmxBlockArgs A, size_t smem_bytes) {
+  constexpr int RT = NTH / 16; // row groups
+  constexpr int NA = NBM / RT; // rows per thread
+  static_assert(RT <= 32 && NBM % RT == 0, "thread layout");
+  extern __shared__ __align__(16) unsigned char fsm[];
+  __shared__ unsigned long long ckey[2][32];
+  __shared__ int cpos[2][32], crow[2][32];
+  __shared__ int at[NBM]; // row at a position
+  __shared__ int flag;
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int tc = tid & 15;
+  const int tr = tid >> 4;
+  const int ilo = A.range ? A.range[0] : 0;
+  const int ihi = A.range ? min(A.range[1], A.nitems) : A.nitems;
+  for (int it = ilo + blockIdx.x; it < ihi; it += gridDim.x) {
+    const TmxItem item = A.items[it];
+    const TmxSlot sl = A.slots[item.slot];
+    const ClassDesc D = describe<1>(sl.nmax, item.m, item.cls);
+    const int nb = D.nb;
+    if (nb <= 0) {
+      continue;
+    }
+    if (nb > NBM || nb > A.max_nb) {
+      if (tid == 0) {
+        atomicOr(&A.status[sl.grain], TMX_ST_TOO_LARGE);
+      }
+      continue;
+    }
+    cplx *Qs = A.scratch + item.scratch;
+    const int lds = nb | 1;
+    const bool inplace = (size_t)nb * lds * sizeof(cplx) > smem_bytes;
+    const int lda = inplace ? nb : lds;
+    cplx *Am = inplace ? Qs : reinterpret_cast<cplx *>(fsm);
+    if (!inplace) {
+      for (int r = tr; r < nb; r += RT) {
+        for (int k = tc; k < nb; k += 16) {
+          Am[r * lda + k] = Qs[(int64_t)r * nb + k];
+        }
+      }
+    }
+    if (tid == 0) {
+      flag = 0;
+    }
+    int pos[NA];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+      pos[a] = tr + RT * a;
+    }
+    __syncthreads();
+    // candidate of column i among this thread's rows (threads of the column)
+    const auto post = [&](int i, int buf) {
+      double best = 0.;
+      unsigned long long key = 0ull;
+      int bp = 0x7fffffff, br = 0;
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        const int r = tr + RT * a;
+        if (r < nb && pos[a] >= i) {
+          double v = cabs_dev(Am[r * lda + i]);
+          v = (v >= 0.) ? v : 0.; // (NaN is no candidate)
+          if (key == 0ull || v > best || (v == best && pos[a] < bp)) {
+            best = v;
+            bp = pos[a];
+            br = r;
+            key = (unsigned long long)__double_as_longlong(v) | (1ull << 63);
+          }
+        }
+      }
+      ckey[buf][tr] = key;
+      cpos[buf][tr] = bp;
+      crow[buf][tr] = br;
+    };
+    if (tc == 0) {
+      post(0, 0);
+    }
+    __syncthreads();
+    for (int i = 0; i < nb; ++i) {
+      const int buf = i & 1;
+      int bi, wl;
+      const unsigned long long key = (lane < RT) ? ckey[buf][lane] : 0ull;
+      warp_argmax(key, (lane < RT) ? cpos[buf][lane] : 0x7fffffff, bi, wl);
+      const int p = crow[buf][wl];
+      if (tid == 0) {
+        at[i] = p;
+        if (!(__longlong_as_double((long long)(ckey[buf][wl] & ~(1ull << 63))) > 0.)) {
+          flag = 1;
+        }
+      }
+      const cplx *pr = Am + p * lda;
+      const cplx pinv = cinv_lu(pr[i]);
+      cplx l[NA];
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        const int r = tr + RT * a;
+        // the row that was at position i takes the pivot's old position
+        if (r == p) {
+          pos[a] = i;
+        } else if (pos[a] == i) {
+          pos[a] = bi;
+        }
+        l[a] = (r < nb && pos[a] > i) ? mul_xx(Am[r * lda + i], pinv) : mkc(0., 0.);
+      }
+      __syncwarp(); // the row's 16 threads have read column i
+      if (tc == (i & 15)) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+          const int r = tr + RT * a;
+          if (r < nb && pos[a] > i) {
+            Am[r * lda + i] = l[a];
+          }
+        }
+      }
+      // columns i + 1, i + 2, ..: column i + 1 first, its threads post the
+      // next step's candidates before the rest
+      for (int k = i + 1 + ((tc - i - 1) & 15); k < nb; k += 16) {
+        const cplx u = pr[k];
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+          const int r = tr + RT * a;
+          if (r < nb && pos[a] > i) {
+            Am[r * lda + k] = csub(Am[r * lda + k], mul_xy(l[a], u));
+          }
+        }
+        if (k == i + 1) {
+          post(k, buf ^ 1);
+        }
+      }
+      __syncthreads();
+    }
+    if (tid == 0 && flag) {
+      atomicOr(&A.status[sl.grain], TMX_ST_SINGULAR);
+    }
+    int *ps = reinterpret_cast<int *>(Qs + 2 * (int64_t)nb * nb);
+    for (int j = tid; j < nb; j += NTH) {
+      ps[j] = at[j];
+    }
+    if (!inplace) {
+      for (int r = tr; r < nb; r += RT) {
+        for (int k = tc; k < nb; k += 16) {
+          Qs[(int64_t)r * nb + k] = Am[r * lda + k];
+        }
+      }
+    }
+    if (A.lu) {
+      // factors (unit-lower L below, U on and above the diagonal) and the
+      // column gather index, for the tangent solves
+      cplx *Ls = A.lu + item.scratch;
+      for (int r = tr; r < nb; r += RT) {
+        const cplx *s = Am + at[r] * lda;
+        for (int k = tc; k < nb; k += 16) {
+          Ls[(int64_t)r * nb + k] = s[k];
+        }
+      }
+      int *pl = reinterpret_cast<int *>(Ls + (int64_t)nb * nb);
+      for (int j = tid; j < nb; j += NTH) {
+        pl[at[j]] = j;
+      }
+    }
+    __syncthreads(); // shared memory is reused by the next item
+  }
+}
+
+// Solve T_c Q_c = -RgQ_c with k_factor's factors: CTA per NTH / C rows of an
+// item, C lanes per row, the row in registers (column c + C t in x[t] of lane
+// c, steps in blocks of C columns so that x is indexed statically), the
+// factors copied to shared memory in position order (read in place for
+// classes whose factors exceed it).
+template <int NBM, int NTH, int C>
+__global__ void __launch_bounds__(NTH, (NBM > 64) ? 1 : 2)
+    k_solve(TmxBlockArgs A, int chunks, size_t smem_bytes) {
+  constexpr int NT = NBM / C;
+  constexpr int ROWS = NTH / C;
+  extern __shared__ __align__(16) unsigned char fsm[];
+  __shared__ cplx uinv[NBM];
+  __shared__ int at[NBM];
+  const int tid = threadIdx.x;
+  const int c = tid % C;
+  const int ilo = A.range ? A.range[0] : 0;
+  const int ihi = A.range ? min(A.range[1], A.nitems) : A.nitems;
+  for (int64_t u0 = (int64_t)ilo * chunks + blockIdx.x; u0 < (int64_t)ihi * chunks;
+       u0 += gridDim.x) {
+    const TmxItem item = A.items[u0 / chunks];
+    const TmxSlot sl = A.slots[item.slot];
+    const int N = sl.nmax;
+    const int m = item.m;
+    const ClassDesc D = describe<1>(N, m, item.cls);
+    const int nb = D.nb;
+    const int a0 = (int)(u0 % chunks) * ROWS;
+    if (nb > NBM || nb > A.max_nb || a0 >= nb) {
+      continue;
+    }
+    const cplx *Qs = A.scratch + item.scratch;
+    const cplx *Rs = Qs + (int64_t)nb * nb;
+    const int *ps = reinterpret_cast<const int *>(Rs + (int64_t)nb * nb);
+    const int lds = nb | 1;
+    const bool inplace = (size_t)nb * lds * sizeof(cplx) > smem_bytes;
+    for (int j = tid; j < nb; j += NTH) {
+      const int p = ps[j];
+      at[j] = p;
+      uinv[j] = cinv_lu(Qs[(int64_t)p * nb + j]);
+    }
+    __syncthreads();
+    cplx *Fm = reinterpret_cast<cplx *>(fsm);
+    if (!inplace) {
+      for (int j = tid >> 5; j < nb; j += NTH / 32) {
+        const cplx *s = Qs + (int64_t)at[j] * nb;
+        for (int k = tid & 31; k < nb; k += 32) {
+          cp16(Fm + j * lds + k, s + k);
+        }
+      }
+      cp_commit();
+    }
+    const int a = a0 + tid / C;
+    const bool act = a < nb;
+    cplx x[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const int k = c + C * t;
+      const cplx v = (act && k < nb) ? Rs[(int64_t)a * nb + k] : mkc(0., 0.);
+      x[t] = mkc(-v.x, -v.y);
+    }
+    cp_wait_all();
+    __syncthreads();
+    // Z U = X (forward over columns)
+#pragma unroll
+    for (int tj = 0; tj < NT; ++tj) {
+      if (tj * C < nb) {
+        for (int cj = 0; cj < C; ++cj) {
+          const int j = tj * C + cj;
+          if (j >= nb) {
+            break;
+          }
+          if (c == cj) {
+            // (column 0 of the classes up to 64: see mul_yx)
+            x[tj] = (NBM <= 64 && j == 0) ? mul_yx(x[tj], uinv[j]) : mul_xy(x[tj], uinv[j]);
+          }
+          cplx xj;
+          xj.x = __shfl_sync(0xffffffffu, x[tj].x, cj, C);
+          xj.y = __shfl_sync(0xffffffffu, x[tj].y, cj, C);
+          const cplx *ur = inplace ? Qs + (int64_t)at[j] * nb : Fm + j * lds;
+#pragma unroll
+          for (int t = tj; t < NT; ++t) {
+            const int k = c + C * t;
+            if (k > j && k < nb) {
+              x[t] = csub(x[t], mul_xy(xj, ur[k]));
+            }
+          }
+        }
+      }
+    }
+    // Y L = Z (backward over columns, L unit lower)
+#pragma unroll
+    for (int tj = NT - 1; tj >= 0; --tj) {
+      if (tj * C < nb) {
+        for (int cj = min(C, nb - tj * C) - 1; cj >= 0; --cj) {
+          const int j = tj * C + cj;
+          cplx xj;
+          xj.x = __shfl_sync(0xffffffffu, x[tj].x, cj, C);
+          xj.y = __shfl_sync(0xffffffffu, x[tj].y, cj, C);
+          const cplx *lr = inplace ? Qs + (int64_t)at[j] * nb : Fm + j * lds;
+#pragma unroll
+          for (int t = 0; t <= tj; ++t) {
+            const int k = c + C * t;
+            if (k < j) {
+              x[t] = csub(x[t], mul_xy(xj, lr[k]));
+            }
+          }
+        }
+      }
+    }
+    // write out: T_c[a][at[k]] = Y[a][k]
+    if (act) {
+      int ia, na;
+      member(D, a, ia, na);
+      if (sl.tout < 0) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const int k = c + C * t;
+          if (k < nb && at[k] == a) {
+            A.diag[sl.diag + ia * N + (na - 1)] = x[t];
+          }
+        }
+      } else {
+        cplx *Tr = A.tout + sl.tout + block_offset(N, m) +
+                   (int64_t)(ia * D.nbb + (na - D.nmin)) * (2 * D.nbb);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const int k = c + C * t;
+          if (k < nb) {
+            int ib, nbn;
+            member(D, at[k], ib, nbn);
+            Tr[ib * D.nbb + (nbn - D.nmin)] = x[t];
+          }
+        }
+      }
+    }
+    __syncthreads(); // shared memory is reused by the next chunk
+  }
+}
+
+// dynamic shared memory a CTA may use for the factors (227 KB per block, less
+// the static arrays)
+#define TMX_FACTOR_SMEM_MAX (221u * 1024u)
+
+template <bool LEAN, int NBM, int NTHF, int NTHS, int C>
+static void launch_apart(const TmxBlockArgs &a, cudaStream_t stream) {
+  const int max_nb = std::max(1, std::min(a.max_nb, NBM));
+  const int rt = asm_row_tiles(max_nb), ct = asm_col_tiles(max_nb);
+  const int chunks = (max_nb + NTHS / C - 1) / (NTHS / C);
+  // one tile, item or row chunk per CTA (see launch_warp_variant)
+  const auto ctas = [&](int per_item) {
+    const int64_t n = (int64_t)std::max(1, a.nitems) * per_item;
+    return (unsigned)((a.max_ctas > 0) ? std::min<int64_t>(n, a.max_ctas) : n);
+  };
+  constexpr size_t asm_smem =
+      4 * TMX_ASM_WG * (TMX_ASM_ROWS + TMX_ASM_COLS + 4) * sizeof(cplx) +
+      TMX_ASM_WG * ((TMX_ASM_ROWS + TMX_ASM_COLS) * 6 + TMX_NS) * sizeof(double);
+  cudaFuncSetAttribute(k_assemble<LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)asm_smem);
+  k_assemble<LEAN><<<ctas(rt * ct), 256, asm_smem, stream>>>(a, rt, ct);
+  // factors in shared memory up to 118 members, above that in the scratch
+  const size_t smem = std::min<size_t>((size_t)max_nb * (max_nb | 1) * sizeof(cplx),
+                                       TMX_FACTOR_SMEM_MAX);
+  cudaFuncSetAttribute(k_factor<NBM, NTHF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem);
+  cudaFuncSetAttribute(k_solve<NBM, NTHS, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem);
+  k_factor<NBM, NTHF><<<ctas(1), NTHF, smem, stream>>>(a, smem);
+  k_solve<NBM, NTHS, C><<<ctas(chunks), NTHS, smem, stream>>>(a, chunks, smem);
 }
 
 int tmx_block_family_capacity(int family) {
@@ -1720,12 +1676,10 @@ void tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream) {
     launch_cta32(a, stream);
     return;
   case TMX_BLOCKS_CTA64:
-    launch_cta64(a, stream);
+    launch_apart<true, 64, 256, 512, 8>(a, stream);
     return;
-  default: {
-    const size_t smem = tmx_block_smem_bytes(a.max_nb, a.chunk_nodes);
-    launch_variant<4, 4, 256, 1>(a, smem, stream);
-  }
+  default:
+    launch_apart<false, 128, 512, 512, 16>(a, stream);
   }
 }
 

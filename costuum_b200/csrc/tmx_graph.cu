@@ -235,7 +235,7 @@ __global__ void k_gm_round(TmxGState *G, int rs, const int32_t *__restrict__ don
   unsigned long long lu_need = 0;
   for (int j = tpl_off[N]; j < tpl_off[N + 1]; ++j) {
     const int nb = tpl[2 * j + 1];
-    lu_need += 2ull * nb * nb;
+    lu_need += (unsigned long long)tmx_item_scratch(nb);
   }
   const unsigned long long lu0 = atomicAdd(&G->lu_used, lu_need);
   if (toff + ts > t_cap || lu0 + lu_need > lu_cap) {
@@ -275,7 +275,7 @@ __global__ void k_gm_round(TmxGState *G, int rs, const int32_t *__restrict__ don
     t.cls = (int16_t)(mc & 0xff);
     t.scratch = (int64_t)lu;
     bitems[b][pos] = t;
-    lu += 2ull * nb * nb;
+    lu += (unsigned long long)tmx_item_scratch(nb);
   }
 }
 

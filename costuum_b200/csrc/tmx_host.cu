@@ -656,7 +656,7 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
   int64_t scr_total = 0;
   for (int64_t i = 0; i < nitems; ++i) {
     items[i].scratch = scr_total;
-    scr_total += 2 * (int64_t)inb[i] * inb[i];
+    scr_total += tmx_item_scratch(inb[i]);
   }
   ctx->p2_scr_total = scr_total;
   if (keep_T && (size_t)t_total * sizeof(cplx) > ctx->T.cap) {
@@ -800,7 +800,6 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
       B.diag = nullptr;
       B.status = (int32_t *)ctx->status.p;
       B.max_nb = inb[i0];
-      B.chunk_nodes = tmx_host_chunk_nodes(B.max_nb);
       B.lu = keep_lu ? (cplx *)ctx->lu.p : lu_keep;
       B.family = dispatch_family(ctx, B.max_nb);
       // the round's flops are booked on its first launch
@@ -1147,7 +1146,7 @@ static int gm_compute(tmx_ctx *ctx) {
           const int b = gm_bucket(nb);
           bc[b] += 1;
           nbmax_b[b] = std::max(nbmax_b[b], nb);
-          lun[N] += 2 * (int64_t)nb * nb;
+          lun[N] += tmx_item_scratch(nb);
         }
       }
     }
@@ -1204,7 +1203,7 @@ static int gm_compute(tmx_ctx *ctx) {
       (rc = ensure(ctx, ctx->keep_arena, arena_cap * sizeof(double))) ||
       (rc = ensure(ctx, ctx->gm_tab, ncap * (int64_t)glf * Kg * Kg * TMX_NQ * sizeof(double))) ||
       (rc = ensure(ctx, ctx->gm_nsc, ncap * (int64_t)glf * Kg * TMX_NS * sizeof(double))) ||
-      (rc = ensure(ctx, ctx->gm_scr, 4 * ncap * 2 * (int64_t)cmK * cmK * sizeof(cplx))) ||
+      (rc = ensure(ctx, ctx->gm_scr, 4 * ncap * tmx_item_scratch(cmK) * sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->gm_diag, ncap * 2 * (int64_t)Kg * sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->gm_slots, ncap * sizeof(TmxSlot))) ||
       (rc = ensure(ctx, ctx->gm_items, 4 * ncap * sizeof(TmxItem))) ||
@@ -1387,7 +1386,6 @@ static int gm_compute(tmx_ctx *ctx) {
         B.diag = (cplx *)ctx->gm_diag.p;
         B.status = (int32_t *)ctx->status.p;
         B.max_nb = (k + 1) / 2;
-        B.chunk_nodes = tmx_host_chunk_nodes(B.max_nb);
         B.family = ctx->dispatch[gm_bucket(B.max_nb)];
         B.max_ctas = 148 * 8;
         tmx_launch_blocks(B, cs);
@@ -1410,7 +1408,7 @@ static int gm_compute(tmx_ctx *ctx) {
         kb.tab_stride = (int64_t)glf * k * k * TMX_NQ;
         kb.nsc_stride = (int64_t)glf * k * TMX_NS;
         kb.diag_stride = 2 * (int64_t)k;
-        kb.scr_stride = 2 * (int64_t)((k + 1) / 2) * ((k + 1) / 2);
+        kb.scr_stride = tmx_item_scratch((k + 1) / 2);
         KA.tab = (const double *)ctx->gm_tab.p;
         KA.nsc = (const double *)ctx->gm_nsc.p;
         KA.arena = (double *)ctx->keep_arena.p;
@@ -1441,7 +1439,7 @@ static int gm_compute(tmx_ctx *ctx) {
           b.tab_stride = (int64_t)glf * ks * ks * TMX_NQ;
           b.nsc_stride = (int64_t)glf * ks * TMX_NS;
           b.diag_stride = 2 * (int64_t)ks;
-          b.scr_stride = 2 * (int64_t)cm * cm;
+          b.scr_stride = tmx_item_scratch(cm);
           b.slot = q * chunk;
           b.tab = tab_t;
           b.nsc = nsc_t;
@@ -1477,7 +1475,6 @@ static int gm_compute(tmx_ctx *ctx) {
         B.diag = (cplx *)ctx->gm_diag.p;
         B.status = (int32_t *)ctx->status.p;
         B.max_nb = (kl + 1) / 2;
-        B.chunk_nodes = tmx_host_chunk_nodes(B.max_nb);
         B.family = ctx->dispatch[gm_bucket(B.max_nb)];
         tmx_launch_blocks(B, cs);
         for (int q = 0; q < gk; ++q) {
@@ -1606,7 +1603,6 @@ static int gm_compute(tmx_ctx *ctx) {
           R.diag = nullptr;
           R.status = (int32_t *)ctx->status.p;
           R.max_nb = nbmax_b[b];
-          R.chunk_nodes = tmx_host_chunk_nodes(R.max_nb);
           R.lu = (cplx *)ctx->gm_lu.p;
           R.family = ctx->dispatch[b];
           R.max_ctas = TMX_GM_ROUND_CTAS;
@@ -1965,7 +1961,7 @@ int tmx_batch_compute(tmx_ctx *ctx) {
       b.tab_stride = (int64_t)glf * ks * ks * TMX_NQ;
       b.nsc_stride = (int64_t)glf * ks * TMX_NS;
       b.diag_stride = 2 * (int64_t)ks;
-      b.scr_stride = 2 * (int64_t)cm * cm;
+      b.scr_stride = tmx_item_scratch(cm);
       if (G == 1) {
         const size_t per_slot = (b.tab_stride + b.nsc_stride) * sizeof(double) +
                                 (4 * b.scr_stride + b.diag_stride) * sizeof(cplx);
@@ -2030,7 +2026,6 @@ int tmx_batch_compute(tmx_ctx *ctx) {
       B.diag = (cplx *)ctx->diag.p;
       B.status = (int32_t *)ctx->status.p;
       B.max_nb = (kl + 1) / 2;
-      B.chunk_nodes = tmx_host_chunk_nodes(B.max_nb);
       B.family = dispatch_family(ctx, B.max_nb);
       // (flops of the upper bound of slots: the profiled figure is an
       // estimate until the group's length is known)

@@ -59,6 +59,15 @@ struct TmxItem {
   int64_t scratch; // offset (complex elements) of this item's Q/RgQ scratch
 };
 
+// complex elements of an item's scratch: Q and RgQ of the class, then the row
+// order of its factors (32-bit integers)
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int64_t tmx_item_scratch(int64_t nb) {
+  return 2 * nb * nb + (nb + 3) / 4;
+}
+
 // Per-slot descriptor for the block kernel.
 struct TmxSlot {
   int32_t grain;  // grain index

@@ -57,14 +57,13 @@ struct TmxBlockArgs {
   const double *nsc;
   const double *wig;           // Wigner buffer
   const int64_t *wig_off;      // per Wigner set: offset of m = 0 (doubles)
-  double2 *scratch;            // per-item Q / RgQ scratch
+  double2 *scratch;            // per-item scratch (tmx_item_scratch)
   double2 *tout;               // T-matrix storage (complex)
   double2 *diag;               // chain-mode diagonal buffer
   int32_t *status;             // per grain status bits
-  int chunk_nodes;             // quadrature nodes per shared-memory chunk
   int max_nb;                  // largest class size in this launch
   double2 *lu = nullptr;       // if set: LU factors + pivots saved per item
-                               // at the item's scratch offset (2 nb^2)
+                               // at the item's scratch offset
   int family = -1;             // tmx_block_family to run, -1: by max_nb
   // device-driven launches (CUDA graph): items [range[0], range[1]) of
   // `items` (clamped to nitems) instead of [0, nitems); at most max_ctas
@@ -74,7 +73,6 @@ struct TmxBlockArgs {
 };
 // largest class size each tmx_block_family can run
 int tmx_block_family_capacity(int family);
-size_t tmx_block_smem_bytes(int max_nb, int chunk_nodes);
 void tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream);
 
 // slots and m = 0 items of one order step from the active list

@@ -241,7 +241,6 @@ extern "C" int tmx_tmatrix_fixed_noalloc(double r_ev, double wavelength,
   B.diag = nullptr;
   B.status = reinterpret_cast<int32_t *>(base + NA_STATUS);
   B.max_nb = max_nb;
-  B.chunk_nodes = tmx_host_chunk_nodes(max_nb);
   tmx_launch_blocks(B, st);
   NA_CK(cudaGetLastError());
   // the grain's status bits (singular pivot, non-finite entries) into the

@@ -102,7 +102,7 @@ int m0_step(tmx_ctx *ctx, const std::vector<int32_t> &g, const std::vector<int> 
   for (size_t i = 0; i < its.size(); ++i) {
     items[i] = its[i].it;
     items[i].scratch = scr;
-    scr += 2 * (int64_t)its[i].nb * its[i].nb;
+    scr += tmx_item_scratch(its[i].nb);
   }
   if ((rc = ensure(ctx, ctx->tab, std::max<int64_t>(1, tab) * sizeof(double))) ||
       (rc = ensure(ctx, ctx->nsc, std::max<int64_t>(1, nsc) * sizeof(double))) ||
@@ -143,7 +143,6 @@ int m0_step(tmx_ctx *ctx, const std::vector<int32_t> &g, const std::vector<int> 
       B.diag = (cplx *)ctx->diag.p;
       B.status = (int32_t *)ctx->status.p;
       B.max_nb = its[i0].nb;
-      B.chunk_nodes = tmx_host_chunk_nodes(B.max_nb);
       B.family = dispatch_family(ctx, B.max_nb);
       tmx_launch_blocks(B, st);
       LAUNCHED();
