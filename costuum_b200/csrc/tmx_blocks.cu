@@ -1864,85 +1864,119 @@ void tmx_launch_keep_tables(const TmxKeepArgs &K, int max_entries,
 // The reference's quadruple loop over (n1, n2, m1, m2 = m1) visits every
 // entry of every m block once, so Qsca = sum_m f_m ||T_m||_F^2 and
 // Qext = sum_m f_m sum_n Re(T_m[(0,n),(0,n)] + T_m[(0,n),(1,n)] +
-// T_m[(1,n),(0,n)] + T_m[(1,n),(1,n)]), f_0 = 1, f_m = 2. One block per
-// grain reads each (contiguous) block coalesced; the reduction order is fixed.
+// T_m[(1,n),(0,n)] + T_m[(1,n),(1,n)]), f_0 = 1, f_m = 2.
+//
+// A grain's blocks are one contiguous range of T, so |T|^2 is summed over that
+// range without regard to blocks (weight 1 up to the end of block 0, 2 after
+// it), all loads of a thread independent; the diagonals are read on their own,
+// a warp per block. Grains of more than 24 orders are shared by 4 or 16 CTAs
+// (blockIdx.y): the last one to finish adds the partial sums in order, so the
+// result depends on the grain alone. Bound by reading T: 28 grains of order 99
+// (21 MB each) 1.99 -> 0.15 ms, 96 grains of orders 16..50 0.28 -> 0.038 ms
+// against one CTA per grain that went block by block.
 #define QS_THREADS 256
-// Qsca and Qext sums of the grains of one block round (TMatrixQTask,
-// TMatrixResource.hpp:1136-1210): one CTA per slot, thread t adds the
-// entries t, t + 256, ... of every m block in order (|T|^2, and Re T on the
-// block diagonals), then a warp tree and the warp partial sums in order.
-// Row and column of an entry advance incrementally (no division per entry).
+__host__ __device__ static inline int qsum_parts(int N) {
+  return N <= 24 ? 1 : N <= 48 ? 4 : TMX_QSUM_PARTS;
+}
+
 __global__ void __launch_bounds__(QS_THREADS)
-    k_qsums(const TmxSlot *__restrict__ slots, int ns,
-            const cplx *__restrict__ T, double *q_out,
+    k_qsums(const TmxSlot *__restrict__ slots, int ns, const cplx *__restrict__ T,
+            double *q_out, double *part, unsigned *ticket,
             const int32_t *__restrict__ range) {
+  __shared__ double red[2][QS_THREADS / 32];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int slo = range ? range[0] : 0;
   const int shi = range ? min(range[1], ns) : ns;
   for (int s = slo + blockIdx.x; s < shi; s += gridDim.x) {
-  const TmxSlot sl = slots[s];
-  const int N = sl.nmax;
-  const cplx *Tg = T + sl.tout;
-  double qs = 0., qe = 0.;
-  for (int m = 0; m <= N && N > 0; ++m) {
-    const int nb = (m == 0) ? N : N + 1 - m;
-    const int w = 2 * nb;
-    const double f = (m > 0) ? 2. : 1.;
-    const cplx *B = Tg + block_offset(N, m);
-    const int dq = QS_THREADS / w, dr = QS_THREADS % w;
-    int row = threadIdx.x / w, col = threadIdx.x % w;
-    double bs = 0., be = 0.;
-    for (int u = threadIdx.x; u < w * w; u += QS_THREADS) {
-      const cplx v = B[u];
-      bs += cnorm2(v);
-      const int rm = (row >= nb) ? row - nb : row;
-      const int cm = (col >= nb) ? col - nb : col;
-      if (rm == cm) {
-        be += v.x;
+    const TmxSlot sl = slots[s];
+    const int N = sl.nmax;
+    const int np = qsum_parts(N);
+    const int ip = blockIdx.y;
+    if (ip >= np) {
+      continue;
+    }
+    const cplx *Tg = T + sl.tout;
+    double qs = 0., qe = 0.;
+    if (N > 0) {
+      const int64_t total = block_offset(N, N + 1);
+      const int64_t first = 4 * (int64_t)N * N;
+      const int64_t chunk = (total + np - 1) / np;
+      const int64_t end = min(total, (ip + 1) * chunk);
+#pragma unroll 4
+      for (int64_t u = ip * chunk + threadIdx.x; u < end; u += QS_THREADS) {
+        const cplx v = Tg[u];
+        qs += (u < first) ? cnorm2(v) : 2. * cnorm2(v);
       }
-      row += dq;
-      col += dr;
-      if (col >= w) {
-        col -= w;
-        ++row;
+      for (int m = ip * (QS_THREADS / 32) + warp; m <= N; m += np * (QS_THREADS / 32)) {
+        const int nb = (m == 0) ? N : N + 1 - m;
+        const int w = 2 * nb;
+        const cplx *B = Tg + block_offset(N, m);
+        double be = 0.;
+        for (int r = lane; r < nb; r += 32) {
+          const cplx *d = B + (int64_t)r * w + r;
+          const cplx *e = d + (int64_t)nb * w;
+          be += (d[0].x + d[nb].x) + (e[0].x + e[nb].x);
+        }
+        qe += (m > 0) ? 2. * be : be;
       }
     }
-    qs += f * bs;
-    qe += f * be;
-  }
-  __shared__ double red[2][QS_THREADS / 32];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    qs += __shfl_down_sync(0xffffffffu, qs, o);
-    qe += __shfl_down_sync(0xffffffffu, qe, o);
-  }
-  const int warp = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    red[0][warp] = qs;
-    red[1][warp] = qe;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0., b = 0.;
-    for (int i = 0; i < QS_THREADS / 32; ++i) {
-      a += red[0][i];
-      b += red[1][i];
+    for (int o = 16; o > 0; o >>= 1) {
+      qs += __shfl_down_sync(0xffffffffu, qs, o);
+      qe += __shfl_down_sync(0xffffffffu, qe, o);
     }
-    q_out[2 * sl.grain] = a;
-    q_out[2 * sl.grain + 1] = b;
-  }
-  // red is reused by the next slot
-  __syncthreads();
+    if (lane == 0) {
+      red[0][warp] = qs;
+      red[1][warp] = qe;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double a = 0., b = 0.;
+      for (int i = 0; i < QS_THREADS / 32; ++i) {
+        a += red[0][i];
+        b += red[1][i];
+      }
+      if (np == 1) {
+        q_out[2 * sl.grain] = a;
+        q_out[2 * sl.grain + 1] = b;
+      } else {
+        volatile double *pg = part + (int64_t)sl.grain * 2 * TMX_QSUM_PARTS;
+        pg[2 * ip] = a;
+        pg[2 * ip + 1] = b;
+        __threadfence();
+        if (atomicAdd(&ticket[sl.grain], 1u) == (unsigned)(np - 1)) {
+          __threadfence();
+          a = b = 0.;
+          for (int i = 0; i < np; ++i) {
+            a += pg[2 * i];
+            b += pg[2 * i + 1];
+          }
+          q_out[2 * sl.grain] = a;
+          q_out[2 * sl.grain + 1] = b;
+          ticket[sl.grain] = 0u; // ready for the grain's next batch
+        }
+      }
+    }
+    // red is reused by the next slot
+    __syncthreads();
   }
 }
 
-void tmx_launch_qsums(const TmxSlot *slots, int ns, const cplx *T,
-                      double *q_out, cudaStream_t stream, const int32_t *range,
-                      int max_ctas) {
+size_t tmx_qsum_part_bytes(int64_t n) {
+  return (size_t)n * (2 * TMX_QSUM_PARTS * sizeof(double) + sizeof(unsigned));
+}
+
+void tmx_launch_qsums(const TmxSlot *slots, int ns, const cplx *T, double *q_out,
+                      double *part, int64_t n, int nmax, cudaStream_t stream,
+                      const int32_t *range, int max_ctas) {
   if (ns <= 0) {
     return;
   }
   const int blocks = (max_ctas > 0) ? std::min(ns, max_ctas) : ns;
-  k_qsums<<<blocks, QS_THREADS, 0, stream>>>(slots, ns, T, q_out, range);
+  unsigned *ticket = reinterpret_cast<unsigned *>(part + 2 * TMX_QSUM_PARTS * n);
+  k_qsums<<<dim3(blocks, qsum_parts(nmax)), QS_THREADS, 0, stream>>>(
+      slots, ns, T, q_out, part, ticket, range);
 }
 
 // ------------------------------------------------------------ chain prep --

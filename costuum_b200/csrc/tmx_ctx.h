@@ -56,6 +56,8 @@ struct tmx_ctx {
   // batch buffers
   DevBuf grains, state, state0, act0, act1, actinit, count, slots, items, tab,
       nsc, scratch, diag, T, q, status, probe;
+  DevBuf q_part;    // partial Q sums of the larger grains
+  int64_t q_n = -1; // grains q and q_part are laid out for
   // uploaded batch (device-resident inputs)
   bool uploaded = false;
   int64_t up_n = 0;

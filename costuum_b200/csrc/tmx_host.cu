@@ -375,7 +375,7 @@ void tmx_destroy(tmx_ctx *ctx) {
                     &ctx->wig_off, &ctx->grains, &ctx->state,  &ctx->act0,
                     &ctx->act1,  &ctx->count,  &ctx->slots,   &ctx->items,
                     &ctx->tab,   &ctx->nsc,    &ctx->scratch, &ctx->diag,
-                    &ctx->T,     &ctx->q,
+                    &ctx->T,     &ctx->q,     &ctx->q_part,
                     &ctx->status, &ctx->probe};
   for (DevBuf *b : bufs) {
     if (b->p) {
@@ -532,6 +532,23 @@ int tmx_batch_upload(tmx_ctx *ctx, int64_t n, const double *r_ev,
 // rounds below t_base). The schedule is kept in the context (p2 buffers and
 // ctx->p2_*) for the tangent kernels. Host-side setup runs on ctx->stream
 // (Wigner tables), which the round then waits for.
+// buffers of the Q sums of the batch's n grains; the counters behind the
+// partial sums start at zero wherever n puts them
+static int ensure_qsums(tmx_ctx *ctx) {
+  if (ctx->q_n == ctx->n) {
+    return TMX_OK;
+  }
+  const size_t bytes = std::max<size_t>(16, tmx_qsum_part_bytes(ctx->n));
+  int rc;
+  if ((rc = ensure(ctx, ctx->q, std::max<int64_t>(1, 2 * ctx->n) * sizeof(double))) ||
+      (rc = ensure(ctx, ctx->q_part, bytes))) {
+    return rc;
+  }
+  CK(cudaMemsetAsync(ctx->q_part.p, 0, bytes, ctx->stream));
+  ctx->q_n = ctx->n;
+  return TMX_OK;
+}
+
 static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
                             cudaStream_t st, int64_t t_base, bool keep_T,
                             int64_t *t_end, bool temp = false,
@@ -540,7 +557,8 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
   NvtxRange blocks_range("tmx_blocks");
   const int np2 = (int)p2.size();
   const int64_t wig_used0 = ctx->wig_used;
-  const void *T_before = ctx->T.p, *q_before = ctx->q.p;
+  const void *T_before = ctx->T.p;
+  const int64_t q_before = ctx->q_n;
   if (!keep_T) {
     ctx->sink_done = 0; // a new set of T-matrices starts at offset 0
   }
@@ -683,12 +701,12 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
       (rc = ensure(ctx, ctx->lu, std::max<int64_t>(1, scr_total) * sizeof(cplx)))) {
     return rc;
   }
-  if (ctx->q.cap < (size_t)2 * ctx->n * sizeof(double)) {
+  if (ctx->q_n != ctx->n) {
     // Q sums of every grain of the batch; rounds on the round streams may
     // still write the old buffer
     CK(cudaStreamSynchronize(ctx->stream2));
     CK(cudaStreamSynchronize(ctx->stream3));
-    if ((rc = ensure(ctx, ctx->q, std::max<int64_t>(1, 2 * ctx->n) * sizeof(double)))) {
+    if ((rc = ensure_qsums(ctx))) {
       return rc;
     }
   }
@@ -696,7 +714,7 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
     return TMX_OK;
   }
   if (st != ctx->stream && (!temp || ctx->wig_used != wig_used0 ||
-                            ctx->T.p != T_before || ctx->q.p != q_before)) {
+                            ctx->T.p != T_before || ctx->q_n != q_before)) {
     // new Wigner tables or a moved T / Q-sum buffer above are ordered on
     // ctx->stream (a round of the order loop that needs none of them does
     // not wait for the orders queued there)
@@ -844,7 +862,12 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
   if (fork) {
     CK(cudaEventDestroy(fork));
   }
-  tmx_launch_qsums(dslots, np2, (const cplx *)ctx->T.p, (double *)ctx->q.p, st);
+  int nmax_round = 0;
+  for (const TmxSlot &sl : slots) {
+    nmax_round = std::max(nmax_round, sl.nmax);
+  }
+  tmx_launch_qsums(dslots, np2, (const cplx *)ctx->T.p, (double *)ctx->q.p,
+                   (double *)ctx->q_part.p, ctx->n, nmax_round, st);
   LAUNCHED();
   // the round's T-matrices to the caller's page-locked sink, on the copy
   // stream once the round is done: the copy overlaps the order loop and the
@@ -1220,7 +1243,7 @@ static int gm_compute(tmx_ctx *ctx) {
       (rc = ensure(ctx, ctx->T, t_cap * sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->gm_lu, lu_cap * sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->gm_luscr, lu_cap * sizeof(cplx))) ||
-      (rc = ensure(ctx, ctx->q, 2 * n * sizeof(double)))) {
+      (rc = ensure_qsums(ctx))) {
     return rc;
   }
   TmxItem *bitems[TMX_GM_BUCKETS];
@@ -1254,7 +1277,7 @@ static int gm_compute(tmx_ctx *ctx) {
                           &ctx->gm_items, &ctx->gm_rslots, &ctx->gm_bitems, &ctx->gm_bptr,
                           &ctx->gm_bcap, &ctx->gm_tpl, &ctx->gm_tpl_off, &ctx->gm_full,
                           &ctx->gm_tsize, &ctx->gm_toff, &ctx->T, &ctx->gm_lu,
-                          &ctx->gm_luscr, &ctx->q, &ctx->state, &ctx->status, &ctx->grains,
+                          &ctx->gm_luscr, &ctx->q, &ctx->q_part, &ctx->state, &ctx->status, &ctx->grains,
                           &ctx->gl_x, &ctx->gl_w, &ctx->gl_off, &ctx->wig, &ctx->wig_off}) {
     key.push_back((uint64_t)(uintptr_t)b->p);
   }
@@ -1617,7 +1640,8 @@ static int gm_compute(tmx_ctx *ctx) {
           }
         }
         tmx_launch_qsums((const TmxSlot *)ctx->gm_rslots.p, (int)n, (const cplx *)ctx->T.p,
-                         (double *)ctx->q.p, rs, &G->srng[rsl][0], 148 * 4);
+                         (double *)ctx->q.p, (double *)ctx->q_part.p, n, Kg, rs,
+                         &G->srng[rsl][0], 148 * 4);
         tmx_launch_gm_round_end(G, 5 + nbk, rs);
         CK(cudaGetLastError());
         return 0;

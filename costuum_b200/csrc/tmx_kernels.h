@@ -202,13 +202,18 @@ struct TmxKeepArgs {
 void tmx_launch_keep_tables(const TmxKeepArgs &K, int max_entries,
                             cudaStream_t stream);
 
-// full Q sums over all m blocks (TMatrixQTask) of the grains of a block round: q_out[2 g], q_out[2 g + 1]
-// for g = slots[s].grain
-// (range: slots [range[0], range[1]) of the ns, read on the device; at most
-// max_ctas CTAs, 0: one per slot)
+// full Q sums over all m blocks (TMatrixQTask) of the grains of a block round:
+// q_out[2 g], q_out[2 g + 1] for g = slots[s].grain; part has
+// tmx_qsum_part_bytes(n) for a batch of n grains (partial sums and counters of
+// the larger grains, the counters zero before the first launch); nmax >= every
+// order (range: slots [range[0], range[1]) of the ns, read on the device; at
+// most max_ctas CTAs and as many per part of a grain, 0: one per slot)
+#define TMX_QSUM_PARTS 16
+size_t tmx_qsum_part_bytes(int64_t n);
 void tmx_launch_qsums(const TmxSlot *slots, int ns, const double2 *T,
-                      double *q_out, cudaStream_t stream,
-                      const int32_t *range = nullptr, int max_ctas = 0);
+                      double *q_out, double *part, int64_t n, int nmax,
+                      cudaStream_t stream, const int32_t *range = nullptr,
+                      int max_ctas = 0);
 
 // FP64 throughput probes (DFMA pipe and DMMA tensor pipe)
 void tmx_launch_probe_dfma(double *out, int iters, int blocks,
