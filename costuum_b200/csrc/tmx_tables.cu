@@ -30,6 +30,11 @@ __device__ __forceinline__ int bessel_nstart(int bessel_start, int nmax,
   return min(hi, 800);
 }
 
+// The upward products read the kept ratios this many orders ahead: the ratios
+// of orders above 48 lie in the output slots (global memory), whose latency
+// the chain of products would otherwise see once per order.
+#define TMX_RHO_WIN 8
+
 // Spherical j_n and [z j_n]'/z, n = 1..nmax, for a real argument, by the
 // downward ratio recurrence rho_n = j_n / j_{n-1} started at n = nstart with
 // rho ~ z / (2 nstart + 1), then j_n = rho_n j_{n-1} upward
@@ -53,12 +58,30 @@ __device__ static void bessel_j_real(int nmax, int nstart, double z,
   const double j0 = sin(z) * zinv;
   double jprev = rho[0] * j0;
   *reinterpret_cast<double2 *>(out) = make_double2(jprev, j0 - jprev * zinv);
-  for (int i = 1; i < nmax; ++i) {
-    const double ji = rho[i * rs] * jprev;
-    const double ip1 = i + 1.;
-    *reinterpret_cast<double2 *>(out + i * stride) =
-        make_double2(ji, jprev - ip1 * zinv * ji);
-    jprev = ji;
+  double win[TMX_RHO_WIN];
+#pragma unroll
+  for (int t = 0; t < TMX_RHO_WIN; ++t) {
+    win[t] = (1 + t < nmax) ? rho[(1 + t) * rs] : 0.;
+  }
+  for (int i0 = 1; i0 < nmax; i0 += TMX_RHO_WIN) {
+    double nxt[TMX_RHO_WIN];
+#pragma unroll
+    for (int t = 0; t < TMX_RHO_WIN; ++t) {
+      const int i = i0 + TMX_RHO_WIN + t;
+      nxt[t] = (i < nmax) ? rho[i * rs] : 0.;
+    }
+#pragma unroll
+    for (int t = 0; t < TMX_RHO_WIN; ++t) {
+      const int i = i0 + t;
+      if (i < nmax) {
+        const double ji = win[t] * jprev;
+        const double ip1 = i + 1.;
+        *reinterpret_cast<double2 *>(out + i * stride) =
+            make_double2(ji, jprev - ip1 * zinv * ji);
+        jprev = ji;
+      }
+      win[t] = nxt[t];
+    }
   }
 }
 
@@ -126,21 +149,39 @@ __device__ static void bessel_j_complex(int nmax, int nstart, cplx z,
   cplx *o = reinterpret_cast<cplx *>(out);
   o[0] = jprev;
   o[1] = csub(j0, cmul(jprev, zinv));
-  for (int i = 1; i < nmax; ++i) {
-    const cplx ji = cmul(rho[i * rs], jprev);
-    const cplx dji = csub(jprev, cmul(cscale(zinv, i + 1.), ji));
-    cplx *oi = reinterpret_cast<cplx *>(out + i * stride);
-    oi[0] = ji;
-    oi[1] = dji;
-    jprev = ji;
+  cplx win[TMX_RHO_WIN];
+#pragma unroll
+  for (int t = 0; t < TMX_RHO_WIN; ++t) {
+    win[t] = (1 + t < nmax) ? rho[(1 + t) * rs] : mkc(0., 0.);
+  }
+  for (int i0 = 1; i0 < nmax; i0 += TMX_RHO_WIN) {
+    cplx nxt[TMX_RHO_WIN];
+#pragma unroll
+    for (int t = 0; t < TMX_RHO_WIN; ++t) {
+      const int i = i0 + TMX_RHO_WIN + t;
+      nxt[t] = (i < nmax) ? rho[i * rs] : mkc(0., 0.);
+    }
+#pragma unroll
+    for (int t = 0; t < TMX_RHO_WIN; ++t) {
+      const int i = i0 + t;
+      if (i < nmax) {
+        const cplx ji = cmul(win[t], jprev);
+        const cplx dji = csub(jprev, cmul(cscale(zinv, i + 1.), ji));
+        cplx *oi = reinterpret_cast<cplx *>(out + i * stride);
+        oi[0] = ji;
+        oi[1] = dji;
+        jprev = ji;
+      }
+      win[t] = nxt[t];
+    }
   }
 }
 
 // Node scalars follow GaussBasedResources::execute (GaussBasedResources.hpp:
 // 132-152), get_r_dr_spheroid (SpecialFunctions.hpp:872-893) and
 // InteractionTask::execute (InteractionResource.hpp:478-527).
-// Tables of node g of one slot; kind 0: real-argument tables and node
-// scalars, kind 1: complex-argument tables. Ratio columns in shared memory,
+// Tables of node g of one slot; kind 0: j_n of the real argument and node
+// scalars, kind 1: j_n of the complex argument, kind 2: y_n. Ratio columns in shared memory,
 // i < rho_smem: the complex recurrence uses the complex entries tid + nt i
 // of trho, the real one the doubles rtid + rnt i.
 __device__ __forceinline__ void table_node(const TmxSlot &sl,
@@ -169,7 +210,9 @@ __device__ __forceinline__ void table_node(const TmxSlot &sl,
     const double drr = r2oa2 * c * sn * d2m1;
     const double r = sqrt(r2);
     double *T = tab + sl.tab + (int64_t)g * N * TMX_NQ;
-    if (kind == 0) {
+    if (kind == 2) {
+      bessel_y_real(N, G.k * r * G.r_ev, T + TMX_Q_Y, TMX_NQ);
+    } else if (kind == 0) {
       const double kr = G.k * r * G.r_ev;
       const double krinv = 1. / kr;
       const cplx krmr = mkc(G.mr * G.k * r * G.r_ev, G.mi * G.k * r * G.r_ev);
@@ -205,7 +248,6 @@ __device__ __forceinline__ void table_node(const TmxSlot &sl,
         bessel_j_real(N, bessel_nstart(bessel_start, N, kr), kr, T + TMX_Q_J,
                       TMX_NQ, T + TMX_Q_J, TMX_NQ);
       }
-      bessel_y_real(N, kr, T + TMX_Q_Y, TMX_NQ);
     } else {
       const cplx krmr = mkc(G.mr * G.k * r * G.r_ev, G.mi * G.k * r * G.r_ev);
       const int ns = bessel_nstart(bessel_start, N, hypot(krmr.x, krmr.y));
@@ -219,9 +261,10 @@ __device__ __forceinline__ void table_node(const TmxSlot &sl,
   }
 }
 
-// Grid (slot, node chunk, kind): kind 0 threads do the real-argument tables
-// and node scalars of node g, kind 1 threads the complex-argument tables, so
-// every warp runs one recurrence type.
+// Grid (slot, node chunk, kind): every warp runs one recurrence type, and the
+// three of a node run side by side (a few grains at orders of 100 to 200 leave
+// the launch bound by one thread's chain: 9 grains 89 -> 39 us per order with y_n
+// beside j_n and the ratios read ahead).
 __global__ void k_tables(const TmxSlot *__restrict__ slots, int nslots,
                          const TmxGrain *__restrict__ grains,
                          const double *__restrict__ gl_x,
@@ -262,15 +305,15 @@ __global__ void k_tables_dev(const TmxSlot *__restrict__ slots, int nslots,
   const int ns = min(nslots, *nact);
   const int ng = *ng_dev;
   const int nch = (ng + 31) >> 5;
-  const int64_t ntask = (int64_t)ns * nch * 2;
+  const int64_t ntask = (int64_t)ns * nch * 3;
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   for (int64_t t = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); t < ntask;
        t += (int64_t)gridDim.x * wpb) {
-    const int s = (int)(t / (2 * nch));
-    const int rem = (int)(t - (int64_t)s * 2 * nch);
-    const int kind = rem & 1;
-    const int g = (rem >> 1) * 32 + lane;
+    const int s = (int)(t / (3 * nch));
+    const int rem = (int)(t - (int64_t)s * 3 * nch);
+    const int kind = rem % 3;
+    const int g = (rem / 3) * 32 + lane;
     const TmxSlot sl = slots[s];
     if (g < sl.ngauss) {
       table_node(sl, grains, gl_x, gl_w, gl_off, tab, nsc, bessel_start, rho_smem, g,
@@ -379,9 +422,10 @@ void tmx_launch_tables(const TmxSlot *slots, int nslots, const TmxGrain *grains,
   // one thread per node: a warp per slot and argument kind when every slot
   // has at most 32 nodes (the order loop up to order 16), else chunks of 64
   const int threads = (ngmax <= 32) ? 32 : 64;
-  // ratios in shared memory for orders up to 48, sized by the launch's
-  // largest order (more CTAs per SM for small orders)
-  const int rho_smem = std::max(1, std::min(48, nmax_max));
+  // ratios in shared memory for launches of orders up to 48, sized by the
+  // largest one; launches of larger orders keep them in the output slots and
+  // need no shared memory (with 48 rows of it per thread eight warps fit an SM)
+  const int rho_smem = (nmax_max <= 48) ? std::max(1, nmax_max) : 0;
   const size_t smem = (size_t)threads * rho_smem * sizeof(cplx);
   static int attr_dev = -1;
   int dev = 0;
@@ -391,7 +435,7 @@ void tmx_launch_tables(const TmxSlot *slots, int nslots, const TmxGrain *grains,
                          (int)(64 * 48 * sizeof(cplx)));
     attr_dev = dev;
   }
-  dim3 grid(nslots, (ngmax + threads - 1) / threads, 2);
+  dim3 grid(nslots, (ngmax + threads - 1) / threads, 3);
   k_tables<<<grid, threads, smem, stream>>>(slots, nslots, grains, gl_x, gl_w,
                                             gl_off, tab, nsc, bessel_start,
                                             rho_smem);
