@@ -1685,104 +1685,113 @@ void tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream) {
 
 // ----------------------------------------------------------- convergence --
 
-// One thread per active slot: m = 0 sums of the latest order in the
-// reference's order (TMatrixResource.hpp:743-756) and the convergence test
-// (:758-775). Unconverged slots that have orders left go to the next list.
+// The m = 0 sums of every (active slot, order of the group), one thread each,
+// in the reference's order (TMatrixResource.hpp:743-756); then one thread per
+// slot applies the convergence test (:758-775) order by order until the order
+// is final. Unconverged slots that have orders left go to the next list.
+// One launch per group: with few grains left the kernels of the loop are
+// shorter than their launches (eight orders of one grain: eight of 3 us -> one
+// of 6 us).
+#define CV_THREADS 128
 __global__ void k_converge(const int32_t *__restrict__ active, int nactive,
+                           const __grid_constant__ TmxChainGroup g, int lg,
                            const TmxSlot *__restrict__ slots,
                            const cplx *__restrict__ diag, TmxChainState *state,
-                           double tolerance, int order, int last_order,
+                           double tolerance, int last_order,
                            int32_t *next_active, int32_t *next_count,
                            int32_t *done_list, int32_t *done_ord,
                            int32_t *done_pos, int32_t *done_count,
-                           const int32_t *nact_dev, int base,
-                           const int32_t *order_dev) {
-  if (order_dev) {
-    order = *order_dev;
+                           const int32_t *nact_dev, int base) {
+  __shared__ double sq[CV_THREADS], se[CV_THREADS];
+  // order s of the group and slot p: 2^lg threads per slot
+  const int s = threadIdx.x & ((1 << lg) - 1);
+  const int p = (blockIdx.x * CV_THREADS + threadIdx.x) >> lg;
+  const bool have = p < nactive && (!nact_dev || base + p < *nact_dev);
+  if (have && s < g.n) {
+    const TmxSlot sl = slots[g.base[s].slot + p];
+    const cplx *dg = diag + sl.diag;
+    const int N = g.order0 + s;
+    double qs = 0., qe = 0.;
+#pragma unroll 4
+    for (int n = 1; n < N + 1; ++n) {
+      const double dn1 = 2. * n + 1.;
+      const cplx a = dg[n - 1];
+      const cplx b = dg[N + n - 1];
+      qs += dn1 * (cnorm2(a) + cnorm2(b));
+      qe += dn1 * (a.x + b.x);
+    }
+    sq[threadIdx.x] = qs;
+    se[threadIdx.x] = qe;
   }
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nactive || (nact_dev && base + p >= *nact_dev)) {
+  __syncthreads();
+  if (!have || s != 0) {
     return;
   }
-  const int g = active[p];
-  {
-    // speculative orders: a grain whose order became final at an earlier
-    // order of the same group is not touched again
-    const TmxChainState s0 = state[g];
-    if (s0.converged || (s0.status & (TMX_ST_NAN | TMX_ST_NOT_CONVERGED))) {
-      return;
-    }
-  }
-  const TmxSlot sl = slots[p];
-  const cplx *dg = diag + sl.diag;
-  const int N = order;
-  double qs = 0., qe = 0.;
-  for (int n = 1; n < N + 1; ++n) {
-    const double dn1 = 2. * n + 1.;
-    const cplx a = dg[n - 1];
-    const cplx b = dg[N + n - 1];
-    qs += dn1 * (cnorm2(a) + cnorm2(b));
-    qe += dn1 * (a.x + b.x);
-  }
-  TmxChainState st = state[g];
-  const double old_qs = st.qsca, old_qe = st.qext;
-  st.qsca = qs;
-  st.qext = qe;
-  st.nmax = N;
-  st.ngauss = sl.ngauss;
-  if (st.dqs_t == -2.) {
-    st.dqs_t = -1.;
-    st.dqe_t = -1.;
-  } else {
-    st.dqs_t = fabs((old_qs - qs) / qs);
-    st.dqe_t = fabs((old_qe - qe) / qe);
-  }
-  if (st.dqs_t > 0.) {
-    st.dqs = st.dqs_t;
-    st.dqe = st.dqe_t;
-    if (st.dqs_t <= tolerance && st.dqe_t <= tolerance) {
-      st.converged = 1;
-    }
-  }
-  bool finite = isfinite(qs) && isfinite(qe);
-  if (!finite) {
-    st.status |= TMX_ST_NAN;
-  }
+  const int gr = active[p];
+  TmxChainState st = state[gr];
   bool stays = false;
-  if (!st.converged && finite) {
-    if (order < last_order) {
-      const int q = atomicAdd(next_count, 1);
-      next_active[q] = g;
-      stays = true;
+  for (int t = 0; t < g.n; ++t) {
+    const double qs = sq[threadIdx.x + t], qe = se[threadIdx.x + t];
+    const int order = g.order0 + t;
+    const double old_qs = st.qsca, old_qe = st.qext;
+    st.qsca = qs;
+    st.qext = qe;
+    st.nmax = order;
+    st.ngauss = g.glf * order;
+    if (st.dqs_t == -2.) {
+      st.dqs_t = -1.;
+      st.dqe_t = -1.;
     } else {
+      st.dqs_t = fabs((old_qs - qs) / qs);
+      st.dqe_t = fabs((old_qe - qe) / qe);
+    }
+    if (st.dqs_t > 0.) {
+      st.dqs = st.dqs_t;
+      st.dqe = st.dqe_t;
+      if (st.dqs_t <= tolerance && st.dqe_t <= tolerance) {
+        st.converged = 1;
+      }
+    }
+    const bool finite = isfinite(qs) && isfinite(qe);
+    if (!finite) {
+      st.status |= TMX_ST_NAN;
+    }
+    stays = !st.converged && finite && order < last_order;
+    if (!st.converged && finite && !stays) {
       st.status |= TMX_ST_NOT_CONVERGED;
     }
+    if (!stays) {
+      break;
+    }
   }
-  state[g] = st;
-  if (!stays) {
+  state[gr] = st;
+  if (stays) {
+    const int q = atomicAdd(next_count, 1);
+    next_active[q] = gr;
+  } else {
     // the grain's order is final: its blocks may start
     const int q = atomicAdd(done_count, 1);
-    done_list[q] = g;
-    done_ord[q] = order;
+    done_list[q] = gr;
+    done_ord[q] = st.nmax;
     done_pos[q] = p;
   }
 }
 
-void tmx_launch_converge(const int32_t *active, int nactive,
+void tmx_launch_converge(const int32_t *active, int nactive, const TmxChainGroup &g,
                          const TmxSlot *slots, const double2 *diag,
-                         TmxChainState *state, double tolerance, int order,
-                         int last_order, int32_t *next_active,
-                         int32_t *next_count, int32_t *done_list,
-                         int32_t *done_ord, int32_t *done_pos,
-                         int32_t *done_count, const int32_t *nact_dev,
-                         int base, cudaStream_t stream, const int32_t *order_dev) {
+                         TmxChainState *state, double tolerance, int last_order,
+                         int32_t *next_active, int32_t *next_count,
+                         int32_t *done_list, int32_t *done_ord, int32_t *done_pos,
+                         int32_t *done_count, const int32_t *nact_dev, int base,
+                         cudaStream_t stream) {
   if (nactive <= 0) {
     return;
   }
-  k_converge<<<(nactive + 127) / 128, 128, 0, stream>>>(
-      active, nactive, slots, diag, state, tolerance, order, last_order,
-      next_active, next_count, done_list, done_ord, done_pos, done_count,
-      nact_dev, base, order_dev);
+  const int lg = g.n <= 1 ? 0 : g.n <= 2 ? 1 : g.n <= 4 ? 2 : 3;
+  const int per = CV_THREADS >> lg;
+  k_converge<<<(nactive + per - 1) / per, CV_THREADS, 0, stream>>>(
+      active, nactive, g, lg, slots, diag, state, tolerance, last_order, next_active,
+      next_count, done_list, done_ord, done_pos, done_count, nact_dev, base);
 }
 
 // ------------------------------------------------------------- kept tables --
@@ -1981,16 +1990,18 @@ void tmx_launch_qsums(const TmxSlot *slots, int ns, const cplx *T, double *q_out
 
 // ------------------------------------------------------------ chain prep --
 
-// Slots and items of one order step: active position p gets the tables at
-// p * strides and the four m = 0 classes as items 4p .. 4p + 3.
+// Slots and items of a group of orders (blockIdx.y): active position p gets the
+// tables at p * strides and the four m = 0 classes as items 4p .. 4p + 3.
 __global__ void k_chain_prep(const int32_t *__restrict__ active, int nactive,
                              const int32_t *__restrict__ nact_dev, int base,
-                             int order, int ngauss, int wig_n, TmxChainBase b,
-                             TmxSlot *slots, TmxItem *items) {
+                             const __grid_constant__ TmxChainGroup g, TmxSlot *slots,
+                             TmxItem *items) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nactive) {
     return;
   }
+  const TmxChainBase &b = g.base[blockIdx.y];
+  const int order = g.order0 + (int)blockIdx.y;
   // positions past the list's length on the device (the host launched for
   // an upper bound) get an empty slot: order 0 has no classes and no nodes,
   // so every kernel of the step skips it
@@ -1998,8 +2009,8 @@ __global__ void k_chain_prep(const int32_t *__restrict__ active, int nactive,
   TmxSlot s;
   s.grain = valid ? active[p] : 0;
   s.nmax = valid ? order : 0;
-  s.ngauss = valid ? ngauss : 0;
-  s.wig_n = wig_n;
+  s.ngauss = valid ? g.glf * order : 0;
+  s.wig_n = g.wig[blockIdx.y];
   s.tab = b.tab + p * b.tab_stride;
   s.nsc = b.nsc + p * b.nsc_stride;
   s.tout = -1;
@@ -2016,12 +2027,12 @@ __global__ void k_chain_prep(const int32_t *__restrict__ active, int nactive,
 }
 
 void tmx_launch_chain_prep(const int32_t *active, int nactive,
-                           const int32_t *nact_dev, int base, int order,
-                           int ngauss, int wig_n, const TmxChainBase &b,
-                           TmxSlot *slots, TmxItem *items, cudaStream_t stream) {
+                           const int32_t *nact_dev, int base,
+                           const TmxChainGroup &g, TmxSlot *slots, TmxItem *items,
+                           cudaStream_t stream) {
   if (nactive <= 0) {
     return;
   }
-  k_chain_prep<<<(nactive + 127) / 128, 128, 0, stream>>>(
-      active, nactive, nact_dev, base, order, ngauss, wig_n, b, slots, items);
+  k_chain_prep<<<dim3((nactive + 127) / 128, g.n), 128, 0, stream>>>(
+      active, nactive, nact_dev, base, g, slots, items);
 }

@@ -1412,9 +1412,13 @@ static int gm_compute(tmx_ctx *ctx) {
         B.family = ctx->dispatch[gm_bucket(B.max_nb)];
         B.max_ctas = 148 * 8;
         tmx_launch_blocks(B, cs);
-        tmx_launch_converge(act_in, (int)n, (const TmxSlot *)ctx->gm_slots.p,
+        TmxChainGroup one = {};
+        one.n = 1;
+        one.order0 = k;
+        one.glf = glf;
+        tmx_launch_converge(act_in, (int)n, one, (const TmxSlot *)ctx->gm_slots.p,
                             (const cplx *)ctx->gm_diag.p, (TmxChainState *)ctx->state.p,
-                            S.tolerance, k, K, act_out, &G->cnt[out], (int32_t *)ctx->done.p,
+                            S.tolerance, K, act_out, &G->cnt[out], (int32_t *)ctx->done.p,
                             (int32_t *)ctx->done.p + n, (int32_t *)ctx->done_pos.p,
                             &G->cnt[1], &G->cnt[in], 0, cs);
         TmxKeepArgs KA;
@@ -1453,9 +1457,14 @@ static int gm_compute(tmx_ctx *ctx) {
       // length empty; after the group its surviving list becomes the input
       // list of order k + gk (the same parity)
       auto group_body = [&](int gk, int chunk) -> int {
-        TmxChainBase base[TMX_MAX_GROUP];
+        TmxChainGroup grp = {};
+        grp.n = gk;
+        grp.order0 = k;
+        grp.glf = glf;
+        TmxChainBase *base = grp.base;
         int64_t tab_t = 0, nsc_t = 0, diag_t = 0, scr_t = 0;
         for (int q = 0; q < gk; ++q) {
+          grp.wig[q] = m0_sets[j + q];
           const int ks = k + q;
           const int cm = (ks + 1) / 2;
           TmxChainBase &b = base[q];
@@ -1473,11 +1482,8 @@ static int gm_compute(tmx_ctx *ctx) {
           diag_t += chunk * b.diag_stride;
           scr_t += 4 * chunk * b.scr_stride;
         }
-        for (int q = 0; q < gk; ++q) {
-          tmx_launch_chain_prep(act_in, chunk, &G->cnt[in], 0, k + q, glf * (k + q),
-                                m0_sets[j + q], base[q], (TmxSlot *)ctx->gm_slots.p,
-                                (TmxItem *)ctx->gm_items.p, cs);
-        }
+        tmx_launch_chain_prep(act_in, chunk, &G->cnt[in], 0, grp,
+                              (TmxSlot *)ctx->gm_slots.p, (TmxItem *)ctx->gm_items.p, cs);
         const int kl = k + gk - 1;
         tmx_launch_tables((const TmxSlot *)ctx->gm_slots.p, gk * chunk,
                           (const TmxGrain *)ctx->grains.p, (const double *)ctx->gl_x.p,
@@ -1500,15 +1506,12 @@ static int gm_compute(tmx_ctx *ctx) {
         B.max_nb = (kl + 1) / 2;
         B.family = ctx->dispatch[gm_bucket(B.max_nb)];
         tmx_launch_blocks(B, cs);
-        for (int q = 0; q < gk; ++q) {
-          // (the output list after the group is the one of its last order)
-          CK(cudaMemsetAsync(&G->cnt[out], 0, sizeof(int32_t), cs));
-          tmx_launch_converge(act_in, chunk, (const TmxSlot *)ctx->gm_slots.p + base[q].slot,
-                              (const cplx *)ctx->gm_diag.p, (TmxChainState *)ctx->state.p,
-                              S.tolerance, k + q, K, act_out, &G->cnt[out],
-                              (int32_t *)ctx->done.p, (int32_t *)ctx->done.p + n,
-                              (int32_t *)ctx->done_pos.p, &G->cnt[1], &G->cnt[in], 0, cs);
-        }
+        CK(cudaMemsetAsync(&G->cnt[out], 0, sizeof(int32_t), cs));
+        tmx_launch_converge(act_in, chunk, grp, (const TmxSlot *)ctx->gm_slots.p,
+                            (const cplx *)ctx->gm_diag.p, (TmxChainState *)ctx->state.p,
+                            S.tolerance, K, act_out, &G->cnt[out], (int32_t *)ctx->done.p,
+                            (int32_t *)ctx->done.p + n, (int32_t *)ctx->done_pos.p,
+                            &G->cnt[1], &G->cnt[in], 0, cs);
         TmxKeepArgs KA;
         KA.done_list = (const int32_t *)ctx->done.p;
         KA.done_ord = (const int32_t *)ctx->done.p + n;
@@ -1529,7 +1532,7 @@ static int gm_compute(tmx_ctx *ctx) {
         KA.keep_q = (int64_t *)ctx->keep_q.p;
         tmx_launch_keep_tables(KA, (int)n, cs);
         tmx_launch_gm_relist(G, act_out, act_in, (int)n, in, out, cs);
-        tmx_launch_gm_step_end(G, snap, outz, j, out, in, k + gk, 2 * gk + 5, cs);
+        tmx_launch_gm_step_end(G, snap, outz, j, out, in, k + gk, 7, cs);
         CK(cudaGetLastError());
         return 0;
       };
@@ -1975,10 +1978,15 @@ int tmx_batch_compute(tmx_ctx *ctx) {
     const int32_t *cur_cnt = cnt + (grp.list ? 2 : 0);
     int32_t *nxt_cnt = cnt + (grp.list ? 0 : 2);
     DevBuf *cur = lists[grp.list], *nxt = lists[grp.list ^ 1];
-    std::vector<TmxChainBase> base(G);
+    TmxChainGroup group = {};
+    group.n = G;
+    group.order0 = k;
+    group.glf = glf;
+    TmxChainBase *base = group.base;
     int64_t tab_t = 0, nsc_t = 0, diag_t = 0, scr_t = 0;
     int chunk = nact;
     for (int s = 0; s < G; ++s) {
+      group.wig[s] = chain_sets[k + s - S.min_order];
       const int ks = k + s;
       const int cm = (ks + 1) / 2;
       TmxChainBase &b = base[s];
@@ -2015,12 +2023,9 @@ int tmx_batch_compute(tmx_ctx *ctx) {
     for (int c0 = 0; c0 < nact; c0 += chunk) {
       const int cn = std::min(chunk, nact - c0);
       const int32_t *a = (const int32_t *)cur->p + c0;
-      for (int s = 0; s < G; ++s) {
-        tmx_launch_chain_prep(a, cn, cur_cnt, c0, k + s, glf * (k + s),
-                              chain_sets[k + s - S.min_order], base[s],
-                              (TmxSlot *)ctx->slots.p, (TmxItem *)ctx->items.p, st);
-        LAUNCHED();
-      }
+      tmx_launch_chain_prep(a, cn, cur_cnt, c0, group, (TmxSlot *)ctx->slots.p,
+                            (TmxItem *)ctx->items.p, st);
+      LAUNCHED();
       // slots and items of the group are contiguous: [s][p]
       const int nsl = (G == 1) ? cn : G * chunk;
       cudaEvent_t pe = nullptr;
@@ -2067,19 +2072,12 @@ int tmx_batch_compute(tmx_ctx *ctx) {
       if ((rc2 = prof_end(ctx, 0, pe, fl, nullptr, 0., B.nitems))) {
         return rc2;
       }
-      for (int s = 0; s < G; ++s) {
-        if (G > 1) {
-          // the active list after the group is the one of its last order
-          CK(cudaMemsetAsync(nxt_cnt, 0, sizeof(int32_t), st));
-        }
-        tmx_launch_converge(a, cn, (const TmxSlot *)ctx->slots.p + base[s].slot,
-                            (const cplx *)ctx->diag.p,
-                            (TmxChainState *)ctx->state.p, S.tolerance, k + s, last,
-                            (int32_t *)nxt->p, nxt_cnt, (int32_t *)ctx->done.p,
-                            (int32_t *)ctx->done.p + n, (int32_t *)ctx->done_pos.p,
-                            cnt + 1, cur_cnt, c0, st);
-        LAUNCHED();
-      }
+      tmx_launch_converge(a, cn, group, (const TmxSlot *)ctx->slots.p,
+                          (const cplx *)ctx->diag.p, (TmxChainState *)ctx->state.p,
+                          S.tolerance, last, (int32_t *)nxt->p, nxt_cnt,
+                          (int32_t *)ctx->done.p, (int32_t *)ctx->done.p + n,
+                          (int32_t *)ctx->done_pos.p, cnt + 1, cur_cnt, c0, st);
+      LAUNCHED();
       if (ctx->keep_valid) {
         // the tables of the grains this chunk made final, before the next
         // chunk or group overwrites them

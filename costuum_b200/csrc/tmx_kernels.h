@@ -85,28 +85,34 @@ struct TmxChainBase {
   int64_t diag, diag_stride;
   int64_t scr, scr_stride;
 };
+// the orders of one group: order0 + s with ngauss = glf (order0 + s), the m = 0
+// Wigner set wig[s] and the buffers base[s], s < n
+#define TMX_MAX_GROUP 8
+struct TmxChainGroup {
+  int32_t n, order0, glf;
+  int32_t wig[TMX_MAX_GROUP];
+  TmxChainBase base[TMX_MAX_GROUP];
+};
 // nact_dev (may be NULL): the list's length on the device; positions
 // p >= *nact_dev - base of this launch (for nactive, an upper bound) get empty
 // slots
 void tmx_launch_chain_prep(const int32_t *active, int nactive,
-                           const int32_t *nact_dev, int base, int order,
-                           int ngauss, int wig_n, const TmxChainBase &b,
-                           TmxSlot *slots, TmxItem *items, cudaStream_t stream);
+                           const int32_t *nact_dev, int base,
+                           const TmxChainGroup &g, TmxSlot *slots, TmxItem *items,
+                           cudaStream_t stream);
 
-// convergence step for the active slots of one order
-// m = 0 sums and the convergence test of one order; grains that continue go
-// to next_active, grains whose order is final are appended to done_list
-// (with that order in done_ord); grains already final are skipped
-// (done_pos: the grain's position in `active`)
+// convergence step for the active slots of a group of orders
+// m = 0 sums of every order, then the convergence test order by order until
+// the grain's order is final; grains that continue past the group's last order
+// go to next_active, the others are appended to done_list (with that order in
+// done_ord); done_pos: the grain's position in `active`
 void tmx_launch_converge(const int32_t *active, int nactive,
-                         const TmxSlot *slots, const double2 *diag,
-                         TmxChainState *state, double tolerance, int order,
-                         int last_order, int32_t *next_active,
-                         int32_t *next_count, int32_t *done_list,
-                         int32_t *done_ord, int32_t *done_pos,
-                         int32_t *done_count, const int32_t *nact_dev,
-                         int base, cudaStream_t stream,
-                         const int32_t *order_dev = nullptr);
+                         const TmxChainGroup &g, const TmxSlot *slots,
+                         const double2 *diag, TmxChainState *state, double tolerance,
+                         int last_order, int32_t *next_active, int32_t *next_count,
+                         int32_t *done_list, int32_t *done_ord, int32_t *done_pos,
+                         int32_t *done_count, const int32_t *nact_dev, int base,
+                         cudaStream_t stream);
 
 // state of the device-driven order loop (tmx_graph.cu), in device memory
 #define TMX_GM_BUCKETS 5
@@ -180,7 +186,6 @@ int tmx_gm_add_decide(cudaGraph_t g, const cudaGraphNode_t *deps, size_t nd,
 
 // copies of the final-order tables of the grains that became final in one
 // group of orders, into the batch's table arena (k_keep_tables)
-#define TMX_MAX_GROUP 8
 struct TmxKeepArgs {
   const int32_t *done_list, *done_ord, *done_pos;
   const int32_t *counters;          // [1]: entries in the done list
