@@ -69,11 +69,11 @@ struct tmx_ctx {
   DevBuf cg, cg_off;
   int cg_nmax = 0;
   DevBuf Ta, o_angles, o_phis, o_wts, o_coef, o_shw, o_og, o_work, o_qj,
-      o_S, o_gq, o_gz, o_cq, o_cz, o_pairs, o_grp, o_ins, o_prs, o_rng, o_x;
+      o_S, o_gq, o_gz, o_cq, o_cz, o_orng, o_grp, o_ins, o_prs, o_rng, o_x;
   // plan of the observable kernels: the amplitude groups in chunks that share
   // the buffer of m sums (o_xcap complex per matrix set), one launch per block
   // size (ranges [rng0, rng0 + nrng) of o_rng)
-  int64_t o_npairs = 0, o_xcap = 1;
+  int64_t o_xcap = 1;
   int o_nbmax = 1;
   struct AmpLaunch {
     int rng0 = 0, nrng = 0, lcap = 1;
@@ -84,10 +84,14 @@ struct tmx_ctx {
     std::vector<AmpLaunch> launches;
   };
   std::vector<AmpChunk> o_chunks;
-  // orientation-average work order: pair-major item starts (o_pairs, pmax^2
-  // + 1) and the grains by descending order (o_ord)
+  // orientation average: the grains by descending order (o_ord) and one launch
+  // per range of pairs (ranges [rng0, rng0 + nrng) of o_orng)
   DevBuf o_ord;
-  int o_pmax = 1;
+  struct OrientLaunch {
+    int rng0 = 0, nrng = 0, ncap = 1, chunk = 8;
+    int64_t nitems = 0;
+  };
+  std::vector<OrientLaunch> o_orient;
   // angles of the current plan (o_angles) and their pi / tau columns
   int o_nangles = 0;
   DevBuf o_wcol;

@@ -293,20 +293,23 @@ struct TmxMatSet {
   const double2 *src[4];
   double2 *dst[4];
 };
-// orientation average (coef_set >= 0) or copy of every grain's T-matrix,
-// with the amplitude factors c_{n' n} folded in when fold != 0;
-// work items (pair (n1, n2), grain) pair-major: pair q = (n1 - 1) pmax +
-// n2 - 1 owns items [pstart[q], pstart[q + 1]), for the grains
-// order[0 .. pstart[q + 1] - pstart[q]) (grains by descending nmax, so the
-// grains of order >= max(n1, n2) come first); npairs = sum of nmax^2;
-// mmax >= every nmax; nmat (1 or 4) sets src[k] -> dst[k]
-void tmx_launch_orient_pairs(const TmxObsGrain *og, const int64_t *pstart,
-                             const int32_t *order, int pmax, int64_t npairs,
-                             const TmxMatSet &mats,
-                             int nmat, const double *coeffs, int ncoef,
-                             const int64_t *cg_off, const double *cg,
-                             int cg_nmax, int mmax, int fold,
-                             cudaStream_t stream);
+// work items of one orientation launch: the 2 n - 1 pairs (n1, n2) with
+// max(n1, n2) = n for the ng grains of order >= n, from item base on
+struct TmxOrientRange {
+  int64_t base;
+  int32_t n, ng;
+};
+// orientation average (coef_set >= 0) or copy of every grain's T-matrix; with
+// fold the amplitude factors c_{n' n} are folded in and the result has the
+// compact class layout at half the offsets, without it only the entries of the
+// parity classes are written (dst zeroed before). order: grains by descending
+// nmax; chunk (2, 4 or 8) grains share a warp; ncap >= every n; nmat (1 .. 4)
+// sets src[k] -> dst[k]
+void tmx_launch_orient(const TmxObsGrain *og, const int32_t *order,
+                       const TmxOrientRange *rng, int nrng, int64_t nitems, int ncap,
+                       int chunk, const TmxMatSet &mats, int nmat,
+                       const double *coeffs, int ncoef, const int64_t *cg_off,
+                       const double *cg, int cg_nmax, int fold, cudaStream_t stream);
 // m sums X of nmat (1 .. 4) averaged sets (compact class layout, src[k]) into
 // x + k xstride: nitems items in the nrng ranges, blocks of at most lcap
 // orders, groups of at most nin incoming angles; wpi / wtau: the plan's pi and

@@ -3,7 +3,7 @@
 //   k_cg            Clebsch-Gordan rows <n1 m n2 -m | N 0>, m >= 0
 //                   (SpecialFunctions::get_clebsch_gordan_coefficients,
 //                   SpecialFunctions.hpp:1131-1244)
-//   k_orient_avg    AlignmentAverageTask::execute (AlignmentAverageTask.hpp:
+//   k_orient        AlignmentAverageTask::execute (AlignmentAverageTask.hpp:
 //                   115-215), restructured: the m1 sum does not depend on m,
 //                   so it is formed once per (n1, n2, N) and reused for every
 //                   m (O(N^4) instead of O(N^5))
@@ -189,168 +189,204 @@ __device__ __forceinline__ cplx c_fold(int nin, int nout, double a, cplx z) {
   }
 }
 
-// One warp per (grain, n1, n2). AlignmentAverageTask::execute (Alignment
-// AverageTask.hpp:115-215) forms, for every m,
+// D += A B for one m8n8k4 FP64 tensor-core tile: lane l holds A[l / 4][l % 4],
+// B[l % 4][l / 4] and D[l / 4][2 (l % 4) + {0, 1}]
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, "
+      "{%0, %1};\n"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
+// AlignmentAverageTask::execute (AlignmentAverageTask.hpp:115-215) forms, for
+// every m,
 //   Ta_m = sum_N' p_N' (-1)^m CG(n1 m n2 -m|N'0) sum_m1 f(m1) (-1)^m1
 //          CG(n1 m1 n2 -m1|N'0) T_m1,
 // with f = 1 for m1 = 0 and 2 otherwise; the m1 sum does not depend on m, so
-// pass 1 forms it once per N' (lanes over N') and pass 2 contracts over N'
-// (lanes over m): O(n^2) per pair instead of O(n^3). Even N' - |n1 - n2|
-// couple the (0,0) and (1,1) sub-blocks, odd ones (0,1) and (1,0). Grains
-// without an orientation distribution (coef_set < 0) are copied. Either way
-// the output carries the factor c_{n2 n1} of the amplitude sums, so that
-// the amplitude kernel contracts Ta with real vectors only.
-// Shared memory per warp and matrix: t[4][M + 1] and S[2][2M + 1] complex.
-// NMAT matrices (a T-matrix and its tangents) share the Clebsch-Gordan
-// reads and the loops; each is summed in the same order as alone.
-template <int NMAT>
-__global__ void __launch_bounds__(256)
-k_orient_pairs(const TmxObsGrain *__restrict__ og,
-               const int64_t *__restrict__ pstart,
-               const int32_t *__restrict__ order, int pmax,
-               int64_t npairs, TmxMatSet mats, const double *__restrict__ coeffs,
-               int ncoef, const int64_t *__restrict__ cg_off,
-               const double *__restrict__ cg, int cg_nmax, int wcap, int fold) {
-  extern __shared__ cplx osh[];
+// pass 1 forms it once per N' and pass 2 contracts over N': O(n^2) per pair
+// instead of O(n^3). T couples (0,0) and (1,1) for even n1 + n2 and (0,1) and
+// (1,0) for odd ones, and only the N' of that parity contribute, so of the two
+// sub-block pairs and the 2 M + 1 rows of the Clebsch-Gordan table one half is
+// left (M = min(n1, n2)).
+//
+// One warp per (pair, chunk of 2 NT grains): both passes are products of the
+// pair's Clebsch-Gordan rows with 8 NT real columns (grain, sub-block, re/im)
+// on the FP64 tensor pipe; t and S = p_N' CG t go through shared memory, whose
+// rows are 4 doubles off a multiple of 16 (the fragments' 4 x 4 doubles hit
+// distinct banks). A chunk shares each row it reads, so the table is read once
+// per 2 NT grains. Grains without an orientation distribution (coef_set < 0)
+// are copied. With fold the output carries the factor c_{n2 n1} of the
+// amplitude sums, so that the amplitude kernel contracts with real vectors.
+// Measured (B200), one warp per (pair, grain) with FMA dot products over all
+// rows and sub-blocks -> this kernel: 96 grains of orders 16..50 0.59 -> 0.23
+// ms; 1920 grains of orders 10..99 6.7 -> 2.9 ms; 1024 grains and their three
+// tangents 1.44 -> 0.54 ms. Bound by the scattered 16-byte T reads (half of
+// each sector) and, above order 63, by the table reads of few grains.
+template <int NT>
+__global__ void __launch_bounds__(128)
+k_orient(const TmxObsGrain *__restrict__ og, const int32_t *__restrict__ order,
+         const TmxOrientRange *__restrict__ rng, int nrng, int64_t nitems, int ncap,
+         TmxMatSet mats, const double *__restrict__ coeffs, int ncoef,
+         const int64_t *__restrict__ cg_off, const double *__restrict__ cg,
+         int cg_nmax, int fold) {
+  constexpr int G = 2 * NT;       // grains per chunk
+  constexpr int LD = 8 * NT + 4;  // row of t and S
+  constexpr int CB = 8;           // table entries in flight per lane
+  extern __shared__ double osm[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  const int nwarps = blockDim.x >> 5;
-  cplx *tv = osh + (int64_t)warp * wcap * NMAT;
-  for (int64_t w = (int64_t)blockIdx.x * nwarps + warp; w < npairs;
-       w += (int64_t)gridDim.x * nwarps) {
-    // work item w = (pair (n1, n2), grain): pair-major, so that the warps
-    // of a CTA (and CTAs running together) contract the same Clebsch-Gordan
-    // rows for different grains and read them from cache. Pair
-    // q = (n1 - 1) pmax + (n2 - 1) owns items [pstart[q], pstart[q + 1]),
-    // one per grain of order >= max(n1, n2), in the order `order` (grains by
-    // descending order).
-    int lo = 0, hi = pmax * pmax - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (pstart[mid] <= w) {
-        lo = mid;
-      } else {
-        hi = mid - 1;
-      }
+  const int q = lane & 3;
+  const int rr = lane >> 2;
+  const int64_t w = (int64_t)blockIdx.x * 4 + warp;
+  if (w >= nitems) {
+    return;
+  }
+  const int rows = (ncap + 7) & ~7;
+  double *t = osm + (int64_t)warp * 2 * rows * LD; // [m][LD]
+  double *S = t + rows * LD;                       // [N'][LD]
+  int lo = 0, hi = nrng - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (rng[mid].base <= w) {
+      lo = mid;
+    } else {
+      hi = mid - 1;
     }
-    const int n1 = lo / pmax + 1;
-    const int n2 = lo % pmax + 1;
-    const TmxObsGrain G = og[order[w - pstart[lo]]];
-    const int N = G.nmax;
-    const int M = min(n1, n2);
-    // fold = 0: the plain averaged T-matrix (c = 1: i^0 times 1)
-    const double afold = fold ? a_fac(n1) * a_fac(n2) : 1.;
-    const int nfold = fold ? n1 : n2 - 1;
-    if (G.coef_set < 0) {
-      for (int m = lane; m <= M; m += 32) {
-        for (int q = 0; q < 4; ++q) {
-          const int i1 = q >> 1, i2 = q & 1;
-          const int64_t e = telem(N, m, i1, n1, i2, n2);
-          const int64_t ed = fold ? celem(N, m, i1, n1, i2, n2) : e;
-          if (ed < 0) {
-            continue;
-          }
+  }
+  const TmxOrientRange R = rng[lo];
+  const int nch = (R.ng + G - 1) / G;
+  const int pr = (int)((w - R.base) / nch);
+  const int g0 = (int)((w - R.base) % nch) * G;
+  const int n1 = (pr < R.n) ? R.n : pr - R.n + 1;
+  const int n2 = (pr < R.n) ? pr + 1 : R.n;
+  const int M = min(n1, n2);
+  const int par = (n1 + n2) & 1;
+  const cplx *src = mat_src(mats, blockIdx.y);
+  cplx *dst = mat_dst(mats, blockIdx.y);
+  // t[m][4 grain + 2 block + re/im]: block 0 is (0, par), block 1 (1, 1 - par)
+  bool avg_any = false;
+  {
+    const int e = lane % (2 * G);
+    const int blk = e & 1;
+    const bool have = g0 + (e >> 1) < R.ng;
+    const TmxObsGrain gr = og[order[have ? g0 + (e >> 1) : 0]];
+    const bool avg = have && gr.coef_set >= 0;
+    avg_any = __any_sync(0xffffffffu, avg);
+    for (int m = lane / (2 * G); m < ((M + 4) & ~3); m += 32 / (2 * G)) {
+      cplx v = mkc(0., 0.);
+      if (have && m <= M) {
+        v = src[gr.t_off + telem(gr.nmax, m, blk, n1, blk ^ par, n2)];
+        // f(m) (-1)^m is a power of two with a sign: the product is exact
+        const double f = avg ? ((m == 0) ? 1. : 2.) * ((m & 1) ? -1. : 1.) : 1.;
+        v = cscale(v, f);
+      }
+      *reinterpret_cast<cplx *>(t + m * LD + 2 * e) = v;
+    }
+  }
+  __syncwarp();
+  // (no table where nothing is averaged)
+  const double *C = avg_any ? cg + cg_off[(n1 - 1) * cg_nmax + (n2 - 1)] : nullptr;
+  const int nrow = M + 1 - par; // N' of the pair's parity: j = 2 jr + par
+  // the grains of this lane's output columns
+  int gN[NT], gset[NT];
+  int64_t goff[NT];
 #pragma unroll
-          for (int k = 0; k < NMAT; ++k) {
-            mats.dst[k][(fold ? G.t_off / 2 : G.t_off) + ed] =
-                c_fold(n2, nfold, afold, mats.src[k][G.t_off + e]);
+  for (int j = 0; j < NT; ++j) {
+    const int g = g0 + 2 * j + (q >> 1);
+    gN[j] = 0;
+    gset[j] = -1;
+    goff[j] = 0;
+    if (g < R.ng) {
+      const TmxObsGrain gr = og[order[g]];
+      gN[j] = gr.nmax;
+      gset[j] = gr.coef_set;
+      goff[j] = gr.t_off;
+    }
+  }
+  if (avg_any) {
+    // pass 1: S(N') = p_N' sum_m1 CG t
+    const int Nlo = abs(n1 - n2);
+    for (int r0 = 0; r0 < nrow; r0 += 8) {
+      const int jr = r0 + rr;
+      const double *Cr = C + (int64_t)(2 * jr + par) * (M + 1);
+      double acc[NT][2];
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        acc[j][0] = acc[j][1] = 0.;
+      }
+      for (int k0 = 0; k0 <= M; k0 += 4 * CB) {
+        double a[CB];
+#pragma unroll
+        for (int b = 0; b < CB; ++b) {
+          const int m = k0 + 4 * b + q;
+          a[b] = (jr < nrow && m <= M) ? Cr[m] : 0.;
+        }
+#pragma unroll
+        for (int b = 0; b < CB; ++b) {
+          if (k0 + 4 * b <= M) {
+            const double *tb = t + (k0 + 4 * b + q) * LD + rr;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+              dmma(acc[j][0], acc[j][1], a[b], tb[8 * j]);
+            }
           }
         }
       }
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const double p = (jr < nrow && gset[j] >= 0)
+                             ? coeffs[(int64_t)gset[j] * ncoef + Nlo + 2 * jr + par]
+                             : 0.;
+        *reinterpret_cast<double2 *>(S + jr * LD + 8 * j + 2 * q) =
+            make_double2(acc[j][0] * p, acc[j][1] * p);
+      }
+    }
+    __syncwarp();
+  }
+  // pass 2: Ta_m = (-1)^m sum_N' CG S
+  const double afold = fold ? a_fac(n1) * a_fac(n2) : 1.;
+  const int nfold = fold ? n1 : n2 - 1; // (c = 1: i^0 times 1)
+  const int i1 = q & 1, i2 = i1 ^ par;
+  for (int m0 = 0; m0 <= M; m0 += 8) {
+    const int m = m0 + rr;
+    double acc[NT][2];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      acc[j][0] = acc[j][1] = 0.;
+    }
+    for (int k0 = 0; avg_any && k0 < nrow; k0 += 4 * CB) {
+      double a[CB];
+#pragma unroll
+      for (int b = 0; b < CB; ++b) {
+        const int jr = k0 + 4 * b + q;
+        a[b] = (m <= M && jr < nrow) ? C[(int64_t)(2 * jr + par) * (M + 1) + m] : 0.;
+      }
+#pragma unroll
+      for (int b = 0; b < CB; ++b) {
+        if (k0 + 4 * b < nrow) {
+          const double *sb = S + (k0 + 4 * b + q) * LD + rr;
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            dmma(acc[j][0], acc[j][1], a[b], sb[8 * j]);
+          }
+        }
+      }
+    }
+    if (m > M || (m == 0 && i1 != i2)) {
       continue;
     }
-    const double *p = coeffs + (int64_t)G.coef_set * ncoef;
-    const int nN = 2 * M + 1;
-    const int Nlo = abs(n1 - n2);
-    const double *C = cg + cg_off[(n1 - 1) * cg_nmax + (n2 - 1)];
-    // per matrix k: t00, t11, t01, t10 [M + 1] and S [2 (2M + 1)] at tv + k wcap
-    const int o11 = M + 1, o01 = 2 * (M + 1), o10 = 3 * (M + 1), oS = 4 * (M + 1);
-    for (int m1 = lane; m1 <= M; m1 += 32) {
-      // f(m1) (-1)^m1 is a power of two with a sign: the product is exact
-      const double f = ((m1 == 0) ? 1. : 2.) * ((m1 & 1) ? -1. : 1.);
+    const double ms = (m & 1) ? -1. : 1.;
 #pragma unroll
-      for (int k = 0; k < NMAT; ++k) {
-        const cplx *Tg = mats.src[k] + G.t_off;
-        cplx *t = tv + k * wcap;
-        t[m1] = cscale(Tg[telem(N, m1, 0, n1, 0, n2)], f);
-        t[o11 + m1] = cscale(Tg[telem(N, m1, 1, n1, 1, n2)], f);
-        t[o01 + m1] = cscale(Tg[telem(N, m1, 0, n1, 1, n2)], f);
-        t[o10 + m1] = cscale(Tg[telem(N, m1, 1, n1, 0, n2)], f);
+    for (int j = 0; j < NT; ++j) {
+      if (gN[j] > 0) {
+        const cplx v = (gset[j] >= 0)
+                           ? mkc(ms * acc[j][0], ms * acc[j][1])
+                           : *reinterpret_cast<const cplx *>(t + m * LD + 8 * j + 2 * q);
+        const int64_t o = fold ? goff[j] / 2 + celem(gN[j], m, i1, n1, i2, n2)
+                               : goff[j] + telem(gN[j], m, i1, n1, i2, n2);
+        dst[o] = c_fold(n2, nfold, afold, v);
       }
     }
-    __syncwarp();
-    // pass 1: S(N') for the two sub-blocks of its parity
-    for (int j = lane; j < nN; j += 32) {
-      const double *Cr = C + (int64_t)j * (M + 1);
-      const int oa = (j & 1) ? o01 : 0;
-      const int ob = (j & 1) ? o10 : o11;
-      cplx sa[NMAT], sb[NMAT];
-#pragma unroll
-      for (int k = 0; k < NMAT; ++k) {
-        sa[k] = sb[k] = mkc(0., 0.);
-      }
-      for (int m1 = 0; m1 <= M; ++m1) {
-        const double c = Cr[m1];
-#pragma unroll
-        for (int k = 0; k < NMAT; ++k) {
-          cfma(sa[k], tv[k * wcap + oa + m1], c);
-          cfma(sb[k], tv[k * wcap + ob + m1], c);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < NMAT; ++k) {
-        tv[k * wcap + oS + 2 * j] = sa[k];
-        tv[k * wcap + oS + 2 * j + 1] = sb[k];
-      }
-    }
-    __syncwarp();
-    // pass 2: Ta_m = sum_N' p_N' (-1)^m CG(m) S(N')
-    for (int m = lane; m <= M; m += 32) {
-      cplx e00[NMAT], e11[NMAT], e01[NMAT], e10[NMAT];
-#pragma unroll
-      for (int k = 0; k < NMAT; ++k) {
-        e00[k] = e11[k] = e01[k] = e10[k] = mkc(0., 0.);
-      }
-      const double ms = (m & 1) ? -1. : 1.;
-      for (int j = 0; j < nN; j += 2) {
-        const double f = ms * p[Nlo + j] * C[(int64_t)j * (M + 1) + m];
-#pragma unroll
-        for (int k = 0; k < NMAT; ++k) {
-          cfma(e00[k], tv[k * wcap + oS + 2 * j], f);
-          cfma(e11[k], tv[k * wcap + oS + 2 * j + 1], f);
-        }
-      }
-      for (int j = 1; j < nN; j += 2) {
-        const double f = ms * p[Nlo + j] * C[(int64_t)j * (M + 1) + m];
-#pragma unroll
-        for (int k = 0; k < NMAT; ++k) {
-          cfma(e01[k], tv[k * wcap + oS + 2 * j], f);
-          cfma(e10[k], tv[k * wcap + oS + 2 * j + 1], f);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < NMAT; ++k) {
-        if (fold) {
-          cplx *Tag = mats.dst[k] + G.t_off / 2;
-          const bool same = ((n1 + n2) & 1) == 0;
-          const int64_t ea = celem(N, m, 0, n1, same ? 0 : 1, n2);
-          const int64_t eb = celem(N, m, 1, n1, same ? 1 : 0, n2);
-          if (ea >= 0) {
-            Tag[ea] = c_fold(n2, nfold, afold, same ? e00[k] : e01[k]);
-          }
-          if (eb >= 0) {
-            Tag[eb] = c_fold(n2, nfold, afold, same ? e11[k] : e10[k]);
-          }
-          continue;
-        }
-        cplx *Tag = mats.dst[k] + G.t_off;
-        Tag[telem(N, m, 0, n1, 0, n2)] = c_fold(n2, nfold, afold, e00[k]);
-        Tag[telem(N, m, 1, n1, 1, n2)] = c_fold(n2, nfold, afold, e11[k]);
-        Tag[telem(N, m, 0, n1, 1, n2)] = c_fold(n2, nfold, afold, e01[k]);
-        Tag[telem(N, m, 1, n1, 0, n2)] = c_fold(n2, nfold, afold, e10[k]);
-      }
-    }
-    __syncwarp();
   }
 }
 
@@ -447,15 +483,6 @@ __global__ void k_wigner_cols(const TmxAngle *__restrict__ angles, int nangles,
   const int m = (int)(u - (int64_t)a * (nmax + 1));
   const TmxAngle A = angles[a];
   wigner_col(A.c, A.s, A.si, nmax, m, pi + u * nmax, tau + u * nmax, 1);
-}
-
-// D += A B for one m8n8k4 FP64 tensor-core tile: lane l holds A[l / 4][l % 4],
-// B[l % 4][l / 4] and D[l / 4][2 (l % 4) + {0, 1}]
-__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, "
-      "{%0, %1};\n"
-      : "+d"(d0), "+d"(d1)
-      : "d"(a), "d"(b));
 }
 
 // parity class c of block m of order N: members (i = 0, n = f0 + 2 j), j <
@@ -871,45 +898,34 @@ void tmx_launch_cg(int nmax, const int64_t *cg_off, double *cg, double *work,
   k_cg<<<blocks, 128, 0, stream>>>(nmax, cg_off, cg, work);
 }
 
-void tmx_launch_orient_pairs(const TmxObsGrain *og, const int64_t *pstart,
-                             const int32_t *order, int pmax, int64_t npairs,
-                             const TmxMatSet &mats,
-                             int nmat, const double *coeffs, int ncoef,
-                             const int64_t *cg_off, const double *cg,
-                             int cg_nmax, int mmax, int fold,
-                             cudaStream_t stream) {
-  if (npairs <= 0) {
+template <int NT>
+static void launch_orient(const TmxObsGrain *og, const int32_t *order,
+                          const TmxOrientRange *rng, int nrng, int64_t nitems, int ncap,
+                          const TmxMatSet &mats, int nmat, const double *coeffs,
+                          int ncoef, const int64_t *cg_off, const double *cg,
+                          int cg_nmax, int fold, cudaStream_t stream) {
+  // t and S: rows of M + 1 <= ncap + 1 orders, padded to tiles
+  const int rows = ncap + 1;
+  const size_t smem = (size_t)4 * 2 * ((rows + 7) & ~7) * (8 * NT + 4) * sizeof(double);
+  cudaFuncSetAttribute(k_orient<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem);
+  k_orient<NT><<<dim3((unsigned)((nitems + 3) / 4), nmat), 128, smem, stream>>>(
+      og, order, rng, nrng, nitems, rows, mats, coeffs, ncoef, cg_off, cg, cg_nmax, fold);
+}
+
+void tmx_launch_orient(const TmxObsGrain *og, const int32_t *order,
+                       const TmxOrientRange *rng, int nrng, int64_t nitems, int ncap,
+                       int chunk, const TmxMatSet &mats, int nmat,
+                       const double *coeffs, int ncoef, const int64_t *cg_off,
+                       const double *cg, int cg_nmax, int fold, cudaStream_t stream) {
+  if (nitems <= 0) {
     return;
   }
-  const int wcap = 4 * (mmax + 1) + 2 * (2 * mmax + 1);
-  const size_t smem = (size_t)8 * wcap * nmat * sizeof(double2);
-  const int64_t want = (npairs + 7) / 8;
-  const int blocks = (int)std::min<int64_t>(want, 148 * 8);
-  if (nmat == 4 || nmat == 3) {
-    // four warps per CTA: the matrices' buffers of 8 warps would leave room
-    // for one CTA per SM
-    const size_t smem4 = (size_t)4 * wcap * nmat * sizeof(double2);
-    const int blocks4 = (int)std::min<int64_t>((npairs + 3) / 4, 148 * 16);
-    if (nmat == 4) {
-      cudaFuncSetAttribute(k_orient_pairs<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem4);
-      k_orient_pairs<4><<<blocks4, 128, smem4, stream>>>(og, pstart, order, pmax, npairs,
-                                                         mats, coeffs, ncoef, cg_off, cg,
-                                                         cg_nmax, wcap, fold);
-    } else {
-      cudaFuncSetAttribute(k_orient_pairs<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem4);
-      k_orient_pairs<3><<<blocks4, 128, smem4, stream>>>(og, pstart, order, pmax, npairs,
-                                                         mats, coeffs, ncoef, cg_off, cg,
-                                                         cg_nmax, wcap, fold);
-    }
-  } else {
-    cudaFuncSetAttribute(k_orient_pairs<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    k_orient_pairs<1><<<blocks, 256, smem, stream>>>(og, pstart, order, pmax, npairs,
-                                                     mats, coeffs, ncoef, cg_off, cg,
-                                                     cg_nmax, wcap, fold);
-  }
+  const auto run = [&](auto f) {
+    f(og, order, rng, nrng, nitems, ncap, mats, nmat, coeffs, ncoef, cg_off, cg, cg_nmax,
+      fold, stream);
+  };
+  run(chunk <= 2 ? launch_orient<1> : chunk <= 4 ? launch_orient<2> : launch_orient<4>);
 }
 
 void tmx_launch_wigner_cols(const TmxAngle *angles, int nangles, int nmax,

@@ -454,9 +454,8 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
   ++ctx->plan_seq;
   cudaStream_t st = ctx->stream;
   const int64_t n = (int64_t)og.size();
-  // orientation-average work items, pair-major (tmx_launch_orient_pairs):
-  // grains by descending order; pair (n1, n2) has one item per grain of
-  // order >= max(n1, n2)
+  // orientation-average work items (tmx_launch_orient): grains by descending
+  // order, so that those of order >= n are the first at_least[n]
   int nbmax = 1;
   for (int64_t g = 0; g < n; ++g) {
     nbmax = std::max(nbmax, og[g].nmax);
@@ -477,15 +476,31 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
   for (int k = nbmax; k >= 1; --k) {
     at_least[k] += at_least[k + 1];
   }
-  std::vector<int64_t> base((size_t)nbmax * nbmax + 1, 0);
-  int64_t npairs = 0;
-  for (int n1 = 1; n1 <= nbmax; ++n1) {
-    for (int n2 = 1; n2 <= nbmax; ++n2) {
-      base[(size_t)(n1 - 1) * nbmax + (n2 - 1)] = npairs;
-      npairs += at_least[std::max(n1, n2)];
+  // one launch per range of n = max(n1, n2), largest first: shared memory is
+  // sized by the range, and so is the chunk of grains per warp -- eight where
+  // their rows leave room for a dozen warps per SM (n < 32), four above, and
+  // no more than there are grains (idle columns cost as much as used ones)
+  std::vector<TmxOrientRange> orng;
+  ctx->o_orient.clear();
+  const int oedge[] = {TMX_MAX_NB, 63, 31, 15, 0}; // M + 1 rows in tiles of 8
+  for (int b = 0; b < 4; ++b) {
+    tmx_ctx::OrientLaunch la;
+    la.rng0 = (int)orng.size();
+    const int top = std::min(oedge[b], nbmax);
+    const int64_t most = (top > oedge[b + 1]) ? at_least[oedge[b + 1] + 1] : 0;
+    la.chunk = most <= 2 ? 2 : (most <= 4 || oedge[b] > 31) ? 4 : 8;
+    la.ncap = top;
+    for (int nn = top; nn > oedge[b + 1]; --nn) {
+      if (at_least[nn] > 0) {
+        orng.push_back({la.nitems, nn, (int32_t)at_least[nn]});
+        la.nitems += (2 * nn - 1) * ((at_least[nn] + la.chunk - 1) / la.chunk);
+      }
+    }
+    la.nrng = (int)orng.size() - la.rng0;
+    if (la.nitems > 0) {
+      ctx->o_orient.push_back(la);
     }
   }
-  base.back() = npairs;
   if ((rc0 = ensure(ctx, ctx->o_ord, std::max<size_t>(1, order.size()) * sizeof(int32_t)))) {
     return rc0;
   }
@@ -573,7 +588,7 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
     CK(cudaMemcpyAsync(buf.p, src, bytes, cudaMemcpyHostToDevice, st));
     return TMX_OK;
   };
-  if ((rc = put(ctx->o_pairs, base.data(), base.size() * sizeof(int64_t))) ||
+  if ((rc = put(ctx->o_orng, orng.data(), orng.size() * sizeof(TmxOrientRange))) ||
       (rc = put(ctx->o_grp, grp.data(), grp.size() * sizeof(TmxAmpGroup))) ||
       (rc = put(ctx->o_ins, plan.ins.data(), plan.ins.size() * sizeof(int32_t))) ||
       (rc = put(ctx->o_prs, plan.pairs.data(), plan.pairs.size() * sizeof(TmxAmpPair))) ||
@@ -581,9 +596,7 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
     return rc;
   }
   CK(cudaStreamSynchronize(st));
-  ctx->o_npairs = npairs;
   ctx->o_nbmax = nbmax;
-  ctx->o_pmax = nbmax;
   ctx->o_xcap = x_max;
   if (ctx->profiling) {
     // flops of one matrix set over the kernels' index spaces: the
@@ -597,7 +610,7 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
         for (int a = 1; a <= N; ++a) {
           for (int b = 1; b <= N; ++b) {
             const double M = std::min(a, b);
-            fo += 16. * (2. * M + 1.) * (M + 1.);
+            fo += 16. * (M + 1.) * (M + 1.);
           }
         }
       }
@@ -611,6 +624,19 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
     }
     ctx->o_fl_orient = fo;
     ctx->o_fl_amp = fa;
+  }
+  return TMX_OK;
+}
+
+// the plan's orientation launches on ctx->stream
+int launch_orient(tmx_ctx *ctx, const TmxMatSet &mats, int nmat, int ncoef, int fold) {
+  for (const tmx_ctx::OrientLaunch &la : ctx->o_orient) {
+    tmx_launch_orient((const TmxObsGrain *)ctx->o_og.p, (const int32_t *)ctx->o_ord.p,
+                      (const TmxOrientRange *)ctx->o_orng.p + la.rng0, la.nrng, la.nitems,
+                      la.ncap, la.chunk, mats, nmat, (const double *)ctx->o_coef.p, ncoef,
+                      (const int64_t *)ctx->cg_off.p, (const double *)ctx->cg.p,
+                      ctx->cg_nmax, fold, ctx->stream);
+    LAUNCHED();
   }
   return TMX_OK;
 }
@@ -633,7 +659,7 @@ int run_amplitudes(tmx_ctx *ctx, const cplx *const *Tsrc, int nmat,
     CK(cudaMemsetAsync(S_out[k], 0, std::max<int64_t>(0, s_total) * 4 * sizeof(cplx),
                        st));
   }
-  if (t_total <= 0 || ctx->o_npairs <= 0) {
+  if (t_total <= 0 || ctx->o_orient.empty()) {
     return TMX_OK;
   }
   TmxMatSet avg = {}, amp = {};
@@ -650,14 +676,9 @@ int run_amplitudes(tmx_ctx *ctx, const cplx *const *Tsrc, int nmat,
   if ((rc = prof_begin(ctx, TMX_PROF_ORIENT, &pe))) {
     return rc;
   }
-  tmx_launch_orient_pairs((const TmxObsGrain *)ctx->o_og.p,
-                          (const int64_t *)ctx->o_pairs.p, (const int32_t *)ctx->o_ord.p,
-                          ctx->o_pmax, ctx->o_npairs, avg, nmat,
-                          (const double *)ctx->o_coef.p,
-                          ncoef, (const int64_t *)ctx->cg_off.p,
-                          (const double *)ctx->cg.p, ctx->cg_nmax, ctx->o_nbmax, 1,
-                          st);
-  LAUNCHED();
+  if ((rc = launch_orient(ctx, avg, nmat, ncoef, 1))) {
+    return rc;
+  }
   // T-matrices in and averaged T-matrices (compact, half the size) out
   if ((rc = prof_end(ctx, TMX_PROF_ORIENT, pe, nmat * ctx->o_fl_orient, st,
                      1.5 * nmat * t_total * sizeof(cplx)))) {
@@ -1826,17 +1847,15 @@ extern "C" int tmx_batch_orientation_average(tmx_ctx *ctx, const double *coeffs,
   if ((rc = upload_obs_plan(ctx, og, AmpPlan(), {}))) {
     return rc;
   }
-  if (t_total > 0 && ctx->o_npairs > 0) {
+  if (t_total > 0 && !ctx->o_orient.empty()) {
     TmxMatSet avg = {};
     avg.src[0] = (const cplx *)ctx->T.p;
     avg.dst[0] = (cplx *)ctx->Ta.p;
-    tmx_launch_orient_pairs((const TmxObsGrain *)ctx->o_og.p,
-                            (const int64_t *)ctx->o_pairs.p,
-                            (const int32_t *)ctx->o_ord.p, ctx->o_pmax, ctx->o_npairs,
-                            avg, 1, (const double *)ctx->o_coef.p, ncoef,
-                            (const int64_t *)ctx->cg_off.p, (const double *)ctx->cg.p,
-                            ctx->cg_nmax, ctx->o_nbmax, 0, st);
-    LAUNCHED();
+    // (the entries between the parity classes stay zero)
+    CK(cudaMemsetAsync(ctx->Ta.p, 0, t_total * sizeof(cplx), st));
+    if ((rc = launch_orient(ctx, avg, 1, ncoef, 0))) {
+      return rc;
+    }
     std::swap(ctx->T, ctx->Ta);
   }
   CK(cudaStreamSynchronize(st));
