@@ -63,20 +63,6 @@ __device__ __forceinline__ void a_side_row(double j, double dj, double y,
   f[3 * ts] = mkc(an * (dd * dj + q * j), an * (dd * dy + q * y));
 }
 
-template <bool LEAN = false>
-__device__ __forceinline__ void a_side(const ClassDesc &D, int a, int N, int g,
-                                       const double *__restrict__ T,
-                                       const double *__restrict__ S,
-                                       const double *__restrict__ Wg, cplx *f,
-                                       int ts, int m = 1) {
-  int i, n;
-  member(D, a, i, n);
-  const double *t = T + ((int64_t)g * N + (n - 1)) * TMX_NQ;
-  const double *w = Wg + ((int64_t)g * N + (n - 1)) * 2;
-  a_side_row<LEAN>(t[TMX_Q_J], t[TMX_Q_DJ], t[TMX_Q_Y], t[TMX_Q_DY], w[0], w[1],
-                   S + (int64_t)g * TMX_NS, n, f, ts, m);
-}
-
 // B-side vectors of column member (ib, n) at one node for the rows of block
 // index ia, stored to wr[t * ts]. LEAN as for a_side.
 struct BSide {
@@ -138,22 +124,6 @@ __device__ __forceinline__ void b_side_row(const ClassDesc &D, int ib, int n,
   for (int rg = 0; rg < ngroups; ++rg) {
     b_side_terms<LEAN>(B, (rg == 0) ? D.iA : D.iB, ib, m, k2, k2mr, w + rg * gs, ts);
   }
-}
-
-template <bool LEAN = false>
-__device__ __forceinline__ void b_side(const ClassDesc &D, int b, int N, int m,
-                                       int g, int ngroups,
-                                       const double *__restrict__ T,
-                                       const double *__restrict__ S,
-                                       const double *__restrict__ Wg, double k2,
-                                       cplx k2mr, cplx *w, int ts, int gs) {
-  int ib, n;
-  member(D, b, ib, n);
-  const double *t = T + ((int64_t)g * N + (n - 1)) * TMX_NQ;
-  const double *wg = Wg + ((int64_t)g * N + (n - 1)) * 2;
-  b_side_row<LEAN>(D, ib, n, m, mkc(t[TMX_Q_JM_RE], t[TMX_Q_JM_IM]),
-                   mkc(t[TMX_Q_DJM_RE], t[TMX_Q_DJM_IM]), wg[0], wg[1],
-                   S + (int64_t)g * TMX_NS, ngroups, k2, k2mr, w, ts, gs);
 }
 
 // zero A-side / B-side entries (padding and nodes past ngauss)
@@ -305,6 +275,25 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
       : "d"(a), "d"(b));
 }
 
+// Complex products with their roundings spelled out (the compiler may contract
+// either product of a sum, and large elongated grains amplify the last bit of
+// a factor by many orders of magnitude): mul_xy fuses the x x and y x products,
+// mul_xx the x x and x y ones, mul_yx the y y and x y ones. Every kernel forms l = q / u
+// with mul_xx and updates with mul_xy, so that a class has the same factors and
+// the same T, bit for bit, whichever kernel runs it.
+__device__ __forceinline__ cplx mul_xy(cplx a, cplx b) {
+  return mkc(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
+             __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
+}
+__device__ __forceinline__ cplx mul_xx(cplx a, cplx b) {
+  return mkc(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
+             __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ cplx mul_yx(cplx a, cplx b) {
+  return mkc(__fma_rn(-a.y, b.y, __dmul_rn(a.x, b.x)),
+             __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
+
 // ------------------------------------------ LU and solves in registers --
 //
 // Row r of a class matrix lives in the registers of the C lanes
@@ -325,6 +314,31 @@ __device__ __forceinline__ void warp_argmax(unsigned long long key, int pos,
   const unsigned bal = __ballot_sync(0xffffffffu, top && (unsigned)pos == mp);
   best_pos = (int)mp;
   best_lane = __ffs(bal) - 1;
+}
+
+// Pivot of one elimination step over the lanes' candidates c (have: the lane has
+// one): the first position with the largest |c|, as warp_argmax finds it from
+// hypot. |c|^2 decides unless another candidate comes within rounding of the
+// largest one (or the squares leave the range of doubles): then the hypots do.
+// Returns whether the pivot is non-zero.
+__device__ __forceinline__ bool warp_pivot(cplx c, bool have, int pos, int &best_pos,
+                                           int &best_lane) {
+  double s = have ? fma(c.x, c.x, c.y * c.y) : 0.;
+  s = (s >= 0.) ? s : 0.; // (NaN is no candidate)
+  const unsigned long long top = 1ull << 63;
+  warp_argmax(have ? (unsigned long long)__double_as_longlong(s) | top : 0ull, pos,
+              best_pos, best_lane);
+  const double best = __shfl_sync(0xffffffffu, s, best_lane);
+  const bool close = have && s >= best * (1. - 0x1p-40);
+  const bool odd = __popc(__ballot_sync(0xffffffffu, close)) != 1;
+  if (odd || !(best > 0x1p-900 && best < 0x1p900)) {
+    double av = have ? cabs_dev(c) : 0.;
+    av = (av >= 0.) ? av : 0.;
+    warp_argmax(have ? (unsigned long long)__double_as_longlong(av) | top : 0ull, pos,
+                best_pos, best_lane);
+    return __shfl_sync(0xffffffffu, av, best_lane) > 0.;
+  }
+  return true;
 }
 
 // In-place LU with partial pivoting of the nb x nb matrix Q (row stride LD,
@@ -759,32 +773,53 @@ static void launch_warp_variant(const TmxBlockArgs &a, cudaStream_t stream) {
 
 // ------------------------------------------ four warps per item (<= 32) --
 //
-// Classes of 17..32 members: one CTA of four warps per item. The warps
-// build each chunk of TMX_WG32 nodes together (one barrier), warp w then
-// accumulates column tile w (columns 8w..8w+7) over all four row tiles on
-// the FP64 tensor pipe (as in k_blocks_warp's tensor path), and warp 0
-// factors and solves with one lane per row (no barriers inside the LU).
+// Classes of 17..32 members: one CTA of four warps per item.
+// Assembly: chunks of TMX_WG32 nodes; thread t builds padded row and column
+// t % 32 of node t / 32 from staged table rows (copied with cp.async while the
+// previous chunk is contracted), then the warps share the 8 x 8 tiles (rows
+// padded per group, so that a tile has one set of W) evenly on the FP64 tensor
+// pipe, K = (node, term) ascending.
+// LU: lane r of every warp holds row r of the columns w, w + 4, .. of its warp
+// w in registers. Per step the owner of the pivot column has put it into
+// shared memory; each warp finds the pivot itself (lanes in parallel: |q|,
+// 1 / q), takes the pivot row by shuffles and updates its columns, the owner
+// of the next column first: one barrier per step, no row exchanges.
+// Solve: four lanes per row, in registers.
+// Measured (B200): 80 items of 17..20 members alone on the chip 61 -> 40 us, 3018
+// items of 17..32 members, 32..100 nodes, 0.74 -> 0.62 ms, against table rows
+// loaded in the build, tiles split by column and the LU on warp 0. Bound by
+// latency at 12 warps per SM (issue slots 42 %, FP64 and DMMA pipes together
+// 52 % busy). 166 registers and three CTAs: at 128 registers (four CTAs) the
+// contraction spills, 49 us and 0.61 ms; eight warps per item 35 us and 0.68 ms.
 
 #define TMX_WG32 4
 
-__host__ __device__ constexpr int cta32_elems() {
-  // F[WG][4][32] + W[2][WG][4][32], or Q, RgQ [32][33], 1/U_jj, indices
-  return (12 * TMX_WG32 * 32 > 2 * 32 * 33 + 3 * 32) ? 12 * TMX_WG32 * 32
-                                                      : 2 * 32 * 33 + 3 * 32;
-}
+struct Cta32 {
+  static constexpr int NBM = 32, LD = NBM + 1, LDK = NBM + 2;
+  // F[4 WG][LDK], W[2][4 WG][LDK] (rows padded by two: the four terms and two
+  // members that eight lanes read fall into distinct banks), then the staged
+  // rows; or Q, RgQ [32][33] and 1 / U_jj
+  static constexpr int CHUNK = 12 * TMX_WG32 * LDK;
+  static constexpr int STAGE = TMX_WG32 * (NBM * TMX_ROW + TMX_NS) / 2;
+  static constexpr int SOLVE = 2 * NBM * LD + NBM;
+  static constexpr int ELEMS = CHUNK + STAGE > SOLVE ? CHUNK + STAGE : SOLVE;
+};
 
-__global__ void __launch_bounds__(128, 4) k_blocks_cta32(TmxBlockArgs A) {
-  constexpr int NBM = 32;
-  constexpr int LD = NBM + 1;
+__global__ void __launch_bounds__(128, 3) k_blocks_cta32(TmxBlockArgs A) {
+  constexpr int NBM = Cta32::NBM, LD = Cta32::LD, LDK = Cta32::LDK, WG = TMX_WG32;
+  constexpr int NTILE = 4; // tiles per warp
   extern __shared__ __align__(16) unsigned char tmx_c32smem[];
+  __shared__ cplx colbuf[2][NBM];
+  __shared__ int at[NBM];      // row at a position
+  __shared__ double an_s[NBM]; // a_n of the members
   cplx *base = reinterpret_cast<cplx *>(tmx_c32smem);
-  cplx *Fs = base;                   // [WG][4][NBM]
-  cplx *Ws = Fs + TMX_WG32 * 4 * NBM; // [2][WG][4][NBM]
-  cplx *Qm = base;                   // [NBM][LD]  (after the assembly)
-  cplx *Rm = Qm + NBM * LD;          // [NBM][LD]
-  cplx *uinv = Rm + NBM * LD;        // [NBM]
-  int *perm = reinterpret_cast<int *>(uinv + NBM); // [NBM]
-  int *piv = perm + NBM;                           // [NBM]
+  cplx *Fs = base;
+  cplx *Ws = Fs + 4 * WG * LDK;
+  double *stg = reinterpret_cast<double *>(base + Cta32::CHUNK);
+  const double *stgS = stg + WG * NBM * TMX_ROW;
+  cplx *Qm = base; // (after the assembly)
+  cplx *Rm = Qm + NBM * LD;
+  cplx *uinv = Rm + NBM * LD;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int wib = tid >> 5;
@@ -795,233 +830,356 @@ __global__ void __launch_bounds__(128, 4) k_blocks_cta32(TmxBlockArgs A) {
   for (int it = ilo + blockIdx.x; it < ihi; it += gridDim.x) {
     const TmxItem item = A.items[it];
     const TmxSlot sl = A.slots[item.slot];
-    const TmxGrain Gr = A.grains[sl.grain];
     const int N = sl.nmax;
     const int ng = sl.ngauss;
     const int m = item.m;
-    const ClassDesc D = describe<1>(N, m, item.cls);
+    const ClassDesc D = describe<8>(N, m, item.cls);
     const int nb = D.nb;
     if (nb <= 0) {
       continue;
     }
-    if (nb > NBM) {
+    if (nb > NBM || D.NRp > NBM) {
       if (tid == 0) {
         atomicOr(&A.status[sl.grain], TMX_ST_TOO_LARGE);
       }
       continue;
     }
+    const TmxGrain Gr = A.grains[sl.grain];
     const double *T = A.tab + sl.tab;
     const double *S = A.nsc + sl.nsc;
     const double *Wg = A.wig + A.wig_off[sl.wig_n] + (int64_t)m * ng * N * 2;
     const double k2 = Gr.k * Gr.k;
     const cplx k2mr = mkc(Gr.mr * k2, Gr.mi * k2);
     const int ngroups = (D.R1 > 0 && m > 0) ? 2 : 1;
-    const int nrt = (nb + 7) >> 3;
-    const int col = wib * 8 + rr; // B-fragment column of this lane
-    double acc[4][4][2];
+    const int nt = (m == 0) ? 2 : 4; // terms per node
+    // this thread's 16-byte pieces of a node's rows (5 per member)
+    const double *src[2];
+    int stride[2], dst[2];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int j = 0; j < 2; ++j) {
+      const int p = tid + 128 * j;
+      const int a = p / 5, piece = p - 5 * a;
+      int ia, n;
+      member(D, a, ia, n);
+      const bool have = a < nb;
+      n = have ? n : 1;
+      src[j] = (piece < 4) ? T + (int64_t)(n - 1) * TMX_NQ + 2 * piece
+                           : Wg + (int64_t)(n - 1) * 2;
+      stride[j] = (piece < 4) ? N * TMX_NQ : 2 * N;
+      dst[j] = have ? a * TMX_ROW + 2 * piece : -1;
+    }
+    const auto issue = [&](int g0) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (dst[j] >= 0) {
+          const double *sp = src[j] + (int64_t)g0 * stride[j];
+#pragma unroll
+          for (int gl = 0; gl < WG; ++gl) {
+            if (g0 + gl < ng) {
+              cp16(stg + gl * NBM * TMX_ROW + dst[j], sp);
+            }
+            sp += stride[j];
+          }
+        }
+      }
+      if (tid < WG * (TMX_NS / 2) && g0 + tid / (TMX_NS / 2) < ng) {
+        cp16(stg + WG * NBM * TMX_ROW + 2 * tid, S + (int64_t)g0 * TMX_NS + 2 * tid);
+      }
+      cp_commit();
+    };
+    issue(0);
+    // this thread's padded row and its column of node gl
+    const int gl = wib;
+    const int ra = (lane < D.NRp) ? padded_member(D, lane) : -1;
+    const bool wcol = (lane & ~7) < nb;
+    int ri, rn, ci, cn;
+    member(D, max(ra, 0), ri, rn);
+    member(D, lane, ci, cn);
+    if (tid < nb) {
+      an_s[tid] = a_n(cn);
+    }
+    // this warp's tiles
+    const int nct = (nb + 7) >> 3;
+    const int ntl = (D.NRp >> 3) * nct;
+    int fo[NTILE], wo[NTILE];
+    double acc[NTILE][4][2];
+#pragma unroll
+    for (int i = 0; i < NTILE; ++i) {
+      const int t = wib + 4 * i;
+      const int row = (t / nct) * 8;
+      fo[i] = q * LDK + row + rr;
+      wo[i] = ((row < D.R0p ? 0 : 4 * WG) + q) * LDK + (t % nct) * 8 + rr;
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
-        acc[r][p][0] = acc[r][p][1] = 0.;
+        acc[i][p][0] = acc[i][p][1] = 0.;
       }
     }
-    for (int g0 = 0; g0 < ng; g0 += TMX_WG32) {
-      __syncthreads();
-      for (int u = tid; u < TMX_WG32 * nb; u += 128) {
-        const int gl = u / nb;
-        const int a = u - gl * nb;
-        cplx *fp = Fs + gl * 4 * NBM + a;
-        cplx *wp = Ws + gl * 4 * NBM + a;
-        if (g0 + gl < ng) {
-          a_side<true>(D, a, N, g0 + gl, T, S, Wg, fp, NBM, m);
-          b_side<true>(D, a, N, m, g0 + gl, ngroups, T, S, Wg, k2, k2mr, wp, NBM,
-                       TMX_WG32 * 4 * NBM);
+    for (int g0 = 0; g0 < ng; g0 += WG) {
+      cp_wait_all();
+      __syncthreads(); // the chunk's rows are there; F and W are free
+      const bool live = g0 + gl < ng;
+      const double *ns = stgS + gl * TMX_NS;
+      if (lane < D.NRp) {
+        cplx v[4] = {mkc(0., 0.), mkc(0., 0.), mkc(0., 0.), mkc(0., 0.)};
+        if (live && ra >= 0) {
+          const double *r = stg + (gl * NBM + ra) * TMX_ROW;
+          const double2 jd = *reinterpret_cast<const double2 *>(r + TMX_Q_J);
+          const double2 yd = *reinterpret_cast<const double2 *>(r + TMX_Q_Y);
+          const double2 wd = *reinterpret_cast<const double2 *>(r + TMX_NQ);
+          a_side_row<true>(jd.x, jd.y, yd.x, yd.y, wd.x, wd.y, ns, rn, v, 1, m);
+        }
+        cplx *o = Fs + gl * nt * LDK + lane;
+        if (m == 0) {
+          o[0] = v[1];
+          o[LDK] = v[3];
         } else {
-          zero_side(fp, NBM, 4);
-          for (int g = 0; g < ngroups; ++g) {
-            zero_side(wp + g * TMX_WG32 * 4 * NBM, NBM, 4);
+          o[0] = v[0];
+          o[LDK] = v[1];
+          o[2 * LDK] = v[2];
+          o[3 * LDK] = v[3];
+        }
+      }
+      if (wcol) {
+        BSide B = {};
+        const bool have = live && lane < nb;
+        if (have) {
+          const double *r = stg + (gl * NBM + lane) * TMX_ROW;
+          const double2 jm = *reinterpret_cast<const double2 *>(r + TMX_Q_JM_RE);
+          const double2 djm = *reinterpret_cast<const double2 *>(r + TMX_Q_DJM_RE);
+          const double2 wd = *reinterpret_cast<const double2 *>(r + TMX_NQ);
+          B = b_side_node<true>(cn, m, jm, djm, wd.x, wd.y, ns);
+        }
+        for (int g = 0; g < ngroups; ++g) {
+          cplx v[4] = {mkc(0., 0.), mkc(0., 0.), mkc(0., 0.), mkc(0., 0.)};
+          if (have) {
+            b_side_terms<true>(B, (g == 0) ? D.iA : D.iB, ci, m, k2, k2mr, v, 1);
+          }
+          cplx *o = Ws + (g * 4 * WG + gl * nt) * LDK + lane;
+          if (m == 0) {
+            o[0] = v[1];
+            o[LDK] = v[3];
+          } else {
+            o[0] = v[0];
+            o[LDK] = v[1];
+            o[2 * LDK] = v[2];
+            o[3 * LDK] = v[3];
           }
         }
       }
       __syncthreads();
-      if (wib * 8 < nb) {
-        const int gmax = min(TMX_WG32, ng - g0);
-        const int nsl = (m == 0) ? (gmax + 1) >> 1 : gmax;
-        for (int sx = 0; sx < nsl; ++sx) {
-          const int gl = (m == 0) ? 2 * sx + (q >> 1) : sx;
-          const int t = (m == 0) ? 1 + 2 * (q & 1) : q;
-          cplx w[2];
+      if (g0 + WG < ng) {
+        issue(g0 + WG);
+      }
+      const int kmax = min(WG, ng - g0) * nt;
+      for (int k0 = 0; k0 < kmax; k0 += 4) {
 #pragma unroll
-          for (int g = 0; g < 2; ++g) {
-            w[g] = (col < nb && g < ngroups)
-                       ? Ws[((g * TMX_WG32 + gl) * 4 + t) * NBM + col]
-                       : mkc(0., 0.);
-          }
-#pragma unroll
-          for (int rti = 0; rti < 4; ++rti) {
-            if (rti < nrt) {
-              const int row = rti * 8 + rr;
-              const cplx f = (row < nb) ? Fs[(gl * 4 + t) * NBM + row] : mkc(0., 0.);
-              const int grp = (row < D.R0) ? 0 : 1;
-              const int lo = rti * 8, hi = min(rti * 8 + 8, nb);
-#pragma unroll
-              for (int g = 0; g < 2; ++g) {
-                const bool present = (g == 0) ? (lo < D.R0) : (ngroups == 2 && hi > D.R0);
-                if (present) {
-                  const double fj = (grp == g) ? f.x : 0.;
-                  const double fy = (grp == g) ? f.y : 0.;
-                  double *a4 = &acc[rti][0][0];
-                  dmma(a4[0], a4[1], fj, w[g].x);
-                  dmma(a4[2], a4[3], fj, w[g].y);
-                  dmma(a4[4], a4[5], fy, w[g].x);
-                  dmma(a4[6], a4[7], fy, w[g].y);
-                }
-              }
-            }
+        for (int i = 0; i < NTILE; ++i) {
+          if (wib + 4 * i < ntl) {
+            const cplx f = Fs[fo[i] + k0 * LDK];
+            const cplx w = Ws[wo[i] + k0 * LDK];
+            dmma(acc[i][0][0], acc[i][0][1], f.x, w.x); // jr
+            dmma(acc[i][1][0], acc[i][1][1], f.x, w.y); // ji
+            dmma(acc[i][2][0], acc[i][2][1], f.y, w.x); // yr
+            dmma(acc[i][3][0], acc[i][3][1], f.y, w.y); // yi
           }
         }
       }
-    }
-    // a_n of each member once per item (in the 1/U_jj slots, free until the
-    // LU)
-    double *an_s = reinterpret_cast<double *>(uinv);
-    if (tid < nb) {
-      int ia, na;
-      member(D, tid, ia, na);
-      an_s[tid] = a_n(na);
     }
     __syncthreads();
     // Q = G^j + i G^y, RgQ = G^j (times a_n1 a_n2), into the chunk buffers
 #pragma unroll
-    for (int rti = 0; rti < 4; ++rti) {
+    for (int i = 0; i < NTILE; ++i) {
+      const int t = wib + 4 * i;
+      const int a = (t < ntl) ? padded_member(D, (t / nct) * 8 + rr) : -1;
+      if (a >= 0) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int a = rti * 8 + rr;
-        const int b = wib * 8 + 2 * q + i;
-        if (a < nb && b < nb) {
-          const double sc = an_s[a] * an_s[b];
-          const double jr = acc[rti][0][i], ji = acc[rti][1][i];
-          const double yr = acc[rti][2][i], yi = acc[rti][3][i];
-          Qm[a * LD + b] = mkc((jr - yi) * sc, (ji + yr) * sc);
-          Rm[a * LD + b] = mkc(jr * sc, ji * sc);
+        for (int e = 0; e < 2; ++e) {
+          const int b = (t % nct) * 8 + 2 * q + e;
+          if (b < nb) {
+            const double sc = an_s[a] * an_s[b];
+            const double jr = acc[i][0][e], ji = acc[i][1][e];
+            const double yr = acc[i][2][e], yi = acc[i][3][e];
+            Qm[a * LD + b] = mkc((jr - yi) * sc, (ji + yr) * sc);
+            Rm[a * LD + b] = mkc(jr * sc, ji * sc);
+          }
         }
       }
     }
-    // every warp's column tiles of Q are in place before warp 0 factors
     __syncthreads();
+    // ---------------------------------------------------------------- LU
+    cplx x[NBM / 4]; // row `lane`, columns wib + 4 t
+    bool singular = false;
+    int pos = lane;
+#pragma unroll
+    for (int t = 0; t < NBM / 4; ++t) {
+      const int k = wib + 4 * t;
+      x[t] = (lane < nb && k < nb) ? Qm[lane * LD + k] : mkc(0., 0.);
+    }
     if (wib == 0) {
-      // LU in place in Qm, lane r updates row r
-      bool singular = false;
-      for (int i = 0; i < nb; ++i) {
-        double best = (lane >= i && lane < nb) ? cabs_dev(Qm[lane * LD + i]) : -1.;
-        int bi = lane;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-          if (ov > best || (ov == best && oi < bi)) {
-            best = ov;
-            bi = oi;
-          }
-        }
-        singular = singular || !(best > 0.);
-        if (lane == 0) {
-          piv[i] = bi;
-        }
-        if (bi != i) {
-          for (int k = lane; k < nb; k += 32) {
-            const cplx t = Qm[i * LD + k];
-            Qm[i * LD + k] = Qm[bi * LD + k];
-            Qm[bi * LD + k] = t;
-          }
-        }
-        __syncwarp();
-        if (lane > i && lane < nb) {
-          const cplx pinv = cinv_lu(Qm[i * LD + i]);
-          const cplx l = cmul(Qm[lane * LD + i], pinv);
-          Qm[lane * LD + i] = l;
-          // four entries at a time: all loads before the stores (the pivot
-          // row is only read in this step), so the updates overlap
-          cplx *qr = Qm + lane * LD;
-          const cplx *pr = Qm + i * LD;
-          int k = i + 1;
-          for (; k + 3 < nb; k += 4) {
-            cplx a0 = qr[k], a1 = qr[k + 1], a2 = qr[k + 2], a3 = qr[k + 3];
-            const cplx b0 = pr[k], b1 = pr[k + 1], b2 = pr[k + 2], b3 = pr[k + 3];
-            a0 = csub(a0, cmul(l, b0));
-            a1 = csub(a1, cmul(l, b1));
-            a2 = csub(a2, cmul(l, b2));
-            a3 = csub(a3, cmul(l, b3));
-            qr[k] = a0;
-            qr[k + 1] = a1;
-            qr[k + 2] = a2;
-            qr[k + 3] = a3;
-          }
-          for (; k < nb; ++k) {
-            qr[k] = csub(qr[k], cmul(l, pr[k]));
-          }
-        }
-        __syncwarp();
-      }
-      if (lane < nb) {
-        uinv[lane] = cinv_lu(Qm[lane * LD + lane]);
-      }
-      if (lane == 0) {
-        // column exchanges of Matrix::plu_inverse step 4, as a gather index
-        for (int j = 0; j < nb; ++j) {
-          perm[j] = j;
-        }
-        for (int j = nb - 1; j >= 0; --j) {
-          const int p = piv[j];
-          const int t = perm[j];
-          perm[j] = perm[p];
-          perm[p] = t;
-        }
-        if (singular) {
-          atomicOr(&A.status[sl.grain], TMX_ST_SINGULAR);
-        }
-      }
+      colbuf[0][lane] = x[0];
     }
     __syncthreads();
-    // solve T_c Q_c = -RgQ_c: four lanes per row, row 8 w + lane / 4
-    solve_rows<NBM, 4>(Rm, Qm, LD, uinv, nb, wib * 8 + (lane >> 2), lane & 3);
+    for (int i = 0; i < nb; ++i) {
+      const cplx c = colbuf[i & 1][lane];
+      cplx pinv = cinv_lu(c);
+      int bi, wl;
+      singular = !warp_pivot(c, lane < nb && pos >= i, pos, bi, wl) || singular;
+      pinv.x = __shfl_sync(0xffffffffu, pinv.x, wl);
+      pinv.y = __shfl_sync(0xffffffffu, pinv.y, wl);
+      // the row that was at position i takes the pivot's old position
+      if (lane == wl) {
+        pos = i;
+      } else if (pos == i) {
+        pos = bi;
+      }
+      const bool elim = lane < nb && pos > i;
+      const cplx l = mul_xx(c, pinv);
+      // columns in two halves; within a live half all are computed (and the
+      // finished ones left alone), so that their shuffles and products overlap
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (wib + 4 * (4 * h + 3) >= i) {
+          cplx u[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            u[t].x = __shfl_sync(0xffffffffu, x[4 * h + t].x, wl);
+            u[t].y = __shfl_sync(0xffffffffu, x[4 * h + t].y, wl);
+          }
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const int k = wib + 4 * (4 * h + t);
+            cplx v = csub(x[4 * h + t], mul_xy(l, u[t]));
+            v = (k == i) ? l : v;
+            if (elim && k >= i) {
+              x[4 * h + t] = v;
+            }
+            if (k == i + 1) {
+              colbuf[k & 1][lane] = x[4 * h + t];
+            }
+          }
+        }
+      }
+      __syncthreads();
+    }
+    // factors in position order
+    if (lane < nb) {
+#pragma unroll
+      for (int t = 0; t < NBM / 4; ++t) {
+        const int k = wib + 4 * t;
+        if (k < nb) {
+          Qm[pos * LD + k] = x[t];
+          if (k == pos) {
+            uinv[k] = cinv_lu(x[t]);
+          }
+        }
+      }
+      if (wib == 0) {
+        at[pos] = lane;
+      }
+    }
+    if (tid == 0 && singular) {
+      atomicOr(&A.status[sl.grain], TMX_ST_SINGULAR);
+    }
     __syncthreads();
     if (A.lu) {
+      // factors and the column gather index, for the tangent solves
       cplx *Ls = A.lu + item.scratch;
       for (int u = tid; u < nb * nb; u += 128) {
         Ls[u] = Qm[(u / nb) * LD + (u % nb)];
       }
       int *ps = reinterpret_cast<int *>(Ls + (int64_t)nb * nb);
-      for (int j = tid; j < nb; j += 128) {
-        ps[j] = perm[j];
-      }
-    }
-    // write out: T_c[a][b] = Y[a][perm[b]]
-    if (sl.tout < 0) {
       if (tid < nb) {
-        int ia, na;
-        member(D, tid, ia, na);
-        A.diag[sl.diag + ia * N + (na - 1)] = Rm[tid * LD + perm[tid]];
-      }
-    } else {
-      cplx *Tb = A.tout + sl.tout + block_offset(N, m);
-      const int w2 = 2 * D.nbb;
-      for (int u = tid; u < nb * nb; u += 128) {
-        const int a = u / nb;
-        const int b = u - a * nb;
-        int ia, na, ib, nbn;
-        member(D, a, ia, na);
-        member(D, b, ib, nbn);
-        Tb[(int64_t)(ia * D.nbb + (na - D.nmin)) * w2 + ib * D.nbb + (nbn - D.nmin)] =
-            Rm[a * LD + perm[b]];
+        ps[tid] = pos; // (warp 0: lane = row)
       }
     }
+    // ------------------------------------------ solve T_c Q_c = -RgQ_c
+    // four lanes per row: row a, columns c + 4 t in y[t]
+    const int a = tid >> 2, c = tid & 3;
+    const bool act = a < nb;
+    cplx y[NBM / 4];
+#pragma unroll
+    for (int t = 0; t < NBM / 4; ++t) {
+      const int k = c + 4 * t;
+      const cplx v = (act && k < nb) ? Rm[a * LD + k] : mkc(0., 0.);
+      y[t] = mkc(-v.x, -v.y);
+    }
+    // Z U = X (forward over columns)
+#pragma unroll
+    for (int tj = 0; tj < NBM / 4; ++tj) {
+      if (tj * 4 < nb) {
+        for (int cj = 0; cj < 4; ++cj) {
+          const int j = tj * 4 + cj;
+          if (j >= nb) {
+            break;
+          }
+          if (c == cj) {
+            // (column 0: see mul_yx)
+            y[tj] = (j == 0) ? mul_yx(y[tj], uinv[j]) : mul_xy(y[tj], uinv[j]);
+          }
+          cplx yj;
+          yj.x = __shfl_sync(0xffffffffu, y[tj].x, cj, 4);
+          yj.y = __shfl_sync(0xffffffffu, y[tj].y, cj, 4);
+#pragma unroll
+          for (int t = tj; t < NBM / 4; ++t) {
+            const int k = c + 4 * t;
+            if (k > j && k < nb) {
+              y[t] = csub(y[t], mul_xy(yj, Qm[j * LD + k]));
+            }
+          }
+        }
+      }
+    }
+    // Y L = Z (backward over columns, L unit lower)
+#pragma unroll
+    for (int tj = NBM / 4 - 1; tj >= 0; --tj) {
+      if (tj * 4 < nb) {
+        for (int cj = min(4, nb - tj * 4) - 1; cj >= 0; --cj) {
+          const int j = tj * 4 + cj;
+          cplx yj;
+          yj.x = __shfl_sync(0xffffffffu, y[tj].x, cj, 4);
+          yj.y = __shfl_sync(0xffffffffu, y[tj].y, cj, 4);
+#pragma unroll
+          for (int t = 0; t <= tj; ++t) {
+            const int k = c + 4 * t;
+            if (k < j) {
+              y[t] = csub(y[t], mul_xy(yj, Qm[j * LD + k]));
+            }
+          }
+        }
+      }
+    }
+    // write out: T_c[a][at[k]] = Y[a][k]
+    if (act) {
+      int ia, na;
+      member(D, a, ia, na);
+      if (sl.tout < 0) {
+#pragma unroll
+        for (int t = 0; t < NBM / 4; ++t) {
+          const int k = c + 4 * t;
+          if (k < nb && at[k] == a) {
+            A.diag[sl.diag + ia * N + (na - 1)] = y[t];
+          }
+        }
+      } else {
+        cplx *Tr = A.tout + sl.tout + block_offset(N, m) +
+                   (int64_t)(ia * D.nbb + (na - D.nmin)) * (2 * D.nbb);
+#pragma unroll
+        for (int t = 0; t < NBM / 4; ++t) {
+          const int k = c + 4 * t;
+          if (k < nb) {
+            int ib, nbn;
+            member(D, at[k], ib, nbn);
+            Tr[ib * D.nbb + (nbn - D.nmin)] = y[t];
+          }
+        }
+      }
+    }
+    __syncthreads(); // shared memory is reused by the next item
   }
 }
 
 static void launch_cta32(const TmxBlockArgs &a, cudaStream_t stream) {
-  const size_t smem = (size_t)cta32_elems() * sizeof(cplx);
+  const size_t smem = (size_t)Cta32::ELEMS * sizeof(cplx);
   cudaFuncSetAttribute(k_blocks_cta32, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)smem);
   // one item per CTA (see launch_warp_variant)
@@ -1267,25 +1425,6 @@ __global__ void __launch_bounds__(256, 3) k_assemble(TmxBlockArgs A, int rtiles,
     }
     __syncthreads(); // stage and chunk buffers are reused by the next tile
   }
-}
-
-// Complex products with their roundings spelled out (the compiler may contract
-// either product of a sum, and large elongated grains amplify the last bit of
-// a factor by many orders of magnitude): mul_xy fuses the x x and y x products,
-// mul_xx the x x and x y ones, mul_yx the y y and x y ones. They are the forms
-// that keep T-matrices the same, bit for bit, as those of one-CTA-per-item
-// kernels with compiler-chosen contractions.
-__device__ __forceinline__ cplx mul_xy(cplx a, cplx b) {
-  return mkc(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
-             __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
-}
-__device__ __forceinline__ cplx mul_xx(cplx a, cplx b) {
-  return mkc(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
-             __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
-}
-__device__ __forceinline__ cplx mul_yx(cplx a, cplx b) {
-  return mkc(__fma_rn(-a.y, b.y, __dmul_rn(a.x, b.x)),
-             __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
 
 // LU of Q_c, one item per CTA, in shared memory (in the scratch itself for
