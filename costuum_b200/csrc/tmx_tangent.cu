@@ -196,7 +196,7 @@ __device__ void build_chunk_tangent(const ClassDesc &D, const AsmLayout &L,
   }
 }
 
-// One block per (item, parameter).
+// One block per (item, parameter): classes above 32 members.
 template <int TR, int TC, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_tangent(TmxTangentArgs A, size_t smem_bytes) {
@@ -317,61 +317,6 @@ __global__ void __launch_bounds__(NT, MINB)
   __syncthreads();
 
   // ---------------------------------------- solve with the saved factors
-  if constexpr (NT == 128) {
-    // classes of up to 32 members: T_c and the factors in shared memory,
-    // B = dRgQ + T_c dQ by all threads, then the register solve with four
-    // lanes per row (row tid / 4)
-    constexpr int LF = 33;
-    if (nb <= 32) {
-      cplx *Am = reinterpret_cast<cplx *>(tmx_tsmem);
-      cplx *Tc = Am + 32 * LF;
-      cplx *Xs = Tc + 32 * LF;
-      cplx *uinv = Xs + 32 * LF;
-      int *perm = reinterpret_cast<int *>(uinv + 32);
-      const cplx *Ls = A.lu + item.scratch;
-      const int *ps = reinterpret_cast<const int *>(Ls + (int64_t)nb * nb);
-      const cplx *Tb = A.T + sl.tout + block_offset(N, m);
-      const int w2 = 2 * D.nbb;
-      for (int u = threadIdx.x; u < nb * nb; u += NT) {
-        const int a = u / nb;
-        const int k = u - a * nb;
-        Am[a * LF + k] = Ls[u];
-        int ia, na, ik, nk;
-        member(D, a, ia, na);
-        member(D, k, ik, nk);
-        Tc[a * LF + k] = Tb[(int64_t)(ia * D.nbb + (na - D.nmin)) * w2 + ik * D.nbb +
-                            (nk - D.nmin)];
-      }
-      for (int j = threadIdx.x; j < nb; j += NT) {
-        perm[j] = ps[j];
-        uinv[j] = cinv_lu(Ls[(int64_t)j * nb + j]);
-      }
-      __syncthreads();
-      for (int u = threadIdx.x; u < nb * nb; u += NT) {
-        const int a = u / nb;
-        const int b = u - a * nb;
-        cplx acc = dR[u];
-        for (int k = 0; k < nb; ++k) {
-          acc = cadd(acc, cmul(Tc[a * LF + k], dQ[(int64_t)k * nb + b]));
-        }
-        Xs[a * LF + b] = acc;
-      }
-      __syncthreads();
-      solve_rows<32, 4>(Xs, Am, LF, uinv, nb, threadIdx.x >> 2, threadIdx.x & 3);
-      __syncthreads();
-      cplx *dTb = A.dT + param * A.dT_stride + sl.tout + block_offset(N, m);
-      for (int u = threadIdx.x; u < nb * nb; u += NT) {
-        const int a = u / nb;
-        const int b = u - a * nb;
-        int ia, na, ib, nbn;
-        member(D, a, ia, na);
-        member(D, b, ib, nbn);
-        dTb[(int64_t)(ia * D.nbb + (na - D.nmin)) * w2 + ib * D.nbb + (nbn - D.nmin)] =
-            Xs[a * LF + perm[b]];
-      }
-      return;
-    }
-  }
   const int lda = nb | 1;
   cplx *Am = reinterpret_cast<cplx *>(tmx_tsmem);
   cplx *uinv = Am + (int64_t)nb * lda;
@@ -450,198 +395,404 @@ __global__ void __launch_bounds__(NT, MINB)
   }
 }
 
-// ------------------------------------------------- warp-per-item variant --
+// -------------------------------------- all three parameters of an item --
 //
-// (item, parameter) pairs of classes with at most 16 members: one warp each,
-// four per CTA, synchronised by __syncwarp only (as the forward warp kernel).
-// Assembly: lane (rt, ct) accumulates rows rt * TR.. and columns ct, ct + 4,
-// .. over chunks of TMX_TWG nodes. Solve: lane r forms row r of
-// X = -(dRgQ + T_c dQ) and runs both triangular solves with the saved
-// factors on it.
+// Classes of at most 32 members. With U = z dF/dz, V = z dW/dw (w = m z the
+// argument of the B side; every weight kept) and L = (d ln r^2 / dd) / 2:
+//   dW/dm = V + W'/m (W': the terms whose factor is m k^2, which are t = 0, 1
+//   for rows of block index 0 and t = 2, 3 for those of 1),
+//   dF/dR = U / R, dW/dR = (m / R) V,
+//   dF/dd = L U + e_F, dW/dd = L (m V + 2 W) + e_W (e: the d(r'/r)/dd terms).
+// So with V' = V + W'/m and U' = U - F' (F': F at the terms of W'),
+//   dQ/dm = sum F V' = A,  dQ/dR = (m A + B) / R with B = sum U' W,
+//   dQ/dd = sum F (L (m V' + 2 W) + e_W) + (L U' + e_F) W:
+// four products of four terms per node instead of the twenty terms of three
+// passes, and one build of F, U, W and V instead of three. The products run on
+// the FP64 tensor pipe, one 8 x 8 tile (three accumulator sets) per warp, one
+// item per CTA; rows are padded per row group, padding is neither cleared nor
+// written out. Then x = -(dRgQ + T_c dQ) and both triangular solves with the
+// saved factors, C lanes per (parameter, row). dQ/dR leaves out 2 Q / R of the
+// weights' R^2 and dRgQ the same of RgQ: they cancel in dRgQ + T dQ.
+// Bound by the FP64 pipe (about 2/3 products, 1/3 build) and by the barriers
+// of the chunks; 1024 grains of orders 4 to 20, four rounds: classes of at
+// most 8 0.70 ms (a warp per item and parameter, entries in registers: 1.67),
+// 9..16 0.92 ms (1.90), 17..32 0.73 ms (128 threads per item and parameter:
+// 1.58). Measured and not taken: 3 nodes per chunk for more CTAs per SM (0.79
+// and 0.96 ms), 4 lanes per row for classes of at most 8 (0.96 ms).
+// NC: largest class; NR: its padded rows; WG: nodes per chunk.
+template <int NC, int NR, int NTH, int WG>
+struct TangentTile {
+  static constexpr int LA = NR + 2, LB = NC + 2; // (bank-conflict-free fragments)
+  static constexpr int ROW = 10;                 // staged row: Bessel 8, Wigner 2
+  static constexpr int A_ELEMS = 12 * WG * LA, B_ELEMS = 24 * WG * LB;
+  static constexpr int STAGE = WG * (NC * ROW + TMX_NS); // doubles
+  static constexpr int LD = NC + 1, MAT = NC * LD;
+  static constexpr size_t CHUNK_BYTES =
+      (size_t)(A_ELEMS + B_ELEMS) * sizeof(cplx) + STAGE * sizeof(double);
+  static constexpr size_t SOLVE_BYTES = (size_t)7 * MAT * sizeof(cplx);
+  static constexpr size_t BYTES = CHUNK_BYTES > SOLVE_BYTES ? CHUNK_BYTES : SOLVE_BYTES;
+};
 
-#define TMX_TWG 2 // quadrature nodes per warp chunk
-
-template <int NBM>
-__host__ __device__ constexpr int tangent_warp_elems() {
-  // chunk buffers F[WG][8][NBM] + W[2][WG][8][NBM], or in the solve phase
-  // dQ, X, LU, T_c ([NBM][NBM + 1] each), 1/U_jj and the gather index
-  return (24 * TMX_TWG * NBM > 4 * NBM * (NBM + 1) + 2 * NBM)
-             ? 24 * TMX_TWG * NBM
-             : 4 * NBM * (NBM + 1) + 2 * NBM;
+__device__ __forceinline__ void tdmma(double *d, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, "
+      "{%0, %1};\n"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
 }
 
-template <int TR, int TC, int MINB>
-__global__ void __launch_bounds__(128, MINB)
-    k_tangent_warp(TmxTangentArgs A) {
-  constexpr int NBM = (8 * TR > 4 * TC) ? 8 * TR : 4 * TC;
-  constexpr int LD = NBM + 1;
-  extern __shared__ __align__(16) unsigned char tmx_twsmem[];
-  const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  cplx *base = reinterpret_cast<cplx *>(tmx_twsmem) + wib * tangent_warp_elems<NBM>();
-  cplx *Fs = base;                       // [WG][8][NBM]
-  cplx *Ws = Fs + 8 * TMX_TWG * NBM;     // [2][WG][8][NBM]
-  cplx *dQm = base;                      // [NBM][LD]  (after the assembly)
-  cplx *Xm = dQm + NBM * LD;             // [NBM][LD]
-  cplx *LUm = Xm + NBM * LD;             // [NBM][LD]
-  cplx *Tcm = LUm + NBM * LD;            // [NBM][LD]
-  cplx *uinv = Tcm + NBM * LD;           // [NBM]
-  int *perm = reinterpret_cast<int *>(uinv + NBM);
-  __shared__ double an_w[4][NBM];
-  double *an_tab = an_w[wib];
-  const int rt = lane >> 2;
-  const int ct = lane & 3;
-  const int64_t nwork = (int64_t)A.nitems * A.nparams;
-  for (int64_t w = (int64_t)blockIdx.x * 4 + wib; w < nwork;
-       w += (int64_t)gridDim.x * 4) {
-    const int it = (int)(w / A.nparams);
-    const int param = (int)(w % A.nparams);
-    const TmxItem item = A.items[it];
-    const TmxSlot sl = A.slots[item.slot];
-    const TmxGrain Gr = A.grains[sl.grain];
-    const int N = sl.nmax;
-    const int ng = sl.ngauss;
-    const int m = item.m;
-    const ClassDesc D = describe<TR>(N, m, item.cls);
-    const int nb = D.nb;
-    if (nb <= 0 || nb > NBM || D.NRp > NBM) {
-      continue;
+template <int NC, int NR, int NTH, int WG, int C, int MINB>
+__global__ void __launch_bounds__(NTH, MINB) k_tangent_tile(TmxTangentArgs A) {
+  using Z = TangentTile<NC, NR, NTH, WG>;
+  constexpr int LA = Z::LA, LB = Z::LB, LD = Z::LD, ROW = Z::ROW;
+  constexpr int NT = NC / C;
+  static_assert(NR / 8 * (NC / 8) <= NTH / 32 && 3 * NC <= NTH / C, "thread layout");
+  __shared__ double an_s[NC];
+  __shared__ cplx uinv[NC];
+  __shared__ int at[NC]; // class member of a solved column
+  cplx *As = reinterpret_cast<cplx *>(tmx_tsmem); // [F, U', Ud][WG][4][LA]
+  cplx *Bs = As + Z::A_ELEMS;                     // [group][V', W, Wd][WG][4][LB]
+  double *stg = reinterpret_cast<double *>(Bs + Z::B_ELEMS);
+  double *stgS = stg + WG * NC * ROW;
+  cplx *dQ = As;              // (after the assembly) [3][NC][LD]
+  cplx *dR = dQ + 3 * Z::MAT; // [3][NC][LD]
+  cplx *Tc = dR + 3 * Z::MAT; // [NC][LD]
+  cplx *LU = dQ;              // (after x)
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const int q = lane & 3;
+  const int rr = lane >> 2;
+  const TmxItem item = A.items[blockIdx.x];
+  const TmxSlot sl = A.slots[item.slot];
+  const int N = sl.nmax;
+  const int ng = sl.ngauss;
+  const int m = item.m;
+  const ClassDesc D = describe<8>(N, m, item.cls);
+  const int nb = D.nb;
+  if (nb <= 0 || nb > NC || D.NRp > NR) {
+    return;
+  }
+  const TmxGrain Gr = A.grains[sl.grain];
+  const double *T = A.tab + sl.tab;
+  const double *S = A.nsc + sl.nsc;
+  const double *Wg = A.wig + A.wig_off[sl.wig_n] + (int64_t)m * ng * N * 2;
+  const double k2 = Gr.k * Gr.k;
+  const cplx mc = mkc(Gr.mr, Gr.mi);
+  const cplx minv = cinv_lu(mc);
+  const cplx k2mr = mkc(Gr.mr * k2, Gr.mi * k2);
+  const int ngroups = (D.R1 > 0 && m > 0) ? 2 : 1;
+  const auto stage = [&](int g0) {
+    const int live = min(WG, ng - g0);
+    for (int u = tid; u < live * nb * 5; u += NTH) {
+      const int gl = u / (nb * 5);
+      const int v = u - gl * nb * 5;
+      const int a = v / 5, p = v - 5 * a;
+      int ia, n;
+      member(D, a, ia, n);
+      const int64_t o = (int64_t)(g0 + gl) * N + (n - 1);
+      const double *src = (p < 4) ? T + o * TMX_NQ + 2 * p : Wg + o * 2;
+      const unsigned dst =
+          (unsigned)__cvta_generic_to_shared(stg + (gl * NC + a) * ROW + 2 * p);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src)
+                   : "memory");
     }
-    const double *T = A.tab + sl.tab;
-    const double *S = A.nsc + sl.nsc;
-    const double *Wg = A.wig + A.wig_off[sl.wig_n] + (int64_t)m * ng * N * 2;
-    const double k2 = Gr.k * Gr.k;
-    const cplx k2mr = mkc(Gr.mr * k2, Gr.mi * k2);
-    AsmLayout L;
-    L.G = TMX_TWG;
-    L.NRp = NBM;
-    L.CT = 0;
-    L.ncol = NBM;
-    L.ngroups = (D.R1 > 0 && m > 0) ? 2 : 1;
-    const int tstep = (m == 0) ? 2 : 1;
-    const int t0 = (m == 0) ? 1 : 0;
-    const int per_node = (param == P_M) ? 4 : 8;
-    const int rgl = (rt * TR < D.R0p) ? 0 : 1;
-    __syncwarp();
-    if (lane < nb) {
-      int ia, na;
-      member(D, lane, ia, na);
-      an_tab[lane] = a_n(na);
+    for (int u = tid; u < live * (TMX_NS / 2); u += NTH) {
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(stgS + 2 * u);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst),
+                   "l"(S + (int64_t)g0 * TMX_NS + 2 * u)
+                   : "memory");
     }
-
-    // -------------------------------------------------- tangent assembly
-    double aj[TR][TC][2], ay[TR][TC][2];
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  stage(0);
+  if (tid < nb) {
+    int ia, n;
+    member(D, tid, ia, n);
+    an_s[tid] = a_n(n);
+  }
+  // this warp's tile
+  const int nct = (nb + 7) >> 3;
+  const int trow = (warp / nct) * 8, tcol = (warp % nct) * 8;
+  const bool tile = trow < D.NRp;
+  const cplx *fr = As + q * LA + trow + rr;
+  const cplx *wr = Bs + (trow < D.R0p ? 0 : Z::B_ELEMS / 2) + q * LB + tcol + rr;
+  double aA[4][2], aB[4][2], aD[4][2]; // (j re, j im, y re, y im)
 #pragma unroll
-    for (int r = 0; r < TR; ++r) {
+  for (int e = 0; e < 4; ++e) {
+    aA[e][0] = aA[e][1] = aB[e][0] = aB[e][1] = aD[e][0] = aD[e][1] = 0.;
+  }
+  for (int g0 = 0; g0 < ng; g0 += WG) {
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads(); // the chunk's rows are there; the fragments are free
+    const int live = min(WG, ng - g0);
+    const int nunit = live * nb;
+    for (int u = tid; u < nunit * (1 + ngroups); u += NTH) {
+      const int side = u / nunit; // 0: A side, 1, 2: B side of group 0, 1
+      const int v = u - side * nunit;
+      const int gl = v / nb;
+      const int a = v - gl * nb;
+      int ib, n;
+      member(D, a, ib, n);
+      const double *r = stg + (gl * NC + a) * ROW;
+      const double *s = stgS + gl * TMX_NS;
+      const double d = r[8], dd = r[9];
+      const double nn = n * (n + 1.);
+      const double z = s[TMX_NS_KR];
+      const double drr = s[TMX_NS_DRR], ddrr = s[TMX_NS_DDRR_DD];
+      const double L = 0.5 * s[TMX_NS_DLNR2_DD];
+      if (side == 0) {
+        const double iz = s[TMX_NS_KRINV];
+        const int row = (a < D.R0) ? a : D.R0p + a - D.R0;
+        cplx *o = As + gl * 4 * LA + row;
+        const double qd = nn * drr * d, qe = nn * ddrr * d * iz;
+        double F[2][4], U[2][4], E[2];
 #pragma unroll
-      for (int c = 0; c < TC; ++c) {
-        aj[r][c][0] = aj[r][c][1] = ay[r][c][0] = ay[r][c][1] = 0.;
+        for (int y = 0; y < 2; ++y) {
+          const double h = r[2 * y], dh = r[2 * y + 1];
+          const double hi = h * iz;
+          const double zh = z * dh - h;            // z h'
+          const double zdh = nn * hi - z * h - dh; // z (dh)'
+          F[y][0] = d * h;
+          F[y][1] = dd * h;
+          F[y][2] = d * dh;
+          F[y][3] = dd * dh + qd * hi;
+          U[y][0] = d * zh;
+          U[y][1] = dd * zh;
+          U[y][2] = d * zdh;
+          U[y][3] = dd * zdh + qd * (dh - 2. * hi);
+          E[y] = qe * h;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const bool mr = (t < 2) == (ib == 0);
+          const cplx f = mkc(F[0][t], F[1][t]);
+          const cplx g = mr ? mkc(U[0][t] - f.x, U[1][t] - f.y) : mkc(U[0][t], U[1][t]);
+          o[t * LA] = f;
+          o[(4 * WG + t) * LA] = g;
+          o[(8 * WG + t) * LA] = (t == 3) ? mkc(L * g.x + E[0], L * g.y + E[1])
+                                          : mkc(L * g.x, L * g.y);
+        }
+        continue;
+      }
+      const int ia = (side == 1) ? D.iA : D.iB;
+      const bool dg = ia == ib;
+      const cplx jm = mkc(r[4], r[5]), djm = mkc(r[6], r[7]);
+      const cplx iw = mkc(s[TMX_NS_KRMRINV_RE], s[TMX_NS_KRMRINV_IM]);
+      const cplx jw = cmul(jm, iw), djw = cmul(djm, iw), jw2 = cmul(jw, iw);
+      const cplx jp = csub(djm, jw);                           // j'
+      const cplx djp = csub(csub(cscale(jw2, nn), jm), djw);   // (dj)'
+      const cplx jwp = csub(djw, cscale(jw2, 2.));             // (j / w)'
+      const double qd = nn * drr * d;
+      const double wr2 = s[TMX_NS_W] * s[TMX_NS_R2];
+      const double beta = s[TMX_NS_SININV] * m * wr2;
+      const double wm = (double)(m * m) * s[TMX_NS_SIN2INV] * wr2;
+      const cplx c1 = (ia == 0) ? k2mr : mkc(k2, 0.);
+      const cplx c2 = (ia == 0) ? mkc(k2, 0.) : k2mr;
+      const cplx ch = dg ? c1 : mkc(-c1.y * beta, c1.x * beta);
+      const cplx cl = dg ? mkc(-c2.x, -c2.y) : mkc(-c2.y * beta, c2.x * beta);
+      // weights of the terms' G (in the order of the terms)
+      const double w0 = dg ? wm : 1., w1 = dg ? wr2 : 1.;
+      const cplx G1 = cscale(djm, d), G2 = cadd(cscale(djm, dd), cscale(jw, qd));
+      const cplx G3 = cscale(jm, d), G4 = cscale(jm, dd);
+      const cplx P1 = cscale(djp, z * d);
+      const cplx P2 = cadd(cscale(djp, z * dd), cscale(jwp, z * qd));
+      const cplx P3 = cscale(jp, z * d), P4 = cscale(jp, z * dd);
+      const cplx ex = cscale(jw, nn * d * ddrr); // of G2
+      cplx *o = Bs + (side == 1 ? 0 : Z::B_ELEMS / 2) + gl * 4 * LB + a;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const cplx g = dg ? (t == 0 ? G1 : t == 1 ? G2 : t == 2 ? G3 : G4)
+                          : (t == 0 ? G4 : t == 1 ? G3 : t == 2 ? G2 : G1);
+        const cplx pv = dg ? (t == 0 ? P1 : t == 1 ? P2 : t == 2 ? P3 : P4)
+                           : (t == 0 ? P4 : t == 1 ? P3 : t == 2 ? P2 : P1);
+        const cplx cw = cscale((t < 2) ? ch : cl, (t & 1) ? w1 : w0);
+        const cplx W = cmul(cw, g);
+        cplx V = cmul(cw, pv);
+        if ((t < 2) == (ia == 0)) {
+          V = cadd(V, cmul(W, minv));
+        }
+        const cplx mv = cmul(mc, V);
+        cplx X = mkc(L * (mv.x + 2. * W.x), L * (mv.y + 2. * W.y));
+        if (dg ? t == 1 : t == 2) {
+          X = cadd(X, cmul(cw, ex));
+        }
+        o[t * LB] = V;
+        o[(4 * WG + t) * LB] = W;
+        o[(8 * WG + t) * LB] = X;
       }
     }
-    for (int g0 = 0; g0 < ng; g0 += TMX_TWG) {
-      __syncwarp();
-      build_chunk_tangent(D, L, NBM, N, m, ng, g0, param, Gr.r_ev, T, S, Wg, k2,
-                          k2mr, Fs, Ws, lane, 32, an_tab);
-      __syncwarp();
-      const int gmax = min(TMX_TWG, ng - g0);
-      for (int gl = 0; gl < gmax; ++gl) {
-        for (int ts = t0; ts < per_node; ts += tstep) {
-          const int kk = 8 * gl + ts;
-          const cplx *fr = Fs + kk * NBM + rt * TR;
-          const cplx *wr = Ws + (rgl * 8 * TMX_TWG + kk) * NBM + ct;
-          cplx wv[TC];
+    __syncthreads();
+    if (g0 + WG < ng) {
+      stage(g0 + WG);
+    }
+    if (tile) {
+      for (int gl = 0; gl < live; ++gl) {
+        const cplx f = fr[gl * 4 * LA], u = fr[(4 * WG + gl * 4) * LA],
+                   e = fr[(8 * WG + gl * 4) * LA];
+        const cplx v = wr[gl * 4 * LB], w = wr[(4 * WG + gl * 4) * LB],
+                   x = wr[(8 * WG + gl * 4) * LB];
+        tdmma(aA[0], f.x, v.x);
+        tdmma(aA[1], f.x, v.y);
+        tdmma(aA[2], f.y, v.x);
+        tdmma(aA[3], f.y, v.y);
+        tdmma(aB[0], u.x, w.x);
+        tdmma(aB[1], u.x, w.y);
+        tdmma(aB[2], u.y, w.x);
+        tdmma(aB[3], u.y, w.y);
+        tdmma(aD[0], f.x, x.x);
+        tdmma(aD[1], f.x, x.y);
+        tdmma(aD[2], f.y, x.x);
+        tdmma(aD[3], f.y, x.y);
+        tdmma(aD[0], e.x, w.x);
+        tdmma(aD[1], e.x, w.y);
+        tdmma(aD[2], e.y, w.x);
+        tdmma(aD[3], e.y, w.y);
+      }
+    }
+  }
+  __syncthreads();
+  // dQ = dG^j + i dG^y, dRgQ = dG^j, by parameter
+  const int ra = tile ? padded_member(D, trow + rr) : -1;
+  if (ra >= 0) {
+    const double ri = 1. / Gr.r_ev;
 #pragma unroll
-          for (int c = 0; c < TC; ++c) {
-            wv[c] = wr[4 * c];
-          }
+    for (int e = 0; e < 2; ++e) {
+      const int b = tcol + 2 * q + e;
+      if (b < nb) {
+        const double sc = an_s[ra] * an_s[b];
+        const int o = ra * LD + b;
+        const cplx Rm = mkc(aA[0][e] * sc, aA[1][e] * sc);
+        const cplx Qm = mkc((aA[0][e] - aA[3][e]) * sc, (aA[1][e] + aA[2][e]) * sc);
+        const cplx Rb = mkc(aB[0][e] * sc, aB[1][e] * sc);
+        const cplx Qb = mkc((aB[0][e] - aB[3][e]) * sc, (aB[1][e] + aB[2][e]) * sc);
+        dR[P_M * Z::MAT + o] = Rm;
+        dQ[P_M * Z::MAT + o] = Qm;
+        dR[P_R * Z::MAT + o] = cscale(cadd(cmul(mc, Rm), Rb), ri);
+        dQ[P_R * Z::MAT + o] = cscale(cadd(cmul(mc, Qm), Qb), ri);
+        dR[P_D * Z::MAT + o] = mkc(aD[0][e] * sc, aD[1][e] * sc);
+        dQ[P_D * Z::MAT + o] =
+            mkc((aD[0][e] - aD[3][e]) * sc, (aD[1][e] + aD[2][e]) * sc);
+      }
+    }
+  }
+  // T_c (class order) of the forward solve, 1 / U_jj and the column order
+  const cplx *Ls = A.lu + item.scratch;
+  const int *ps = reinterpret_cast<const int *>(Ls + (int64_t)nb * nb);
+  const cplx *Tb = A.T + sl.tout + block_offset(N, m);
+  const int w2 = 2 * D.nbb;
+  for (int u = tid; u < nb * nb; u += NTH) {
+    const int a = u / nb;
+    const int k = u - a * nb;
+    int ia, na, ik, nk;
+    member(D, a, ia, na);
+    member(D, k, ik, nk);
+    Tc[a * LD + k] =
+        Tb[(int64_t)(ia * D.nbb + (na - D.nmin)) * w2 + ik * D.nbb + (nk - D.nmin)];
+  }
+  for (int j = tid; j < nb; j += NTH) {
+    at[ps[j]] = j;
+    uinv[j] = cinv_lu(Ls[(int64_t)j * nb + j]);
+  }
+  __syncthreads();
+  // x = -(dRgQ + T_c dQ) of row a of parameter p: columns c + C t in x[t]
+  const int c = tid % C;
+  const int p = (tid / C) / NC, a = (tid / C) % NC;
+  const bool act = p < A.nparams && p < 3 && a < nb;
+  cplx x[NT];
 #pragma unroll
-          for (int r = 0; r < TR; ++r) {
-            const cplx f = fr[r];
+  for (int t = 0; t < NT; ++t) {
+    const int k = c + C * t;
+    x[t] = (act && k < nb) ? dR[p * Z::MAT + a * LD + k] : mkc(0., 0.);
+  }
+  if (act) {
+    for (int k = 0; k < nb; ++k) {
+      const cplx tk = Tc[a * LD + k];
+      const cplx *qk = dQ + p * Z::MAT + k * LD + c;
 #pragma unroll
-            for (int c = 0; c < TC; ++c) {
-              aj[r][c][0] = fma(f.x, wv[c].x, aj[r][c][0]);
-              aj[r][c][1] = fma(f.x, wv[c].y, aj[r][c][1]);
-              ay[r][c][0] = fma(f.y, wv[c].x, ay[r][c][0]);
-              ay[r][c][1] = fma(f.y, wv[c].y, ay[r][c][1]);
-            }
+      for (int t = 0; t < NT; ++t) {
+        if (c + C * t < nb) {
+          const cplx v = qk[C * t];
+          x[t].x = fma(tk.x, v.x, fma(-tk.y, v.y, x[t].x));
+          x[t].y = fma(tk.x, v.y, fma(tk.y, v.x, x[t].y));
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    x[t] = mkc(-x[t].x, -x[t].y);
+  }
+  __syncthreads(); // dQ is free
+  for (int u = tid; u < nb * nb; u += NTH) {
+    LU[(u / nb) * LD + (u % nb)] = Ls[u];
+  }
+  __syncthreads();
+  // X U = x (forward over columns), then Y L = X (backward, L unit lower)
+#pragma unroll
+  for (int tj = 0; tj < NT; ++tj) {
+    if (tj * C < nb) {
+      for (int cj = 0; cj < C; ++cj) {
+        const int j = tj * C + cj;
+        if (j >= nb) {
+          break;
+        }
+        if (c == cj) {
+          x[tj] = cmul(x[tj], uinv[j]);
+        }
+        cplx xj;
+        xj.x = __shfl_sync(0xffffffffu, x[tj].x, cj, C);
+        xj.y = __shfl_sync(0xffffffffu, x[tj].y, cj, C);
+#pragma unroll
+        for (int t = tj; t < NT; ++t) {
+          const int k = c + C * t;
+          if (k > j && k < nb) {
+            x[t] = csub(x[t], cmul(xj, LU[j * LD + k]));
           }
         }
       }
     }
-    __syncwarp();
-    // dQ = dG^j + i dG^y into dQm, dRgQ = dG^j into Xm
+  }
 #pragma unroll
-    for (int r = 0; r < TR; ++r) {
-      const int a = padded_member(D, rt * TR + r);
+  for (int tj = NT - 1; tj >= 0; --tj) {
+    if (tj * C < nb) {
+      for (int cj = min(C, nb - tj * C) - 1; cj >= 0; --cj) {
+        const int j = tj * C + cj;
+        cplx xj;
+        xj.x = __shfl_sync(0xffffffffu, x[tj].x, cj, C);
+        xj.y = __shfl_sync(0xffffffffu, x[tj].y, cj, C);
 #pragma unroll
-      for (int c = 0; c < TC; ++c) {
-        const int b = ct + 4 * c;
-        if (a >= 0 && b < nb) {
-          dQm[a * LD + b] = mkc(aj[r][c][0] - ay[r][c][1], aj[r][c][1] + ay[r][c][0]);
-          Xm[a * LD + b] = mkc(aj[r][c][0], aj[r][c][1]);
+        for (int t = 0; t <= tj; ++t) {
+          const int k = c + C * t;
+          if (k < j) {
+            x[t] = csub(x[t], cmul(xj, LU[j * LD + k]));
+          }
         }
       }
     }
-    // saved factors, gather index and T_c (class order) of the forward solve
-    const cplx *Ls = A.lu + item.scratch;
-    const int *ps = reinterpret_cast<const int *>(Ls + (int64_t)nb * nb);
-    const cplx *Tb = A.T + sl.tout + block_offset(N, m);
-    const int w2 = 2 * D.nbb;
-    for (int u = lane; u < nb * nb; u += 32) {
-      const int a = u / nb;
-      const int k = u - a * nb;
-      LUm[a * LD + k] = Ls[u];
-      int ia, na, ik, nk;
-      member(D, a, ia, na);
-      member(D, k, ik, nk);
-      Tcm[a * LD + k] = Tb[(int64_t)(ia * D.nbb + (na - D.nmin)) * w2 + ik * D.nbb +
-                           (nk - D.nmin)];
-    }
-    for (int j = lane; j < nb; j += 32) {
-      perm[j] = ps[j];
-      uinv[j] = cinv_lu(Ls[(int64_t)j * nb + j]);
-    }
-    __syncwarp();
-    // ------------------- B = dRgQ + T_c dQ; the solve takes X = -B and
-    // solves X U = -B, then Y L = X
-    for (int u = lane; u < nb * nb; u += 32) {
-      const int a = u / nb;
-      const int b = u - a * nb;
-      cplx acc = Xm[a * LD + b];
-      for (int k = 0; k < nb; ++k) {
-        acc = cadd(acc, cmul(Tcm[a * LD + k], dQm[k * LD + b]));
+  }
+  if (act) {
+    int ia, na;
+    member(D, a, ia, na);
+    cplx *dTr = A.dT + p * A.dT_stride + sl.tout + block_offset(N, m) +
+                (int64_t)(ia * D.nbb + (na - D.nmin)) * w2;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const int k = c + C * t;
+      if (k < nb) {
+        int ib, nbn;
+        member(D, at[k], ib, nbn);
+        dTr[ib * D.nbb + (nbn - D.nmin)] = x[t];
       }
-      Xm[a * LD + b] = acc;
     }
-    __syncwarp();
-    solve_rows<NBM, 32 / NBM>(Xm, LUm, LD, uinv, nb, lane / (32 / NBM),
-                              lane % (32 / NBM));
-    __syncwarp();
-    cplx *dTb = A.dT + param * A.dT_stride + sl.tout + block_offset(N, m);
-    for (int u = lane; u < nb * nb; u += 32) {
-      const int a = u / nb;
-      const int b = u - a * nb;
-      int ia, na, ib, nbn;
-      member(D, a, ia, na);
-      member(D, b, ib, nbn);
-      dTb[(int64_t)(ia * D.nbb + (na - D.nmin)) * w2 + ib * D.nbb + (nbn - D.nmin)] =
-          Xm[a * LD + perm[b]];
-    }
-    __syncwarp();
   }
 }
 
-template <int TR, int TC, int MINB>
-static void launch_tangent_warp(const TmxTangentArgs &a, cudaStream_t stream) {
-  constexpr int NBM = (8 * TR > 4 * TC) ? 8 * TR : 4 * TC;
-  const size_t smem = (size_t)4 * tangent_warp_elems<NBM>() * sizeof(cplx);
-  cudaFuncSetAttribute(k_tangent_warp<TR, TC, MINB>,
+template <int NC, int NR, int NTH, int WG, int C, int MINB>
+static void launch_tangent_tile(const TmxTangentArgs &a, cudaStream_t stream) {
+  constexpr size_t smem = TangentTile<NC, NR, NTH, WG>::BYTES;
+  cudaFuncSetAttribute(k_tangent_tile<NC, NR, NTH, WG, C, MINB>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  // one (item, parameter) per warp: CTAs retire quickly, so that the
-  // launches of the other size buckets running beside this one get SMs
-  const int64_t work = (int64_t)a.nitems * a.nparams;
-  const int blocks = (int)std::max<int64_t>(1, (work + 3) / 4);
-  k_tangent_warp<TR, TC, MINB><<<blocks, 128, smem, stream>>>(a);
+  k_tangent_tile<NC, NR, NTH, WG, C, MINB><<<a.nitems, NTH, smem, stream>>>(a);
 }
 
 size_t tmx_tangent_smem_bytes(int max_nb, int chunk_nodes) {
@@ -658,12 +809,6 @@ size_t tmx_tangent_smem_bytes(int max_nb, int chunk_nodes) {
   const size_t full = lu + (size_t)max_nb * lda * sizeof(cplx);
   if (full <= 200 * 1024) {
     lu_total = full;
-  }
-  if (max_nb <= 32) {
-    // solve of the 128-thread kernel: factors, T_c and B (32 x 33 each),
-    // 1/U_jj and the gather index
-    const size_t small = (size_t)(3 * 32 * 33 + 32) * sizeof(cplx) + 32 * sizeof(int);
-    lu_total = std::max(lu_total, small);
   }
   return asm_bytes > lu_total ? asm_bytes : lu_total;
 }
@@ -691,18 +836,21 @@ void tmx_launch_tangents(const TmxTangentArgs &a, cudaStream_t stream) {
   if (a.nitems <= 0 || a.nparams <= 0) {
     return;
   }
+  // One variant per padded size: the tile count sets the warps of a CTA, the
+  // class size its shared memory (33, 47 and 118 KB: 6, 4 and 1 CTAs per SM).
+  // Above 32 the three parameters' matrices no longer fit (7 nb^2 entries) and
+  // each parameter has a CTA of its own.
   if (a.max_nb <= 8) {
-    launch_tangent_warp<1, 2, 3>(a, stream);
+    launch_tangent_tile<8, 16, 64, 4, 2, 6>(a, stream);
     return;
   }
   if (a.max_nb <= 16) {
-    launch_tangent_warp<2, 4, 2>(a, stream);
+    launch_tangent_tile<16, 16, 128, 4, 2, 4>(a, stream);
     return;
   }
-  const size_t smem = tmx_tangent_smem_bytes(a.max_nb, a.chunk_nodes);
   if (a.max_nb <= 32) {
-    launch_tangent<2, 4, 128, 3>(a, smem, stream);
-  } else {
-    launch_tangent<4, 4, 256, 1>(a, smem, stream);
+    launch_tangent_tile<32, 32, 512, 4, 4, 1>(a, stream);
+    return;
   }
+  launch_tangent<4, 4, 256, 1>(a, tmx_tangent_smem_bytes(a.max_nb, a.chunk_nodes), stream);
 }
