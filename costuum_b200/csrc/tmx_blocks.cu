@@ -1830,8 +1830,10 @@ void tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream) {
 // is final. Unconverged slots that have orders left go to the next list.
 // One launch per group: with few grains left the kernels of the loop are
 // shorter than their launches (eight orders of one grain: eight of 3 us -> one
-// of 6 us).
+// of 6 us). Bound by the latency of the diagonal's loads: CV_LOADS orders are
+// read ahead of their additions.
 #define CV_THREADS 128
+#define CV_LOADS 8
 __global__ void k_converge(const int32_t *__restrict__ active, int nactive,
                            const __grid_constant__ TmxChainGroup g, int lg,
                            const TmxSlot *__restrict__ slots,
@@ -1846,18 +1848,33 @@ __global__ void k_converge(const int32_t *__restrict__ active, int nactive,
   const int s = threadIdx.x & ((1 << lg) - 1);
   const int p = (blockIdx.x * CV_THREADS + threadIdx.x) >> lg;
   const bool have = p < nactive && (!nact_dev || base + p < *nact_dev);
+  int gr = 0;
+  TmxChainState st;
+  if (have && s == 0) { // (read beside the sums)
+    gr = active[p];
+    st = state[gr];
+  }
   if (have && s < g.n) {
     const TmxSlot sl = slots[g.base[s].slot + p];
     const cplx *dg = diag + sl.diag;
     const int N = g.order0 + s;
     double qs = 0., qe = 0.;
-#pragma unroll 4
-    for (int n = 1; n < N + 1; ++n) {
-      const double dn1 = 2. * n + 1.;
-      const cplx a = dg[n - 1];
-      const cplx b = dg[N + n - 1];
-      qs += dn1 * (cnorm2(a) + cnorm2(b));
-      qe += dn1 * (a.x + b.x);
+    for (int n0 = 1; n0 < N + 1; n0 += CV_LOADS) {
+      cplx a[CV_LOADS], b[CV_LOADS];
+#pragma unroll
+      for (int i = 0; i < CV_LOADS; ++i) {
+        const int n = min(n0 + i, N);
+        a[i] = dg[n - 1];
+        b[i] = dg[N + n - 1];
+      }
+#pragma unroll
+      for (int i = 0; i < CV_LOADS; ++i) {
+        if (n0 + i < N + 1) {
+          const double dn1 = 2. * (n0 + i) + 1.;
+          qs += dn1 * (cnorm2(a[i]) + cnorm2(b[i]));
+          qe += dn1 * (a[i].x + b[i].x);
+        }
+      }
     }
     sq[threadIdx.x] = qs;
     se[threadIdx.x] = qe;
@@ -1866,8 +1883,6 @@ __global__ void k_converge(const int32_t *__restrict__ active, int nactive,
   if (!have || s != 0) {
     return;
   }
-  const int gr = active[p];
-  TmxChainState st = state[gr];
   bool stays = false;
   for (int t = 0; t < g.n; ++t) {
     const double qs = sq[threadIdx.x + t], qe = se[threadIdx.x + t];
@@ -1943,41 +1958,64 @@ void tmx_launch_converge(const int32_t *active, int nactive, const TmxChainGroup
 // reserved offset (in doubles, a multiple of 16), recorded per grain and per
 // done-list entry; -1 where the arena is full (the round then recomputes
 // them). One CTA per entry, grid-stride; the last CTA to finish moves *next
-// to the end of the range.
-__global__ void k_keep_tables(TmxKeepArgs K) {
+// to the end of the range. Part of the order loop's chain and bound by the
+// latency of its loads (13 to 130 KB per entry): 512 threads with four 16-byte
+// loads in flight each, the first ones beside the reservation. 4096 grains,
+// 19 launches: 453 -> 184 us (128 threads, one load after the other: up to
+// 42 us for the 115 KB of an order 30); the batch 5.85 -> 5.30 ms together
+// with the loads of k_converge (203 -> 173 us).
+#define KT_THREADS 512
+#define KT_LOADS 4
+__global__ void __launch_bounds__(KT_THREADS)
+    k_keep_tables(const __grid_constant__ TmxKeepArgs K) {
   __shared__ long long s_off;
   __shared__ unsigned s_last;
-  if (K.order0_dev) {
-    K.order0 = *K.order0_dev;
-    K.base[0] = *K.base_dev;
-  }
+  const int order0 = K.order0_dev ? *K.order0_dev : K.order0;
   const int begin = *K.next;
   const int end = K.counters[1];
   for (int q = begin + blockIdx.x; q < end; q += gridDim.x) {
     const int g = K.done_list[q];
-    const int s = K.done_ord[q] - K.order0;
+    const int s = K.done_ord[q] - order0;
     const int p = K.done_pos[q];
-    const TmxChainBase b = K.base[s];
+    const TmxChainBase &b = K.order0_dev ? *K.base_dev : K.base[s];
     const int64_t tsz = b.tab_stride, nsz = b.nsc_stride;
-    const int64_t want = ((tsz + 15) & ~(int64_t)15) + ((nsz + 15) & ~(int64_t)15);
+    const int64_t tpad = (tsz + 15) & ~(int64_t)15;
+    const int64_t want = tpad + ((nsz + 15) & ~(int64_t)15);
     if (threadIdx.x == 0) {
       const long long off =
           (long long)atomicAdd(K.used, (unsigned long long)want);
       s_off = (off + want <= K.cap) ? off : -1;
     }
+    const double2 *ts = reinterpret_cast<const double2 *>(K.tab + b.tab + p * tsz);
+    const double2 *ns = reinterpret_cast<const double2 *>(K.nsc + b.nsc + p * nsz);
+    const int nt = (int)(tsz / 2), nn = nt + (int)(nsz / 2);
+    double2 v[KT_LOADS];
+    const auto load = [&](int u0) {
+#pragma unroll
+      for (int i = 0; i < KT_LOADS; ++i) {
+        const int u = u0 + i * KT_THREADS;
+        if (u < nn) {
+          v[i] = u < nt ? ts[u] : ns[u - nt];
+        }
+      }
+    };
+    load(threadIdx.x); // (beside the reservation)
     __syncthreads();
     const long long off = s_off;
     if (off >= 0) {
-      const double2 *ts = reinterpret_cast<const double2 *>(K.tab + b.tab + p * tsz);
       double2 *td = reinterpret_cast<double2 *>(K.arena + off);
-      for (int64_t u = threadIdx.x; u < tsz / 2; u += blockDim.x) {
-        td[u] = ts[u];
-      }
-      const int64_t noff = off + ((tsz + 15) & ~(int64_t)15);
-      const double2 *ns = reinterpret_cast<const double2 *>(K.nsc + b.nsc + p * nsz);
-      double2 *nd = reinterpret_cast<double2 *>(K.arena + noff);
-      for (int64_t u = threadIdx.x; u < nsz / 2; u += blockDim.x) {
-        nd[u] = ns[u];
+      double2 *nd = reinterpret_cast<double2 *>(K.arena + off + tpad);
+      for (int u0 = threadIdx.x; u0 < nn; u0 += KT_LOADS * KT_THREADS) {
+        if (u0 != threadIdx.x) {
+          load(u0);
+        }
+#pragma unroll
+        for (int i = 0; i < KT_LOADS; ++i) {
+          const int u = u0 + i * KT_THREADS;
+          if (u < nn) {
+            *(u < nt ? td + u : nd + (u - nt)) = v[i];
+          }
+        }
       }
     }
     if (threadIdx.x == 0) {
@@ -2003,7 +2041,7 @@ __global__ void k_keep_tables(TmxKeepArgs K) {
 void tmx_launch_keep_tables(const TmxKeepArgs &K, int max_entries,
                             cudaStream_t stream) {
   const int blocks = std::max(1, std::min(max_entries, 148 * 4));
-  k_keep_tables<<<blocks, 128, 0, stream>>>(K);
+  k_keep_tables<<<blocks, KT_THREADS, 0, stream>>>(K);
 }
 
 // ------------------------------------------------------------- Q sums ------
