@@ -21,6 +21,7 @@
 //  * T = -RgQ Q^-1 by two triangular solves on the LU factors instead of the
 //    explicit inverse followed by a product.
 #include <algorithm>
+#include <type_traits>
 
 #include "tmx_blocks_common.cuh"
 
@@ -1197,13 +1198,13 @@ static void launch_cta32(const TmxBlockArgs &a, cudaStream_t stream) {
 // scratch), one CTA per item factors Q (k_factor), and the solves are split by
 // rows again (k_solve).
 // Measured (B200), one CTA per item for everything -> the three kernels: 1154
-// items of 33..50 members, 66..100 nodes: 1.41 -> 0.50 + 0.23 + 0.16 ms; 1960
-// items of 65..99 members, 198 nodes: 15.4 -> 5.96 + 1.99 + 1.79 ms; the m = 0
-// classes of nine grains at orders 129..199: 1.42 -> 0.39 ms per order.
+// items of 33..50 members, 66..100 nodes: 1.41 -> 0.50 + 0.13 + 0.16 ms; 1960
+// items of 65..99 members, 198 nodes: 15.4 -> 5.96 + 1.44 + 1.59 ms; the m = 0
+// classes of nine grains at orders 129..199: 1.42 -> 0.33 ms per order.
 // k_assemble is bound by the issue of its build phase (32 x 64 tiles with two
 // CTAs per SM took 0.53 and 6.9 ms; three chunks of table rows in flight
-// instead of one 0.56 and 7.1), k_factor by its shared-memory traffic, k_solve
-// by the FP64 pipe and the chain of its columns.
+// instead of one 0.56 and 7.1), k_solve by the FP64 pipe and the chain of its
+// columns.
 
 #define TMX_ASM_ROWS 32
 #define TMX_ASM_COLS 32
@@ -1430,25 +1431,33 @@ __global__ void __launch_bounds__(256, 3) k_assemble(TmxBlockArgs A, int rtiles,
 // LU of Q_c, one item per CTA, in shared memory (in the scratch itself for
 // classes whose factors exceed it).
 //
-// Thread (tr, tc) of a (NTH / 16) x 16 grid owns rows tr, tr + NTH / 16, ..
-// and columns tc, tc + 16, ..; rows stay in place and carry a position (the
-// pivot of step i is the first position with the largest |Q_ri|, as in
-// Matrix::plu_inverse). A step has one barrier: the threads of column i + 1
-// post their largest candidate of the next step right after updating it,
-// behind the barrier every warp reduces the candidates itself, and the l of a
-// row are formed by the 16 threads that share it. The factors go back to the
-// scratch with their rows in place, and the row at each position beside them.
-template <int NBM, int NTH>
-__global__ void __launch_bounds__(NTH, (NBM > 64) ? 1 : 2)
+// Rows stay in place; at[s] is the row at position s (the pivot of step i is
+// the first position with the largest |Q_ri|, as in Matrix::plu_inverse), so
+// the rows still to be eliminated are those at positions above i. Warp 0 runs
+// one column ahead: while the other UW warps apply step i to the columns from
+// i + 2 on, it updates column i + 1, finds the pivot of step i + 1 and writes
+// the l of its column; a step has one barrier. It applies a step's exchange of
+// positions to at[] while the others still read it, so they take the row at
+// the exchanged position from the posted exchange instead. The factors go back
+// to the scratch with their rows in place, and the row at each position beside
+// them.
+// Bound by the shared-memory traffic of the updates while many rows are left,
+// by the latency of warp 0's column afterwards. All warps searching and
+// inverting the pivot themselves kept the FP64 pipe busy with copies of the
+// same work: 1154 items of 33..50 members 0.227 -> 0.134 ms, 1960 items of
+// 65..99 1.99 -> 1.44 ms, one item of 100 0.19 -> 0.14 ms. Measured and not
+// taken: update warps only beside, not on, warp 0's scheduler (0.194 and 1.88
+// ms); three CTAs per SM for up to 64 members (0.153 ms).
+template <int NBM, int UW, int MINB>
+__global__ void __launch_bounds__(32 + 32 * UW, MINB)
     k_factor(TmxBlockArgs A, size_t smem_bytes) {
-  constexpr int RT = NTH / 16; // row groups
-  constexpr int NA = NBM / RT; // rows per thread
-  static_assert(RT <= 32 && NBM % RT == 0, "thread layout");
+  constexpr int NTH = 32 + 32 * UW;
+  constexpr int CT = NTH / 16; // row groups of the copies
+  constexpr int RT = 2 * UW;   // row groups of the updates
+  constexpr int NA = (NBM + RT - 1) / RT; // rows per thread
   extern __shared__ __align__(16) unsigned char fsm[];
-  __shared__ unsigned long long ckey[2][32];
-  __shared__ int cpos[2][32], crow[2][32];
-  __shared__ int at[NBM]; // row at a position
-  __shared__ int flag;
+  __shared__ int at[NBM];                // row at a position
+  __shared__ int prow[2], pbi[2], pold[2]; // pivot row, its position, the row at i
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int tc = tid & 15;
@@ -1471,133 +1480,215 @@ __global__ void __launch_bounds__(NTH, (NBM > 64) ? 1 : 2)
     }
     cplx *Qs = A.scratch + item.scratch;
     const int lds = nb | 1;
-    const bool inplace = (size_t)nb * lds * sizeof(cplx) > smem_bytes;
-    const int lda = inplace ? nb : lds;
-    cplx *Am = inplace ? Qs : reinterpret_cast<cplx *>(fsm);
-    if (!inplace) {
-      for (int r = tr; r < nb; r += RT) {
-        for (int k = tc; k < nb; k += 16) {
-          Am[r * lda + k] = Qs[(int64_t)r * nb + k];
-        }
+    // (one body per address space: generic accesses to shared memory are slower)
+    const auto factors = [&](auto ip) {
+      constexpr bool inplace = decltype(ip)::value;
+      const int lda = inplace ? nb : lds;
+      cplx *Am;
+      if constexpr (inplace) {
+        Am = Qs;
+      } else {
+        Am = reinterpret_cast<cplx *>(fsm);
       }
-    }
-    if (tid == 0) {
-      flag = 0;
-    }
-    int pos[NA];
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-      pos[a] = tr + RT * a;
-    }
-    __syncthreads();
-    // candidate of column i among this thread's rows (threads of the column)
-    const auto post = [&](int i, int buf) {
-      double best = 0.;
-      unsigned long long key = 0ull;
-      int bp = 0x7fffffff, br = 0;
-#pragma unroll
-      for (int a = 0; a < NA; ++a) {
-        const int r = tr + RT * a;
-        if (r < nb && pos[a] >= i) {
-          double v = cabs_dev(Am[r * lda + i]);
-          v = (v >= 0.) ? v : 0.; // (NaN is no candidate)
-          if (key == 0ull || v > best || (v == best && pos[a] < bp)) {
-            best = v;
-            bp = pos[a];
-            br = r;
-            key = (unsigned long long)__double_as_longlong(v) | (1ull << 63);
+      if (!inplace) {
+        for (int r = tr; r < nb; r += CT) {
+          for (int k = tc; k < nb; k += 16) {
+            Am[r * lda + k] = Qs[(int64_t)r * nb + k];
           }
         }
       }
-      ckey[buf][tr] = key;
-      cpos[buf][tr] = bp;
-      crow[buf][tr] = br;
-    };
-    if (tc == 0) {
-      post(0, 0);
-    }
-    __syncthreads();
-    for (int i = 0; i < nb; ++i) {
-      const int buf = i & 1;
-      int bi, wl;
-      const unsigned long long key = (lane < RT) ? ckey[buf][lane] : 0ull;
-      warp_argmax(key, (lane < RT) ? cpos[buf][lane] : 0x7fffffff, bi, wl);
-      const int p = crow[buf][wl];
-      if (tid == 0) {
-        at[i] = p;
-        if (!(__longlong_as_double((long long)(ckey[buf][wl] & ~(1ull << 63))) > 0.)) {
-          flag = 1;
-        }
-      }
-      const cplx *pr = Am + p * lda;
-      const cplx pinv = cinv_lu(pr[i]);
-      cplx l[NA];
-#pragma unroll
-      for (int a = 0; a < NA; ++a) {
-        const int r = tr + RT * a;
-        // the row that was at position i takes the pivot's old position
-        if (r == p) {
-          pos[a] = i;
-        } else if (pos[a] == i) {
-          pos[a] = bi;
-        }
-        l[a] = (r < nb && pos[a] > i) ? mul_xx(Am[r * lda + i], pinv) : mkc(0., 0.);
-      }
-      __syncwarp(); // the row's 16 threads have read column i
-      if (tc == (i & 15)) {
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-          const int r = tr + RT * a;
-          if (r < nb && pos[a] > i) {
-            Am[r * lda + i] = l[a];
-          }
-        }
-      }
-      // columns i + 1, i + 2, ..: column i + 1 first, its threads post the
-      // next step's candidates before the rest
-      for (int k = i + 1 + ((tc - i - 1) & 15); k < nb; k += 16) {
-        const cplx u = pr[k];
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-          const int r = tr + RT * a;
-          if (r < nb && pos[a] > i) {
-            Am[r * lda + k] = csub(Am[r * lda + k], mul_xy(l[a], u));
-          }
-        }
-        if (k == i + 1) {
-          post(k, buf ^ 1);
-        }
+      for (int j = tid; j < nb; j += NTH) {
+        at[j] = j;
       }
       __syncthreads();
-    }
-    if (tid == 0 && flag) {
-      atomicOr(&A.status[sl.grain], TMX_ST_SINGULAR);
-    }
-    int *ps = reinterpret_cast<int *>(Qs + 2 * (int64_t)nb * nb);
-    for (int j = tid; j < nb; j += NTH) {
-      ps[j] = at[j];
-    }
-    if (!inplace) {
-      for (int r = tr; r < nb; r += RT) {
-        for (int k = tc; k < nb; k += 16) {
-          Qs[(int64_t)r * nb + k] = Am[r * lda + k];
+      bool flag = false; // (warp 0) a pivot was zero
+      // column j by warp 0: NP positions per lane; pr: pivot row of step j - 1
+      const auto panel = [&](auto np, int j, const cplx *pr) {
+        constexpr int NP = decltype(np)::value;
+        cplx v[NP];
+        double t[NP];
+        int r[NP];
+  #pragma unroll
+        for (int a = 0; a < NP; ++a) {
+          const int s = j + lane + 32 * a;
+          r[a] = (s < nb) ? at[s] : 0;
+          v[a] = (s < nb) ? Am[r[a] * lda + j] : mkc(0., 0.);
+          if (j > 0) {
+            const cplx l = (s < nb) ? Am[r[a] * lda + j - 1] : mkc(0., 0.);
+            v[a] = csub(v[a], mul_xy(l, pr[j]));
+          }
         }
-      }
-    }
-    if (A.lu) {
-      // factors (unit-lower L below, U on and above the diagonal) and the
-      // column gather index, for the tangent solves
-      cplx *Ls = A.lu + item.scratch;
-      for (int r = tr; r < nb; r += RT) {
-        const cplx *s = Am + at[r] * lda;
-        for (int k = tc; k < nb; k += 16) {
-          Ls[(int64_t)r * nb + k] = s[k];
+        const unsigned long long top = 1ull << 63;
+        double best = 0.;
+        int lp = 0x7fffffff, lr = 0, bi, wl;
+        cplx lv = mkc(0., 0.);
+        const auto pick = [&]() { // largest t of this lane, first on ties
+          best = 0.;
+          lp = 0x7fffffff;
+  #pragma unroll
+          for (int a = 0; a < NP; ++a) {
+            const int s = j + lane + 32 * a;
+            t[a] = (t[a] >= 0.) ? t[a] : 0.; // (NaN is no candidate)
+            if (s < nb && (lp == 0x7fffffff || t[a] > best)) {
+              best = t[a];
+              lp = s;
+              lr = r[a];
+              lv = v[a];
+            }
+          }
+        };
+  #pragma unroll
+        for (int a = 0; a < NP; ++a) {
+          t[a] = fma(v[a].x, v[a].x, v[a].y * v[a].y);
         }
+        pick();
+        cplx pinv = cinv_lu(lv);
+        warp_argmax(lp < nb ? (unsigned long long)__double_as_longlong(best) | top : 0ull,
+                    lp, bi, wl);
+        best = __shfl_sync(0xffffffffu, best, wl);
+        // |Q|^2 decides unless others come within rounding (see warp_pivot)
+        unsigned close = 0;
+  #pragma unroll
+        for (int a = 0; a < NP; ++a) {
+          close += (j + lane + 32 * a < nb && t[a] >= best * (1. - 0x1p-40)) ? 1u : 0u;
+        }
+        if (__reduce_add_sync(0xffffffffu, close) != 1u ||
+            !(best > 0x1p-900 && best < 0x1p900)) {
+  #pragma unroll
+          for (int a = 0; a < NP; ++a) {
+            t[a] = cabs_dev(v[a]);
+          }
+          pick();
+          pinv = cinv_lu(lv);
+          warp_argmax(lp < nb ? (unsigned long long)__double_as_longlong(best) | top : 0ull,
+                      lp, bi, wl);
+          flag = !(__shfl_sync(0xffffffffu, best, wl) > 0.) || flag;
+        }
+        const int p = __shfl_sync(0xffffffffu, lr, wl);
+        pinv.x = __shfl_sync(0xffffffffu, pinv.x, wl);
+        pinv.y = __shfl_sync(0xffffffffu, pinv.y, wl);
+  #pragma unroll
+        for (int a = 0; a < NP; ++a) {
+          if (j + lane + 32 * a < nb) {
+            Am[r[a] * lda + j] = (r[a] == p) ? v[a] : mul_xx(v[a], pinv);
+          }
+        }
+        if (lane == 0) {
+          prow[j & 1] = p;
+          pbi[j & 1] = bi;
+          pold[j & 1] = r[0];
+        }
+      };
+      const auto column = [&](int j, const cplx *pr) {
+        if (nb - j <= 32) {
+          panel(std::integral_constant<int, 1>{}, j, pr);
+        } else if (NBM <= 64 || nb - j <= 64) {
+          panel(std::integral_constant<int, 2>{}, j, pr);
+        } else {
+          panel(std::integral_constant<int, NBM / 32>{}, j, pr);
+        }
+      };
+      if (tid < 32) {
+        column(0, Am);
       }
-      int *pl = reinterpret_cast<int *>(Ls + (int64_t)nb * nb);
+      __syncthreads();
+      for (int i = 0; i < nb; ++i) {
+        const int p = prow[i & 1], bi = pbi[i & 1], o = pold[i & 1];
+        const cplx *pr = Am + p * lda;
+        if (tid < 32) {
+          if (lane == 0) {
+            at[bi] = o;
+            at[i] = p;
+          }
+          __syncwarp();
+          if (i + 1 < nb) {
+            column(i + 1, pr);
+          }
+        } else if (i + 1 + tr - 2 < nb) {
+          const int s0 = i + 1 + tr - 2;
+          cplx l[NA], *row[NA];
+  #pragma unroll
+          for (int a = 0; a < NA; ++a) {
+            const int s = s0 + RT * a;
+            row[a] = Am;
+            l[a] = mkc(0., 0.);
+            if (s < nb) {
+              row[a] = Am + ((s == bi) ? o : at[s]) * lda;
+              l[a] = row[a][i];
+            }
+          }
+          int k = i + 2 + tc;
+          for (; k + 16 < nb; k += 32) {
+            const cplx u0 = pr[k], u1 = pr[k + 16];
+            cplx v0[NA], v1[NA];
+  #pragma unroll
+            for (int a = 0; a < NA; ++a) {
+              if (s0 + RT * a < nb) {
+                v0[a] = row[a][k];
+                v1[a] = row[a][k + 16];
+              }
+            }
+  #pragma unroll
+            for (int a = 0; a < NA; ++a) {
+              if (s0 + RT * a < nb) {
+                row[a][k] = csub(v0[a], mul_xy(l[a], u0));
+                row[a][k + 16] = csub(v1[a], mul_xy(l[a], u1));
+              }
+            }
+          }
+          if (k < nb) {
+            const cplx u = pr[k];
+            cplx v[NA];
+  #pragma unroll
+            for (int a = 0; a < NA; ++a) {
+              if (s0 + RT * a < nb) {
+                v[a] = row[a][k];
+              }
+            }
+  #pragma unroll
+            for (int a = 0; a < NA; ++a) {
+              if (s0 + RT * a < nb) {
+                row[a][k] = csub(v[a], mul_xy(l[a], u));
+              }
+            }
+          }
+        }
+        __syncthreads();
+      }
+      if (tid == 0 && flag) {
+        atomicOr(&A.status[sl.grain], TMX_ST_SINGULAR);
+      }
+      int *ps = reinterpret_cast<int *>(Qs + 2 * (int64_t)nb * nb);
       for (int j = tid; j < nb; j += NTH) {
-        pl[at[j]] = j;
+        ps[j] = at[j];
       }
+      if (!inplace) {
+        for (int r = tr; r < nb; r += CT) {
+          for (int k = tc; k < nb; k += 16) {
+            Qs[(int64_t)r * nb + k] = Am[r * lda + k];
+          }
+        }
+      }
+      if (A.lu) {
+        // factors (unit-lower L below, U on and above the diagonal) and the
+        // column gather index, for the tangent solves
+        cplx *Ls = A.lu + item.scratch;
+        for (int r = tr; r < nb; r += CT) {
+          const cplx *s = Am + at[r] * lda;
+          for (int k = tc; k < nb; k += 16) {
+            Ls[(int64_t)r * nb + k] = s[k];
+          }
+        }
+        int *pl = reinterpret_cast<int *>(Ls + (int64_t)nb * nb);
+        for (int j = tid; j < nb; j += NTH) {
+          pl[at[j]] = j;
+        }
+      }
+    };
+    if (NBM > 64 && (size_t)nb * lds * sizeof(cplx) > smem_bytes) {
+      factors(std::true_type{});
+    } else {
+      factors(std::false_type{});
     }
     __syncthreads(); // shared memory is reused by the next item
   }
@@ -1664,52 +1755,73 @@ __global__ void __launch_bounds__(NTH, (NBM > 64) ? 1 : 2)
     }
     cp_wait_all();
     __syncthreads();
-    // Z U = X (forward over columns)
-#pragma unroll
-    for (int tj = 0; tj < NT; ++tj) {
-      if (tj * C < nb) {
-        for (int cj = 0; cj < C; ++cj) {
-          const int j = tj * C + cj;
-          if (j >= nb) {
-            break;
-          }
-          if (c == cj) {
-            // (column 0 of the classes up to 64: see mul_yx)
-            x[tj] = (NBM <= 64 && j == 0) ? mul_yx(x[tj], uinv[j]) : mul_xy(x[tj], uinv[j]);
-          }
-          cplx xj;
-          xj.x = __shfl_sync(0xffffffffu, x[tj].x, cj, C);
-          xj.y = __shfl_sync(0xffffffffu, x[tj].y, cj, C);
-          const cplx *ur = inplace ? Qs + (int64_t)at[j] * nb : Fm + j * lds;
-#pragma unroll
-          for (int t = tj; t < NT; ++t) {
-            const int k = c + C * t;
-            if (k > j && k < nb) {
-              x[t] = csub(x[t], mul_xy(xj, ur[k]));
+    // Above 64 members a body for shared memory alone beside the general one
+    // (1.59 against 1.79 ms for 1960 items of 65..99 members); up to 64 the
+    // loads that it hoists cost registers (0.18 against 0.16 ms for 1154 items).
+    const auto solves = [&](auto ip) {
+      constexpr bool SPLIT = decltype(ip)::value;
+      // Z U = X (forward over columns)
+  #pragma unroll
+      for (int tj = 0; tj < NT; ++tj) {
+        if (tj * C < nb) {
+          for (int cj = 0; cj < C; ++cj) {
+            const int j = tj * C + cj;
+            if (j >= nb) {
+              break;
+            }
+            if (c == cj) {
+              // (column 0 of the classes up to 64: see mul_yx)
+              x[tj] = (NBM <= 64 && j == 0) ? mul_yx(x[tj], uinv[j]) : mul_xy(x[tj], uinv[j]);
+            }
+            cplx xj;
+            xj.x = __shfl_sync(0xffffffffu, x[tj].x, cj, C);
+            xj.y = __shfl_sync(0xffffffffu, x[tj].y, cj, C);
+            const cplx *ur;
+            if constexpr (SPLIT) {
+              ur = reinterpret_cast<const cplx *>(fsm) + j * lds;
+            } else {
+              ur = inplace ? Qs + (int64_t)at[j] * nb : Fm + j * lds;
+            }
+  #pragma unroll
+            for (int t = tj; t < NT; ++t) {
+              const int k = c + C * t;
+              if (k > j && k < nb) {
+                x[t] = csub(x[t], mul_xy(xj, ur[k]));
+              }
             }
           }
         }
       }
-    }
-    // Y L = Z (backward over columns, L unit lower)
-#pragma unroll
-    for (int tj = NT - 1; tj >= 0; --tj) {
-      if (tj * C < nb) {
-        for (int cj = min(C, nb - tj * C) - 1; cj >= 0; --cj) {
-          const int j = tj * C + cj;
-          cplx xj;
-          xj.x = __shfl_sync(0xffffffffu, x[tj].x, cj, C);
-          xj.y = __shfl_sync(0xffffffffu, x[tj].y, cj, C);
-          const cplx *lr = inplace ? Qs + (int64_t)at[j] * nb : Fm + j * lds;
-#pragma unroll
-          for (int t = 0; t <= tj; ++t) {
-            const int k = c + C * t;
-            if (k < j) {
-              x[t] = csub(x[t], mul_xy(xj, lr[k]));
+      // Y L = Z (backward over columns, L unit lower)
+  #pragma unroll
+      for (int tj = NT - 1; tj >= 0; --tj) {
+        if (tj * C < nb) {
+          for (int cj = min(C, nb - tj * C) - 1; cj >= 0; --cj) {
+            const int j = tj * C + cj;
+            cplx xj;
+            xj.x = __shfl_sync(0xffffffffu, x[tj].x, cj, C);
+            xj.y = __shfl_sync(0xffffffffu, x[tj].y, cj, C);
+            const cplx *lr;
+            if constexpr (SPLIT) {
+              lr = reinterpret_cast<const cplx *>(fsm) + j * lds;
+            } else {
+              lr = inplace ? Qs + (int64_t)at[j] * nb : Fm + j * lds;
+            }
+  #pragma unroll
+            for (int t = 0; t <= tj; ++t) {
+              const int k = c + C * t;
+              if (k < j) {
+                x[t] = csub(x[t], mul_xy(xj, lr[k]));
+              }
             }
           }
         }
       }
+    };
+    if (NBM > 64 && !inplace) {
+      solves(std::true_type{});
+    } else {
+      solves(std::false_type{});
     }
     // write out: T_c[a][at[k]] = Y[a][k]
     if (act) {
@@ -1745,7 +1857,7 @@ __global__ void __launch_bounds__(NTH, (NBM > 64) ? 1 : 2)
 // the static arrays)
 #define TMX_FACTOR_SMEM_MAX (221u * 1024u)
 
-template <bool LEAN, int NBM, int NTHF, int NTHS, int C>
+template <bool LEAN, int NBM, int UW, int MINB, int NTHS, int C>
 static void launch_apart(const TmxBlockArgs &a, cudaStream_t stream) {
   const int max_nb = std::max(1, std::min(a.max_nb, NBM));
   const int rt = asm_row_tiles(max_nb), ct = asm_col_tiles(max_nb);
@@ -1764,11 +1876,11 @@ static void launch_apart(const TmxBlockArgs &a, cudaStream_t stream) {
   // factors in shared memory up to 118 members, above that in the scratch
   const size_t smem = std::min<size_t>((size_t)max_nb * (max_nb | 1) * sizeof(cplx),
                                        TMX_FACTOR_SMEM_MAX);
-  cudaFuncSetAttribute(k_factor<NBM, NTHF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaFuncSetAttribute(k_factor<NBM, UW, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)smem);
   cudaFuncSetAttribute(k_solve<NBM, NTHS, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)smem);
-  k_factor<NBM, NTHF><<<ctas(1), NTHF, smem, stream>>>(a, smem);
+  k_factor<NBM, UW, MINB><<<ctas(1), 32 + 32 * UW, smem, stream>>>(a, smem);
   k_solve<NBM, NTHS, C><<<ctas(chunks), NTHS, smem, stream>>>(a, chunks, smem);
 }
 
@@ -1815,10 +1927,10 @@ void tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream) {
     launch_cta32(a, stream);
     return;
   case TMX_BLOCKS_CTA64:
-    launch_apart<true, 64, 256, 512, 8>(a, stream);
+    launch_apart<true, 64, 8, 2, 512, 8>(a, stream);
     return;
   default:
-    launch_apart<false, 128, 512, 512, 16>(a, stream);
+    launch_apart<false, 128, 15, 1, 512, 16>(a, stream);
   }
 }
 
