@@ -268,6 +268,9 @@ def workload_config():
             "l2": "flushed between steps (256 MB write); working set > L2"}
 
 
+REF_LIB = os.path.join(ROOT, "oracle", "_ref", "libref_driver.so")
+
+
 def reference_sample(nthreads, step):
     """One bounded sample of the workload through the reference's own task
     objects under QuickSched (oracle/_ref, built from the reference): slice
@@ -310,6 +313,10 @@ def cpu_baseline_block(nthreads, steps=3, warmup=1):
 def run_reference(args):
     rank, world, local = dist_env()
     if rank != 0:
+        return 0
+    if not os.path.exists(REF_LIB):
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "oracle/_ref is not built: the reference's sources are not there"}))
         return 0
     nthreads = os.cpu_count() or 1
     times, done = [], 0
@@ -738,7 +745,7 @@ def run_ours(args):
     out = None
     if rank == 0:
         cpu = None
-        if world == 1 and not args.skip_cpu:
+        if world == 1 and not args.skip_cpu and os.path.exists(REF_LIB):
             cpu = cpu_baseline_block(os.cpu_count() or 1)
         out = {
             "metric": "T-matrices/s (converged, batched)",
@@ -888,7 +895,7 @@ def averaging_leg(ctx, lib, fp64_peak):
     wall = time.perf_counter() - t0
     peak_gbs, peak_src = hbm_peak()
     kernels = {}
-    for k, name in ((2, "k_orient_pairs"), (3, "k_amp"), (4, "k_shape_avg")):
+    for k, name in ((2, "k_orient"), (3, "k_amp"), (4, "k_shape_avg")):
         ms = np.zeros(1)
         n = ctypes.c_int64()
         fl = np.zeros(1)
