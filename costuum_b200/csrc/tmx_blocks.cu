@@ -1199,8 +1199,8 @@ static void launch_cta32(const TmxBlockArgs &a, cudaStream_t stream) {
 // rows again (k_solve).
 // Measured (B200), one CTA per item for everything -> the three kernels: 1154
 // items of 33..50 members, 66..100 nodes: 1.41 -> 0.50 + 0.13 + 0.16 ms; 1960
-// items of 65..99 members, 198 nodes: 15.4 -> 5.96 + 1.44 + 1.59 ms; the m = 0
-// classes of nine grains at orders 129..199: 1.42 -> 0.33 ms per order.
+// items of 65..99 members, 198 nodes: 15.4 -> 5.96 + 1.10 + 1.59 ms; the m = 0
+// classes of nine grains at orders 129..199: 1.42 -> 0.32 ms per order.
 // k_assemble is bound by the issue of its build phase (32 x 64 tiles with two
 // CTAs per SM took 0.53 and 6.9 ms; three chunks of table rows in flight
 // instead of one 0.56 and 7.1), k_solve by the FP64 pipe and the chain of its
@@ -1428,26 +1428,94 @@ __global__ void __launch_bounds__(256, 3) k_assemble(TmxBlockArgs A, int rtiles,
   }
 }
 
+// Pivot of one column over the lanes' candidates c[a] (bit a of live) at
+// positions pos[a], rows r[a]: the first position with the largest |c| (|c|^2
+// decides unless others come within rounding, see warp_pivot). Gives the row p,
+// its position bi, 1 / c and d of the row; returns whether the pivot is zero.
+template <int NP>
+__device__ __forceinline__ bool lane_pivot(const cplx (&c)[NP], const cplx (&d)[NP],
+                                           const int (&pos)[NP], const int (&r)[NP],
+                                           unsigned live, int &p, int &bi, cplx &pinv,
+                                           cplx &dp) {
+  const unsigned long long top = 1ull << 63;
+  double t[NP], best = 0.;
+  int lp = 0x7fffffff, lr = 0, wl;
+  cplx lc = mkc(0., 0.), ld = lc;
+  const auto pick = [&]() { // largest t of this lane, first position on ties
+    best = 0.;
+    lp = 0x7fffffff;
+#pragma unroll
+    for (int a = 0; a < NP; ++a) {
+      t[a] = (t[a] >= 0.) ? t[a] : 0.; // (NaN is no candidate)
+      if ((live >> a & 1u) && (lp == 0x7fffffff || t[a] > best ||
+                               (t[a] == best && pos[a] < lp))) {
+        best = t[a];
+        lp = pos[a];
+        lr = r[a];
+        lc = c[a];
+        ld = d[a];
+      }
+    }
+  };
+  bool zero = false;
+#pragma unroll
+  for (int a = 0; a < NP; ++a) {
+    t[a] = fma(c[a].x, c[a].x, c[a].y * c[a].y);
+  }
+  pick();
+  pinv = cinv_lu(lc);
+  warp_argmax(live ? (unsigned long long)__double_as_longlong(best) | top : 0ull, lp, bi,
+              wl);
+  best = __shfl_sync(0xffffffffu, best, wl);
+  unsigned close = 0;
+#pragma unroll
+  for (int a = 0; a < NP; ++a) {
+    close += ((live >> a & 1u) && t[a] >= best * (1. - 0x1p-40)) ? 1u : 0u;
+  }
+  if (__reduce_add_sync(0xffffffffu, close) != 1u ||
+      !(best > 0x1p-900 && best < 0x1p900)) {
+#pragma unroll
+    for (int a = 0; a < NP; ++a) {
+      t[a] = cabs_dev(c[a]);
+    }
+    pick();
+    pinv = cinv_lu(lc);
+    warp_argmax(live ? (unsigned long long)__double_as_longlong(best) | top : 0ull, lp, bi,
+                wl);
+    zero = !(__shfl_sync(0xffffffffu, best, wl) > 0.);
+  }
+  p = __shfl_sync(0xffffffffu, lr, wl);
+  pinv.x = __shfl_sync(0xffffffffu, pinv.x, wl);
+  pinv.y = __shfl_sync(0xffffffffu, pinv.y, wl);
+  dp.x = __shfl_sync(0xffffffffu, ld.x, wl);
+  dp.y = __shfl_sync(0xffffffffu, ld.y, wl);
+  return zero;
+}
+
 // LU of Q_c, one item per CTA, in shared memory (in the scratch itself for
 // classes whose factors exceed it).
 //
 // Rows stay in place; at[s] is the row at position s (the pivot of step i is
 // the first position with the largest |Q_ri|, as in Matrix::plu_inverse), so
-// the rows still to be eliminated are those at positions above i. Warp 0 runs
-// one column ahead: while the other UW warps apply step i to the columns from
-// i + 2 on, it updates column i + 1, finds the pivot of step i + 1 and writes
-// the l of its column; a step has one barrier. It applies a step's exchange of
-// positions to at[] while the others still read it, so they take the row at
-// the exchanged position from the posted exchange instead. The factors go back
-// to the scratch with their rows in place, and the row at each position beside
-// them.
-// Bound by the shared-memory traffic of the updates while many rows are left,
-// by the latency of warp 0's column afterwards. All warps searching and
-// inverting the pivot themselves kept the FP64 pipe busy with copies of the
-// same work: 1154 items of 33..50 members 0.227 -> 0.134 ms, 1960 items of
-// 65..99 1.99 -> 1.44 ms, one item of 100 0.19 -> 0.14 ms. Measured and not
-// taken: update warps only beside, not on, warp 0's scheduler (0.194 and 1.88
-// ms); three CTAs per SM for up to 64 members (0.153 ms).
+// the rows still to be eliminated are those at positions above i. Steps go in
+// pairs, with one barrier per pair, and warp 0 runs a pair ahead: while the
+// other UW warps apply steps i and i + 1 to the columns from i + 4 on (one load
+// and store per entry for both, the updates in the order of the steps), it
+// updates columns i + 2 and i + 3, finds their pivots and writes their l. The
+// second pivot row of a pair has not had the first step's update then: every
+// reader makes it, and one warp stores it in the phase after. Warp 0 applies
+// the exchanges of positions to at[] while the others still read it, so they
+// take the rows at the exchanged positions from the posted exchanges instead.
+// The factors go back to the scratch with their rows in place, and the row at
+// each position beside them.
+// Bound by the latency of warp 0's columns and, while many rows are left, by
+// the shared-memory traffic of the updates. All warps searching and inverting
+// the pivot themselves -> warp 0 one column ahead -> a pair ahead: 1154 items of
+// 33..50 members 0.227 -> 0.134 -> 0.126 ms, 1960 items of 65..99 1.99 -> 1.44
+// -> 1.10 ms, the m = 0 classes of nine grains at orders 129..199 0.151 ->
+// 0.117 -> 0.098 ms. Measured and not taken (one column ahead): update warps
+// only beside, not on, warp 0's scheduler (0.194 and 1.88 ms); three CTAs per SM
+// for up to 64 members (0.153 ms).
 template <int NBM, int UW, int MINB>
 __global__ void __launch_bounds__(32 + 32 * UW, MINB)
     k_factor(TmxBlockArgs A, size_t smem_bytes) {
@@ -1457,7 +1525,8 @@ __global__ void __launch_bounds__(32 + 32 * UW, MINB)
   constexpr int NA = (NBM + RT - 1) / RT; // rows per thread
   extern __shared__ __align__(16) unsigned char fsm[];
   __shared__ int at[NBM];                // row at a position
-  __shared__ int prow[2], pbi[2], pold[2]; // pivot row, its position, the row at i
+  // pivot rows of a pair of steps, their positions, the rows that gave way
+  __shared__ int prow[2][2], pbi[2][2], pold[2][2];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int tc = tid & 15;
@@ -1502,156 +1571,154 @@ __global__ void __launch_bounds__(32 + 32 * UW, MINB)
       }
       __syncthreads();
       bool flag = false; // (warp 0) a pivot was zero
-      // column j by warp 0: NP positions per lane; pr: pivot row of step j - 1
-      const auto panel = [&](auto np, int j, const cplx *pr) {
+      // columns j and j + 1 by warp 0: NP positions per lane; p0, p1: pivot rows
+      // of the pair before (columns j - 2 and j - 1)
+      const auto panel = [&](auto np, int j, int p0, int p1) {
         constexpr int NP = decltype(np)::value;
-        cplx v[NP];
-        double t[NP];
-        int r[NP];
-  #pragma unroll
+        const bool two = j + 1 < nb;
+        cplx v[NP], w[NP];
+        int r[NP], pos[NP];
+        unsigned live = 0;
+        cplx u0 = mkc(0., 0.), u1 = u0, x0 = u0, x1 = u0;
+        if (j > 0) {
+          const cplx lp = Am[p1 * lda + j - 2];
+          u0 = Am[p0 * lda + j];
+          u1 = csub(Am[p1 * lda + j], mul_xy(lp, u0));
+          if (two) {
+            x0 = Am[p0 * lda + j + 1];
+            x1 = csub(Am[p1 * lda + j + 1], mul_xy(lp, x0));
+          }
+        }
+#pragma unroll
         for (int a = 0; a < NP; ++a) {
-          const int s = j + lane + 32 * a;
-          r[a] = (s < nb) ? at[s] : 0;
-          v[a] = (s < nb) ? Am[r[a] * lda + j] : mkc(0., 0.);
+          pos[a] = j + lane + 32 * a;
+          const bool in = pos[a] < nb;
+          live |= in ? 1u << a : 0u;
+          r[a] = in ? at[pos[a]] : -1;
+          const cplx *row = Am + (in ? r[a] : 0) * lda;
+          v[a] = row[j];
+          w[a] = two ? row[j + 1] : mkc(0., 0.);
           if (j > 0) {
-            const cplx l = (s < nb) ? Am[r[a] * lda + j - 1] : mkc(0., 0.);
-            v[a] = csub(v[a], mul_xy(l, pr[j]));
+            const cplx l0 = row[j - 2], l1 = row[j - 1];
+            v[a] = csub(csub(v[a], mul_xy(l0, u0)), mul_xy(l1, u1));
+            w[a] = csub(csub(w[a], mul_xy(l0, x0)), mul_xy(l1, x1));
           }
         }
-        const unsigned long long top = 1ull << 63;
-        double best = 0.;
-        int lp = 0x7fffffff, lr = 0, bi, wl;
-        cplx lv = mkc(0., 0.);
-        const auto pick = [&]() { // largest t of this lane, first on ties
-          best = 0.;
-          lp = 0x7fffffff;
-  #pragma unroll
+        const int o0 = __shfl_sync(0xffffffffu, r[0], 0);
+        int q0, b0;
+        cplx pinv, x;
+        flag = lane_pivot<NP>(v, w, pos, r, live, q0, b0, pinv, x) || flag;
+#pragma unroll
+        for (int a = 0; a < NP; ++a) {
+          if (r[a] == q0) {
+            live &= ~(1u << a);
+          } else {
+            v[a] = mul_xx(v[a], pinv);
+            w[a] = csub(w[a], mul_xy(v[a], x));
+          }
+          if (r[a] >= 0) {
+            Am[r[a] * lda + j] = v[a];
+          }
+          // the row that was at position j takes the pivot's old position
+          pos[a] = (r[a] == o0) ? b0 : pos[a];
+        }
+        int q1 = -1, b1 = -1;
+        if (two) {
+          flag = lane_pivot<NP>(w, v, pos, r, live, q1, b1, pinv, x) || flag;
+#pragma unroll
           for (int a = 0; a < NP; ++a) {
-            const int s = j + lane + 32 * a;
-            t[a] = (t[a] >= 0.) ? t[a] : 0.; // (NaN is no candidate)
-            if (s < nb && (lp == 0x7fffffff || t[a] > best)) {
-              best = t[a];
-              lp = s;
-              lr = r[a];
-              lv = v[a];
+            if (r[a] >= 0) {
+              Am[r[a] * lda + j + 1] =
+                  (r[a] == q0 || r[a] == q1) ? w[a] : mul_xx(w[a], pinv);
             }
-          }
-        };
-  #pragma unroll
-        for (int a = 0; a < NP; ++a) {
-          t[a] = fma(v[a].x, v[a].x, v[a].y * v[a].y);
-        }
-        pick();
-        cplx pinv = cinv_lu(lv);
-        warp_argmax(lp < nb ? (unsigned long long)__double_as_longlong(best) | top : 0ull,
-                    lp, bi, wl);
-        best = __shfl_sync(0xffffffffu, best, wl);
-        // |Q|^2 decides unless others come within rounding (see warp_pivot)
-        unsigned close = 0;
-  #pragma unroll
-        for (int a = 0; a < NP; ++a) {
-          close += (j + lane + 32 * a < nb && t[a] >= best * (1. - 0x1p-40)) ? 1u : 0u;
-        }
-        if (__reduce_add_sync(0xffffffffu, close) != 1u ||
-            !(best > 0x1p-900 && best < 0x1p900)) {
-  #pragma unroll
-          for (int a = 0; a < NP; ++a) {
-            t[a] = cabs_dev(v[a]);
-          }
-          pick();
-          pinv = cinv_lu(lv);
-          warp_argmax(lp < nb ? (unsigned long long)__double_as_longlong(best) | top : 0ull,
-                      lp, bi, wl);
-          flag = !(__shfl_sync(0xffffffffu, best, wl) > 0.) || flag;
-        }
-        const int p = __shfl_sync(0xffffffffu, lr, wl);
-        pinv.x = __shfl_sync(0xffffffffu, pinv.x, wl);
-        pinv.y = __shfl_sync(0xffffffffu, pinv.y, wl);
-  #pragma unroll
-        for (int a = 0; a < NP; ++a) {
-          if (j + lane + 32 * a < nb) {
-            Am[r[a] * lda + j] = (r[a] == p) ? v[a] : mul_xx(v[a], pinv);
           }
         }
         if (lane == 0) {
-          prow[j & 1] = p;
-          pbi[j & 1] = bi;
-          pold[j & 1] = r[0];
+          const int k = (j >> 1) & 1;
+          prow[k][0] = q0;
+          pbi[k][0] = b0;
+          pold[k][0] = o0;
+          prow[k][1] = q1;
+          pbi[k][1] = b1;
+          pold[k][1] = two ? ((b0 == j + 1) ? o0 : at[j + 1]) : -1;
         }
       };
-      const auto column = [&](int j, const cplx *pr) {
+      const auto columns = [&](int j, int p0, int p1) {
         if (nb - j <= 32) {
-          panel(std::integral_constant<int, 1>{}, j, pr);
+          panel(std::integral_constant<int, 1>{}, j, p0, p1);
         } else if (NBM <= 64 || nb - j <= 64) {
-          panel(std::integral_constant<int, 2>{}, j, pr);
+          panel(std::integral_constant<int, 2>{}, j, p0, p1);
         } else {
-          panel(std::integral_constant<int, NBM / 32>{}, j, pr);
+          panel(std::integral_constant<int, NBM / 32>{}, j, p0, p1);
         }
       };
       if (tid < 32) {
-        column(0, Am);
+        columns(0, 0, 0);
       }
       __syncthreads();
-      for (int i = 0; i < nb; ++i) {
-        const int p = prow[i & 1], bi = pbi[i & 1], o = pold[i & 1];
-        const cplx *pr = Am + p * lda;
+      int d0 = 0, d1 = -1; // pivot rows of the pair before
+      for (int i = 0; i < nb; i += 2) {
+        const int k2 = (i >> 1) & 1;
+        const int p0 = prow[k2][0], bi0 = pbi[k2][0], o0 = pold[k2][0];
+        const int p1 = prow[k2][1], bi1 = pbi[k2][1], o1 = pold[k2][1];
         if (tid < 32) {
           if (lane == 0) {
-            at[bi] = o;
-            at[i] = p;
+            at[bi0] = o0;
+            at[i] = p0;
+            if (p1 >= 0) {
+              at[bi1] = o1;
+              at[i + 1] = p1;
+            }
           }
           __syncwarp();
-          if (i + 1 < nb) {
-            column(i + 1, pr);
+          if (i + 2 < nb) {
+            columns(i + 2, p0, p1);
           }
-        } else if (i + 1 + tr - 2 < nb) {
-          const int s0 = i + 1 + tr - 2;
-          cplx l[NA], *row[NA];
-  #pragma unroll
-          for (int a = 0; a < NA; ++a) {
-            const int s = s0 + RT * a;
-            row[a] = Am;
-            l[a] = mkc(0., 0.);
-            if (s < nb) {
-              row[a] = Am + ((s == bi) ? o : at[s]) * lda;
-              l[a] = row[a][i];
+        } else {
+          if (d1 >= 0 && tr < 4) {
+            // the second pivot row of the pair before, which the others read
+            // without its first update until now
+            const cplx lp = Am[d1 * lda + i - 2];
+            for (int k = i + lane; k < nb; k += 32) {
+              Am[d1 * lda + k] = csub(Am[d1 * lda + k], mul_xy(lp, Am[d0 * lda + k]));
             }
           }
-          int k = i + 2 + tc;
-          for (; k + 16 < nb; k += 32) {
-            const cplx u0 = pr[k], u1 = pr[k + 16];
-            cplx v0[NA], v1[NA];
-  #pragma unroll
+          const int s0 = i + 2 + tr - 2;
+          if (s0 < nb) {
+            const cplx *pr0 = Am + p0 * lda, *pr1 = Am + p1 * lda;
+            const cplx lp = pr1[i];
+            cplx l0[NA], l1[NA], *row[NA];
+#pragma unroll
             for (int a = 0; a < NA; ++a) {
-              if (s0 + RT * a < nb) {
-                v0[a] = row[a][k];
-                v1[a] = row[a][k + 16];
+              const int s = s0 + RT * a;
+              row[a] = Am;
+              l0[a] = l1[a] = mkc(0., 0.);
+              if (s < nb) {
+                row[a] = Am + ((s == bi1) ? o1 : (s == bi0) ? o0 : at[s]) * lda;
+                l0[a] = row[a][i];
+                l1[a] = row[a][i + 1];
               }
             }
-  #pragma unroll
-            for (int a = 0; a < NA; ++a) {
-              if (s0 + RT * a < nb) {
-                row[a][k] = csub(v0[a], mul_xy(l[a], u0));
-                row[a][k + 16] = csub(v1[a], mul_xy(l[a], u1));
+            for (int k = i + 4 + tc; k < nb; k += 16) {
+              const cplx u0 = pr0[k];
+              const cplx u1 = csub(pr1[k], mul_xy(lp, u0));
+              cplx v[NA];
+#pragma unroll
+              for (int a = 0; a < NA; ++a) {
+                if (s0 + RT * a < nb) {
+                  v[a] = row[a][k];
+                }
               }
-            }
-          }
-          if (k < nb) {
-            const cplx u = pr[k];
-            cplx v[NA];
-  #pragma unroll
-            for (int a = 0; a < NA; ++a) {
-              if (s0 + RT * a < nb) {
-                v[a] = row[a][k];
-              }
-            }
-  #pragma unroll
-            for (int a = 0; a < NA; ++a) {
-              if (s0 + RT * a < nb) {
-                row[a][k] = csub(v[a], mul_xy(l[a], u));
+#pragma unroll
+              for (int a = 0; a < NA; ++a) {
+                if (s0 + RT * a < nb) {
+                  row[a][k] = csub(csub(v[a], mul_xy(l0[a], u0)), mul_xy(l1[a], u1));
+                }
               }
             }
           }
+          d0 = p0;
+          d1 = p1;
         }
         __syncthreads();
       }
