@@ -1943,10 +1943,11 @@ static void launch_apart(const TmxBlockArgs &a, cudaStream_t stream) {
   // factors in shared memory up to 118 members, above that in the scratch
   const size_t smem = std::min<size_t>((size_t)max_nb * (max_nb | 1) * sizeof(cplx),
                                        TMX_FACTOR_SMEM_MAX);
+  // (the limit, not this launch's size: another thread may set it in between)
   cudaFuncSetAttribute(k_factor<NBM, UW, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+                       (int)TMX_FACTOR_SMEM_MAX);
   cudaFuncSetAttribute(k_solve<NBM, NTHS, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+                       (int)TMX_FACTOR_SMEM_MAX);
   k_factor<NBM, UW, MINB><<<ctas(1), 32 + 32 * UW, smem, stream>>>(a, smem);
   k_solve<NBM, NTHS, C><<<ctas(chunks), NTHS, smem, stream>>>(a, chunks, smem);
 }

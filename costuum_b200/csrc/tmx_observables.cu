@@ -898,6 +898,11 @@ void tmx_launch_cg(int nmax, const int64_t *cg_off, double *cg, double *work,
   k_cg<<<blocks, 128, 0, stream>>>(nmax, cg_off, cg, work);
 }
 
+// The attribute is the block's limit, not the launch's size: threads with
+// contexts of their own launch the same kernel with different sizes, and one
+// that lowered it between another's set and launch would fail that launch.
+#define TMX_OBS_SMEM_MAX (227 * 1024)
+
 template <int NT>
 static void launch_orient(const TmxObsGrain *og, const int32_t *order,
                           const TmxOrientRange *rng, int nrng, int64_t nitems, int ncap,
@@ -908,7 +913,7 @@ static void launch_orient(const TmxObsGrain *og, const int32_t *order,
   const int rows = ncap + 1;
   const size_t smem = (size_t)4 * 2 * ((rows + 7) & ~7) * (8 * NT + 4) * sizeof(double);
   cudaFuncSetAttribute(k_orient<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+                       TMX_OBS_SMEM_MAX);
   k_orient<NT><<<dim3((unsigned)((nitems + 3) / 4), nmat), 128, smem, stream>>>(
       og, order, rng, nrng, nitems, rows, mats, coeffs, ncoef, cg_off, cg, cg_nmax, fold);
 }
@@ -947,7 +952,7 @@ static void launch_amp(const TmxAmpGroup *groups, const int32_t *ins,
   constexpr int NA = 4 * NT, VS = (NA > 8) ? 18 : 10;
   const size_t smem = (size_t)lcap * (2 * NA * 2 * sizeof(double2) + 2 * VS * sizeof(double));
   cudaFuncSetAttribute(k_amp<NT, NTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+                       TMX_OBS_SMEM_MAX);
   k_amp<NT, NTH><<<dim3((unsigned)nitems, nmat), NTH, smem, stream>>>(
       groups, ins, pairs, rng, nrng, og, mats, wpi, wtau, wnmax, x, xstride, lcap);
 }
