@@ -232,6 +232,8 @@ struct tmx_ctx {
   // round streams, their bucket streams (stream2, stream3, aux[0..5]) and
   // the copy stream
   cudaEvent_t drain_ev[9] = {};
+  // the last set-up on `stream` that block rounds on other streams wait for
+  cudaEvent_t setup_ev = nullptr;
   // device-to-host copies of streamed T-matrices (created with the first
   // sink copy): a round's copy waits for the round, the rounds that follow
   // on the same round stream do not wait for the copy

@@ -414,6 +414,9 @@ void tmx_destroy(tmx_ctx *ctx) {
       cudaEventDestroy(e);
     }
   }
+  if (ctx->setup_ev) {
+    cudaEventDestroy(ctx->setup_ev);
+  }
   if (ctx->gm_exec) {
     cudaGraphExecDestroy(ctx->gm_exec);
   }
@@ -610,12 +613,6 @@ int tmx_batch_upload(tmx_ctx *ctx, int64_t n, const double *r_ev,
   return TMX_OK;
 }
 
-// One round of phase 2: every (grain, m, class) block of the grains in p2 at
-// their orders (ctx->nmax_h / ctx->ngauss_h), launched on stream `st`, with
-// T-matrices from complex offset t_base on (keep_T: T already holds earlier
-// rounds below t_base). The schedule is kept in the context (p2 buffers and
-// ctx->p2_*) for the tangent kernels. Host-side setup runs on ctx->stream
-// (Wigner tables), which the round then waits for.
 // buffers of the Q sums of the batch's n grains; the counters behind the
 // partial sums start at zero wherever n puts them
 static int ensure_qsums(tmx_ctx *ctx) {
@@ -633,6 +630,12 @@ static int ensure_qsums(tmx_ctx *ctx) {
   return TMX_OK;
 }
 
+// One round of phase 2: every (grain, m, class) block of the grains in p2 at
+// their orders (ctx->nmax_h / ctx->ngauss_h), launched on stream `st`, with
+// T-matrices from complex offset t_base on (keep_T: T already holds earlier
+// rounds below t_base). The schedule is kept in the context (p2 buffers and
+// ctx->p2_*) for the tangent kernels. Set-up runs on ctx->stream (Wigner tables,
+// a larger T, the Q sums' counters); the round and those after it wait for it.
 static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
                             cudaStream_t st, int64_t t_base, bool keep_T,
                             int64_t *t_end, bool temp = false,
@@ -642,6 +645,7 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
   const int np2 = (int)p2.size();
   const int64_t wig_used0 = ctx->wig_used;
   const void *T_before = ctx->T.p;
+  const size_t T_cap = ctx->T.cap;
   const int64_t q_before = ctx->q_n;
   if (!keep_T) {
     ctx->sink_done = 0; // a new set of T-matrices starts at offset 0
@@ -797,16 +801,20 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
   if (np2 == 0) {
     return TMX_OK;
   }
-  if (st != ctx->stream && (!temp || ctx->wig_used != wig_used0 ||
-                            ctx->T.p != T_before || ctx->q_n != q_before)) {
-    // new Wigner tables or a moved T / Q-sum buffer above are ordered on
-    // ctx->stream (a round of the order loop that needs none of them does
-    // not wait for the orders queued there)
-    cudaEvent_t ready;
-    CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
-    CK(cudaEventRecord(ready, ctx->stream));
-    CK(cudaStreamWaitEvent(st, ready, 0));
-    CK(cudaEventDestroy(ready));
+  if (st != ctx->stream) {
+    // new Wigner tables, a moved T and the cleared counters of the Q sums are
+    // ordered on ctx->stream, behind the orders queued there. The round that
+    // asked for them waits, and so does every later one: it may run on the
+    // other round stream and reads the same tables and counters. (A batch that
+    // needs none of them does not wait for the orders.)
+    if (!ctx->setup_ev) {
+      CK(cudaEventCreateWithFlags(&ctx->setup_ev, cudaEventDisableTiming));
+    }
+    if (!temp || ctx->wig_used != wig_used0 || ctx->T.p != T_before ||
+        ctx->T.cap != T_cap || ctx->q_n != q_before) {
+      CK(cudaEventRecord(ctx->setup_ev, ctx->stream));
+    }
+    CK(cudaStreamWaitEvent(st, ctx->setup_ev, 0));
   }
   // buffers of this round: the persistent p2 set, or (temp) stream-ordered
   // allocations on `st` that are released after the round's launches
