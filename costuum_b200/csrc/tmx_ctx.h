@@ -13,6 +13,7 @@
 #include "../../include/tmx.h"
 #include "tmx_common.cuh"
 #include "tmx_kernels.h"
+#include "tmx_qsum_state.h"
 
 namespace {
 
@@ -57,7 +58,7 @@ struct tmx_ctx {
   DevBuf grains, state, state0, act0, act1, actinit, count, slots, items, tab,
       nsc, scratch, diag, T, q, status, probe;
   DevBuf q_part;    // partial Q sums of the larger grains
-  int64_t q_n = -1; // grains q and q_part are laid out for
+  TmxQsumState qs;  // what q and q_part are laid out for
   // uploaded batch (device-resident inputs)
   bool uploaded = false;
   int64_t up_n = 0;

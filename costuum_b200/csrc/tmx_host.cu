@@ -616,17 +616,29 @@ int tmx_batch_upload(tmx_ctx *ctx, int64_t n, const double *r_ev,
 // buffers of the Q sums of the batch's n grains; the counters behind the
 // partial sums start at zero wherever n puts them
 static int ensure_qsums(tmx_ctx *ctx) {
-  if (ctx->q_n == ctx->n) {
-    return TMX_OK;
-  }
   const size_t bytes = std::max<size_t>(16, tmx_qsum_part_bytes(ctx->n));
-  int rc;
-  if ((rc = ensure(ctx, ctx->q, std::max<int64_t>(1, 2 * ctx->n) * sizeof(double))) ||
-      (rc = ensure(ctx, ctx->q_part, bytes))) {
-    return rc;
+  return ctx->qs.layout(
+      ctx->n,
+      [&] {
+        const int rc =
+            ensure(ctx, ctx->q, std::max<int64_t>(1, 2 * ctx->n) * sizeof(double));
+        return rc ? rc : ensure(ctx, ctx->q_part, bytes);
+      },
+      [&]() -> int {
+        CK(cudaMemsetAsync(ctx->q_part.p, 0, bytes, ctx->stream));
+        return TMX_OK;
+      });
+}
+
+// start of a batch's block rounds: those of a batch that ended early are waited for
+static int begin_qsums(tmx_ctx *ctx) {
+  if (ctx->qs.begin()) {
+    for (cudaStream_t x : {ctx->stream, ctx->stream2, ctx->stream3, ctx->aux[0],
+                           ctx->aux[1], ctx->aux[2], ctx->aux[3], ctx->aux[4],
+                           ctx->aux[5]}) {
+      CK(cudaStreamSynchronize(x));
+    }
   }
-  CK(cudaMemsetAsync(ctx->q_part.p, 0, bytes, ctx->stream));
-  ctx->q_n = ctx->n;
   return TMX_OK;
 }
 
@@ -642,11 +654,14 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
                             bool keep_lu = false) {
   int rc;
   NvtxRange blocks_range("tmx_blocks");
+  if (!keep_T && (rc = begin_qsums(ctx))) {
+    return rc;
+  }
   const int np2 = (int)p2.size();
   const int64_t wig_used0 = ctx->wig_used;
   const void *T_before = ctx->T.p;
   const size_t T_cap = ctx->T.cap;
-  const int64_t q_before = ctx->q_n;
+  const int64_t q_before = ctx->qs.n;
   if (!keep_T) {
     ctx->sink_done = 0; // a new set of T-matrices starts at offset 0
   }
@@ -789,7 +804,7 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
       (rc = ensure(ctx, ctx->lu, std::max<int64_t>(1, scr_total) * sizeof(cplx)))) {
     return rc;
   }
-  if (ctx->q_n != ctx->n) {
+  if (ctx->qs.n != ctx->n) {
     // Q sums of every grain of the batch; rounds on the round streams may
     // still write the old buffer
     CK(cudaStreamSynchronize(ctx->stream2));
@@ -811,7 +826,7 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
       CK(cudaEventCreateWithFlags(&ctx->setup_ev, cudaEventDisableTiming));
     }
     if (!temp || ctx->wig_used != wig_used0 || ctx->T.p != T_before ||
-        ctx->T.cap != T_cap || ctx->q_n != q_before) {
+        ctx->T.cap != T_cap || ctx->qs.n != q_before) {
       CK(cudaEventRecord(ctx->setup_ev, ctx->stream));
     }
     CK(cudaStreamWaitEvent(st, ctx->setup_ev, 0));
@@ -1086,6 +1101,7 @@ static int finish_blocks(tmx_ctx *ctx, int64_t t_total, int rounds,
   if (ctx->prof_used > 8192 && (rc = prof_resolve(ctx))) {
     return rc;
   }
+  ctx->qs.end();
   ctx->have_batch = true;
   return TMX_OK;
 }
@@ -1146,6 +1162,7 @@ int tmx_rerun_blocks(tmx_ctx *ctx) {
     return rc;
   }
   CK(cudaStreamSynchronize(ctx->stream));
+  ctx->qs.end();
   ctx->p2_t_total = t_end;
   ctx->p2_rounds = 1;
   ctx->lu_ready = true;
@@ -1335,7 +1352,7 @@ static int gm_compute(tmx_ctx *ctx) {
       (rc = ensure(ctx, ctx->T, t_cap * sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->gm_lu, lu_cap * sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->gm_luscr, lu_cap * sizeof(cplx))) ||
-      (rc = ensure_qsums(ctx))) {
+      (rc = begin_qsums(ctx)) || (rc = ensure_qsums(ctx))) {
     return rc;
   }
   TmxItem *bitems[TMX_GM_BUCKETS];
