@@ -1972,9 +1972,9 @@ int tmx_block_family_capacity(int family) {
 // The family given in a.family (set by the host's dispatch table), else the
 // smallest one whose capacity covers a.max_nb. A family whose capacity is
 // below an item's class size flags that grain TMX_ST_TOO_LARGE.
-void tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream) {
+int tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream) {
   if (a.nitems <= 0) {
-    return;
+    return 0;
   }
   int f = a.family;
   if (f < 0 || f >= TMX_BLOCK_FAMILIES) {
@@ -1987,18 +1987,19 @@ void tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream) {
   switch (f) {
   case TMX_BLOCKS_WARP_DFMA:
     launch_warp_variant<1, 2, TMX_WARP_DFMA_MINB, false>(a, stream);
-    return;
+    return 1;
   case TMX_BLOCKS_WARP_DMMA:
     launch_warp_variant<1, 1, TMX_WARP_DMMA_MINB, true>(a, stream);
-    return;
+    return 1;
   case TMX_BLOCKS_CTA32:
     launch_cta32(a, stream);
-    return;
+    return 1;
   case TMX_BLOCKS_CTA64:
     launch_apart<true, 64, 8, 2, 512, 8>(a, stream);
-    return;
+    return 3;
   default:
     launch_apart<false, 128, 15, 1, 512, 16>(a, stream);
+    return 3;
   }
 }
 

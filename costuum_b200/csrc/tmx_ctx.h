@@ -268,11 +268,12 @@ struct tmx_ctx {
     }                                                                          \
   } while (0)
 
-#define LAUNCHED()                                                             \
+#define LAUNCHED_N(n)                                                          \
   do {                                                                         \
-    ++ctx->launches;                                                           \
+    ctx->launches += (n);                                                      \
     CK(cudaGetLastError());                                                    \
   } while (0)
+#define LAUNCHED() LAUNCHED_N(1)
 
 // Makes ctx->stream wait for everything queued so far on the other streams
 // of the context. Every free of a shared buffer (Wigner and quadrature

@@ -944,8 +944,7 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
         CK(cudaEventCreate(&tb));
         CK(cudaEventRecord(ta, bs));
       }
-      tmx_launch_blocks(B, bs);
-      LAUNCHED();
+      LAUNCHED_N(tmx_launch_blocks(B, bs));
       if (ctx->tuning) {
         CK(cudaEventRecord(tb, bs));
         ctx->tune_ev.emplace_back(dispatch_bucket(B.max_nb), ta, tb);
@@ -1390,10 +1389,6 @@ static int gm_compute(tmx_ctx *ctx) {
                           &ctx->gl_x, &ctx->gl_w, &ctx->gl_off, &ctx->wig, &ctx->wig_off}) {
     key.push_back((uint64_t)(uintptr_t)b->p);
   }
-  int nbk = 0; // size buckets a round launches
-  for (int b = 0; b < TMX_GM_BUCKETS; ++b) {
-    nbk += (bcap[b] > 0) ? 1 : 0;
-  }
   if (key != ctx->gm_key || !ctx->gm_exec) {
     if (ctx->gm_exec) {
       CK(cudaGraphExecDestroy(ctx->gm_exec));
@@ -1520,7 +1515,7 @@ static int gm_compute(tmx_ctx *ctx) {
         B.max_nb = (k + 1) / 2;
         B.family = ctx->dispatch[gm_bucket(B.max_nb)];
         B.max_ctas = 148 * 8;
-        tmx_launch_blocks(B, cs);
+        const int nblk = tmx_launch_blocks(B, cs);
         TmxChainGroup one = {};
         one.n = 1;
         one.order0 = k;
@@ -1552,7 +1547,7 @@ static int gm_compute(tmx_ctx *ctx) {
         KA.keep_tab = (int64_t *)ctx->keep_tab.p;
         KA.keep_q = (int64_t *)ctx->keep_q.p;
         tmx_launch_keep_tables(KA, (int)n, cs);
-        tmx_launch_gm_step_end(G, snap, outz, j, out, -1, k + 1, 7, cs);
+        tmx_launch_gm_step_end(G, snap, outz, j, out, -1, k + 1, 6 + nblk, cs);
         CK(cudaGetLastError());
         return 0;
       };
@@ -1614,7 +1609,7 @@ static int gm_compute(tmx_ctx *ctx) {
         B.status = (int32_t *)ctx->status.p;
         B.max_nb = (kl + 1) / 2;
         B.family = ctx->dispatch[gm_bucket(B.max_nb)];
-        tmx_launch_blocks(B, cs);
+        const int nblk = tmx_launch_blocks(B, cs);
         CK(cudaMemsetAsync(&G->cnt[out], 0, sizeof(int32_t), cs));
         tmx_launch_converge(act_in, chunk, grp, (const TmxSlot *)ctx->gm_slots.p,
                             (const cplx *)ctx->gm_diag.p, (TmxChainState *)ctx->state.p,
@@ -1641,7 +1636,7 @@ static int gm_compute(tmx_ctx *ctx) {
         KA.keep_q = (int64_t *)ctx->keep_q.p;
         tmx_launch_keep_tables(KA, (int)n, cs);
         tmx_launch_gm_relist(G, act_out, act_in, (int)n, in, out, cs);
-        tmx_launch_gm_step_end(G, snap, outz, j, out, in, k + gk, 7, cs);
+        tmx_launch_gm_step_end(G, snap, outz, j, out, in, k + gk, 6 + nblk, cs);
         CK(cudaGetLastError());
         return 0;
       };
@@ -1714,6 +1709,7 @@ static int gm_compute(tmx_ctx *ctx) {
         return rc;
       }
       auto exec_body = [&]() -> int {
+        int nblk = 0; // kernels of the size buckets
         for (int b = TMX_GM_BUCKETS - 1; b >= 0; --b) {
           if (bcap[b] == 0) {
             continue;
@@ -1741,7 +1737,7 @@ static int gm_compute(tmx_ctx *ctx) {
           R.lu = (cplx *)ctx->gm_lu.p;
           R.family = ctx->dispatch[b];
           R.max_ctas = TMX_GM_ROUND_CTAS;
-          tmx_launch_blocks(R, bs);
+          nblk += tmx_launch_blocks(R, bs);
         }
         // (joined only after every bucket has forked, so that they run
         // side by side)
@@ -1754,7 +1750,7 @@ static int gm_compute(tmx_ctx *ctx) {
         tmx_launch_qsums((const TmxSlot *)ctx->gm_rslots.p, (int)n, (const cplx *)ctx->T.p,
                          (double *)ctx->q.p, (double *)ctx->q_part.p, n, Kg, rs,
                          &G->srng[rsl][0], 148 * 4);
-        tmx_launch_gm_round_end(G, 5 + nbk, rs);
+        tmx_launch_gm_round_end(G, 5 + nblk, rs);
         CK(cudaGetLastError());
         return 0;
       };
@@ -2176,8 +2172,7 @@ int tmx_batch_compute(tmx_ctx *ctx) {
       if ((rc2 = prof_begin(ctx, 0, &pe))) {
         return rc2;
       }
-      tmx_launch_blocks(B, st);
-      LAUNCHED();
+      LAUNCHED_N(tmx_launch_blocks(B, st));
       if ((rc2 = prof_end(ctx, 0, pe, fl, nullptr, 0., B.nitems))) {
         return rc2;
       }

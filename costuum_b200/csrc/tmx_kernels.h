@@ -73,7 +73,8 @@ struct TmxBlockArgs {
 };
 // largest class size each tmx_block_family can run
 int tmx_block_family_capacity(int family);
-void tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream);
+// returns the kernels launched (0, 1 or, for the families above 32 members, 3)
+int tmx_launch_blocks(const TmxBlockArgs &a, cudaStream_t stream);
 
 // slots and m = 0 items of one order step from the active list
 // buffer offsets of one order's slots in a (possibly speculative) group of

@@ -1344,8 +1344,7 @@ extern "C" int tmx_batch_gradients(tmx_ctx *ctx, int32_t ntheta,
           B.max_nb = max_nb;
           B.family = dispatch_family(ctx, max_nb);
           B.lu = v.lu;
-          tmx_launch_blocks(B, gs);
-          LAUNCHED();
+          LAUNCHED_N(tmx_launch_blocks(B, gs));
         }
         TmxTangentArgs A;
         A.items = v.items + i0;
