@@ -1274,10 +1274,24 @@ extern "C" int tmx_batch_gradients(tmx_ctx *ctx, int32_t ntheta,
     return seg;
   };
   std::vector<RoundView> views;
+  // scratch of a round's tangents: only the classes above 32 members keep dQ
+  // and dRgQ in memory (tmx_launch_tangents). Rounds made by the host lay the
+  // items' scratch out largest first, so theirs is the front of it; a round
+  // made on the device mixes the sizes.
+  auto large_scratch = [](const std::vector<int> &nb) {
+    int64_t s = 0;
+    for (size_t i = 0; i < nb.size() && nb[i] > 32; ++i) {
+      s += tmx_item_scratch(nb[i]);
+    }
+    return s;
+  };
   if (ctx->rounds_lu) {
     for (const auto &r : ctx->rounds_kept) {
-      views.push_back({r.items, r.slots, r.tab, r.nsc, r.lu,
-                       r.seg.empty() ? segments(r.nb) : r.seg, r.scr_total});
+      const bool host = r.seg.empty();
+      const auto seg = host ? segments(r.nb) : r.seg;
+      const bool large = !seg.empty() && seg[0][2] > 32;
+      views.push_back({r.items, r.slots, r.tab, r.nsc, r.lu, seg,
+                       host ? large_scratch(r.nb) : large ? r.scr_total : 0});
     }
   } else {
     if ((rc = ensure(ctx, ctx->lu, std::max<int64_t>(1, ctx->p2_scr_total) * sizeof(cplx)))) {
@@ -1285,7 +1299,8 @@ extern "C" int tmx_batch_gradients(tmx_ctx *ctx, int32_t ntheta,
     }
     views.push_back({(const TmxItem *)ctx->p2items.p, (const TmxSlot *)ctx->p2slots.p,
                      (const double *)ctx->p2tab.p, (const double *)ctx->p2nsc.p,
-                     (cplx *)ctx->lu.p, segments(ctx->p2_nb), ctx->p2_scr_total});
+                     (cplx *)ctx->lu.p, segments(ctx->p2_nb),
+                     large_scratch(ctx->p2_nb)});
   }
   // each round's tangent scratch in its own region: the rounds' size
   // buckets run concurrently
