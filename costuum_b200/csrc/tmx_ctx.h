@@ -81,7 +81,7 @@ struct tmx_ctx {
     int64_t nitems = 0;
   };
   struct AmpChunk {
-    int g0 = 0, g1 = 0, nin = 1, nitem_max = 1;
+    int g0 = 0, g1 = 0, nin = 1, nitem_max = 1, pass = 0;
     std::vector<AmpLaunch> launches;
   };
   std::vector<AmpChunk> o_chunks;
@@ -93,8 +93,9 @@ struct tmx_ctx {
     int64_t nitems = 0;
   };
   std::vector<OrientLaunch> o_orient;
-  // angles of the current plan (o_angles) and their pi / tau columns
-  int o_nangles = 0;
+  // angles of the current plan (o_angles) by pass: first, number; and the pi /
+  // tau columns of one pass
+  std::vector<std::array<int64_t, 2>> o_passes;
   DevBuf o_wcol;
   // flops of one matrix set in the orientation average and the amplitudes
   // of the current plan (counted while profiling)

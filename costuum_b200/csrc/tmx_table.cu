@@ -11,7 +11,6 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
-#include <map>
 #include <system_error>
 #include <thread>
 #include <unordered_map>
@@ -379,62 +378,151 @@ struct AmpJob {
 
 // groups of a set of jobs (TmxAmpGroup without a grain): by distinct incoming
 // angle in order of first use, at most TMX_AMP_NIN of them and about
-// kGroupPairs pairs per group
+// kGroupPairs pairs per group. The pi and tau columns of the plan's angles (16
+// bytes per order and block m of each) are in memory kColumnBytes at a time:
+// where the angles need more, the groups go in passes, each with the angles it
+// uses renumbered, and an angle that several passes use has its columns made in
+// each of them (a column costs as much as one product with one).
 struct AmpPlan {
   static constexpr int kGroupPairs = 512;
+  static constexpr int64_t kColumnBytes = (int64_t)512 << 20;
+  struct Pass {
+    int g0, g1;     // groups
+    int64_t a0, na; // angles
+  };
   std::vector<int32_t> ins;
   std::vector<TmxAmpPair> pairs;
   std::vector<TmxAmpGroup> groups;
+  std::vector<Pass> passes;
+  std::vector<int32_t> angles; // angle of each number of each pass, if split
+  bool split;
+
+  // nang angles in all, orders of at most nmax
+  AmpPlan(int64_t nang, int nmax)
+      : split(nang > pass_angles(nmax)), nang_(nang), cap_(pass_angles(nmax)) {
+    if (split) {
+      number_.resize(nang);
+      number_pass_.assign(nang, -1);
+    }
+    slot_.assign(nang, -1);
+    passes.push_back({0, 0, 0, split ? 0 : nang});
+  }
+
+  // (a group's angles always fit a pass)
+  static int64_t pass_angles(int nmax) {
+    return std::max<int64_t>(kGroupPairs + TMX_AMP_NIN + 1,
+                             kColumnBytes / (16 * (int64_t)(nmax + 1) * nmax));
+  }
 
   // returns the new groups [first, second)
-  std::pair<int, int> add(const std::vector<AmpJob> &jobs) {
+  std::pair<int, int> add(const AmpJob *jobs, size_t n) {
     const int g0 = (int)groups.size();
-    std::map<int32_t, int> seen;
-    std::vector<int32_t> angle;
-    std::vector<std::vector<const AmpJob *>> by;
-    for (const AmpJob &j : jobs) {
-      const auto it = seen.emplace(j.ain, (int)by.size());
-      if (it.second) {
-        angle.push_back(j.ain);
-        by.emplace_back();
+    // jobs by incoming angle: a stable counting sort
+    start_.assign(1, 0);
+    first_.clear();
+    for (size_t j = 0; j < n; ++j) {
+      int32_t &s = slot_[jobs[j].ain];
+      if (s < 0) {
+        s = (int32_t)first_.size();
+        first_.push_back(jobs[j].ain);
+        start_.push_back(0);
       }
-      by[it.first->second].push_back(&j);
+      ++start_[s + 1];
+    }
+    for (size_t a = 1; a < start_.size(); ++a) {
+      start_[a] += start_[a - 1];
+    }
+    sorted_.resize(n);
+    pos_.assign(start_.begin(), start_.end() - 1);
+    for (size_t j = 0; j < n; ++j) {
+      sorted_[pos_[slot_[jobs[j].ain]]++] = (int64_t)j;
     }
     TmxAmpGroup g = {};
-    const auto close = [&]() {
+    const auto close_group = [&]() {
       if (g.npair > 0) {
+        number(g);
         groups.push_back(g);
+        passes.back().g1 = (int)groups.size();
       }
       g = TmxAmpGroup{};
     };
-    for (size_t a = 0; a < by.size(); ++a) {
-      for (size_t j = 0; j < by[a].size(); ++j) {
-        if (g.npair >= kGroupPairs || (j == 0 && g.nin == TMX_AMP_NIN)) {
-          close();
+    for (size_t a = 0; a < first_.size(); ++a) {
+      for (int64_t q = start_[a]; q < start_[a + 1]; ++q) {
+        const AmpJob &J = jobs[sorted_[q]];
+        const bool fresh = q == start_[a];
+        if (g.npair >= kGroupPairs || (fresh && g.nin == TMX_AMP_NIN)) {
+          close_group();
         }
         if (g.npair == 0) {
           g.in0 = (int32_t)ins.size();
           g.pair0 = (int32_t)pairs.size();
         }
-        if (j == 0 || g.nin == 0) {
-          ins.push_back(angle[a]);
+        if (fresh || g.nin == 0) {
+          ins.push_back(J.ain);
           ++g.nin;
         }
         TmxAmpPair p;
         p.in = g.nin - 1;
-        p.angle_out = by[a][j]->aout;
-        p.nphi = by[a][j]->nphi;
+        p.angle_out = J.aout;
+        p.nphi = J.nphi;
         p.pref = g.nitem;
-        p.phi0 = by[a][j]->phi0;
-        p.out = by[a][j]->out;
+        p.phi0 = J.phi0;
+        p.out = J.out;
         pairs.push_back(p);
         ++g.npair;
         g.nitem += p.nphi;
       }
     }
-    close();
+    close_group();
+    for (int32_t a : first_) {
+      slot_[a] = -1;
+    }
     return {g0, (int)groups.size()};
   }
+
+private:
+  // the group's angles by their numbers in its pass, a new one if they do not
+  // fit the present one
+  void number(const TmxAmpGroup &g) {
+    if (!split) {
+      return;
+    }
+    const int64_t before = (int64_t)angles.size();
+    const auto see = [&](int32_t a) {
+      if (number_pass_[a] != (int32_t)passes.size()) {
+        number_pass_[a] = (int32_t)passes.size();
+        number_[a] = (int32_t)((int64_t)angles.size() - passes.back().a0);
+        angles.push_back(a);
+      }
+    };
+    const auto see_all = [&]() {
+      for (int32_t k = 0; k < g.nin; ++k) {
+        see(ins[g.in0 + k]);
+      }
+      for (int32_t k = 0; k < g.npair; ++k) {
+        see(pairs[g.pair0 + k].angle_out);
+      }
+    };
+    see_all();
+    if ((int64_t)angles.size() - passes.back().a0 > cap_) {
+      angles.resize(before);
+      const int n = (int)groups.size();
+      passes.push_back({n, n, before, 0});
+      see_all();
+    }
+    passes.back().na = (int64_t)angles.size() - passes.back().a0;
+    for (int32_t k = 0; k < g.nin; ++k) {
+      ins[g.in0 + k] = number_[ins[g.in0 + k]];
+    }
+    for (int32_t k = 0; k < g.npair; ++k) {
+      int32_t &a = pairs[g.pair0 + k].angle_out;
+      a = number_[a];
+    }
+  }
+
+  int64_t nang_, cap_;
+  std::vector<int32_t> slot_, first_, number_, number_pass_;
+  std::vector<int64_t> start_, pos_, sorted_;
 };
 
 // groups [g0, g1) of a plan for one grain, their S from out0 on
@@ -447,9 +535,10 @@ struct AmpUse {
 // Work plan of the observable kernels for the grains `og` (already on the
 // device in ctx->o_og): the orientation kernel's pair-major order and the
 // amplitude kernel's groups of every grain (`uses`, by descending order) in
-// launches of blocks of similar size.
+// launches of blocks of similar size. ang: the angles the plan's jobs name.
 int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
-                    const AmpPlan &plan, std::vector<AmpUse> uses) {
+                    const std::vector<TmxAngle> &ang, const AmpPlan &plan,
+                    std::vector<AmpUse> uses) {
   int rc0;
   ++ctx->plan_seq;
   cudaStream_t st = ctx->stream;
@@ -515,13 +604,17 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
     return og[a.grain].nmax > og[b.grain].nmax;
   });
   std::vector<TmxAmpGroup> grp;
-  for (const AmpUse &u : uses) {
-    for (int k = u.g0; k < u.g1; ++k) {
-      TmxAmpGroup g = plan.groups[k];
-      g.grain = u.grain;
-      g.out0 = u.out0;
-      grp.push_back(g);
+  std::vector<size_t> pass_end; // groups of the passes, one after the other
+  for (const AmpPlan::Pass &p : plan.passes) {
+    for (const AmpUse &u : uses) {
+      for (int k = std::max(u.g0, p.g0); k < std::min(u.g1, p.g1); ++k) {
+        TmxAmpGroup g = plan.groups[k];
+        g.grain = u.grain;
+        g.out0 = u.out0;
+        grp.push_back(g);
+      }
     }
+    pass_end.push_back(grp.size());
   }
   // chunks of groups whose m sums fit the X buffer, and per chunk one launch
   // per block size: ranges of groups whose block m has lo < L <= hi orders
@@ -529,12 +622,17 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
   std::vector<TmxAmpRange> rng;
   const int64_t x_cap = (int64_t)1 << 24; // complex elements per matrix
   int64_t x_max = 1;
+  int pass = 0;
   for (size_t g0 = 0; g0 < grp.size();) {
+    while (g0 >= pass_end[pass]) {
+      ++pass;
+    }
     tmx_ctx::AmpChunk ch;
     ch.g0 = (int)g0;
+    ch.pass = pass;
     int64_t x = 0;
     size_t g1 = g0;
-    for (; g1 < grp.size(); ++g1) {
+    for (; g1 < pass_end[pass]; ++g1) {
       const int64_t need = (int64_t)grp[g1].npair * (og[grp[g1].grain].nmax + 1) * 4;
       if (g1 > g0 && x + need > x_cap) {
         break;
@@ -588,7 +686,18 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
     CK(cudaMemcpyAsync(buf.p, src, bytes, cudaMemcpyHostToDevice, st));
     return TMX_OK;
   };
-  if ((rc = put(ctx->o_orng, orng.data(), orng.size() * sizeof(TmxOrientRange))) ||
+  // angles of the passes, one after the other
+  std::vector<TmxAngle> by_pass;
+  for (int32_t a : plan.angles) {
+    by_pass.push_back(ang[a]);
+  }
+  const std::vector<TmxAngle> &table = plan.split ? by_pass : ang;
+  ctx->o_passes.clear();
+  for (const AmpPlan::Pass &p : plan.passes) {
+    ctx->o_passes.push_back({p.a0, p.na});
+  }
+  if ((rc = put(ctx->o_angles, table.data(), table.size() * sizeof(TmxAngle))) ||
+      (rc = put(ctx->o_orng, orng.data(), orng.size() * sizeof(TmxOrientRange))) ||
       (rc = put(ctx->o_grp, grp.data(), grp.size() * sizeof(TmxAmpGroup))) ||
       (rc = put(ctx->o_ins, plan.ins.data(), plan.ins.size() * sizeof(int32_t))) ||
       (rc = put(ctx->o_prs, plan.pairs.data(), plan.pairs.size() * sizeof(TmxAmpPair))) ||
@@ -687,20 +796,28 @@ int run_amplitudes(tmx_ctx *ctx, const cplx *const *Tsrc, int nmat,
   if ((rc = prof_begin(ctx, TMX_PROF_AMP, &pe))) {
     return rc;
   }
-  // the pi / tau columns of every angle of the plan, once for all grains
+  // the pi / tau columns of the angles of a pass, once for all grains
   const int wn = ctx->o_nbmax;
-  const size_t wcol = (size_t)ctx->o_nangles * (wn + 1) * wn;
+  int64_t na = 0;
+  for (const auto &p : ctx->o_passes) {
+    na = std::max(na, p[1]);
+  }
+  const size_t wcol = (size_t)na * (wn + 1) * wn;
   if ((rc = ensure(ctx, ctx->o_wcol, std::max<size_t>(1, 2 * wcol) * sizeof(double)))) {
     return rc;
   }
   double *wpi = (double *)ctx->o_wcol.p, *wtau = wpi + wcol;
-  tmx_launch_wigner_cols((const TmxAngle *)ctx->o_angles.p, ctx->o_nangles, wn, wpi,
-                         wtau, st);
-  LAUNCHED();
   const TmxAmpGroup *grp = (const TmxAmpGroup *)ctx->o_grp.p;
   const TmxAmpPair *prs = (const TmxAmpPair *)ctx->o_prs.p;
   const TmxObsGrain *og = (const TmxObsGrain *)ctx->o_og.p;
+  int pass = -1;
   for (const tmx_ctx::AmpChunk &ch : ctx->o_chunks) {
+    if (ch.pass != pass) {
+      pass = ch.pass;
+      tmx_launch_wigner_cols((const TmxAngle *)ctx->o_angles.p + ctx->o_passes[pass][0],
+                             (int)ctx->o_passes[pass][1], wn, wpi, wtau, st);
+      LAUNCHED();
+    }
     for (const tmx_ctx::AmpLaunch &la : ch.launches) {
       tmx_launch_amp(grp, (const int32_t *)ctx->o_ins.p, prs,
                      (const TmxAmpRange *)ctx->o_rng.p + la.rng0, la.nrng, la.nitems,
@@ -811,17 +928,13 @@ extern "C" int tmx_get_table(
       phis.push_back(mkc(cos(ph[i]), sin(ph[i])));
     }
   }
-  if ((rc = ensure(ctx, ctx->o_angles, ang.size() * sizeof(TmxAngle))) ||
-      (rc = ensure(ctx, ctx->o_phis, phis.size() * sizeof(cplx))) ||
+  if ((rc = ensure(ctx, ctx->o_phis, phis.size() * sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->o_wts, std::max<size_t>(1, acc_w.size()) * sizeof(double))) ||
       (rc = ensure(ctx, ctx->o_coef, std::max<int64_t>(1, (int64_t)nsets * ncoef) * sizeof(double))) ||
       (rc = ensure(ctx, ctx->o_shw, nshape * sizeof(double)))) {
     return rc;
   }
   ++ctx->plan_seq; // the observable buffers change below
-  CK(cudaMemcpyAsync(ctx->o_angles.p, ang.data(), ang.size() * sizeof(TmxAngle),
-                     cudaMemcpyHostToDevice, st));
-  ctx->o_nangles = (int)ang.size();
   CK(cudaMemcpyAsync(ctx->o_phis.p, phis.data(), phis.size() * sizeof(cplx),
                      cudaMemcpyHostToDevice, st));
   if (!acc_w.empty()) {
@@ -927,7 +1040,7 @@ extern "C" int tmx_get_table(
     CK(cudaMemcpyAsync(ctx->o_og.p, og.data(), ng * sizeof(TmxObsGrain),
                        cudaMemcpyHostToDevice, st));
     // ---- amplitudes: the same angles for every grain
-    AmpPlan plan;
+    AmpPlan plan((int64_t)ang.size(), nmax_chunk);
     std::vector<AmpUse> uses;
     std::vector<TmxQJob> qj;
     const int64_t per_theta = 1 + (account ? (int64_t)ngauss * ngauss : 0);
@@ -940,12 +1053,12 @@ extern "C" int tmx_get_table(
                         t * per_theta + 1 + (int64_t)ti * ngauss});
       }
     }
-    const auto main_groups = plan.add(jobs);
+    const auto main_groups = plan.add(jobs.data(), jobs.size());
     jobs.clear();
     for (int t = 0; do_sca && t < ntheta; ++t) {
       jobs.push_back({sca_ain, sca_a0 + t, nphi_sca, sca_p0, (int64_t)t * nphi_sca});
     }
-    const auto sca_groups = plan.add(jobs);
+    const auto sca_groups = plan.add(jobs.data(), jobs.size());
     for (int64_t g = 0; g < ng; ++g) {
       if (og[g].nmax <= 0) {
         continue;
@@ -978,7 +1091,7 @@ extern "C" int tmx_get_table(
       CK(cudaMemcpyAsync(ctx->o_qj.p, qj.data(), qj.size() * sizeof(TmxQJob),
                          cudaMemcpyHostToDevice, st));
     }
-    if ((rc = upload_obs_plan(ctx, og, plan, std::move(uses))) ||
+    if ((rc = upload_obs_plan(ctx, og, ang, plan, std::move(uses))) ||
         (ctx->obs_s_valid = false, false) ||
         (rc = run_amplitudes(ctx, (const cplx *)ctx->T.p, t_total, ncoef,
                              (cplx *)ctx->o_S.p, s_total))) {
@@ -1103,12 +1216,16 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
   }
   std::vector<cplx> phis(1, mkc(1., 0.));
   std::vector<TmxObsGrain> og(n);
-  AmpPlan plan;
+  int nmax_b = 1;
+  for (int64_t g = 0; g < n; ++g) {
+    nmax_b = std::max(nmax_b, ctx->nmax_h[g]);
+  }
+  AmpPlan plan(ntheta, nmax_b);
   std::vector<AmpJob> jobs;
   for (int t = 0; t < ntheta; ++t) {
     jobs.push_back({t, t, 1, 0, t});
   }
-  const auto groups = plan.add(jobs);
+  const auto groups = plan.add(jobs.data(), jobs.size());
   std::vector<AmpUse> uses;
   std::vector<TmxQJob> qj;
   qj.reserve((size_t)n * ntheta);
@@ -1136,16 +1253,12 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
       qj.push_back(q);
     }
   }
-  if ((rc = ensure(ctx, ctx->o_angles, std::max(1, ntheta) * sizeof(TmxAngle))) ||
-      (rc = ensure(ctx, ctx->o_phis, sizeof(cplx))) ||
+  if ((rc = ensure(ctx, ctx->o_phis, sizeof(cplx))) ||
       (rc = ensure(ctx, ctx->o_og, std::max<int64_t>(1, n) * sizeof(TmxObsGrain))) ||
       (rc = ensure(ctx, ctx->o_qj, std::max<size_t>(1, qj.size()) * sizeof(TmxQJob))) ||
       (rc = ensure(ctx, ctx->o_coef, std::max(1, ncoef) * sizeof(double)))) {
     return rc;
   }
-  CK(cudaMemcpyAsync(ctx->o_angles.p, ang.data(), ntheta * sizeof(TmxAngle),
-                     cudaMemcpyHostToDevice, st));
-  ctx->o_nangles = ntheta;
   CK(cudaMemcpyAsync(ctx->o_phis.p, phis.data(), sizeof(cplx),
                      cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(ctx->o_og.p, og.data(), n * sizeof(TmxObsGrain),
@@ -1159,16 +1272,10 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
                        cudaMemcpyHostToDevice, st));
   }
   ctx->o_nqj = (int)qj.size();
-  if (coeffs) {
-    int nmax_b = 1;
-    for (int64_t g = 0; g < n; ++g) {
-      nmax_b = std::max(nmax_b, og[g].nmax);
-    }
-    if ((rc = tmx_ensure_cg(ctx, nmax_b))) {
-      return rc;
-    }
+  if (coeffs && (rc = tmx_ensure_cg(ctx, nmax_b))) {
+    return rc;
   }
-  if ((rc = upload_obs_plan(ctx, og, plan, std::move(uses)))) {
+  if ((rc = upload_obs_plan(ctx, og, ang, plan, std::move(uses)))) {
     return rc;
   }
   key.valid = true;
@@ -1633,21 +1740,15 @@ int plain_amplitudes(tmx_ctx *ctx, const std::vector<int32_t> &grain,
       }
       by[grain[j0]].push_back(J);
     }
-    AmpPlan plan;
+    AmpPlan plan((int64_t)used.size(), nbmax);
     std::vector<AmpUse> uses;
     for (int64_t g = 0; g < n; ++g) {
       if (!by[g].empty()) {
-        const auto gr = plan.add(by[g]);
+        const auto gr = plan.add(by[g].data(), by[g].size());
         uses.push_back({(int32_t)g, gr.first, gr.second, 0});
       }
     }
-    if ((rc = ensure(ctx, ctx->o_angles, std::max<size_t>(1, used.size()) * sizeof(TmxAngle)))) {
-      return rc;
-    }
-    CK(cudaMemcpyAsync(ctx->o_angles.p, used.data(), used.size() * sizeof(TmxAngle),
-                       cudaMemcpyHostToDevice, st));
-    ctx->o_nangles = (int)used.size();
-    if ((rc = upload_obs_plan(ctx, og, plan, std::move(uses))) ||
+    if ((rc = upload_obs_plan(ctx, og, used, plan, std::move(uses))) ||
         (rc = run_amplitudes(ctx, (const cplx *)ctx->T.p, ctx->p2_t_total, 1,
                              (cplx *)ctx->o_S.p, ns))) {
       return rc;
@@ -1858,7 +1959,7 @@ extern "C" int tmx_batch_orientation_average(tmx_ctx *ctx, const double *coeffs,
     CK(cudaMemcpyAsync(ctx->o_coef.p, coeffs, (int64_t)nsets * ncoef * sizeof(double),
                        cudaMemcpyHostToDevice, st));
   }
-  if ((rc = upload_obs_plan(ctx, og, AmpPlan(), {}))) {
+  if ((rc = upload_obs_plan(ctx, og, {}, AmpPlan(0, 1), {}))) {
     return rc;
   }
   if (t_total > 0 && !ctx->o_orient.empty()) {
