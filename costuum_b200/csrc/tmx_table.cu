@@ -13,7 +13,6 @@
 #include <cstring>
 #include <system_error>
 #include <thread>
-#include <unordered_map>
 #include <vector>
 
 #include "tmx_ctx.h"
@@ -414,28 +413,40 @@ struct AmpPlan {
                              kColumnBytes / (16 * (int64_t)(nmax + 1) * nmax));
   }
 
-  // returns the new groups [first, second)
-  std::pair<int, int> add(const AmpJob *jobs, size_t n) {
+  // returns the new groups [first, second) of n jobs, the j-th being job(j)
+  template <class Job> std::pair<int, int> add(int32_t n, Job job) {
     const int g0 = (int)groups.size();
-    // jobs by incoming angle: a stable counting sort
+    // jobs by incoming angle: a stable counting sort, left out where they come
+    // in that order
     start_.assign(1, 0);
+    start_.reserve((size_t)n + 1);
     first_.clear();
-    for (size_t j = 0; j < n; ++j) {
-      int32_t &s = slot_[jobs[j].ain];
+    first_.reserve(n);
+    bool in_order = true;
+    for (int32_t j = 0; j < n; ++j) {
+      const int32_t a = job(j).ain;
+      int32_t &s = slot_[a];
       if (s < 0) {
         s = (int32_t)first_.size();
-        first_.push_back(jobs[j].ain);
+        first_.push_back(a);
         start_.push_back(0);
       }
+      in_order = in_order && s + 1 == (int32_t)first_.size();
       ++start_[s + 1];
     }
     for (size_t a = 1; a < start_.size(); ++a) {
       start_[a] += start_[a - 1];
     }
-    sorted_.resize(n);
-    pos_.assign(start_.begin(), start_.end() - 1);
-    for (size_t j = 0; j < n; ++j) {
-      sorted_[pos_[slot_[jobs[j].ain]]++] = (int64_t)j;
+    if (!in_order) {
+      sorted_.resize(n);
+      pos_.assign(start_.begin(), start_.end() - 1);
+      for (int32_t j = 0; j < n; ++j) {
+        sorted_[pos_[slot_[job(j).ain]]++] = j;
+      }
+    }
+    if (pairs.empty()) {
+      pairs.reserve(n);
+      ins.reserve(first_.size());
     }
     TmxAmpGroup g = {};
     const auto close_group = [&]() {
@@ -447,8 +458,8 @@ struct AmpPlan {
       g = TmxAmpGroup{};
     };
     for (size_t a = 0; a < first_.size(); ++a) {
-      for (int64_t q = start_[a]; q < start_[a + 1]; ++q) {
-        const AmpJob &J = jobs[sorted_[q]];
+      for (int32_t q = start_[a]; q < start_[a + 1]; ++q) {
+        const AmpJob J = job(in_order ? q : sorted_[q]);
         const bool fresh = q == start_[a];
         if (g.npair >= kGroupPairs || (fresh && g.nin == TMX_AMP_NIN)) {
           close_group();
@@ -478,6 +489,9 @@ struct AmpPlan {
       slot_[a] = -1;
     }
     return {g0, (int)groups.size()};
+  }
+  std::pair<int, int> add(const std::vector<AmpJob> &jobs) {
+    return add((int32_t)jobs.size(), [&](int32_t j) { return jobs[j]; });
   }
 
 private:
@@ -521,8 +535,7 @@ private:
   }
 
   int64_t nang_, cap_;
-  std::vector<int32_t> slot_, first_, number_, number_pass_;
-  std::vector<int64_t> start_, pos_, sorted_;
+  std::vector<int32_t> slot_, first_, number_, number_pass_, start_, pos_, sorted_;
 };
 
 // groups [g0, g1) of a plan for one grain, their S from out0 on
@@ -1053,12 +1066,12 @@ extern "C" int tmx_get_table(
                         t * per_theta + 1 + (int64_t)ti * ngauss});
       }
     }
-    const auto main_groups = plan.add(jobs.data(), jobs.size());
+    const auto main_groups = plan.add(jobs);
     jobs.clear();
     for (int t = 0; do_sca && t < ntheta; ++t) {
       jobs.push_back({sca_ain, sca_a0 + t, nphi_sca, sca_p0, (int64_t)t * nphi_sca});
     }
-    const auto sca_groups = plan.add(jobs.data(), jobs.size());
+    const auto sca_groups = plan.add(jobs);
     for (int64_t g = 0; g < ng; ++g) {
       if (og[g].nmax <= 0) {
         continue;
@@ -1225,7 +1238,7 @@ int batch_observable_setup(tmx_ctx *ctx, int ntheta, const double *thetas,
   for (int t = 0; t < ntheta; ++t) {
     jobs.push_back({t, t, 1, 0, t});
   }
-  const auto groups = plan.add(jobs.data(), jobs.size());
+  const auto groups = plan.add(jobs);
   std::vector<AmpUse> uses;
   std::vector<TmxQJob> qj;
   qj.reserve((size_t)n * ntheta);
@@ -1674,15 +1687,15 @@ void k_from_s(double k, const zc S[2][2], double *K) {
   K[14] = -K[11];
 }
 
-// Amplitude matrices S^P of jobs (AmpJob with a grain each: incoming and
+// Amplitude matrices S^P of nj jobs (the j-th for grain(j): incoming and
 // outgoing angle, azimuths e^{i(phi_out - phi_in)}) for the T-matrices of the
 // last batch (plain or averaged); ns amplitudes in all, at the jobs' places.
-int plain_amplitudes(tmx_ctx *ctx, const std::vector<int32_t> &grain,
-                     const std::vector<TmxAngle> &ang, const std::vector<AmpJob> &jobs,
-                     const std::vector<cplx> &e1, int64_t ns, std::vector<zc> &S) {
+template <class Grain, class Job>
+int plain_amplitudes(tmx_ctx *ctx, int64_t nj, Grain grain, Job job,
+                     const std::vector<TmxAngle> &ang, const std::vector<cplx> &e1,
+                     int64_t ns, std::vector<zc> &S) {
   cudaStream_t st = ctx->stream;
   const int64_t n = ctx->n;
-  const int64_t nj = (int64_t)grain.size();
   int rc;
   std::vector<TmxObsGrain> og(n);
   int nbmax = 1;
@@ -1699,68 +1712,47 @@ int plain_amplitudes(tmx_ctx *ctx, const std::vector<int32_t> &grain,
       (rc = ensure(ctx, ctx->o_S, std::max<int64_t>(1, ns) * 4 * sizeof(cplx)))) {
     return rc;
   }
-  std::vector<std::vector<AmpJob>> by(n);
-  // angles in use, renumbered per pass: a pass takes jobs until the table of
-  // its angles reaches 512 MB
-  const int64_t max_ang = std::max<int64_t>(
-      2, ((int64_t)512 << 20) / (16 * (int64_t)(nbmax + 1) * nbmax));
-  std::vector<int32_t> local(ang.size());
-  S.assign(4 * ns, zc(0., 0.));
-  std::vector<cplx> Sh(4 * ns);
+  // jobs by grain (a stable counting sort), those of grains without a T left out
+  std::vector<int32_t> start(n + 1, 0);
+  for (int64_t j = 0; j < nj; ++j) {
+    start[grain(j) + 1] += og[grain(j)].nmax > 0 ? 1 : 0;
+  }
+  for (int64_t g = 0; g < n; ++g) {
+    start[g + 1] += start[g];
+  }
+  std::vector<int32_t> by(start[n]);
+  std::vector<int32_t> pos(start.begin(), start.end() - 1);
+  for (int64_t j = 0; j < nj; ++j) {
+    if (og[grain(j)].nmax > 0) {
+      by[pos[grain(j)]++] = (int32_t)j;
+    }
+  }
+  AmpPlan plan((int64_t)ang.size(), nbmax);
+  std::vector<AmpUse> uses;
+  for (int64_t g = 0; g < n; ++g) {
+    if (start[g + 1] > start[g]) {
+      const int32_t *own = by.data() + start[g];
+      const auto gr = plan.add(start[g + 1] - start[g],
+                               [&](int32_t j) { return job(own[j]); });
+      uses.push_back({(int32_t)g, gr.first, gr.second, 0});
+    }
+  }
   ++ctx->plan_seq; // the observable buffers change below
   ctx->obs_s_valid = false;
   CK(cudaMemcpyAsync(ctx->o_og.p, og.data(), n * sizeof(TmxObsGrain),
                      cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(ctx->o_phis.p, e1.data(), e1.size() * sizeof(cplx),
                      cudaMemcpyHostToDevice, st));
-  int64_t j0 = 0;
-  while (j0 < nj) {
-    std::fill(local.begin(), local.end(), -1);
-    std::vector<TmxAngle> used;
-    for (auto &v : by) {
-      v.clear();
-    }
-    const int64_t first = j0;
-    for (; j0 < nj; ++j0) {
-      if (og[grain[j0]].nmax <= 0) {
-        continue;
-      }
-      AmpJob J = jobs[j0];
-      const int fresh = (local[J.ain] < 0) + (local[J.aout] < 0 && J.aout != J.ain);
-      if (j0 > first && (int64_t)used.size() + fresh > max_ang) {
-        break;
-      }
-      for (int32_t *a : {&J.ain, &J.aout}) {
-        int32_t &l = local[*a];
-        if (l < 0) {
-          l = (int32_t)used.size();
-          used.push_back(ang[*a]);
-        }
-        *a = l;
-      }
-      by[grain[j0]].push_back(J);
-    }
-    AmpPlan plan((int64_t)used.size(), nbmax);
-    std::vector<AmpUse> uses;
-    for (int64_t g = 0; g < n; ++g) {
-      if (!by[g].empty()) {
-        const auto gr = plan.add(by[g].data(), by[g].size());
-        uses.push_back({(int32_t)g, gr.first, gr.second, 0});
-      }
-    }
-    if ((rc = upload_obs_plan(ctx, og, used, plan, std::move(uses))) ||
-        (rc = run_amplitudes(ctx, (const cplx *)ctx->T.p, ctx->p2_t_total, 1,
-                             (cplx *)ctx->o_S.p, ns))) {
-      return rc;
-    }
-    CK(cudaMemcpyAsync(Sh.data(), ctx->o_S.p, 4 * ns * sizeof(cplx),
-                       cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    // each pass leaves zeros at the other passes' places
-    for (int64_t i = 0; i < 4 * ns; ++i) {
-      S[i] += zc(Sh[i].x, Sh[i].y);
-    }
+  if ((rc = upload_obs_plan(ctx, og, ang, plan, std::move(uses))) ||
+      (rc = run_amplitudes(ctx, (const cplx *)ctx->T.p, ctx->p2_t_total, 1,
+                           (cplx *)ctx->o_S.p, ns))) {
+    return rc;
   }
+  static_assert(sizeof(zc) == sizeof(cplx), "both are (re, im) in doubles");
+  S.resize(4 * ns);
+  CK(cudaMemcpyAsync(S.data(), ctx->o_S.p, 4 * ns * sizeof(cplx), cudaMemcpyDeviceToHost,
+                     st));
+  CK(cudaStreamSynchronize(st));
   return TMX_OK;
 }
 
@@ -1783,56 +1775,75 @@ int lab_amplitudes(tmx_ctx *ctx, int64_t njobs, const int64_t *grain,
                    const double *theta_in, const double *phi_in,
                    const double *theta_out, const double *phi_out,
                    std::vector<zc> &SL) {
-  std::vector<int32_t> g(njobs);
-  std::vector<AmpJob> jobs(njobs);
+  std::vector<std::array<int32_t, 2>> pair(njobs); // angles in, out
   std::vector<cplx> e1(njobs);
-  std::vector<PDir> din(njobs), dout(njobs);
-  // one angle per distinct particle-frame zenith
+  struct Rot {
+    double in[2][2], out[2][2];
+  };
+  std::vector<Rot> rot(njobs);
+  // Particle-frame zeniths that repeat get one number. The numbers seen last
+  // are kept in pairs by hash, in a table that stays in the cache: an angle
+  // pushed out of it gets a second number, which costs its columns again but
+  // nothing else (100,000 jobs with directions of their own: 7 ms in one hash
+  // table of all angles, 2.5 ms in this one).
   std::vector<TmxAngle> ang;
-  std::unordered_map<uint64_t, int32_t> index;
+  ang.reserve(2 * (size_t)njobs);
+  struct Seen {
+    uint32_t tag[2];
+    int32_t number[2];
+  };
+  size_t places = 16;
+  while (places < (size_t)njobs && places < 32768) {
+    places *= 2;
+  }
+  std::vector<Seen> seen(places, Seen{{0, 0}, {-1, -1}});
   const auto angle = [&](const TmxAngle &a) {
     uint64_t h[3];
     memcpy(h, &a, sizeof(h));
     // (cos, sin) name the angle; 1 / sin follows from sin
-    uint64_t key = h[0] ^ (h[1] * 0x9E3779B97F4A7C15ull);
-    for (;;) {
-      const auto it = index.emplace(key, (int32_t)ang.size());
-      if (it.second) {
-        ang.push_back(a);
-      }
-      const int32_t i = it.first->second;
-      if (memcmp(&ang[i], &a, sizeof(a)) == 0) {
+    const uint64_t key = (h[0] ^ (h[1] >> 1)) * 0x9E3779B97F4A7C15ull;
+    const uint32_t tag = (uint32_t)(key >> 32);
+    Seen &e = seen[(key >> 16) & (places - 1)];
+    for (int w = 0; w < 2; ++w) {
+      const int32_t i = e.number[w];
+      if (e.tag[w] == tag && i >= 0 && memcmp(&ang[i], &a, sizeof(a)) == 0) {
         return i;
       }
-      key = key * 6364136223846793005ull + 1442695040888963407ull;
     }
+    e.tag[1] = e.tag[0];
+    e.number[1] = e.number[0];
+    e.tag[0] = tag;
+    e.number[0] = (int32_t)ang.size();
+    ang.push_back(a);
+    return e.number[0];
   };
   for (int64_t j = 0; j < njobs; ++j) {
     const double ca = cos(alpha[j]), sa = sin(alpha[j]);
     const double cb = cos(beta[j]), sb = sin(beta[j]);
-    din[j] = particle_dir(ca, sa, cb, sb, theta_in[j], phi_in[j]);
-    dout[j] = particle_dir(ca, sa, cb, sb, theta_out[j], phi_out[j]);
-    g[j] = (int32_t)grain[j];
-    jobs[j] = {angle(din[j].a), angle(dout[j].a), 1, j, j};
-    e1[j] = mkc(dout[j].cphi * din[j].cphi + dout[j].sphi * din[j].sphi,
-                dout[j].sphi * din[j].cphi - dout[j].cphi * din[j].sphi);
+    const PDir din = particle_dir(ca, sa, cb, sb, theta_in[j], phi_in[j]);
+    const PDir dout = particle_dir(ca, sa, cb, sb, theta_out[j], phi_out[j]);
+    pair[j] = {angle(din.a), angle(dout.a)};
+    e1[j] = mkc(dout.cphi * din.cphi + dout.sphi * din.sphi,
+                dout.sphi * din.cphi - dout.cphi * din.sphi);
+    memcpy(rot[j].in, din.R, sizeof(din.R));
+    memcpy(rot[j].out, dout.R, sizeof(dout.R));
   }
-  std::vector<zc> SP;
-  int rc = plain_amplitudes(ctx, g, ang, jobs, e1, njobs, SP);
+  int rc = plain_amplitudes(
+      ctx, njobs, [&](int64_t j) { return grain[j]; },
+      [&](int64_t j) { return AmpJob{pair[j][0], pair[j][1], 1, j, j}; }, ang, e1, njobs, SL);
   if (rc) {
     return rc;
   }
-  SL.resize(4 * njobs);
   for (int64_t j = 0; j < njobs; ++j) {
-    const zc *S = SP.data() + 4 * j;
-    const double(&Ri)[2][2] = din[j].R;
+    const zc S[4] = {SL[4 * j], SL[4 * j + 1], SL[4 * j + 2], SL[4 * j + 3]};
+    const double(&Ri)[2][2] = rot[j].in;
+    const double(&Rd)[2][2] = rot[j].out;
     double Ro[2][2];
-    const double det = 1. / (dout[j].R[0][0] * dout[j].R[1][1] -
-                             dout[j].R[0][1] * dout[j].R[1][0]);
-    Ro[0][0] = dout[j].R[1][1] * det;
-    Ro[0][1] = -dout[j].R[0][1] * det;
-    Ro[1][0] = -dout[j].R[1][0] * det;
-    Ro[1][1] = dout[j].R[0][0] * det;
+    const double det = 1. / (Rd[0][0] * Rd[1][1] - Rd[0][1] * Rd[1][0]);
+    Ro[0][0] = Rd[1][1] * det;
+    Ro[0][1] = -Rd[0][1] * det;
+    Ro[1][0] = -Rd[1][0] * det;
+    Ro[1][1] = Rd[0][0] * det;
     const zc cS11 = S[0] * Ri[0][0] + S[1] * Ri[1][0];
     const zc cS12 = S[0] * Ri[0][1] + S[1] * Ri[1][1];
     const zc cS21 = S[2] * Ri[0][0] + S[3] * Ri[1][0];
@@ -1881,8 +1892,9 @@ int absorption(tmx_ctx *ctx, int32_t grain, int32_t ntheta, const double *th,
     }
   }
   std::vector<zc> S;
-  int rc = plain_amplitudes(ctx, std::vector<int32_t>(jobs.size(), grain), ang, jobs, e1,
-                            ns, S);
+  int rc = plain_amplitudes(
+      ctx, (int64_t)jobs.size(), [&](int64_t) { return grain; },
+      [&](int64_t j) { return jobs[j]; }, ang, e1, ns, S);
   if (rc) {
     return rc;
   }

@@ -70,3 +70,44 @@ def test_memory_of_many_angles():
     # 512 MB of columns, 264 MB of m sums (8000 x 129 x 4), each with the quarter
     # that buffers grow by; 100 MB for all else
     assert grown <= 1.25 * (512 * 2 ** 20 + 8000 * 129 * 4 * 16) + 100e6
+
+
+def _directions(nj):
+    return np.random.default_rng(4).uniform(0.1, 3.0, (6, nj))
+
+
+def test_directions_of_many_jobs(batch):
+    # two angles of their own per job, the grains' jobs mixed: several passes
+    c, res, _ = batch
+    nj = 6000
+    ti, pi, to, po = _directions(nj)[:4]
+    g = np.arange(nj) % len(ORDERS)
+    Z = c.scattering_matrix(g, ti, pi, to, po)
+    for i, n in enumerate(ORDERS):
+        # the same pairs alone, in groups of the same 16
+        own = np.flatnonzero(g == i)
+        for i0 in range(0, own.size, 800):
+            p = own[i0:i0 + 800]
+            assert np.array_equal(Z[p], c.scattering_matrix(i, ti[p], pi[p], to[p], po[p]))
+        pick = own[[0, 1, 15, 16, 503, 504, 505, 1007, 1008, 1009, 1999]]
+        S, scale = _amplitudes(res.tmatrix(i), n, K, np.cos(ti[pick]), np.cos(to[pick]),
+                               po[pick] - pi[pick])
+        # (as in the test of one grain's angle pairs)
+        d = scale * 2.0 ** -53 * 16 * (2 * n + 4)
+        tol = 4 * np.max(np.abs(S), axis=0) * d + 4 * d * d
+        assert np.all(np.abs(Z[pick, 0, 0] - 0.5 * np.sum(np.abs(S) ** 2, axis=0)) <= tol)
+
+
+def test_a_pass_costs_its_own_launches(batch):
+    # at order 128 a pass holds 1016 such jobs; another one adds its columns,
+    # four sizes of blocks and the azimuths, and the T-matrices are not copied
+    # again
+    c, _, _ = batch
+
+    def launches(nj):
+        a = _directions(nj)
+        before = c.kernel_launches
+        c.scattering_matrix(0, *a[:4])
+        return c.kernel_launches - before
+    assert launches(2000) - launches(1000) <= 6
+    assert launches(3000) - launches(2000) <= 6
