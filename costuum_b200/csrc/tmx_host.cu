@@ -864,15 +864,15 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
     if ((rc = prof_begin(ctx, 1, &pe, st))) {
       return rc;
     }
-    int ngmax = 1, nmmax = 1;
+    int ngmax = 1;
     for (const TmxSlot &sl : slots) {
       ngmax = std::max(ngmax, sl.ngauss);
-      nmmax = std::max(nmmax, sl.nmax);
     }
     tmx_launch_tables(dslots, np2, (const TmxGrain *)ctx->grains.p,
                       (const double *)ctx->gl_x.p, (const double *)ctx->gl_w.p,
                       (const int64_t *)ctx->gl_off.p, tab, nsc,
-                      ctx->up_sched.bessel_start, ngmax, nmmax, st);
+                      ctx->up_sched.bessel_start, ngmax, tmx_tables_rho(slots.data(), np2),
+                      st);
     LAUNCHED();
     if ((rc = prof_end(ctx, 1, pe, 0., st, 0., np2))) {
       return rc;

@@ -261,30 +261,35 @@ __device__ __forceinline__ void table_node(const TmxSlot &sl,
   }
 }
 
-// Grid (slot, node chunk, kind): every warp runs one recurrence type, and the
-// three of a node run side by side (a few grains at orders of 100 to 200 leave
-// the launch bound by one thread's chain: 9 grains 89 -> 39 us per order with y_n
-// beside j_n and the ratios read ahead).
-__global__ void k_tables(const TmxSlot *__restrict__ slots, int nslots,
+// Grid (slot, chunk of 32 nodes), a warp per kind: every warp runs one
+// recurrence type, and the three of a node run side by side (a few grains at
+// orders of 100 to 200 leave the launch bound by one thread's chain: 9 grains
+// 89 -> 39 us per order with y_n beside j_n and the ratios read ahead). The
+// CTA's shared memory holds the ratios of its complex warp and of its real one.
+#define TMX_TAB_NODES 32
+__global__ void __launch_bounds__(3 * TMX_TAB_NODES) k_tables(const TmxSlot *__restrict__ slots, int nslots,
                          const TmxGrain *__restrict__ grains,
                          const double *__restrict__ gl_x,
                          const double *__restrict__ gl_w,
                          const int64_t *__restrict__ gl_off, double *tab,
                          double *nsc, int bessel_start, int rho_smem) {
-  // ratio buffers: a shared-memory column per thread (rho_smem rows), or
-  // the output slots themselves when the orders exceed rho_smem
+  // ratio buffers: a shared-memory column per node (rho_smem rows), or the
+  // output slots themselves when the orders exceed rho_smem
   extern __shared__ cplx trho[];
+  cplx *rreal = trho + rho_smem * TMX_TAB_NODES; // (doubles)
+  const int lane = threadIdx.x & (TMX_TAB_NODES - 1);
+  const int kind = threadIdx.x / TMX_TAB_NODES;
   const int s = blockIdx.x;
   if (s >= nslots) {
     return;
   }
   const TmxSlot sl = slots[s];
-  const int g = blockIdx.y * blockDim.x + threadIdx.x;
+  const int g = blockIdx.y * TMX_TAB_NODES + lane;
   if (g >= sl.ngauss) {
     return;
   }
-  table_node(sl, grains, gl_x, gl_w, gl_off, tab, nsc, bessel_start, rho_smem, g,
-             blockIdx.z, trho, threadIdx.x, blockDim.x, threadIdx.x, blockDim.x);
+  table_node(sl, grains, gl_x, gl_w, gl_off, tab, nsc, bessel_start, rho_smem, g, kind,
+             kind == 1 ? trho : rreal, lane, TMX_TAB_NODES, lane, TMX_TAB_NODES);
 }
 
 // Device-driven form (CUDA graph): the slots [0, *nact) of one order, whose
@@ -411,34 +416,45 @@ __global__ void k_wigner(const TmxWigJob *__restrict__ jobs, int njobs,
 
 // --------------------------------------------------------- launchers ------
 
+// Shared memory for the ratios (24 bytes per order and node) keeps them out of
+// the output slots, whose traffic bounds a launch that fills the chip; a launch
+// of larger orders is bound by its chains and needs the warps. A launch with
+// both follows the quarter of its work (orders x nodes): 1000 slots of order 40
+// and one of 60 take 166 us with shared memory, 294 without it, 100 of order 100
+// and one of 60 take 260 and 207 us, 300 of order 60 beside 500 of 24 143 and
+// 269 us. In CTAs of one kind each, which all took the memory of the complex
+// ratios, and with no memory for any slot of a launch above order 48, these took
+// 387, 215 and 329 us (1000 of order 40 alone 213, now 168 us).
+int tmx_tables_rho(const TmxSlot *slots, int nslots) {
+  int top = 0;
+  int64_t small = 0, all = 0;
+  for (int s = 0; s < nslots; ++s) {
+    const int64_t work = (int64_t)slots[s].nmax * slots[s].ngauss;
+    all += work;
+    if (slots[s].nmax <= TMX_RHO_SMEM_NMAX) {
+      small += work;
+      top = std::max(top, slots[s].nmax);
+    }
+  }
+  return 4 * small >= all ? top : TMX_RHO_SMEM_NMAX + 1;
+}
+
 void tmx_launch_tables(const TmxSlot *slots, int nslots, const TmxGrain *grains,
                        const double *gl_x, const double *gl_w,
                        const int64_t *gl_off, double *tab, double *nsc,
-                       int bessel_start, int ngmax, int nmax_max,
+                       int bessel_start, int ngmax, int rho_nmax,
                        cudaStream_t stream) {
   if (nslots <= 0 || ngmax <= 0) {
     return;
   }
-  // one thread per node: a warp per slot and argument kind when every slot
-  // has at most 32 nodes (the order loop up to order 16), else chunks of 64
-  const int threads = (ngmax <= 32) ? 32 : 64;
-  // ratios in shared memory for launches of orders up to 48, sized by the
-  // largest one; launches of larger orders keep them in the output slots and
-  // need no shared memory (with 48 rows of it per thread eight warps fit an SM)
-  const int rho_smem = (nmax_max <= 48) ? std::max(1, nmax_max) : 0;
-  const size_t smem = (size_t)threads * rho_smem * sizeof(cplx);
-  static int attr_dev = -1;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (attr_dev != dev) {
-    cudaFuncSetAttribute(k_tables, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(64 * 48 * sizeof(cplx)));
-    attr_dev = dev;
-  }
-  dim3 grid(nslots, (ngmax + threads - 1) / threads, 3);
-  k_tables<<<grid, threads, smem, stream>>>(slots, nslots, grains, gl_x, gl_w,
-                                            gl_off, tab, nsc, bessel_start,
-                                            rho_smem);
+  // (at most 48 KB, so that no limit has to be raised)
+  const int rho_smem = (rho_nmax <= TMX_RHO_SMEM_NMAX) ? std::max(0, rho_nmax) : 0;
+  const size_t smem =
+      (size_t)TMX_TAB_NODES * rho_smem * (sizeof(cplx) + sizeof(double));
+  const dim3 grid(nslots, (ngmax + TMX_TAB_NODES - 1) / TMX_TAB_NODES);
+  k_tables<<<grid, 3 * TMX_TAB_NODES, smem, stream>>>(slots, nslots, grains, gl_x, gl_w,
+                                                      gl_off, tab, nsc, bessel_start,
+                                                      rho_smem);
 }
 
 void tmx_launch_tables_dev(const TmxSlot *slots, int nslots, const int32_t *nact,
