@@ -21,12 +21,12 @@
 #include <functional>
 #include <map>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <tuple>
 #include <vector>
 
 #include "tmx_ctx.h"
+#include "tmx_idle.h"
 
 // ----------------------------------------------------- Gauss-Legendre ----
 
@@ -220,38 +220,22 @@ int tmx_host_chunk_nodes(int max_nb) {
 // one), as long as a small particle's whole computation, and programs on the
 // plain path make a context per particle. So a destroyed context leaves its
 // shell, idle and without any of its buffers, for the next context on that
-// device: at most kShells of them, each keeping kShellPool bytes of its pool
-// mapped; the rest goes back to the device. One particle with its observables:
+// device: at most kShells of them per device, each keeping kShellPool bytes of
+// its pool mapped; the rest goes back to the device. One particle with its observables:
 // 8.0 -> 3.3 ms (create and destroy 3.1 to 4.9 -> 0.3 ms).
 struct CtxShell {
-  int device;
   cudaStream_t stream, stream2, stream3, aux[6];
   cudaMemPool_t pool;
   int32_t *pinned;
 };
-static constexpr size_t kShells = 4;
+static constexpr int kShells = 4;
 static constexpr size_t kShellPool = (size_t)32 << 20;
-static std::mutex g_shell_mutex;
-// (never destroyed: a process may end with idle shells after the driver is gone)
-static std::vector<CtxShell> &idle_shells() {
-  static auto *v = new std::vector<CtxShell>();
-  return *v;
-}
+static TmxIdle<CtxShell, kShells, 64> g_idle_shells;
 
 static bool take_shell(tmx_ctx *ctx) {
   CtxShell s = {};
-  {
-    std::lock_guard<std::mutex> lock(g_shell_mutex);
-    std::vector<CtxShell> &v = idle_shells();
-    size_t i = v.size();
-    while (i > 0 && v[i - 1].device != ctx->device) {
-      --i;
-    }
-    if (i == 0) {
-      return false;
-    }
-    s = v[i - 1];
-    v.erase(v.begin() + (i - 1));
+  if (!g_idle_shells.take(ctx->device, s)) {
+    return false;
   }
   // (handles of a device that was reset meanwhile are of no use)
   if (cudaStreamQuery(s.stream) != cudaSuccess) {
@@ -277,16 +261,9 @@ static bool keep_shell(tmx_ctx *ctx) {
     cudaGetLastError();
     return false;
   }
-  CtxShell s = {ctx->device, ctx->stream, ctx->stream2, ctx->stream3, {}, ctx->pool,
-                ctx->pinned};
+  CtxShell s = {ctx->stream, ctx->stream2, ctx->stream3, {}, ctx->pool, ctx->pinned};
   std::copy(ctx->aux, ctx->aux + 6, s.aux);
-  std::lock_guard<std::mutex> lock(g_shell_mutex);
-  std::vector<CtxShell> &v = idle_shells();
-  if (v.size() >= kShells) {
-    return false;
-  }
-  v.push_back(s);
-  return true;
+  return g_idle_shells.put(ctx->device, s);
 }
 
 static int make_shell(tmx_ctx *ctx) {
