@@ -25,6 +25,8 @@
 #include <tuple>
 #include <vector>
 
+#include <cuda.h>
+
 #include "tmx_ctx.h"
 #include "tmx_idle.h"
 
@@ -227,20 +229,38 @@ struct CtxShell {
   cudaStream_t stream, stream2, stream3, aux[6];
   cudaMemPool_t pool;
   int32_t *pinned;
+  unsigned long long owner; // CUDA context they belong to (cuda_context_id)
 };
 static constexpr int kShells = 4;
 static constexpr size_t kShellPool = (size_t)32 << 20;
 static TmxIdle<CtxShell, kShells, 64> g_idle_shells;
 
+// Number of the calling thread's CUDA context, another one after a reset of its
+// device; 0 if the driver does not tell.
+static unsigned long long cuda_context_id() {
+  using Fn = CUresult (*)(CUcontext, unsigned long long *);
+  void *fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  unsigned long long id = 0;
+  if (cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+      found != cudaDriverEntryPointSuccess || !fn ||
+      reinterpret_cast<Fn>(fn)(nullptr, &id) != CUDA_SUCCESS) {
+    cudaGetLastError();
+    return 0;
+  }
+  return id;
+}
+
 static bool take_shell(tmx_ctx *ctx) {
   CtxShell s = {};
-  if (!g_idle_shells.take(ctx->device, s)) {
-    return false;
-  }
-  // (handles of a device that was reset meanwhile are of no use)
-  if (cudaStreamQuery(s.stream) != cudaSuccess) {
-    return false;
-  }
+  const unsigned long long id = cuda_context_id();
+  // (those of a device that was reset meanwhile are gone: their handles may name
+  // other streams by now, and none of them may be used or destroyed)
+  do {
+    if (!g_idle_shells.take(ctx->device, s)) {
+      return false;
+    }
+  } while (s.owner != id);
   ctx->stream = s.stream;
   ctx->stream2 = s.stream2;
   ctx->stream3 = s.stream3;
@@ -261,9 +281,10 @@ static bool keep_shell(tmx_ctx *ctx) {
     cudaGetLastError();
     return false;
   }
-  CtxShell s = {ctx->stream, ctx->stream2, ctx->stream3, {}, ctx->pool, ctx->pinned};
+  CtxShell s = {ctx->stream, ctx->stream2, ctx->stream3, {}, ctx->pool, ctx->pinned,
+                cuda_context_id()};
   std::copy(ctx->aux, ctx->aux + 6, s.aux);
-  return g_idle_shells.put(ctx->device, s);
+  return s.owner != 0 && g_idle_shells.put(ctx->device, s);
 }
 
 static int make_shell(tmx_ctx *ctx) {
