@@ -863,13 +863,15 @@ static int run_blocks_round(tmx_ctx *ctx, const std::vector<int32_t> &p2,
       return rc;
     }
     int ngmax = 1;
+    bool same_ng = true;
     for (const TmxSlot &sl : slots) {
       ngmax = std::max(ngmax, sl.ngauss);
+      same_ng = same_ng && sl.ngauss == slots[0].ngauss;
     }
     tmx_launch_tables(dslots, np2, (const TmxGrain *)ctx->grains.p,
                       (const double *)ctx->gl_x.p, (const double *)ctx->gl_w.p,
                       (const int64_t *)ctx->gl_off.p, tab, nsc,
-                      ctx->up_sched.bessel_start, ngmax, tmx_tables_rho(slots.data(), np2),
+                      ctx->up_sched.bessel_start, ngmax, same_ng, tmx_tables_rho(slots.data(), np2),
                       st);
     LAUNCHED();
     if ((rc = prof_end(ctx, 1, pe, 0., st, 0., np2))) {
@@ -1591,7 +1593,7 @@ static int gm_compute(tmx_ctx *ctx) {
                           (const TmxGrain *)ctx->grains.p, (const double *)ctx->gl_x.p,
                           (const double *)ctx->gl_w.p, (const int64_t *)ctx->gl_off.p,
                           (double *)ctx->gm_tab.p, (double *)ctx->gm_nsc.p, S.bessel_start,
-                          glf * kl, kl, cs);
+                          glf * kl, false, kl, cs);
         TmxBlockArgs B;
         B.items = (const TmxItem *)ctx->gm_items.p;
         B.nitems = 4 * gk * chunk;
@@ -2139,7 +2141,7 @@ int tmx_batch_compute(tmx_ctx *ctx) {
                         (const TmxGrain *)ctx->grains.p,
                         (const double *)ctx->gl_x.p, (const double *)ctx->gl_w.p,
                         (const int64_t *)ctx->gl_off.p, (double *)ctx->tab.p,
-                        (double *)ctx->nsc.p, S.bessel_start, glf * kl, kl, st);
+                        (double *)ctx->nsc.p, S.bessel_start, glf * kl, G == 1, kl, st);
       LAUNCHED();
       if ((rc2 = prof_end(ctx, 1, pe, 0., nullptr, 0., nsl))) {
         return rc2;

@@ -27,14 +27,15 @@ struct TmxChainState {
   int32_t status;
 };
 
-// node scalars and Bessel tables of every slot; ngmax >= every slot's ngauss;
+// node scalars and Bessel tables of every slot; ngmax >= every slot's ngauss
+// (same_ng: each has ngmax nodes, or none);
 // slots of orders up to rho_nmax keep the ratios of their recurrences in shared
 // memory if rho_nmax <= TMX_RHO_SMEM_NMAX (above it no slot does)
 #define TMX_RHO_SMEM_NMAX 64
 void tmx_launch_tables(const TmxSlot *slots, int nslots, const TmxGrain *grains,
                        const double *gl_x, const double *gl_w,
                        const int64_t *gl_off, double *tab, double *nsc,
-                       int bessel_start, int ngmax, int rho_nmax,
+                       int bessel_start, int ngmax, bool same_ng, int rho_nmax,
                        cudaStream_t stream);
 // rho_nmax of a launch of these slots
 int tmx_tables_rho(const TmxSlot *slots, int nslots);

@@ -119,7 +119,7 @@ int m0_step(tmx_ctx *ctx, const std::vector<int32_t> &g, const std::vector<int> 
                     (const double *)ctx->gl_x.p, (const double *)ctx->gl_w.p,
                     (const int64_t *)ctx->gl_off.p, (double *)ctx->tab.p,
                     (double *)ctx->nsc.p, ctx->up_sched.bessel_start, ngmax,
-                    tmx_tables_rho(slots.data(), ns), st);
+                    false, tmx_tables_rho(slots.data(), ns), st);
   LAUNCHED();
   const int edges[] = {1 << 30, 64, 32, 16, 8, 0};
   size_t i0 = 0;

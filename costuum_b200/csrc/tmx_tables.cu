@@ -30,9 +30,9 @@ __device__ __forceinline__ int bessel_nstart(int bessel_start, int nmax,
   return min(hi, 800);
 }
 
-// The upward products read the kept ratios this many orders ahead: the ratios
-// of orders above 48 lie in the output slots (global memory), whose latency
-// the chain of products would otherwise see once per order.
+// The upward products read kept ratios that lie in the output slots (global
+// memory) this many orders ahead (AHEAD), whose latency the chain of products
+// would otherwise see once per order.
 #define TMX_RHO_WIN 8
 
 // Spherical j_n and [z j_n]'/z, n = 1..nmax, for a real argument, by the
@@ -42,6 +42,7 @@ __device__ __forceinline__ int bessel_nstart(int bessel_start, int nmax,
 // The ratios go to rho[(n-1) * rs] (shared memory, or the output slots
 // themselves); out[(n-1) * stride + {0, 1}] = (j_n, [z j_n]'/z), stored as
 // one 16-byte pair.
+template <bool AHEAD>
 __device__ static void bessel_j_real(int nmax, int nstart, double z,
                                      double *out, int stride, double *rho,
                                      int rs) {
@@ -58,6 +59,16 @@ __device__ static void bessel_j_real(int nmax, int nstart, double z,
   const double j0 = sin(z) * zinv;
   double jprev = rho[0] * j0;
   *reinterpret_cast<double2 *>(out) = make_double2(jprev, j0 - jprev * zinv);
+  if (!AHEAD) {
+    for (int i = 1; i < nmax; ++i) {
+      const double ji = rho[i * rs] * jprev;
+      const double ip1 = i + 1.;
+      *reinterpret_cast<double2 *>(out + i * stride) =
+          make_double2(ji, jprev - ip1 * zinv * ji);
+      jprev = ji;
+    }
+    return;
+  }
   double win[TMX_RHO_WIN];
 #pragma unroll
   for (int t = 0; t < TMX_RHO_WIN; ++t) {
@@ -129,6 +140,7 @@ __device__ static cplx csin_dev(cplx z) {
 // few bits.
 // out[(n-1) * stride + {0,1,2,3}] = (Re j, Im j, Re dj, Im dj), stored as
 // two 16-byte pairs; the ratios go to rho[(n-1) * rs].
+template <bool AHEAD>
 __device__ static void bessel_j_complex(int nmax, int nstart, cplx z,
                                         double *out, int stride, cplx *rho,
                                         int rs) {
@@ -149,6 +161,17 @@ __device__ static void bessel_j_complex(int nmax, int nstart, cplx z,
   cplx *o = reinterpret_cast<cplx *>(out);
   o[0] = jprev;
   o[1] = csub(j0, cmul(jprev, zinv));
+  if (!AHEAD) {
+    for (int i = 1; i < nmax; ++i) {
+      const cplx ji = cmul(rho[i * rs], jprev);
+      const cplx dji = csub(jprev, cmul(cscale(zinv, i + 1.), ji));
+      cplx *oi = reinterpret_cast<cplx *>(out + i * stride);
+      oi[0] = ji;
+      oi[1] = dji;
+      jprev = ji;
+    }
+    return;
+  }
   cplx win[TMX_RHO_WIN];
 #pragma unroll
   for (int t = 0; t < TMX_RHO_WIN; ++t) {
@@ -191,8 +214,8 @@ __device__ __forceinline__ void table_node(const TmxSlot &sl,
                                            const int64_t *__restrict__ gl_off,
                                            double *tab, double *nsc,
                                            int bessel_start, int rho_smem,
-                                           int g, int kind, cplx *trho, int tid,
-                                           int nt, int rtid, int rnt) {
+                                           int g, int kind, bool with_y, cplx *trho,
+                                           int tid, int nt, int rtid, int rnt) {
   const TmxGrain G = grains[sl.grain];
   const int N = sl.nmax;
   const int ng = sl.ngauss;
@@ -242,54 +265,71 @@ __device__ __forceinline__ void table_node(const TmxSlot &sl,
       S[TMX_NS_PAD] = 0.;
       S[TMX_NS_PAD2] = 0.;
       if (N <= rho_smem) {
-        bessel_j_real(N, bessel_nstart(bessel_start, N, kr), kr, T + TMX_Q_J,
-                      TMX_NQ, reinterpret_cast<double *>(trho) + rtid, rnt);
+        bessel_j_real<false>(N, bessel_nstart(bessel_start, N, kr), kr, T + TMX_Q_J,
+                             TMX_NQ, reinterpret_cast<double *>(trho) + rtid, rnt);
       } else {
-        bessel_j_real(N, bessel_nstart(bessel_start, N, kr), kr, T + TMX_Q_J,
-                      TMX_NQ, T + TMX_Q_J, TMX_NQ);
+        bessel_j_real<true>(N, bessel_nstart(bessel_start, N, kr), kr, T + TMX_Q_J,
+                            TMX_NQ, T + TMX_Q_J, TMX_NQ);
+      }
+      if (with_y) {
+        bessel_y_real(N, kr, T + TMX_Q_Y, TMX_NQ);
       }
     } else {
       const cplx krmr = mkc(G.mr * G.k * r * G.r_ev, G.mi * G.k * r * G.r_ev);
       const int ns = bessel_nstart(bessel_start, N, hypot(krmr.x, krmr.y));
       if (N <= rho_smem) {
-        bessel_j_complex(N, ns, krmr, T + TMX_Q_JM_RE, TMX_NQ, trho + tid, nt);
+        bessel_j_complex<false>(N, ns, krmr, T + TMX_Q_JM_RE, TMX_NQ, trho + tid, nt);
       } else {
-        bessel_j_complex(N, ns, krmr, T + TMX_Q_JM_RE, TMX_NQ,
-                         reinterpret_cast<cplx *>(T + TMX_Q_JM_RE), TMX_NQ / 2);
+        bessel_j_complex<true>(N, ns, krmr, T + TMX_Q_JM_RE, TMX_NQ,
+                               reinterpret_cast<cplx *>(T + TMX_Q_JM_RE), TMX_NQ / 2);
       }
     }
   }
 }
 
-// Grid (slot, chunk of 32 nodes), a warp per kind: every warp runs one
-// recurrence type, and the three of a node run side by side (a few grains at
-// orders of 100 to 200 leave the launch bound by one thread's chain: 9 grains
-// 89 -> 39 us per order with y_n beside j_n and the ratios read ahead). The
-// CTA's shared memory holds the ratios of its complex warp and of its real one.
+// Two layouts, the same arithmetic per node:
+// A CTA of three warps, one per kind, for 32 nodes (grid: slot, chunk; or, where
+// all slots have ng_all nodes, the nodes of all slots one after the other, so
+// that no lane is left over). The three of a node run side by side (a few
+// grains at orders of 100 to 200 leave the launch bound by one thread's chain: 9
+// grains of order 120 93 -> 38 us with y_n beside j_n and the ratios read ahead),
+// and the shared memory holds the ratios of the complex and the real warp: 1000
+// slots of order 40 178 us with a CTA per kind, 166 with this one; 4000 of order
+// 10 50 and 48, of order 17 119 and 135, 2000 of order 24 137 and 127 us.
+// A CTA per kind for 32 or 64 nodes (grid: slot, chunk, kind), y_n after j_n.
 #define TMX_TAB_NODES 32
-__global__ void __launch_bounds__(3 * TMX_TAB_NODES) k_tables(const TmxSlot *__restrict__ slots, int nslots,
-                         const TmxGrain *__restrict__ grains,
-                         const double *__restrict__ gl_x,
-                         const double *__restrict__ gl_w,
-                         const int64_t *__restrict__ gl_off, double *tab,
-                         double *nsc, int bessel_start, int rho_smem) {
+__global__ void __launch_bounds__(3 * TMX_TAB_NODES)
+    k_tables(const TmxSlot *__restrict__ slots, int nslots,
+             const TmxGrain *__restrict__ grains, const double *__restrict__ gl_x,
+             const double *__restrict__ gl_w, const int64_t *__restrict__ gl_off,
+             double *tab, double *nsc, int bessel_start, int rho_smem, int ng_all) {
   // ratio buffers: a shared-memory column per node (rho_smem rows), or the
   // output slots themselves when the orders exceed rho_smem
   extern __shared__ cplx trho[];
-  cplx *rreal = trho + rho_smem * TMX_TAB_NODES; // (doubles)
-  const int lane = threadIdx.x & (TMX_TAB_NODES - 1);
-  const int kind = threadIdx.x / TMX_TAB_NODES;
-  const int s = blockIdx.x;
+  const bool beside = blockDim.x == 3 * TMX_TAB_NODES;
+  const int nodes = beside ? TMX_TAB_NODES : blockDim.x;
+  const int kind = beside ? threadIdx.x / TMX_TAB_NODES : blockIdx.z;
+  const int lane = beside ? threadIdx.x & (TMX_TAB_NODES - 1) : threadIdx.x;
+  cplx *rho = trho;
+  if (beside && kind == 0) {
+    rho += rho_smem * TMX_TAB_NODES; // (doubles, behind the complex warp's)
+  }
+  int s = blockIdx.x;
+  int g = blockIdx.y * nodes + lane;
+  if (ng_all > 0) {
+    const int64_t u = (int64_t)blockIdx.x * TMX_TAB_NODES + lane;
+    s = (int)(u / ng_all);
+    g = (int)(u - (int64_t)s * ng_all);
+  }
   if (s >= nslots) {
     return;
   }
   const TmxSlot sl = slots[s];
-  const int g = blockIdx.y * TMX_TAB_NODES + lane;
   if (g >= sl.ngauss) {
     return;
   }
   table_node(sl, grains, gl_x, gl_w, gl_off, tab, nsc, bessel_start, rho_smem, g, kind,
-             kind == 1 ? trho : rreal, lane, TMX_TAB_NODES, lane, TMX_TAB_NODES);
+             !beside, rho, lane, nodes, lane, nodes);
 }
 
 // Device-driven form (CUDA graph): the slots [0, *nact) of one order, whose
@@ -322,7 +362,8 @@ __global__ void k_tables_dev(const TmxSlot *__restrict__ slots, int nslots,
     const TmxSlot sl = slots[s];
     if (g < sl.ngauss) {
       table_node(sl, grains, gl_x, gl_w, gl_off, tab, nsc, bessel_start, rho_smem, g,
-                 kind, trho, threadIdx.x, blockDim.x, 2 * threadIdx.x, 2 * blockDim.x);
+                 kind, false, trho, threadIdx.x, blockDim.x, 2 * threadIdx.x,
+                 2 * blockDim.x);
     }
   }
 }
@@ -442,19 +483,36 @@ int tmx_tables_rho(const TmxSlot *slots, int nslots) {
 void tmx_launch_tables(const TmxSlot *slots, int nslots, const TmxGrain *grains,
                        const double *gl_x, const double *gl_w,
                        const int64_t *gl_off, double *tab, double *nsc,
-                       int bessel_start, int ngmax, int rho_nmax,
+                       int bessel_start, int ngmax, bool same_ng, int rho_nmax,
                        cudaStream_t stream) {
   if (nslots <= 0 || ngmax <= 0) {
     return;
   }
-  // (at most 48 KB, so that no limit has to be raised)
+  // (at most 48 KB in either layout, so that no limit has to be raised)
   const int rho_smem = (rho_nmax <= TMX_RHO_SMEM_NMAX) ? std::max(0, rho_nmax) : 0;
-  const size_t smem =
-      (size_t)TMX_TAB_NODES * rho_smem * (sizeof(cplx) + sizeof(double));
-  const dim3 grid(nslots, (ngmax + TMX_TAB_NODES - 1) / TMX_TAB_NODES);
-  k_tables<<<grid, 3 * TMX_TAB_NODES, smem, stream>>>(slots, nslots, grains, gl_x, gl_w,
-                                                      gl_off, tab, nsc, bessel_start,
-                                                      rho_smem);
+  // small orders of several node counts leave lanes over, and warps of their own
+  // give them back: 1000 slots of orders 8..15 24.9 -> 20.5 us, 3000 of 8..23 88
+  // -> 83; the other way round where the ratios' memory limits the warps, 2000 of
+  // 8..32 100 -> 98, 1000 of 20..32 90 -> 80, 200 of 30..48 51 -> 45 us
+  if (!same_ng && rho_smem > 0 && rho_smem <= 24) {
+    const int nodes = (ngmax <= TMX_TAB_NODES) ? TMX_TAB_NODES : 2 * TMX_TAB_NODES;
+    k_tables<<<dim3(nslots, (ngmax + nodes - 1) / nodes, 2), nodes,
+               (size_t)nodes * rho_smem * sizeof(cplx), stream>>>(
+        slots, nslots, grains, gl_x, gl_w, gl_off, tab, nsc, bessel_start, rho_smem, 0);
+    return;
+  }
+  // (packed where a launch fills the chip; the chains of large orders run better
+  // slot by slot: 100 of order 100 229 and 206 us)
+  const bool pack = same_ng && rho_smem > 0;
+  const int64_t total = (int64_t)nslots * ngmax;
+  dim3 grid(nslots, (ngmax + TMX_TAB_NODES - 1) / TMX_TAB_NODES);
+  if (pack) {
+    grid = dim3((unsigned)((total + TMX_TAB_NODES - 1) / TMX_TAB_NODES));
+  }
+  k_tables<<<grid, 3 * TMX_TAB_NODES,
+             (size_t)TMX_TAB_NODES * rho_smem * (sizeof(cplx) + sizeof(double)), stream>>>(
+      slots, nslots, grains, gl_x, gl_w, gl_off, tab, nsc, bessel_start, rho_smem,
+      pack ? ngmax : 0);
 }
 
 void tmx_launch_tables_dev(const TmxSlot *slots, int nslots, const int32_t *nact,
