@@ -279,9 +279,13 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 // Complex products with their roundings spelled out (the compiler may contract
 // either product of a sum, and large elongated grains amplify the last bit of
 // a factor by many orders of magnitude): mul_xy fuses the x x and y x products,
-// mul_xx the x x and x y ones, mul_yx the y y and x y ones. Every kernel forms l = q / u
-// with mul_xx and updates with mul_xy, so that a class has the same factors and
-// the same T, bit for bit, whichever kernel runs it.
+// mul_xx the x x and x y ones, mul_yx the y y and x y ones. k_blocks_cta32,
+// k_factor and k_solve form l = q / u with mul_xx and update with mul_xy; the warp
+// kernels leave their products to the compiler, which contracts them alike. So
+// the families for up to 64 members give a class the same T, bit for bit. The
+// family for up to 128 (k_assemble<false>) applies the a_n to the node vectors
+// instead of the finished entries: its T differs in the last bits, and so may a
+// context whose dispatch table names it for smaller classes.
 __device__ __forceinline__ cplx mul_xy(cplx a, cplx b) {
   return mkc(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
              __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));

@@ -256,7 +256,7 @@ enum tmx_block_family {
   TMX_FAMILY_WARP_DMMA = 1, /* one warp per item, DMMA m8n8k4 tiles; nb <= 16 */
   TMX_FAMILY_CTA32 = 2,     /* four warps per item; nb <= 32 */
   TMX_FAMILY_CTA64 = 3,     /* assembly, factors and solves apart; nb <= 64 */
-  TMX_FAMILY_CTA = 4        /* as CTA64; nb <= 128 */
+  TMX_FAMILY_CTA = 4        /* as CTA64; nb <= 128; other last bits than the rest */
 };
 #define TMX_DISPATCH_BUCKETS 5
 #define TMX_DISPATCH_FAMILIES 5
