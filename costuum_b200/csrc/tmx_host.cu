@@ -223,8 +223,14 @@ int tmx_host_chunk_nodes(int max_nb) {
 // plain path make a context per particle. So a destroyed context leaves its
 // shell, idle and without any of its buffers, for the next context on that
 // device: at most kShells of them per device, each keeping kShellPool bytes of
-// its pool mapped; the rest goes back to the device. One particle with its observables:
-// 8.0 -> 3.3 ms (create and destroy 3.1 to 4.9 -> 0.3 ms).
+// its pool mapped; the rest goes back to the device. One particle with its
+// observables, medians of 120 in four processes: 8.0 to 9.1 -> 2.6 ms (create
+// and destroy 4.0 to 4.6 -> 0.3 ms), size parameter 11: 11.7 to 16.6 -> 4.6 ms.
+// kShellPool covers what such a particle takes (one and two of the 32 MB pieces a
+// pool grows by). Where it does not, every object maps the rest and gives it back,
+// up to hundreds of ms at times: with one piece kept and the Clebsch-Gordan work
+// space at full size the means were 3.4 to 11 instead of 2.9 ms and, at size
+// parameter 11, 9 to 26 instead of 5.1 ms.
 struct CtxShell {
   cudaStream_t stream, stream2, stream3, aux[6];
   cudaMemPool_t pool;
@@ -232,7 +238,7 @@ struct CtxShell {
   unsigned long long owner; // CUDA context they belong to (cuda_context_id)
 };
 static constexpr int kShells = 4;
-static constexpr size_t kShellPool = (size_t)32 << 20;
+static constexpr size_t kShellPool = (size_t)64 << 20;
 static TmxIdle<CtxShell, kShells, 64> g_idle_shells;
 
 // Number of the calling thread's CUDA context, another one after a reset of its

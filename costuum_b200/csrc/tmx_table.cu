@@ -1175,7 +1175,10 @@ int tmx_ensure_cg(tmx_ctx *ctx, int nmax) {
       tot += (int64_t)(2 * M + 1) * (M + 1);
     }
   }
-  const int blocks = 4 * 148;
+  // a thread per row of the table, as many as stay resident at most; each has two
+  // rows of work space
+  const int64_t rows = (int64_t)nmax * nmax * (2 * nmax + 1);
+  const int blocks = (int)std::min<int64_t>(4 * 148, (rows + 127) / 128);
   int rc;
   if ((rc = ensure(ctx, ctx->cg, tot * sizeof(double))) ||
       (rc = ensure(ctx, ctx->cg_off, off.size() * sizeof(int64_t))) ||
