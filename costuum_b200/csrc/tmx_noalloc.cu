@@ -54,6 +54,8 @@ static constexpr size_t NA_SCR =
                           sizeof(double));
 // Q/RgQ scratch: sum over items of 2 nb^2 complex is below the complex size
 // of the T-matrix itself, 4 nmax^2 + 4 sum_m (nmax + 1 - m)^2 = 49856 at 32
+// (classes of at most 32 members keep both on chip and do not use it; the larger
+// ones, which do, need tmx_item_scratch)
 static constexpr size_t NA_SCR_ELEMS = 49856;
 static constexpr size_t NA_END = NA_SCR + NA_SCR_ELEMS * sizeof(cplx);
 static_assert(NA_END <= TMX_NOALLOC_BYTES, "static scratch layout too large");

@@ -722,7 +722,7 @@ int upload_obs_plan(tmx_ctx *ctx, const std::vector<TmxObsGrain> &og,
   ctx->o_xcap = x_max;
   if (ctx->profiling) {
     // flops of one matrix set over the kernels' index spaces: the
-    // orientation average 16 (2M + 1)(M + 1) per (n1, n2), M = min(n1, n2),
+    // orientation average 16 (M + 1)^2 per (n1, n2), M = min(n1, n2),
     // of every averaged grain; the amplitudes 16 L^2 per m block (L orders)
     // and incoming angle and 32 L per pair
     double fo = 0., fa = 0.;
